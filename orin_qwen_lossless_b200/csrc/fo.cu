@@ -985,6 +985,30 @@ bool fo_mm_ids_supported(const bf16n_weight & w, const bf16n_weight * up) {
     return !up || (fo_supported(*up) && up->K == w.K && up->rows == w.rows);
 }
 
+// whole experts the fused kernel's shared memory lists (and the two-pass form takes)
+void fo_require_expert_count(bool glu, int n_experts) {
+    require(fo_mm_shm(glu, n_experts) <= (size_t) device_info().smem_optin, "too many experts for the fragment-order batched kernel's shared memory");
+}
+
+// Scratch of the two-pass form (prefill_fo_two_pass), 0 where the fused kernel is taken. The fused kernel decodes an
+// expert once per 96 of its tokens on 16 warps per SM, the two-pass form once on 26, but sends the weights through memory as
+// BF16 (two bytes written and read per weight). Measured, fused / two-pass in us, at 16, 64, 80, 96 and 256 pairs per expert:
+//   gate/up + SwiGLU (512 x 2048), 256 experts: 609 / 593, 643 / 602, 743 / 602, 1017 / 605, 1950 / 959
+//                                   16 experts:  93 / 72,   97 / 73,   99 / 72,   99 / 74,  184 / 123
+//   down (2048 x 512), 256 experts:             304 / 309, 357 / 330, 395 / 334, 548 / 336, 1119 / 529
+//                       16 experts:              28 / 37,   32 / 40,   33 / 39,   56 / 39,   83 / 57
+// hence the two lines; a call with few pairs per expert is left alone although a pair of matrices would gain a little.
+// At most 512 MiB (128 experts of the gate/up pair at a time), the order of the call's own FP32 outputs at 8192 tokens.
+constexpr int64_t FO_TWO_PASS_GLU = 16, FO_TWO_PASS_ONE = 80; // routed pairs per expert
+constexpr size_t FO_SCRATCH_MAX = (size_t) 512 << 20;
+
+size_t fo_mm_ids_scratch_bytes(const bf16n_weight & w, const bf16n_weight * up, int n_experts, int n_tok, int n_used) {
+    const size_t per_expert = (size_t) (w.rows / n_experts) * (size_t) w.K * 2 * (up ? 2 : 1);
+    if ((w.rows / n_experts) % (up ? 128 : 256) || per_expert > FO_SCRATCH_MAX) { return 0; }
+    if ((int64_t) n_tok * n_used < (up ? FO_TWO_PASS_GLU : FO_TWO_PASS_ONE) * n_experts) { return 0; }
+    return per_expert * std::min<size_t>((size_t) n_experts, FO_SCRATCH_MAX / per_expert);
+}
+
 void fo_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
                const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
                cudaStream_t st) {
@@ -1000,7 +1024,7 @@ void fo_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_b
     require(a.rows_per_expert % BAND == 0, "rows per expert must be whole 16-row bands");
     a.n_units = w.rows / BAND * a.C;
     const size_t shm = fo_mm_shm(up != nullptr, n_experts);
-    require(shm <= (size_t) device_info().smem_optin, "too many experts for the fragment-order batched kernel's shared memory");
+    fo_require_expert_count(up != nullptr, n_experts);
     const unsigned grid = (unsigned) device_info().sms; // persistent: the items are counted on the device from the bounds
     if (up) { k_fo_mm_ids<true><<<grid, FO_WARPS * 32, shm, st>>>(a); } else { k_fo_mm_ids<false><<<grid, FO_WARPS * 32, shm, st>>>(a); }
     check_launch();

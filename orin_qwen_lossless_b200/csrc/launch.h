@@ -103,6 +103,8 @@ void peer_wait(uint32_t * local_header, int n_peers_mask, cudaStream_t st);
 
 // ep_prefill.cu: expert-parallel prefill, rows exchanged with peer stores
 size_t ep_layout_fill(bf16n_ep_layout & l);
+void fo_require_expert_count(bool glu, int n_experts);
+size_t fo_mm_ids_scratch_bytes(const bf16n_weight & w, const bf16n_weight * up, int n_experts, int n_tok, int n_used);
 void ep_dispatch(const bf16n_ep_layout & l, const void * x_bf16, int64_t x_row, const int32_t * ids, int n_tok, int n_used, int n_experts,
                  int32_t * plan, cudaStream_t st);
 void ep_inbox_ids(const bf16n_ep_layout & l, int32_t * ids_out, cudaStream_t st);
@@ -151,3 +153,8 @@ void prefill_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void 
                     int n_tok, int n_used, cudaStream_t st);
 
 } // namespace b16
+void expand_tiles_fo(const bf16n_weight & w, const bf16n_weight * up, int n_experts, int e0, int n, const int32_t * bounds, void * images,
+                     cudaStream_t st);
+bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
+                         const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
+                         void * scratch, size_t scratch_bytes, cudaStream_t st);

@@ -770,35 +770,37 @@ size_t prefill_workspace_bytes(const bf16n_weight & w, const bf16n_weight * up) 
 
 namespace {
 
+// tensor-core pass over decoded tiles: experts [0, n_experts) of `bounds` and `images`
+void tile_mm(const void * images, const PrefillArgs & a, const int32_t * bounds, int n_experts, int64_t K, bool glu, cudaStream_t st) {
+    const int rows_per_block = glu ? TM_N / 2 : TM_N;
+    TileMmArgs t = {};
+    t.images = (const unsigned char *) images;
+    t.x = a.x; t.x_row = a.x_row;
+    t.ids_src1 = a.ids_src1; t.ids_dst = a.ids_dst; t.bounds = bounds;
+    t.dst = a.dst; t.dst_col = a.dst_col; t.dst_bf16 = a.dst_bf16;
+    t.vec_ok = a.vec_ok;
+    t.bulk_ok = ((uintptr_t) a.dst % 16) == 0 && (a.dst_col * (a.dst_bf16 ? 2 : 4)) % 16 == 0;
+    t.n_experts = n_experts;
+    t.blocks_per_expert = (int) (a.rows_per_expert / rows_per_block);
+    t.ktiles = (int) (K / 64);
+    const unsigned grid = (unsigned) std::min<int64_t>(device_info().sms, (int64_t) n_experts * t.blocks_per_expert);
+    if (glu) { k_tile_mm<true><<<grid, TM_THREADS, TM_SMEM, st>>>(t); }
+    else { k_tile_mm<false><<<grid, TM_THREADS, TM_SMEM, st>>>(t); }
+    check_launch();
+}
+
 // decode pass (expand_tiles.cu) + tensor-core pass over the decoded tiles
 bool two_pass(const bf16n_weight & w, const bf16n_weight * up, const PrefillArgs & a, int n_experts, cudaStream_t st) {
     const size_t need = prefill_workspace_bytes(w, up);
     const int rows_per_block = up ? TM_N / 2 : TM_N;
     if (need == 0 || need > g_workspace_bytes || a.rows_per_expert % rows_per_block || ((uintptr_t) g_workspace % 1024)) { return false; }
     expand_tiles(w, up, n_experts, a.bounds, g_workspace, st);
-    TileMmArgs t = {};
-    t.images = (const unsigned char *) g_workspace;
-    t.x = a.x; t.x_row = a.x_row;
-    t.ids_src1 = a.ids_src1; t.ids_dst = a.ids_dst; t.bounds = a.bounds;
-    t.dst = a.dst; t.dst_col = a.dst_col; t.dst_bf16 = a.dst_bf16;
-    t.vec_ok = a.vec_ok;
-    t.bulk_ok = ((uintptr_t) a.dst % 16) == 0 && (a.dst_col * (a.dst_bf16 ? 2 : 4)) % 16 == 0;
-    t.n_experts = n_experts;
-    t.blocks_per_expert = (int) (a.rows_per_expert / rows_per_block);
-    t.ktiles = (int) (w.K / 64);
-    const unsigned grid = (unsigned) std::min<int64_t>(device_info().sms, (int64_t) n_experts * t.blocks_per_expert);
-    if (up) { k_tile_mm<true><<<grid, TM_THREADS, TM_SMEM, st>>>(t); }
-    else { k_tile_mm<false><<<grid, TM_THREADS, TM_SMEM, st>>>(t); }
-    check_launch();
+    tile_mm(g_workspace, a, a.bounds, n_experts, w.K, up != nullptr, st);
     return true;
 }
 
-} // namespace
-
-void prefill_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
-                    const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
-                    int n_tok, int n_used, cudaStream_t st) {
-    (void) n_tok; (void) n_used;
+PrefillArgs batch_args(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
+                       const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts) {
     PrefillArgs a = {};
     a.w0 = view_of(w);
     a.w1 = up ? view_of(*up) : a.w0;
@@ -809,6 +811,35 @@ void prefill_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void 
     a.n_experts = n_experts;
     a.rows_per_expert = w.rows / n_experts;
     require(((uintptr_t) x_bf16 % 16) == 0 && (x_row * 2) % 16 == 0, "batched activations must be 16-byte aligned rows");
+    return a;
+}
+
+} // namespace
+
+// Fragment-order experts with the caller's scratch: decode into images and multiply, as many experts at a time as the
+// scratch holds. False: the scratch holds no expert, or the rows are not whole row blocks (the fused kernel serves both).
+bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
+                         const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
+                         void * scratch, size_t scratch_bytes, cudaStream_t st) {
+    const size_t per_expert = (size_t) (w.rows / n_experts) * (size_t) w.K * 2 * (up ? 2 : 1);
+    const int64_t rows_per_block = up ? TM_N / 2 : TM_N;
+    if (!scratch || (w.rows / n_experts) % rows_per_block || ((uintptr_t) scratch % 1024) || scratch_bytes < per_expert) { return false; }
+    const PrefillArgs a = batch_args(w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16, dst_col, n_experts);
+    const int fit = (int) std::min<size_t>((size_t) n_experts, scratch_bytes / per_expert);
+    const int ranges = (n_experts + fit - 1) / fit, step = (n_experts + ranges - 1) / ranges; // ranges of equal size
+    for (int e0 = 0; e0 < n_experts; e0 += step) {
+        const int n = std::min(step, n_experts - e0);
+        expand_tiles_fo(w, up, n_experts, e0, n, bounds + e0, scratch, st);
+        tile_mm(scratch, a, bounds + e0, n, w.K, up != nullptr, st);
+    }
+    return true;
+}
+
+void prefill_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
+                    const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
+                    int n_tok, int n_used, cudaStream_t st) {
+    (void) n_tok; (void) n_used;
+    const PrefillArgs a = batch_args(w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16, dst_col, n_experts);
     const int rows_out = (up ? DEC_WARPS / 2 : DEC_WARPS) * w.R;
     require(a.rows_per_expert % rows_out == 0, "rows per expert must be a multiple of the batched kernel's row block");
     if (g_workspace && two_pass(w, up, a, n_experts, st)) { return; }

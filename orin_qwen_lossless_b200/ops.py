@@ -640,6 +640,21 @@ def moe_mm_ids(x: torch.Tensor, topk_ids: torch.Tensor, w: Weight, n_experts: in
         raise RuntimeError("bf16n.moe_mm_ids: x must be contiguous bf16")
     if n_experts <= 0 or w.meta.rows % n_experts:
         raise RuntimeError("bf16n.moe_mm_ids: rows must split into n_experts")
+def _mm_ids_scratch(cw, cu, n_experts: int, T: int, n_used: int, device) -> torch.Tensor | None:
+    """Memory for the decoded tiles of one batched call on fragment-order experts, from torch's allocator and back to it
+    when the call has been enqueued; None where the fused kernel is the faster one, under stream capture (a graph would
+    keep the memory) and when the memory is not to be had."""
+    if torch.cuda.is_current_stream_capturing():
+        return None
+    need = lib().bf16n_mm_ids_scratch_bytes(C.byref(cw), C.byref(cu) if cu is not None else None, n_experts, T, n_used)
+    if need == 0:
+        return None
+    try:
+        return torch.empty(need + 1024, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
     T, n_used = topk_ids.shape
     N = w.meta.rows // n_experts
     per_slot = x.dim() == 3
@@ -654,9 +669,12 @@ def moe_mm_ids(x: torch.Tensor, topk_ids: torch.Tensor, w: Weight, n_experts: in
     if _auto_workspace and not torch.cuda.is_current_stream_capturing():
         ensure_workspace((w, up))
     with torch.cuda.device(x.device):
-        check(lib().bf16n_mm_ids(C.byref(cw), C.byref(cu) if cu is not None else None, x.data_ptr(), w.meta.K,
-                                 src1.data_ptr(), dst.data_ptr(), bounds.data_ptr(), y.data_ptr(),
-                                 int(out_dtype == torch.bfloat16), N, n_experts, T, n_used, _stream()))
+        scratch = _mm_ids_scratch(cw, cu, n_experts, T, n_used, x.device) if w.meta.frag_order else None
+        if scratch is None:
+            check(lib().bf16n_mm_ids(*args, _stream()))
+        else:
+            off = (-scratch.data_ptr()) % 1024
+            check(lib().bf16n_mm_ids_scratch(*args, scratch.data_ptr() + off, scratch.numel() - off, _stream()))
     return y
 
 
