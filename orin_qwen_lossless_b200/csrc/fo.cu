@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const Pair
         if (bytes <= FO_SPLIT_CAP) {
             const uint32_t landed = mbar_wait(bar, 0u);
             if (landed) {
-                StagedReader rd;
+                WindowReader rd;
                 rd.open(smem_u32(buf) + 4 * (w0 - (w0 & ~3u) + my), landed);
                 by_members(rd, smem_u32(lut));
             } else { // the copy never arrived: the flag reports it and the band's outputs become NaN
@@ -827,7 +827,7 @@ __global__ void __launch_bounds__(1024) k_fo_gemv_staged(const PairView w, const
                     break;
                 }
                 parity ^= 1u << bi;
-                StagedReader rd;
+                WindowReader rd;
                 rd.open(smem_u32(buf + bi * FO_CAP) + 4 * cur.my, landed);
                 body(rd, smem_u32(lut));
             } else {

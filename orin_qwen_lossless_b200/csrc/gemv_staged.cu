@@ -9,9 +9,8 @@
 //     mixed-precision fma (BF16 x BF16 + FP32, exact products, one rounding: the same bits as FP32 fma of the widened
 //     values);
 //   * reads the sign|mantissa plane with 16-byte streaming loads, one row ahead;
-//   * walks the bit streams with a 64-bit buffer, a one-word look-ahead and a refill test every second code whose
-//     bookkeeping needs no masking: table entries carry the code length in their low bits and the funnel shifts use
-//     only the low 5 bits of their shift operand.
+//   * walks the bit streams with the window reader (staged.cuh), whose bookkeeping needs no masking: table entries carry the
+//     code length in their low bits and the funnel shifts use only the low 5 bits of their shift operand.
 // Units that do not fit the buffer (codes much longer than average) are decoded straight from global memory.
 // Products are summed in the format's order (see gemv.cu), so results equal the general kernel's bit for bit.
 #include "staged.cuh"
@@ -128,7 +127,7 @@ __global__ void __launch_bounds__(512, 1) k_pair_gemv_staged(const PairView w, c
             // nothing to compute; the block still reaches its end (and, with peers, its announcement)
         } else if (staged) {
             parity ^= 1u;
-            StagedReader rd;
+            WindowReader rd;
             rd.open(smem_u32(buf) + 4 * cur.my, landed);
             mine = unit_rows<C, TX>(rd, smem_u32(lut), k, pl, R, x, lane);
         } else {

@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(256) k_expert_units(const ExpertMat m0, const 
             if (lane == 0) { atomicOr(&g_wait_expired, 1u); }
             mine = __int_as_float(0x7fc00000);
         } else {
-            StagedReader rd;
+            WindowReader rd;
             rd.open(smem_u32(buf) + 4 * my, landed);
             mine = rows(rd, smem_u32(lut));
         }
