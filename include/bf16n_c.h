@@ -158,7 +158,6 @@ int bf16n_mm_ids(const bf16n_weight * w, const bf16n_weight * up, const void * x
  * workspace = NULL withdraws it. bf16n_mm_ids_workspace_bytes returns 0 for matrices the two-pass form does not take
  * (fragment order, NIBBLE, other unit shapes): rows * K * 2 bytes for one matrix, twice that for a gate/up pair. */
 size_t bf16n_mm_ids_workspace_bytes(const bf16n_weight * w, const bf16n_weight * up);
-int bf16n_set_workspace(void * workspace, size_t bytes);
 /* No reference counterpart: the two-pass form for fragment-order experts, with the buffer of this one call. scratch_bytes
  * returns what such a call can use (0: the fused kernel is faster at these sizes, or the matrices have no two-pass form);
  * a smaller buffer is used in more, shorter ranges of experts, and one that holds no expert (or null) runs the fused kernel. The
@@ -167,6 +166,7 @@ size_t bf16n_mm_ids_scratch_bytes(const bf16n_weight * w, const bf16n_weight * u
 int bf16n_mm_ids_scratch(const bf16n_weight * w, const bf16n_weight * up, const void * x_bf16, int64_t x_row,
                          const int32_t * ids_src1, const int32_t * ids_dst, const int32_t * bounds, void * dst, int dst_bf16,
                          int64_t dst_col, int n_experts, int n_tok, int n_used, void * scratch, size_t scratch_bytes, void * stream);
+int bf16n_set_workspace(void * workspace, size_t bytes);
 /* y[t, i] = sum_k w[t, k] * ys[t, k, i] in slot order (FP32). Replaces bf16n::moe_combine (launch.h:81-82,
  * launch.cu:539-572). */
 int bf16n_moe_combine(const float * ys, const void * w, int w_bf16, void * y, int y_bf16, int n_tok, int n_used, int64_t n,

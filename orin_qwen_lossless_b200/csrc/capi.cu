@@ -364,6 +364,27 @@ int bf16n_mm_ids(const bf16n_weight * w, const bf16n_weight * up, const void * x
     });
 }
 
+size_t bf16n_mm_ids_scratch_bytes(const bf16n_weight * w, const bf16n_weight * up, int n_experts, int n_tok, int n_used) {
+    if (!w || !w->fo || (up && !up->fo) || n_experts <= 0 || w->rows % n_experts || n_tok <= 0 || n_used <= 0) { return 0; }
+    return fo_mm_ids_scratch_bytes(*w, up, n_experts, n_tok, n_used);
+}
+
+int bf16n_mm_ids_scratch(const bf16n_weight * w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
+                         const int32_t * ids_dst, const int32_t * bounds, void * dst, int dst_bf16, int64_t dst_col, int n_experts,
+                         int n_tok, int n_used, void * scratch, size_t scratch_bytes, void * stream) {
+    return guarded([&] {
+        ensure_init();
+        check_weight(*w);
+        if (up) { check_weight(*up); }
+        require(n_experts > 0 && w->rows % n_experts == 0, "rows must split evenly into experts");
+        require(fo_mm_ids_supported(*w, up), "mm_ids_scratch: fragment-order experts only");
+        fo_require_expert_count(up != nullptr, n_experts);
+        if (prefill_fo_two_pass(*w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16 != 0, dst_col, n_experts, scratch,
+                                scratch_bytes, (cudaStream_t) stream)) { return; }
+        fo_mm_ids(*w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16 != 0, dst_col, n_experts, (cudaStream_t) stream);
+    });
+}
+
 size_t bf16n_mm_ids_workspace_bytes(const bf16n_weight * w, const bf16n_weight * up) {
     return w ? prefill_workspace_bytes(*w, up) : 0;
 }
@@ -386,27 +407,6 @@ int bf16n_moe_combine(const float * ys, const void * w, int w_bf16, void * y, in
 int bf16n_swiglu(const float * g, const float * u, float * y, int64_t n, void * stream) {
     return guarded([&] {
         ensure_init();
-size_t bf16n_mm_ids_scratch_bytes(const bf16n_weight * w, const bf16n_weight * up, int n_experts, int n_tok, int n_used) {
-    if (!w || !w->fo || (up && !up->fo) || n_experts <= 0 || w->rows % n_experts || n_tok <= 0 || n_used <= 0) { return 0; }
-    return fo_mm_ids_scratch_bytes(*w, up, n_experts, n_tok, n_used);
-}
-
-int bf16n_mm_ids_scratch(const bf16n_weight * w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
-                         const int32_t * ids_dst, const int32_t * bounds, void * dst, int dst_bf16, int64_t dst_col, int n_experts,
-                         int n_tok, int n_used, void * scratch, size_t scratch_bytes, void * stream) {
-    return guarded([&] {
-        ensure_init();
-        check_weight(*w);
-        if (up) { check_weight(*up); }
-        require(n_experts > 0 && w->rows % n_experts == 0, "rows must split evenly into experts");
-        require(fo_mm_ids_supported(*w, up), "mm_ids_scratch: fragment-order experts only");
-        fo_require_expert_count(up != nullptr, n_experts);
-        if (prefill_fo_two_pass(*w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16 != 0, dst_col, n_experts, scratch,
-                                scratch_bytes, (cudaStream_t) stream)) { return; }
-        fo_mm_ids(*w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16 != 0, dst_col, n_experts, (cudaStream_t) stream);
-    });
-}
-
         moe_swiglu(g, u, y, n, (cudaStream_t) stream);
     });
 }

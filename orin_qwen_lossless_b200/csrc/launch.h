@@ -92,6 +92,8 @@ bool fo_mm_ids_supported(const bf16n_weight & w, const bf16n_weight * up);
 void fo_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
                const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
                cudaStream_t st);
+void fo_require_expert_count(bool glu, int n_experts);
+size_t fo_mm_ids_scratch_bytes(const bf16n_weight & w, const bf16n_weight * up, int n_experts, int n_tok, int n_used);
 void fo_expand_store(const bf16n_weight & w, int64_t row0, int64_t nrows, uint16_t * out, cudaStream_t st);
 void fo_expand_compare(const bf16n_weight & w, int64_t row0, int64_t nrows, const uint16_t * src, unsigned long long * total,
                        cudaStream_t st);
@@ -103,8 +105,6 @@ void peer_wait(uint32_t * local_header, int n_peers_mask, cudaStream_t st);
 
 // ep_prefill.cu: expert-parallel prefill, rows exchanged with peer stores
 size_t ep_layout_fill(bf16n_ep_layout & l);
-void fo_require_expert_count(bool glu, int n_experts);
-size_t fo_mm_ids_scratch_bytes(const bf16n_weight & w, const bf16n_weight * up, int n_experts, int n_tok, int n_used);
 void ep_dispatch(const bf16n_ep_layout & l, const void * x_bf16, int64_t x_row, const int32_t * ids, int n_tok, int n_used, int n_experts,
                  int32_t * plan, cudaStream_t st);
 void ep_inbox_ids(const bf16n_ep_layout & l, int32_t * ids_out, cudaStream_t st);
@@ -145,6 +145,11 @@ void prefill_init();
 void expand_tiles_init();
 bool expand_tiles_supported(const bf16n_weight & w);
 void expand_tiles(const bf16n_weight & w, const bf16n_weight * up, int n_experts, const int32_t * bounds, void * images, cudaStream_t st);
+void expand_tiles_fo(const bf16n_weight & w, const bf16n_weight * up, int n_experts, int e0, int n, const int32_t * bounds, void * images,
+                     cudaStream_t st);
+bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
+                         const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
+                         void * scratch, size_t scratch_bytes, cudaStream_t st);
 void prefill_set_workspace(void * p, size_t bytes);
 size_t prefill_workspace_bytes(const bf16n_weight & w, const bf16n_weight * up);
 bool prefill_supported(const bf16n_weight & w, const bf16n_weight * up);
@@ -153,8 +158,3 @@ void prefill_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void 
                     int n_tok, int n_used, cudaStream_t st);
 
 } // namespace b16
-void expand_tiles_fo(const bf16n_weight & w, const bf16n_weight * up, int n_experts, int e0, int n, const int32_t * bounds, void * images,
-                     cudaStream_t st);
-bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
-                         const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
-                         void * scratch, size_t scratch_bytes, cudaStream_t st);

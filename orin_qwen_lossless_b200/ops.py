@@ -628,18 +628,6 @@ def moe_route(topk_ids: torch.Tensor, n_experts: int, per_slot: bool):
     return src1, dst, bounds
 
 
-def moe_mm_ids(x: torch.Tensor, topk_ids: torch.Tensor, w: Weight, n_experts: int, up: Weight | None = None,
-               out_dtype: torch.dtype = torch.float32, route=None) -> torch.Tensor:
-    """Batched routed product (more than 8 tokens). route: the (ids_src1, ids_dst, bounds) of moe_route for these ids and
-    this activation layout, when the caller already has them (moe_experts sorts once for both of its products)."""
-    cw = w.c()
-    cu = up.c() if up is not None else None
-    _check_ids(topk_ids)
-    _check_x(x, w.meta.K)
-    if x.dtype != torch.bfloat16 or not x.is_contiguous():
-        raise RuntimeError("bf16n.moe_mm_ids: x must be contiguous bf16")
-    if n_experts <= 0 or w.meta.rows % n_experts:
-        raise RuntimeError("bf16n.moe_mm_ids: rows must split into n_experts")
 def _mm_ids_scratch(cw, cu, n_experts: int, T: int, n_used: int, device) -> torch.Tensor | None:
     """Memory for the decoded tiles of one batched call on fragment-order experts, from torch's allocator and back to it
     when the call has been enqueued; None where the fused kernel is the faster one, under stream capture (a graph would
@@ -655,6 +643,18 @@ def _mm_ids_scratch(cw, cu, n_experts: int, T: int, n_used: int, device) -> torc
         return None
 
 
+def moe_mm_ids(x: torch.Tensor, topk_ids: torch.Tensor, w: Weight, n_experts: int, up: Weight | None = None,
+               out_dtype: torch.dtype = torch.float32, route=None) -> torch.Tensor:
+    """Batched routed product (more than 8 tokens). route: the (ids_src1, ids_dst, bounds) of moe_route for these ids and
+    this activation layout, when the caller already has them (moe_experts sorts once for both of its products)."""
+    cw = w.c()
+    cu = up.c() if up is not None else None
+    _check_ids(topk_ids)
+    _check_x(x, w.meta.K)
+    if x.dtype != torch.bfloat16 or not x.is_contiguous():
+        raise RuntimeError("bf16n.moe_mm_ids: x must be contiguous bf16")
+    if n_experts <= 0 or w.meta.rows % n_experts:
+        raise RuntimeError("bf16n.moe_mm_ids: rows must split into n_experts")
     T, n_used = topk_ids.shape
     N = w.meta.rows // n_experts
     per_slot = x.dim() == 3
