@@ -998,9 +998,11 @@ void fo_require_expert_count(bool glu, int n_experts) {
 //   down (2048 x 512), 256 experts:             304 / 309, 357 / 330, 395 / 334, 548 / 336, 1119 / 529
 //                       16 experts:              28 / 37,   32 / 40,   33 / 39,   56 / 39,   83 / 57
 // hence the two lines; a call with few pairs per expert is left alone although a pair of matrices would gain a little.
-// At most 512 MiB (128 experts of the gate/up pair at a time), the order of the call's own FP32 outputs at 8192 tokens.
+// At most 1 GiB (256 experts of the gate/up pair at a time, twice the call's own FP32 outputs at 8192 tokens): every range
+// ends with partly empty waves of both passes (gate/up of 256 experts in 1, 2, 4, 16 ranges: 541 / 602 / 664 / 1156 us at
+// 64 pairs per expert, 855 / 957 / 1041 / 1939 at 256), which images that stay in L2 do not make up for.
 constexpr int64_t FO_TWO_PASS_GLU = 16, FO_TWO_PASS_ONE = 80; // routed pairs per expert
-constexpr size_t FO_SCRATCH_MAX = (size_t) 512 << 20;
+constexpr size_t FO_SCRATCH_MAX = (size_t) 1 << 30;
 
 size_t fo_mm_ids_scratch_bytes(const bf16n_weight & w, const bf16n_weight * up, int n_experts, int n_tok, int n_used) {
     const size_t per_expert = (size_t) (w.rows / n_experts) * (size_t) w.K * 2 * (up ? 2 : 1);
