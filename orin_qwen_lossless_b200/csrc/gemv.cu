@@ -4,7 +4,8 @@
 // implies (four accumulators per lane by column & 3, chunks in order, then a xor butterfly), which makes the results
 // independent of the launch geometry and equal, bit for bit, to the reference kernels' order
 // (core/include/bf16n/kernels.cuh:498-535, 958-986, 139-187).
-#include "decode.cuh"
+#include "sinks.cuh"
+#include "staged.cuh"
 #include "launch.h"
 #include <cstdlib>
 
@@ -12,7 +13,6 @@ namespace b16 {
 namespace {
 
 using namespace dev;
-using bf16 = __nv_bfloat16;
 
 // FP32 products of one row-chunk (this lane's 16 weights, as 8 BF16x2 words) with the matching activations
 __device__ __forceinline__ void fma_chunk(const uint32_t (&w)[8], const float4 (&x)[4], float (&a)[4]) {
@@ -321,47 +321,6 @@ __global__ void __launch_bounds__(256) k_nib_gemv(const NibView g, const NibView
 
 // ---------------------------------------------------------------- exact reconstruction (dequant / verify / gather)
 
-struct StoreBF16 { // row-major BF16 output
-    uint16_t * out;
-    int64_t K;
-    __device__ __forceinline__ void chunk(int64_t r, int c, int lane, const uint32_t (&w)[8]) {
-        uint16_t * o = out + r * K + c * CHUNK + 4 * lane;
-#pragma unroll
-        for (int j = 0; j < 4; j++) { *(uint2 *) (o + 128 * j) = make_uint2(w[2 * j], w[2 * j + 1]); }
-    }
-    __device__ __forceinline__ void one(int64_t r, int col, uint32_t bits) { out[r * K + col] = (uint16_t) bits; }
-    __device__ __forceinline__ void finish(int) {}
-};
-
-struct CompareBF16 { // count words that differ from src
-    const uint16_t * src;
-    int64_t K;
-    unsigned long long * total;
-    unsigned int bad;
-    __device__ __forceinline__ void chunk(int64_t r, int c, int lane, const uint32_t (&w)[8]) {
-        const uint16_t * o = src + r * K + c * CHUNK + 4 * lane;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint2 s = __ldg((const uint2 *) (o + 128 * j));
-            const uint32_t d0 = s.x ^ w[2 * j], d1 = s.y ^ w[2 * j + 1];
-            bad += ((d0 & 0xFFFFu) != 0) + ((d0 >> 16) != 0) + ((d1 & 0xFFFFu) != 0) + ((d1 >> 16) != 0);
-        }
-    }
-    // NIBBLE escapes: the dense pass saw +0 where src holds the escaped value, so every escape that matches its source
-    // takes back one counted difference (and a wrong one keeps it)
-    __device__ __forceinline__ void one(int64_t r, int col, uint32_t bits) {
-        const uint32_t s = src[r * K + col];
-        if (s != 0) { bad -= 1; }
-        if (s != bits) { bad += 1; }
-    }
-    __device__ __forceinline__ void finish(int lane) {
-        unsigned int b = bad;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) { b += __shfl_xor_sync(FULL, b, o); }
-        if (lane == 0 && b) { atomicAdd(total, (unsigned long long) b); }
-    }
-};
-
 template <typename Sink>
 __global__ void __launch_bounds__(256) k_pair_expand(const PairView w, int C, int R, bool cm, int64_t row0, int64_t nrows, const Sink sink_in) {
     Sink sink = sink_in;
@@ -649,7 +608,9 @@ void launch_expand(const bf16n_weight & w, int64_t row0, int64_t nrows, const Si
     const unsigned gx = (unsigned) std::max<int64_t>(1, std::min<int64_t>((work + 7) / 8, (int64_t) device_info().sms * 16));
     if (w.format == FMT_NIBBLE) {
         k_nib_expand<Sink><<<gx, 256, 0, st>>>(nib_view(w), C, row0, nrows, sink);
-    } else if (w.format == FMT_HUFPAIR) {
+    } else if (expand_rows_applies(w)) {
+        expand_rows(w, row0, nrows, sink, st);
+    } else if (w.format == FMT_HUFPAIR) { // fewer than four steps of 512 weights to a unit (R = 1 or 2, short rows)
         k_pair_expand<Sink><<<gx, 256, 0, st>>>(pair_view(w), C, w.R, w.cm != 0, row0, nrows, sink);
     } else {
         k_huf_expand<Sink><<<gx, 256, 0, st>>>(huf_view(w), C, w.R, row0, nrows, sink);
@@ -674,7 +635,7 @@ void gemv_init() {
     ATTR((k_pair_glu<8, bf16>), 8 * HP_MAX_PAIRS + 8 * CHUNK * 4);
     ATTR((k_pair_glu<4, float>), 8 * HP_MAX_PAIRS + 4 * CHUNK * 4);
     ATTR((k_pair_glu<4, bf16>), 8 * HP_MAX_PAIRS + 4 * CHUNK * 4);
-#undef ATTR
+    expand_rows_init();
     gemv_staged_init();
     gemv_rings_init();
 }

@@ -54,6 +54,13 @@ __device__ __forceinline__ void grid_dependency_wait() {
 }
 #endif
 
+// expand_rows.cu: exact reconstruction of lane-major HUFPAIR matrices
+namespace dev { struct StoreBF16; struct CompareBF16; }
+void expand_rows_init();
+bool expand_rows_applies(const bf16n_weight & w);
+void expand_rows(const bf16n_weight & w, int64_t row0, int64_t nrows, const dev::StoreBF16 & sink, cudaStream_t st);
+void expand_rows(const bf16n_weight & w, int64_t row0, int64_t nrows, const dev::CompareBF16 & sink, cudaStream_t st);
+
 // gemv.cu
 void gemv_init();
 void gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers = nullptr);
