@@ -108,6 +108,7 @@ int bf16n_sm_count(int * out);
 #define BF16N_FAULT_MOE_DECODE 2u
 #define BF16N_FAULT_FRAG_ORDER 4u
 #define BF16N_FAULT_PREFILL 8u
+#define BF16N_FAULT_ROW_GATHER 16u
 int bf16n_fault_status(unsigned int * flags, void * stream);
 
 /* GEMV (<= a few columns), dense or routed by expert ids. multi_col != 0: dense batches of 2..4 columns decode the
@@ -185,6 +186,12 @@ int bf16n_int4_quantize(const void * w_bf16, int64_t rows, int K, uint8_t * q, f
 int bf16n_int4_gemv(const void * x_bf16, int T, const uint8_t * q, const float * s, int64_t rows, int K, float * y, void * stream);
 int bf16n_int2_quantize(const void * w_bf16, int64_t rows, int K, uint8_t * q, float * s, void * stream);
 int bf16n_int2_gemv(const void * x_bf16, int T, const uint8_t * q, const float * s, int64_t rows, int K, float * y, void * stream);
+/* Draft-token logits from the scores [T, rows] of a k-bit copy: the n_cand largest scores of each token (ties: lowest row) name
+ * the candidates, whose lossless rows are gathered into cand_rows [T * n_cand, K] BF16 and multiplied with x [T, K] in FP32;
+ * out [T, vocab] gets those products and -inf everywhere else. cand [T, n_cand] receives the candidates, in no particular
+ * order. Replaces the topk, row gather, einsum and scatter of engines/vllm/vllm_bf16n/ops.py:222-240. */
+int bf16n_draft_logits(const float * scores, int T, int64_t rows, int n_cand, const bf16n_weight * w, const void * x_bf16, int32_t * cand,
+                       void * cand_rows, float * out, int64_t vocab, void * stream);
 
 /* Router on the GPU: softmax over n_experts logits per token, the k largest (ties: lowest index), weights renormalised
  * to sum 1. The reference core takes ids and weights from its engines (tests/core/test_kernels.py:333-345 synthesise

@@ -17,7 +17,7 @@ std::once_flag g_once;
 int g_init_status = BF16N_OK;
 std::string g_init_error;
 int g_device = -1;                         // the device bf16n_init ran on: the only one this process may launch on
-unsigned int * g_fault_words[4] = {};      // bit i of bf16n_fault_status: gemv_staged, moe_decode, fragment order, prefill
+unsigned int * g_fault_words[5] = {};      // bit i of bf16n_fault_status: gemv_staged, moe_decode, fragment order, prefill, row gather
 std::atomic<uint64_t> g_peer_wait_ns{2000000000ull};
 
 template <typename F>
@@ -50,10 +50,12 @@ void ensure_init() {
             moe_decode_init();
             prefill_init();
             fo_init();
+            draft_init();
             g_fault_words[0] = gemv_staged_fault_word();
             g_fault_words[1] = moe_decode_fault_word();
             g_fault_words[2] = fo_fault_word();
             g_fault_words[3] = prefill_fault_word();
+            g_fault_words[4] = row_gather_fault_word();
         } catch (const std::exception & e) {
             g_init_status = BF16N_ECUDA;
             g_init_error = e.what();
@@ -183,14 +185,14 @@ int bf16n_fault_status(unsigned int * flags, void * stream) {
         require(flags != nullptr, "fault_status: null argument");
         ensure_init();
         cudaStream_t st = (cudaStream_t) stream;
-        unsigned int seen[4] = {0, 0, 0, 0};
-        for (int i = 0; i < 4; i++) {
+        unsigned int seen[5] = {0, 0, 0, 0, 0};
+        for (int i = 0; i < 5; i++) {
             cuda_ok(cudaMemcpyAsync(&seen[i], g_fault_words[i], sizeof(unsigned int), cudaMemcpyDeviceToHost, st), "fault word read");
             cuda_ok(cudaMemsetAsync(g_fault_words[i], 0, sizeof(unsigned int), st), "fault word clear");
         }
         cuda_ok(cudaStreamSynchronize(st), "fault word read");
         *flags = 0;
-        for (int i = 0; i < 4; i++) { if (seen[i]) { *flags |= 1u << i; } }
+        for (int i = 0; i < 5; i++) { if (seen[i]) { *flags |= 1u << i; } }
     });
 }
 
@@ -205,6 +207,26 @@ int bf16n_int4_gemv(const void * x_bf16, int T, const uint8_t * q, const float *
 }
 int bf16n_int2_gemv(const void * x_bf16, int T, const uint8_t * q, const float * s, int64_t rows, int K, float * y, void * stream) {
     return guarded([&] { ensure_init(); draft_gemv(2, x_bf16, T, q, s, rows, K, y, (cudaStream_t) stream); });
+}
+
+int bf16n_draft_logits(const float * scores, int T, int64_t rows, int n_cand, const bf16n_weight * w, const void * x_bf16, int32_t * cand,
+                       void * cand_rows, float * out, int64_t vocab, void * stream) {
+    return guarded([&] {
+        ensure_init();
+        require(scores && w && x_bf16 && cand && cand_rows && out, "draft_logits: null argument");
+        check_weight(*w);
+        require(T >= 1 && T <= 65535 && rows >= 1 && rows <= INT32_MAX - 8192, "draft_logits: sizes out of range");
+        require(n_cand >= 1 && n_cand <= rows && (int64_t) T * n_cand < INT32_MAX, "draft_logits: 1..rows candidates");
+        require(rows <= w->rows && rows <= vocab, "draft_logits: the scores have more rows than the matrix or the logits");
+        require(!w->cm && w->format != FMT_HUFFMAN, "draft_logits: no row gather for this matrix");
+        require(((uintptr_t) x_bf16 | (uintptr_t) cand_rows) % 16 == 0, "draft_logits: x and the row buffer must be 16-byte aligned");
+        cudaStream_t st = (cudaStream_t) stream;
+        draft_select(scores, T, rows, n_cand, cand, out, vocab, st);
+        const int64_t n = (int64_t) T * n_cand;
+        if (frag_order(*w)) { fo_gather_rows(*w, cand, 4, n, cand_rows, true, w->K * 2, 0, st); }
+        else { gather_rows(*w, cand, 4, n, cand_rows, true, w->K * 2, 0, st); }
+        draft_rescore(x_bf16, cand_rows, cand, T, n_cand, (int) w->K, out, vocab, st);
+    });
 }
 
 int bf16n_set_peer_wait_limit_ms(unsigned int ms) {

@@ -435,6 +435,89 @@ __global__ void __launch_bounds__(256) k_pair_rows(const PairView w, int C, int 
     }
 }
 
+// The same gather for few rows (a draft step's candidates, the tokens of a decode batch), where the time is one warp's
+// chain of table lookups from the start of its unit: up to R - 1 rows only to find where the wanted one begins. The unit's
+// streams come into shared memory with one bulk copy, and the rows before the wanted one are passed over with a second
+// table that gives, for 12 bits of stream, the codes that end in them (up to three, two for most) and their length: each
+// lane passes over its own codes, the lanes need not stay in step before the row is read.
+constexpr int ROWS_THREADS = 256;
+template <bool BF>
+__global__ void __launch_bounds__(ROWS_THREADS) k_pair_rows_staged(const PairView w, const AuxHeader * hdr, int C, int R, const char * ids,
+                                                                   int64_t ids_s0, int64_t n, int64_t row0, char * dst, int64_t dst_s1, int rows_per_block,
+                                                                   uint32_t cap, const Opaque k) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    uint32_t * lut = (uint32_t *) smem;                              // code table | codes and bits per 12 bits | one barrier per row | streams
+    uint16_t * many = (uint16_t *) (smem + 4 * HP_MAX_PAIRS);
+    uint64_t * bars = (uint64_t *) (smem + 6 * HP_MAX_PAIRS);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char * buf = smem + 6 * HP_MAX_PAIRS + 128 + (size_t) warp * cap;
+    const uint32_t bar = smem_u32(bars + warp);
+    const bool reads = warp < rows_per_block;
+    if (reads && lane == 0) { mbar_init(bar, 1); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    stage_lut(lut, w.lut, HP_MAX_PAIRS);
+    __syncthreads();
+    for (int i = threadIdx.x; i < HP_MAX_PAIRS; i += ROWS_THREADS) {
+        uint32_t len = 0, count = 0;
+        for (; count < 3; count++) { // a prefix code: a code of at most the bits that are left is decided by them
+            const uint32_t l = lut[(uint32_t) (i << len) & (HP_MAX_PAIRS - 1)] & 31u;
+            if (len + l > (uint32_t) HP_LMAX) { break; }
+            len += l;
+        }
+        many[i] = (uint16_t) (len | count << 8);
+    }
+    grid_dependency_wait(); // the row ids may come from the kernel before this one; everything above is the matrix's own
+    const int64_t i = (int64_t) blockIdx.x * rows_per_block + warp;
+    const bool live = reads && i < n;
+    int64_t gr = 0, gu = 0;
+    uint32_t first = 0, bytes = 0;
+    if (live) {
+        gr = row0 + *(const volatile int32_t *) (ids + i * ids_s0);
+        gu = gr / R;
+        const uint32_t w0 = __ldg(w.ubase + gu), w1 = gu + 1 < (int64_t) hdr->n_a ? __ldg(w.ubase + gu + 1) : (uint32_t) hdr->n_b;
+        const uint32_t start = w0 & ~3u;
+        bytes = ((w1 - start + 4u + 3u) & ~3u) * 4u;
+        if (bytes <= cap && lane == 0) {
+            mbar_expect_tx(bar, bytes);
+            bulk_g2s(smem_u32(buf), w.stream + start, bytes, bar);
+        }
+        first = 4u * (w0 - start + __ldg(w.lrel + gu * 32 + lane));
+    }
+    __syncthreads(); // `many` is complete
+    if (!live) { return; }
+    const int64_t K = (int64_t) C * CHUNK;
+    const uint8_t * pl = w.plane + gr * K + 16 * lane;
+    char * o = dst + i * dst_s1;
+    auto row = [&](auto & rd, uint32_t lut_arg) {
+        for (int c = 0; c < C; c++) {
+            uint32_t e[8], wv[8];
+            rd.take8(lut_arg, k, e);
+            assemble8(ld_stream16(pl + (int64_t) c * CHUNK), e, wv);
+            put_row_chunk<BF>(o, c, lane, wv);
+        }
+    };
+    if (bytes <= cap) {
+        const uint32_t landed = mbar_wait(bar, 0u);
+        if (!landed) { // the copy never arrived: the flag reports it and the row becomes NaN
+            if (lane == 0) { atomicOr(&g_wait_expired, 1u); }
+            const uint32_t nan[8] = {0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u};
+            for (int c = 0; c < C; c++) { put_row_chunk<BF>(o, c, lane, nan); }
+            return;
+        }
+        WindowReader rd;
+        rd.open(smem_u32(buf) + first, landed);
+        rd.skip((int) (gr - gu * R) * C * 8, smem_u32(many), smem_u32(lut), k);
+        row(rd, smem_u32(lut));
+    } else { // more than 3 bits per weight: straight from global memory
+        GlobalReader rd;
+        rd.lut = lut;
+        rd.rd.open(w, gu, lane);
+        uint32_t e[8];
+        for (int c = 0; c < (int) (gr - gu * R) * C; c++) { rd.take8(0u, k, e); }
+        row(rd, 0u);
+    }
+}
+
 template <bool BF>
 __global__ void __launch_bounds__(256) k_nib_rows(const NibView w, int C, const char * ids, int64_t ids_s0, int64_t n, int64_t row0,
                                                    char * dst, int64_t dst_s1) {
@@ -622,6 +705,8 @@ void launch_expand(const bf16n_weight & w, int64_t row0, int64_t nrows, const Si
 
 // ---------------------------------------------------------------- entry points used by the C ABI (capi.cu)
 
+BF16N_DEFINE_FAULT_WORD(row_gather_fault_word)
+
 void gemv_init() {
     const int optin = device_info().smem_optin;
 #define ATTR(KERNEL, BYTES) allow_dynamic_smem((const void *) KERNEL, (int) (BYTES), optin, #KERNEL)
@@ -635,6 +720,8 @@ void gemv_init() {
     ATTR((k_pair_glu<8, bf16>), 8 * HP_MAX_PAIRS + 8 * CHUNK * 4);
     ATTR((k_pair_glu<4, float>), 8 * HP_MAX_PAIRS + 4 * CHUNK * 4);
     ATTR((k_pair_glu<4, bf16>), 8 * HP_MAX_PAIRS + 4 * CHUNK * 4);
+    ATTR(k_pair_rows_staged<true>, 6 * HP_MAX_PAIRS + 128 + 2 * (16 * K_MAX * 3 / 8 + 80));
+    ATTR(k_pair_rows_staged<false>, 6 * HP_MAX_PAIRS + 128 + 2 * (16 * K_MAX * 3 / 8 + 80));
     expand_rows_init();
     gemv_staged_init();
     gemv_rings_init();
@@ -757,6 +844,14 @@ void gather_rows(const bf16n_weight & w, const void * ids, int64_t ids_s0, int64
     if (w.format == FMT_NIBBLE) {
         if (dst_bf16) { k_nib_rows<true><<<gx, 256, 0, st>>>(nib_view(w), C, ip, ids_s0, n, row0, dp, dst_s1); }
         else { k_nib_rows<false><<<gx, 256, 0, st>>>(nib_view(w), C, ip, ids_s0, n, row0, dp, dst_s1); }
+    } else if (n <= (int64_t) device_info().sms * 4) {
+        // few rows: spread over the SMs, at most two to a block (k_pair_rows: eight)
+        const int per = n > device_info().sms * 2 ? 2 : 1;
+        const uint32_t cap = (uint32_t) ((w.R * w.K * 3 / 8 + 64 + 15) & ~15ll);
+        const size_t shm = 6 * HP_MAX_PAIRS + 128 + (size_t) per * cap;
+        const Opaque k = {1u, 4u, ~0u, 32u};
+        launch_chained(dst_bf16 ? k_pair_rows_staged<true> : k_pair_rows_staged<false>, dim3((unsigned) ((n + per - 1) / per)), dim3(ROWS_THREADS), shm,
+                       st, pair_view(w), (const AuxHeader *) w.aux, C, w.R, ip, ids_s0, n, row0, dp, dst_s1, per, cap, k);
     } else {
         if (dst_bf16) { k_pair_rows<true><<<gx, 256, 0, st>>>(pair_view(w), C, w.R, ip, ids_s0, n, row0, dp, dst_s1); }
         else { k_pair_rows<false><<<gx, 256, 0, st>>>(pair_view(w), C, w.R, ip, ids_s0, n, row0, dp, dst_s1); }

@@ -46,6 +46,9 @@ void launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t shm,
     cfg.attrs = &attr; cfg.numAttrs = 1;
     cuda_ok(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...), "kernel launch");
 }
+// Lets the next kernel on the stream begin its own prologue now. Only for kernels in which every block that has work also
+// waits (grid_dependency_wait) before it touches what earlier kernels wrote or read.
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Blocks until every kernel this one depends on has completed and its writes are visible; then lets the next kernel on
 // the stream begin its own prologue.
 __device__ __forceinline__ void grid_dependency_wait() {
@@ -79,6 +82,7 @@ unsigned int * gemv_staged_fault_word();
 unsigned int * moe_decode_fault_word();
 unsigned int * fo_fault_word();
 unsigned int * prefill_fault_word();
+unsigned int * row_gather_fault_word();
 
 // gemv_staged.cu
 void gemv_staged_init();
@@ -146,6 +150,12 @@ void moe_decode_static(const bf16n_weight & gate, const bf16n_weight & up, const
 // draft.cu: draft-only 2-bit / 4-bit copies of an output head
 void draft_quantize(int bits, const void * w_bf16, int64_t rows, int K, uint8_t * q, float * s, cudaStream_t st);
 void draft_gemv(int bits, const void * x_bf16, int T, const uint8_t * q, const float * s, int64_t rows, int K, float * y, cudaStream_t st);
+
+void draft_init();
+// candidates (row ids [T, n_cand]) of FP32 scores [T, rows], and -inf everywhere in out [T, vocab]; then the candidates' exact scores
+void draft_select(const float * scores, int T, int64_t rows, int n_cand, int32_t * cand, float * out, int64_t vocab, cudaStream_t st);
+void draft_rescore(const void * x_bf16, const void * rows_bf16, const int32_t * cand, int T, int n_cand, int K, float * out, int64_t vocab,
+                   cudaStream_t st);
 
 // prefill.cu
 void prefill_init();

@@ -545,7 +545,19 @@ def draft_logits(h: torch.Tensor, w: Weight, head: DraftHead, vocab: int) -> tor
     other entry is -inf. A proposal path: candidate coverage does not guarantee the exact head's argmax."""
     n, K = h.shape
     h = h.contiguous()
-    cand = head.scores(h).topk(head.candidates, dim=-1).indices                   # [n, C]
+    scores = head.scores(h)
+    rows = scores.shape[1]
+    if rows <= min(w.meta.rows, vocab) and w.meta.K == K and w.plane.device == h.device and h.data_ptr() % 16 == 0:
+        cw = w.c()
+        cand = torch.empty((n, head.candidates), dtype=torch.int32, device=h.device)
+        cand_rows = torch.empty((n * head.candidates, K), dtype=torch.bfloat16, device=h.device)
+        out = torch.empty((n, vocab), dtype=torch.float32, device=h.device)
+        with torch.cuda.device(h.device):
+            check(lib().bf16n_draft_logits(scores.data_ptr(), n, rows, head.candidates, C.byref(cw), h.data_ptr(), cand.data_ptr(),
+                                           cand_rows.data_ptr(), out.data_ptr(), vocab, _stream()))
+        return out
+    # a head with padding rows beyond the vocabulary (or an unaligned h)
+    cand = scores.topk(head.candidates, dim=-1).indices                           # [n, C]
     rows = get_rows(cand.reshape(-1), w).view(n, head.candidates, K)              # exact BF16 rows
     exact = torch.einsum("nck,nk->nc", rows.float(), h.float())
     out = torch.full((n, vocab), float("-inf"), dtype=torch.float32, device=h.device)
@@ -668,6 +680,8 @@ def moe_mm_ids(x: torch.Tensor, topk_ids: torch.Tensor, w: Weight, n_experts: in
     src1, dst, bounds = moe_route(topk_ids, n_experts, per_slot) if route is None else route
     if _auto_workspace and not torch.cuda.is_current_stream_capturing():
         ensure_workspace((w, up))
+    args = (C.byref(cw), C.byref(cu) if cu is not None else None, x.data_ptr(), w.meta.K, src1.data_ptr(), dst.data_ptr(),
+            bounds.data_ptr(), y.data_ptr(), int(out_dtype == torch.bfloat16), N, n_experts, T, n_used)
     with torch.cuda.device(x.device):
         scratch = _mm_ids_scratch(cw, cu, n_experts, T, n_used, x.device) if w.meta.frag_order else None
         if scratch is None:
