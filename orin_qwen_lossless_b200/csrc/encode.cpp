@@ -166,7 +166,7 @@ std::vector<uint32_t> canonical_codes(const std::vector<uint8_t> & len, int L) {
 
 // MSB-first bit sink writing whole little-endian u32 words in place
 struct bit_sink {
-    uint32_t * out;
+    uint32_t * out = nullptr;
     uint64_t acc = 0;
     int nb = 0;
     inline void put(uint32_t code, int len) {
@@ -181,13 +181,13 @@ struct bit_sink {
     inline void finish() { if (nb) { *out++ = (uint32_t) (acc << (32 - nb)); } }
 };
 
-template <typename T> void put_at(std::vector<uint8_t> & buf, uint64_t off, const T * src, size_t n) {
+template <typename B, typename T> void put_at(B & buf, uint64_t off, const T * src, size_t n) {
     if (n) { memcpy(buf.data() + off, src, n * sizeof(T)); }
 }
 
 // ------------------------------------------------------------------ NIBBLE
 
-std::vector<uint8_t> encode_nibble(const uint16_t * w, int64_t rows, int64_t K, uint8_t * plane) {
+Bytes encode_nibble(const uint16_t * w, int64_t rows, int64_t K, uint8_t * plane) {
     const int64_t C = K / CHUNK;
     constexpr int64_t BLK = 256;
     const int64_t nblk = (rows + BLK - 1) / BLK;
@@ -247,7 +247,7 @@ std::vector<uint8_t> encode_nibble(const uint16_t * w, int64_t rows, int64_t K, 
     });
     for (int64_t r = 0; r < rows; r++) { esc_off[r + 1] += esc_off[r]; }
     h.n_a = esc_off[rows];
-    std::vector<uint8_t> aux(h.off_d + std::max<uint64_t>(h.n_a, 1) * 4, 0);
+    Bytes aux(h.off_d + std::max<uint64_t>(h.n_a, 1) * 4, 0);
     memcpy(aux.data(), head.data(), head.size());
     memcpy(aux.data(), &h, sizeof h);
     put_at(aux, h.off_c, esc_off.data(), esc_off.size());
@@ -338,32 +338,38 @@ Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, b
     }
 
     const int64_t units = frag_order ? rows / 16 * C : rows / R;
-    // symbols of lane l of unit u, in stream order
-    auto for_lane = [&](int64_t u, int l, auto && emit) {
-        if (!pair) {
-            for (int64_t r = u * R; r < (u + 1) * R; r++) {
-                for (int64_t c = 0; c < C; c++) {
-                    const uint16_t * p = w + r * K + c * CHUNK;
-                    for (int s = 0; s < 16; s++) { emit(expo(p[chunk_col(l, s)])); }
-                }
-            }
-        } else if (frag_order) {
+    // emit(l, a, b): the next two symbols of lane l's stream of unit u, every lane in its stream order. The weights are
+    // walked as they lie in memory, all lanes side by side (lane by lane, a unit's rows would be read 32 times).
+    auto for_unit = [&](int64_t u, auto && emit) {
+        if (pair && frag_order) {
             const int64_t band = u / C, slab = u % C;
             for (int64_t kt = slab * 32; kt < slab * 32 + 32; kt++) {
-                for (int q = 0; q < 4; q++) {
-                    int r, c;
-                    frag_rc(l, q, r, c);
-                    const uint16_t * p = w + (band * 16 + r) * K + kt * 16 + c;
-                    emit(expo(p[0]) | expo(p[1]) << 8);
+                for (int l = 0; l < 32; l++) {
+                    uint32_t sym[4];
+                    for (int q = 0; q < 4; q++) {
+                        int r, c;
+                        frag_rc(l, q, r, c);
+                        const uint16_t * p = w + (band * 16 + r) * K + kt * 16 + c;
+                        sym[q] = expo(p[0]) | expo(p[1]) << 8;
+                    }
+                    emit(l, sym[0], sym[1]);
+                    emit(l, sym[2], sym[3]);
                 }
             }
-        } else {
-            for (int64_t o = 0; o < R * C; o++) {
-                const int64_t r = u * R + (chunk_major ? o % R : o / C), c = chunk_major ? o / R : o % C;
-                const uint16_t * p = w + r * K + c * CHUNK;
-                for (int s = 0; s < 16; s += 2) {
-                    const uint16_t * q = p + chunk_col(l, s);
-                    emit(expo(q[0]) | expo(q[1]) << 8);
+            return;
+        }
+        for (int64_t o = 0; o < R * C; o++) {
+            const int64_t r = u * R + (chunk_major ? o % R : o / C), c = chunk_major ? o / R : o % C;
+            const uint16_t * p = w + r * K + c * CHUNK;
+            for (int j = 0; j < 4; j++) {
+                for (int l = 0; l < 32; l++) { // slots 4 j .. 4 j + 3
+                    const uint16_t * q = p + chunk_col(l, 4 * j);
+                    if (pair) {
+                        emit(l, expo(q[0]) | expo(q[1]) << 8, expo(q[2]) | expo(q[3]) << 8);
+                    } else {
+                        emit(l, expo(q[0]), expo(q[1]));
+                        emit(l, expo(q[2]), expo(q[3]));
+                    }
                 }
             }
         }
@@ -373,11 +379,9 @@ Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, b
     std::vector<uint32_t> lane_words((size_t) units * 32);
     parallel_ranges(units, 8, [&](int64_t u0, int64_t u1, int) {
         for (int64_t u = u0; u < u1; u++) {
-            for (int l = 0; l < 32; l++) {
-                uint64_t bits = 0;
-                for_lane(u, l, [&](uint32_t sym) { bits += cl[sym] & 15u; });
-                lane_words[u * 32 + l] = (uint32_t) ((bits + 31) / 32);
-            }
+            uint32_t bits[32] = {0};
+            for_unit(u, [&](int l, uint32_t a, uint32_t b) { bits[l] += (cl[a] & 15u) + (cl[b] & 15u); });
+            for (int l = 0; l < 32; l++) { lane_words[u * 32 + l] = (bits[l] + 31) / 32; }
         }
     });
     std::vector<uint64_t> unit_start(units + 1, 0);
@@ -405,7 +409,10 @@ Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, b
         stream_off = h.off_c;
     }
     h.n_a = (uint64_t) units; h.n_b = n_words;
-    out.aux.assign(stream_off + (n_words + tail) * 4, 0);
+    out.aux.resize(stream_off + (n_words + tail) * 4);
+    memset(out.aux.data(), 0, HEADER_BYTES);
+    if (pair) { memset(out.aux.data() + h.off_c + (uint64_t) units * 32 * 2, 0, h.off_d - h.off_c - (uint64_t) units * 32 * 2); }
+    memset(out.aux.data() + stream_off + n_words * 4, 0, (size_t) tail * 4);
     memcpy(out.aux.data(), &h, sizeof h);
     put_at(out.aux, h.off_a, lut.data(), lut.size());
 
@@ -438,12 +445,16 @@ Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, b
     parallel_ranges(units, 8, [&](int64_t u0, int64_t u1, int) {
         for (int64_t u = u0; u < u1; u++) {
             uint32_t * at = stream + unit_start[u];
+            bit_sink sink[32];
             for (int l = 0; l < 32; l++) {
-                bit_sink sink{at};
-                for_lane(u, l, [&](uint32_t sym) { sink.put(cl[sym] >> 4, (int) (cl[sym] & 15u)); });
-                sink.finish();
+                sink[l].out = at;
                 at += lane_words[u * 32 + l];
             }
+            for_unit(u, [&](int l, uint32_t a, uint32_t b) { // two codes of at most 12 bits in one put
+                const uint32_t ca = cl[a], cb = cl[b], nb = cb & 15u;
+                sink[l].put((ca >> 4) << nb | cb >> 4, (int) ((ca & 15u) + nb));
+            });
+            for (int l = 0; l < 32; l++) { sink[l].finish(); }
         }
     });
 

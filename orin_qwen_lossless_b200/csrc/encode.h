@@ -4,13 +4,24 @@
 #include "format.h"
 
 #include <cstdint>
+#include <memory>
+#include <utility>
 #include <vector>
 
 namespace b16 {
 
+// Bytes that resize() leaves as the allocator gives them: the encoder writes every one of them, from all threads, and a
+// zero fill beforehand would touch the pages of a large tensor once more, from one thread.
+template <typename T> struct no_fill : std::allocator<T> {
+    template <typename U> struct rebind { using other = no_fill<U>; };
+    template <typename U> void construct(U * p) noexcept { ::new ((void *) p) U; }
+    template <typename U, typename... A> void construct(U * p, A &&... a) { ::new ((void *) p) U(std::forward<A>(a)...); }
+};
+using Bytes = std::vector<uint8_t, no_fill<uint8_t>>;
+
 struct Encoded {
-    std::vector<uint8_t> plane; // rows * K sign|mantissa bytes
-    std::vector<uint8_t> aux;   // 256-byte header + exponent data
+    Bytes plane; // rows * K sign|mantissa bytes
+    Bytes aux;   // 256-byte header + exponent data
     int format = 0;             // format produced (a HUFPAIR request falls back to HUFFMAN above 4096 distinct pairs)
     int R = 0;                  // rows per unit, 0 for NIBBLE
 };

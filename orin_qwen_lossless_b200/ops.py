@@ -118,6 +118,24 @@ def sm_count() -> int:
 
 # ------------------------------------------------------------------ host: encode, policy
 
+class _Encoded:
+    """The encoder's result, freed when the last tensor over its memory is (the tensors are the buffers the encoder wrote,
+    not copies of them)."""
+
+    def __init__(self, handle):
+        self.handle, self.free = handle, lib().bf16n_encoded_free
+
+    def tensor(self, part) -> torch.Tensor:
+        n = C.c_size_t(0)
+        p = part(self.handle, C.byref(n))
+        buf = (C.c_uint8 * n.value).from_address(C.cast(p, C.c_void_p).value)
+        buf.owner = self      # torch.frombuffer keeps buf alive
+        return torch.frombuffer(buf, dtype=torch.uint8)
+
+    def __del__(self):
+        self.free(self.handle)
+
+
 def encode(w: torch.Tensor, fmt: int, R: int, chunk_major: bool, frag_order: bool = False
            ) -> tuple[torch.Tensor, torch.Tensor, Meta]:
     """Encode a BF16 CPU tensor (..., K) on all host cores: (plane uint8 [rows, K], aux uint8 [n], Meta). FMT_HUFPAIR
@@ -133,16 +151,9 @@ def encode(w: torch.Tensor, fmt: int, R: int, chunk_major: bool, frag_order: boo
     rows = wc.numel() // max(K, 1)
     h = C.c_void_p()
     check(lib().bf16n_encode(wc.data_ptr(), rows, K, fmt, R, int(chunk_major), int(frag_order), C.byref(h)))
-    try:
-        n = C.c_size_t(0)
-        p = lib().bf16n_encoded_plane(h, C.byref(n))
-        plane = torch.empty((rows, K), dtype=torch.uint8)
-        C.memmove(plane.data_ptr(), p, n.value)
-        p = lib().bf16n_encoded_aux(h, C.byref(n))
-        aux = torch.empty((n.value,), dtype=torch.uint8)
-        C.memmove(aux.data_ptr(), p, n.value)
-    finally:
-        lib().bf16n_encoded_free(h)
+    owner = _Encoded(h)
+    plane = owner.tensor(lib().bf16n_encoded_plane).view(rows, K)
+    aux = owner.tensor(lib().bf16n_encoded_aux)
     return plane, aux, parse_header(aux)
 
 
