@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(256) k_huf_gemv(const HufView g, const HufView
 // ---------------------------------------------------------------- NIBBLE: one warp per row
 
 template <int C>
-struct NibRow { uint4 sm[C]; uint2 cd[C]; uint4 L; uint32_t e0, e1; };
+struct NibRow { uint4 sm[C]; uint2 cd[C]; uint4 L; uint32_t e0, e1, rec; }; // rec: this lane's first escape record
 
 template <int C>
 __device__ __forceinline__ void nib_load(NibRow<C> & d, const NibView & w, int64_t row, int lane) {
@@ -270,51 +270,105 @@ __device__ __forceinline__ void nib_load(NibRow<C> & d, const NibView & w, int64
     d.L = __ldg(w.row_lut + row);
     d.e0 = __ldg(w.esc_off + row);
     d.e1 = __ldg(w.esc_off + row + 1);
+    d.rec = d.e0 + lane < d.e1 ? __ldg(w.esc + d.e0 + lane) : 0u;
 }
 
-// dot(row, x): dense pass (escaped slots decode to +0), then the row's escapes, then the butterfly
-template <int C, typename TX>
-__device__ __forceinline__ float nib_dot(const NibRow<C> & d, const NibView & w, const TX * __restrict__ x, int lane) {
-    float a[4] = {0.f, 0.f, 0.f, 0.f};
+// the row's BF16 pairs (escaped slots decode to +0), ready before the activations are
+template <int C>
+struct NibWords { uint32_t w[C][8]; uint32_t e0, e1, rec; };
+
+template <int C>
+__device__ __forceinline__ void nib_decode(const NibRow<C> & r, NibWords<C> & d) {
 #pragma unroll
     for (int c = 0; c < C; c++) {
-        uint32_t wv[8];
-        nib_assemble8(d.sm[c], d.cd[c], d.L, wv);
-        float4 xq[4];
+        nib_assemble8(r.sm[c], r.cd[c], r.L, d.w[c]);
 #pragma unroll
-        for (int j = 0; j < 4; j++) { xq[j] = ldg_x4(x, c * CHUNK + 128 * j + 4 * lane); }
-        fma_chunk(wv, xq, a);
+        for (int q = 0; q < 8; q++) { asm volatile("" : "+r"(d.w[c][q])); } // decoded here, not where they are used
     }
-    float acc = (a[0] + a[1]) + (a[2] + a[3]);
-    for (uint32_t i = d.e0 + lane; i < d.e1; i += 32) {
-        const uint32_t rec = __ldg(w.esc + i);
-        acc = fmaf(__uint_as_float(esc_bits(rec) << 16), ldg_x1(x, rec & 0xFFF), acc);
+    d.e0 = r.e0; d.e1 = r.e1; d.rec = r.rec;
+}
+
+// four activations as they lie in memory
+template <typename TX> struct RawX4;
+template <> struct RawX4<float> {
+    uint4 v;
+    __device__ __forceinline__ void load(const float * x) { v = ld_act16(x); }
+    __device__ __forceinline__ float4 f() const { return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)); }
+};
+template <> struct RawX4<bf16> {
+    uint2 v;
+    __device__ __forceinline__ void load(const bf16 * x) { v = ld_act8(x); }
+    __device__ __forceinline__ float4 f() const { return make_float4(bf16lo_f32(v.x), bf16hi_f32(v.x), bf16lo_f32(v.y), bf16hi_f32(v.y)); }
+};
+
+// dots of M decoded rows with x: dense pass, then each row's escapes, then the butterfly. The activations of up to four
+// chunks are requested before the first of them is used: one trip to L2, not one per chunk.
+template <int C, int M, typename TX>
+__device__ __forceinline__ void nib_dots(const NibWords<C> (&d)[M], const NibView * const (&w)[M], const TX * x, int lane, float (&sum)[M]) {
+    constexpr int G = C < 4 ? C : 4;
+    float a[M][4];
+#pragma unroll
+    for (int m = 0; m < M; m++) { a[m][0] = a[m][1] = a[m][2] = a[m][3] = 0.f; }
+#pragma unroll
+    for (int c0 = 0; c0 < C; c0 += G) {
+        RawX4<TX> q[G * 4];
+#pragma unroll
+        for (int i = 0; i < G * 4; i++) { q[i].load(x + (c0 + (i >> 2)) * CHUNK + 128 * (i & 3) + 4 * lane); }
+#pragma unroll
+        for (int c = 0; c < G; c++) {
+            const float4 xq[4] = {q[4 * c].f(), q[4 * c + 1].f(), q[4 * c + 2].f(), q[4 * c + 3].f()};
+#pragma unroll
+            for (int m = 0; m < M; m++) { fma_chunk(d[m].w[c0 + c], xq, a[m]); }
+        }
     }
-    return warp_sum(acc);
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        float acc = (a[m][0] + a[m][1]) + (a[m][2] + a[m][3]);
+        uint32_t rec = d[m].rec;
+        for (uint32_t i = d[m].e0 + lane; i < d[m].e1;) {
+            acc = fmaf(__uint_as_float(esc_bits(rec) << 16), ldg_x1(x, rec & 0xFFF), acc);
+            i += 32;
+            if (i < d[m].e1) { rec = __ldg(w[m]->esc + i); }
+        }
+        sum[m] = warp_sum(acc);
+    }
 }
 
 // GLU: g rows are the gate, v rows the up half (separate matrices, or the same matrix shifted by nrows rows)
+//
+// What bounds it: a decode step is a row of launches that depend on each other, each of a few microseconds. So everything
+// that does not need the kernel before it is done before the wait for it (launch_chained): the warp's first row is loaded, its
+// escapes with it, and decoded to BF16 pairs; its own dependents may start at once, since what they touch before their
+// wait belongs to no kernel (weights) and their wait ends only when this kernel, and with it the one it waits for, is complete.
+// Behind the wait are one trip to L2 for the activations (one per chunk, and two for a gate/up pair, before), the products and the
+// sums. 48 layers of three launches each: 460 -> 349 us; 20 layers at 2 / 4 tokens: 237 / 337 -> 188 / 256 us. Measured and left:
+// activations staged in shared memory once per block, its rows multiplied with up to four columns (359 us; 225 / 360).
+constexpr int nib_blocks(int C, bool glu) { return glu ? (C <= 2 ? 3 : C == 4 ? 2 : 1) : C == 8 ? 2 : C == 4 ? 3 : 4; } // per SM: room for the launches behind
 template <int C, typename TX, bool GLU>
-__global__ void __launch_bounds__(256) k_nib_gemv(const NibView g, const NibView v, Cols p) {
-    // Launched as a programmatic dependent (launch_chained): a warp fetches its first row's weights while the kernel
-    // before it on the stream is still draining, and waits for that kernel only before it reads activations or writes
-    // outputs (expert ids, when there are any, belong to an earlier kernel too).
-    bool waited = p.ids != nullptr;
-    if (waited) { grid_dependency_wait(); }
+__global__ void __launch_bounds__(256, nib_blocks(C, GLU)) k_nib_gemv(const NibView g, const NibView v, Cols p) {
+    constexpr int M = GLU ? 2 : 1;
+    bool waited = p.ids != nullptr; // expert ids, when there are any, belong to an earlier kernel too
+    if (waited) { grid_dependency_wait(); } else { grid_launch_dependents(); }
     const TX * xg; OutVec out; int64_t rbase;
     column<TX>(p, blockIdx.y, xg, out, rbase);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const NibView * w[M];
+    w[0] = &g;
+    if constexpr (GLU) { w[1] = &v; }
     for (int64_t r = (int64_t) blockIdx.x * 8 + warp; r < p.nrows; r += (int64_t) gridDim.x * 8) {
-        NibRow<C> dg, dv;
-        nib_load<C>(dg, g, rbase + r, lane);
-        if (GLU) { nib_load<C>(dv, v, rbase + r, lane); }
+        NibWords<C> d[M];
+        {
+            NibRow<C> row[M];
+#pragma unroll
+            for (int m = 0; m < M; m++) { nib_load<C>(row[m], *w[m], rbase + r, lane); }
+#pragma unroll
+            for (int m = 0; m < M; m++) { nib_decode<C>(row[m], d[m]); }
+        }
         if (!waited) { grid_dependency_wait(); waited = true; }
-        const float gs = nib_dot<C, TX>(dg, g, xg, lane);
-        if (GLU) {
-            const float vs = nib_dot<C, TX>(dv, v, xg, lane);
-            if (lane == 0) { out.put(r, vs * silu_f(gs)); }
-        } else if (lane == 0) {
-            out.put(r, gs);
+        float s[M];
+        nib_dots<C, M, TX>(d, w, xg, lane, s);
+        if (lane == 0) {
+            if constexpr (GLU) { out.put(r, s[1] * silu_f(s[0])); } else { out.put(r, s[0]); }
         }
     }
 }
@@ -560,6 +614,18 @@ dim3 row_geometry(int64_t work, int ncols) { // 8 warps per block, one work item
     return dim3((unsigned) std::max<int64_t>(1, std::min<int64_t>((work + 7) / 8, cap)), (unsigned) ncols);
 }
 
+template <typename TX, bool GLU>
+void launch_nib(const NibView & g, const NibView & v, const Cols & p, int64_t K, int ncols, cudaStream_t st) {
+    const dim3 grid = row_geometry(p.nrows, ncols);
+    switch (K / CHUNK) {
+        case 1: launch_chained(k_nib_gemv<1, TX, GLU>, grid, dim3(256), 0, st, g, v, p); break;
+        case 2: launch_chained(k_nib_gemv<2, TX, GLU>, grid, dim3(256), 0, st, g, v, p); break;
+        case 4: launch_chained(k_nib_gemv<4, TX, GLU>, grid, dim3(256), 0, st, g, v, p); break;
+        case 8: launch_chained(k_nib_gemv<8, TX, GLU>, grid, dim3(256), 0, st, g, v, p); break;
+        default: fail_invalid("unsupported K");
+    }
+}
+
 // Mid-size dense HUFPAIR matrices (256 units up to 4 per SM) with several columns: one staged decode per column over all
 // SMs instead of the general kernel's shared decode, whose warps read their lane streams straight from global memory
 // (4096 x 2048, R = 8: 29 -> 19 us at 4 tokens, 54 -> 33 us at 8; from 1024 units on the two forms are level).
@@ -634,15 +700,7 @@ void launch_gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t 
             }
         }
     } else if (w.format == FMT_NIBBLE) {
-        const dim3 grid = row_geometry(a.nrows, a.ncols);
-        const NibView v = nib_view(w);
-        switch (C) {
-            case 1: launch_chained(k_nib_gemv<1, TX, false>, grid, dim3(256), 0, st, v, v, p); break;
-            case 2: launch_chained(k_nib_gemv<2, TX, false>, grid, dim3(256), 0, st, v, v, p); break;
-            case 4: launch_chained(k_nib_gemv<4, TX, false>, grid, dim3(256), 0, st, v, v, p); break;
-            case 8: launch_chained(k_nib_gemv<8, TX, false>, grid, dim3(256), 0, st, v, v, p); break;
-            default: fail_invalid("unsupported K");
-        }
+        launch_nib<TX, false>(nib_view(w), nib_view(w), p, w.K, a.ncols, st);
     } else {
         const dim3 grid = row_geometry(a.nrows / w.R, a.ncols);
         const size_t shm = (4u << HUF_LMAX) + w.K * 4;
@@ -656,15 +714,7 @@ void launch_glu(const bf16n_weight & g, const NibView * up_nib, const bf16n_weig
     const Cols p = make_cols(a);
     const int C = (int) (g.K / CHUNK);
     if (g.format == FMT_NIBBLE) {
-        const dim3 grid = row_geometry(a.nrows, a.ncols);
-        const NibView gv = nib_view(g), uv = up_nib ? *up_nib : nib_view(*u);
-        switch (C) {
-            case 1: launch_chained(k_nib_gemv<1, TX, true>, grid, dim3(256), 0, st, gv, uv, p); break;
-            case 2: launch_chained(k_nib_gemv<2, TX, true>, grid, dim3(256), 0, st, gv, uv, p); break;
-            case 4: launch_chained(k_nib_gemv<4, TX, true>, grid, dim3(256), 0, st, gv, uv, p); break;
-            case 8: launch_chained(k_nib_gemv<8, TX, true>, grid, dim3(256), 0, st, gv, uv, p); break;
-            default: fail_invalid("unsupported K");
-        }
+        launch_nib<TX, true>(nib_view(g), up_nib ? *up_nib : nib_view(*u), p, g.K, a.ncols, st);
     } else if (g.format == FMT_HUFPAIR) {
         dim3 grid; int threads;
         unit_geometry(a.nrows / g.R, a.ncols, 16, grid, threads);
@@ -740,7 +790,7 @@ struct NibItem { // one dense NIBBLE product of a group
     NibView v;
     const char * x; char * y;
     int64_t x_tok, y_tok, row0, nrows;
-    int ncols, chunks, first_block, blocks; // blocks [first_block, first_block + blocks) of the grid serve this item
+    int ncols, chunks, first_block, blocks; // `blocks` blocks from first_block on serve each column
     bool x_bf16, y_bf16;
 };
 struct NibGroup { int n; NibItem item[GROUP_MAX]; };
@@ -750,37 +800,43 @@ __device__ __forceinline__ void nib_item_rows(const NibItem & it, int block, int
     const TX * xg = (const TX *) (it.x + col * it.x_tok);
     const OutVec out = {it.y + col * it.y_tok, it.y_bf16};
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const NibView * w[1] = {&it.v};
     bool waited = false;
     for (int64_t r = (int64_t) block * 8 + warp; r < it.nrows; r += (int64_t) it.blocks * 8) {
-        NibRow<C> d;
-        nib_load<C>(d, it.v, it.row0 + r, lane);
+        NibWords<C> d[1];
+        {
+            NibRow<C> row;
+            nib_load<C>(row, it.v, it.row0 + r, lane);
+            nib_decode<C>(row, d[0]);
+        }
         if (!waited) { grid_dependency_wait(); waited = true; } // weights first, then the activations an earlier kernel may have written
-        const float s = nib_dot<C, TX>(d, it.v, xg, lane);
-        if (lane == 0) { out.put(r, s); }
+        float s[1];
+        nib_dots<C, 1, TX>(d, w, xg, lane, s);
+        if (lane == 0) { out.put(r, s[0]); }
     }
     if (!waited) { grid_dependency_wait(); }
 }
 
 // Every block belongs to one item of the group (a prefix table of block ranges); within its item it is a block of the
-// single-product kernel: same loads, same order of operations, so the results are the same bits.
-__global__ void __launch_bounds__(256) k_nib_gemv_group(const NibGroup g) {
+// single-product kernel: same loads, same order of operations, so the results are the same bits. WIDE adds rows of 4096
+// columns and the registers for them; without, three blocks fit an SM and the 352 blocks of a layer's three products are
+// resident at once (two left a second wave).
+template <bool WIDE>
+__global__ void __launch_bounds__(256, WIDE ? 1 : 3) k_nib_gemv_group(const NibGroup g) {
+    grid_launch_dependents(); // as in k_nib_gemv
     int m = 0;
     while (m + 1 < g.n && (int) blockIdx.x >= g.item[m + 1].first_block) { m++; }
     const NibItem & it = g.item[m];
-    const int local = (int) blockIdx.x - it.first_block;
-    const int col = local / (it.blocks / it.ncols), block = local % (it.blocks / it.ncols);
-    NibItem one = it;
-    one.blocks = it.blocks / it.ncols;
-    const int key = it.chunks * 2 + (it.x_bf16 ? 1 : 0);
-    switch (key) {
-        case 2: nib_item_rows<1, float>(one, block, col); break;
-        case 3: nib_item_rows<1, bf16>(one, block, col); break;
-        case 4: nib_item_rows<2, float>(one, block, col); break;
-        case 5: nib_item_rows<2, bf16>(one, block, col); break;
-        case 8: nib_item_rows<4, float>(one, block, col); break;
-        case 9: nib_item_rows<4, bf16>(one, block, col); break;
-        case 16: nib_item_rows<8, float>(one, block, col); break;
-        case 17: nib_item_rows<8, bf16>(one, block, col); break;
+    const int local = (int) blockIdx.x - it.first_block, col = local / it.blocks, block = local % it.blocks;
+    switch (it.chunks * 2 + (it.x_bf16 ? 1 : 0)) {
+        case 2: nib_item_rows<1, float>(it, block, col); break;
+        case 3: nib_item_rows<1, bf16>(it, block, col); break;
+        case 4: nib_item_rows<2, float>(it, block, col); break;
+        case 5: nib_item_rows<2, bf16>(it, block, col); break;
+        case 8: nib_item_rows<4, float>(it, block, col); break;
+        case 9: nib_item_rows<4, bf16>(it, block, col); break;
+        case 16: if constexpr (WIDE) { nib_item_rows<8, float>(it, block, col); } break;
+        case 17: if constexpr (WIDE) { nib_item_rows<8, bf16>(it, block, col); } break;
         default: grid_dependency_wait(); break;
     }
 }
@@ -799,6 +855,7 @@ void gemv_group(const bf16n_weight * w, const bf16n_mmv_args * a, int n, cudaStr
     while (i < n) {
         NibGroup g = {};
         int blocks = 0;
+        bool wide = false;
         while (i < n && g.n < GROUP_MAX) {
             NibItem & it = g.item[g.n++];
             it.v = nib_view(w[i]);
@@ -808,11 +865,12 @@ void gemv_group(const bf16n_weight * w, const bf16n_mmv_args * a, int n, cudaStr
             it.x_bf16 = a[i].x_bf16 != 0; it.y_bf16 = a[i].y_bf16 != 0;
             const dim3 geo = row_geometry(a[i].nrows, a[i].ncols);
             it.first_block = blocks;
-            it.blocks = (int) geo.x * a[i].ncols;
-            blocks += it.blocks;
+            wide = wide || it.chunks > 4;
+            it.blocks = (int) geo.x;
+            blocks += it.blocks * it.ncols;
             i++;
         }
-        launch_chained(k_nib_gemv_group, dim3((unsigned) blocks), dim3(256), 0, st, g);
+        launch_chained(wide ? k_nib_gemv_group<true> : k_nib_gemv_group<false>, dim3((unsigned) blocks), dim3(256), 0, st, g);
         check_launch();
     }
 }
