@@ -189,8 +189,8 @@ __global__ void __launch_bounds__(256) k_fo_gemv(const PairView w, int C, Cols p
 // a block holds `nb` bands, a warp decodes exactly one unit. The slabs' partial sums meet in shared memory and are added
 // in slab order. A warp here runs nearly alone on its SM and its unit comes cold from HBM; read lane by lane, every
 // lane's stream line would stall the warp for a trip to L2 at a different moment. So the unit's stream block is copied
-// into the warp's shared-memory buffer with one bulk copy and its plane pulled into L2, both started before the table
-// and the activations are staged, and the plane is read four tile pairs ahead. A unit whose streams do not fit the
+// into the warp's shared-memory buffer with one bulk copy and its plane pulled into L2, both started before the
+// activations are staged, and the plane is read four tile pairs ahead. A unit whose streams do not fit the
 // buffer (more than 3 bits per weight) is read from global memory.
 constexpr uint32_t FO_SPLIT_CAP = (BAND * CHUNK * 3 / 8 + 64 + 15) & ~15u;
 constexpr int FO_GROUP = 2;      // routed columns of one expert that share a decode (4: 80 registers, a block fewer per SM: 96 against 81 us per layer when no experts are shared)
@@ -211,10 +211,16 @@ __device__ __forceinline__ float2 load_x2(const bf16 * p) {
     return make_float2(bf16lo_f32(v), bf16hi_f32(v));
 }
 
+// blockIdx.z picks one of two matrices of a shape (gate and up of a decode step): one launch, whose last wave is partly empty
+// once, and no gap between the two.
+struct FoMat { PairView v; const AuxHeader * hdr; int64_t y_shift; }; // y_shift: bytes from the columns' outputs to this matrix's
+
 template <typename TX, bool MMA, int G = 1>
-__global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const PairView w, const AuxHeader * hdr, int C, Cols p, int nb, int ncols, const Opaque k) {
+__global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const FoMat m0, const FoMat m1, int C, Cols p, int nb, int ncols, const Opaque k) {
     static_assert(!MMA || G == 1, "grouping is for the FMA form");
     extern __shared__ __align__(128) unsigned char smem[];
+    const FoMat & mat = blockIdx.z ? m1 : m0;
+    const PairView & w = mat.v;
     uint32_t * lut = (uint32_t *) smem;
     uint64_t * bars = (uint64_t *) (smem + 4 * HP_MAX_PAIRS); // one per warp
     const int64_t K = (int64_t) C * CHUNK;
@@ -230,9 +236,11 @@ __global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const Pair
     if (lane == 0) { mbar_init(bar, 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncwarp();
+    stage_lut(lut, w.lut); // the matrix's own: while the kernel before this one drains
     grid_dependency_wait(); // activations and expert ids may come from the kernel before this one
     const TX * xg; OutVec out; int64_t rbase;
     column<TX>(p, MMA ? 0 : blockIdx.y, xg, out, rbase);
+    out.p += mat.y_shift;
     int members[G];   // the columns this block multiplies ([0]: its own)
     int m = 1;
     members[0] = MMA ? 0 : (int) blockIdx.y;
@@ -270,7 +278,7 @@ __global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const Pair
     const int64_t unit = active ? (rbase / BAND + b) * C + slab : 0;
     uint32_t w0 = 0, my = 0, bytes = 0;
     if (active) {
-        const uint32_t n_units = (uint32_t) hdr->n_a, n_words = (uint32_t) hdr->n_b;
+        const uint32_t n_units = (uint32_t) mat.hdr->n_a, n_words = (uint32_t) mat.hdr->n_b;
         w0 = __ldg(w.ubase + unit);
         const uint32_t w1 = unit + 1 < (int64_t) n_units ? __ldg(w.ubase + unit + 1) : n_words, start = w0 & ~3u;
         bytes = ((w1 - start + 4u + 3u) & ~3u) * 4u;
@@ -283,7 +291,6 @@ __global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const Pair
             bulk_prefetch_l2(w.plane + unit * (BAND * CHUNK), BAND * CHUNK);
         }
     }
-    stage_lut(lut, w.lut);
     if constexpr (MMA) {
         for (int i = threadIdx.x; i < 8 * (int) K; i += blockDim.x) {
             const int n = i / (int) K, c = i - n * (int) K;
@@ -409,6 +416,7 @@ __global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const Pair
                 else {
                     const TX * xm; OutVec om; int64_t rb;
                     column<TX>(p, members[g], xm, om, rb);
+                    om.p += mat.y_shift;
                     om.put(b * BAND + lane, v);
                 }
             }
@@ -861,6 +869,33 @@ void launch_fo(const bf16n_weight & w, const Cols & p, int ncols_grid, cudaStrea
     launch_chained(k_fo_gemv<NC, TX>, grid, dim3(warps * 32), shm, st, pair_view(w), C, p);
 }
 
+FoMat fo_mat(const bf16n_weight & w, int64_t y_shift = 0) { return {pair_view(w), (const AuxHeader *) w.aux, y_shift}; }
+
+// routed columns, and few bands: a band's slabs side by side
+bool fo_split_applies(const bf16n_weight & w, const bf16n_mmv_args & a) {
+    return w.K / CHUNK <= 8 && a.nrows / BAND * a.ncols < (int64_t) device_info().sms * 64;
+}
+
+// one decode per column (two from four tokens on); with `up`, a second matrix of the shape whose outputs go to up_y
+template <typename TX>
+void fo_split(const bf16n_weight & w, const bf16n_weight * up, void * up_y, const bf16n_mmv_args & a, cudaStream_t st) {
+    const Cols p = make_cols(a);
+    const int C = (int) (w.K / CHUNK), nb = std::max(1, 8 / C);
+    const int64_t bands = p.nrows / BAND;
+    const Opaque k = {1u, 4u, ~0u, 32u};
+    const dim3 grid((unsigned) ((bands + nb - 1) / nb), (unsigned) a.ncols, up ? 2 : 1);
+    const FoMat m0 = fo_mat(w), m1 = up ? fo_mat(*up, (char *) up_y - (char *) a.y) : m0;
+    // routed columns of 4..8 whole tokens: columns with the same expert share one decode (same bits per column).
+    // Measured on one MoE layer whose tokens all pick the same 8 experts: 4 tokens 88.5 us grouped against 93.3
+    // per column; 2 tokens 63.1 against 60.7 (half as many blocks, each with twice the multiply work, on a GPU
+    // that two tokens do not fill), so fewer than four tokens go per column, as in the reference.
+    const bool grouped = a.ids && a.n_used > 0 && a.ncols % a.n_used == 0 && a.ncols >= 4 * a.n_used && a.ncols <= 64;
+    const int g = grouped ? FO_GROUP : 1;
+    const size_t shm = 4 * HP_MAX_PAIRS + 128 + (size_t) w.K * 4 + (size_t) nb * C * 16 * g * 4 + (size_t) nb * C * FO_SPLIT_CAP;
+    launch_chained(grouped ? k_fo_gemv_split<TX, false, FO_GROUP> : k_fo_gemv_split<TX, false>, grid, dim3(nb * C * 32), shm, st, m0, m1, C, p, nb,
+                   grouped ? a.ncols : 1, k);
+}
+
 template <typename TX>
 void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st) {
     Cols p = make_cols(a);
@@ -869,25 +904,8 @@ void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st
     // the split kernels (16384 x 2048: 34.6 against 22.4 us at one token, 35.9 against 35.6 at eight).
     constexpr int64_t big_per_sm = 16;
     if (a.ids || (a.ncols == 1 && (p.nrows / BAND < (int64_t) device_info().sms * big_per_sm || !a.x_bf16))) {
-        const int C = (int) (w.K / CHUNK);
-        const int64_t bands = p.nrows / BAND;
-        if (C <= 8 && bands * a.ncols < (int64_t) device_info().sms * 64) { // few bands: a band's slabs side by side
-            const int nb = std::max(1, 8 / C);
-            const Opaque k = {1u, 4u, ~0u, 32u};
-            const dim3 grid((unsigned) ((bands + nb - 1) / nb), (unsigned) a.ncols);
-            // routed columns of 4..8 whole tokens: columns with the same expert share one decode (same bits per column).
-            // Measured on one MoE layer whose tokens all pick the same 8 experts: 4 tokens 88.5 us grouped against 93.3
-            // per column; 2 tokens 63.1 against 60.7 (half as many blocks, each with twice the multiply work, on a GPU
-            // that two tokens do not fill), so fewer than four tokens go per column, as in the reference.
-            const bool grouped = a.ids && a.n_used > 0 && a.ncols % a.n_used == 0 && a.ncols >= 4 * a.n_used && a.ncols <= 64;
-            const int g = grouped ? FO_GROUP : 1;
-            const size_t shm = 4 * HP_MAX_PAIRS + 128 + (size_t) w.K * 4 + (size_t) nb * C * 16 * g * 4 + (size_t) nb * C * FO_SPLIT_CAP;
-            if (grouped) {
-                launch_chained(k_fo_gemv_split<TX, false, FO_GROUP>, grid, dim3(nb * C * 32), shm, st, pair_view(w), (const AuxHeader *) w.aux, C, p,
-                               nb, a.ncols, k);
-            } else {
-                launch_chained(k_fo_gemv_split<TX, false>, grid, dim3(nb * C * 32), shm, st, pair_view(w), (const AuxHeader *) w.aux, C, p, nb, 1, k);
-            }
+        if (fo_split_applies(w, a)) {
+            fo_split<TX>(w, nullptr, nullptr, a, st);
         } else {
             launch_fo<1, TX>(w, p, a.ids ? a.ncols : 1, st);
         }
@@ -928,7 +946,7 @@ void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st
                                        (size_t) nb * C * FO_SPLIT_CAP;
                     const Opaque k = {1u, 4u, ~0u, 32u};
                     launch_chained(k_fo_gemv_split<bf16, true>, dim3((unsigned) ((bands + nb - 1) / nb)), dim3(nb * C * 32), shm, st,
-                                   pair_view(w), (const AuxHeader *) w.aux, C, q, nb, nc, k);
+                                   fo_mat(w), fo_mat(w), C, q, nb, nc, k);
                 }
             } else {
                 const int warps = bands >= sms * 32 ? 8 : bands >= sms * 8 ? 4 : 2;
@@ -1034,6 +1052,17 @@ void fo_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_b
 
 void fo_gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st) {
     if (a.x_bf16) { fo_gemv_t<bf16>(w, a, st); } else { fo_gemv_t<float>(w, a, st); }
+}
+
+void fo_gemv_two(const bf16n_weight & w, const bf16n_weight & up, const bf16n_mmv_args & a, void * up_y, cudaStream_t st) {
+    if (fo_split_applies(w, a)) {
+        if (a.x_bf16) { fo_split<bf16>(w, &up, up_y, a, st); } else { fo_split<float>(w, &up, up_y, a, st); }
+        return;
+    }
+    bf16n_mmv_args u = a;
+    u.y = up_y;
+    fo_gemv(w, a, st);
+    fo_gemv(up, u, st);
 }
 
 void fo_expand_store(const bf16n_weight & w, int64_t row0, int64_t nrows, uint16_t * out, cudaStream_t st) {

@@ -99,6 +99,7 @@ void gemv_rings(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t s
 void fo_init();
 bool fo_supported(const bf16n_weight & w);
 void fo_gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st);
+void fo_gemv_two(const bf16n_weight & w, const bf16n_weight & up, const bf16n_mmv_args & a, void * up_y, cudaStream_t st); // routed columns
 bool fo_mm_ids_supported(const bf16n_weight & w, const bf16n_weight * up);
 void fo_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
                const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,

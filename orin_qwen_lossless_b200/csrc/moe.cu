@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(32) k_topk(const float * __restrict__ logits, 
 
 __global__ void k_swiglu(const float * __restrict__ g, const float * __restrict__ u, float * __restrict__ y, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x) {
-        y[i] = silu_f(g[i]) * u[i];
+        y[i] = silu_f(ld_act_f32(g + i)) * ld_act_f32(u + i);
     }
 }
 
@@ -192,7 +192,7 @@ void moe_combine(const float * ys, const void * w, bool w_bf16, void * y, bool y
 void moe_swiglu(const float * g, const float * u, float * y, int64_t n, cudaStream_t st) {
     if (n == 0) { return; }
     const unsigned blocks = (unsigned) std::min<int64_t>((n + 255) / 256, (int64_t) device_info().sms * 8);
-    k_swiglu<<<blocks, 256, 0, st>>>(g, u, y, n);
+    launch_chained(k_swiglu, dim3(blocks), dim3(256), 0, st, g, u, y, n);
     check_launch();
 }
 

@@ -345,7 +345,7 @@ void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_
 }
 
 // The same step over fragment-order experts (the layout the vLLM policy gives expert stacks): routed products through the
-// fragment-order GEMV (one decode per (token, slot) column, a band's slabs on separate warps), SwiGLU in place, the
+// fragment-order GEMV (one decode per (token, slot) column, a band's slabs on separate warps; gate and up in one launch), SwiGLU in place, the
 // slot-order combine. All experts on this GPU (no expert slice). Same scratch layout as moe_decode.
 void moe_decode_frag_order(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_weight & down, const void * x, bool x_bf16,
                            int64_t x_tok, const int32_t * ids, const float * weights, int n_tok, int n_used, int n_experts,
@@ -359,8 +359,8 @@ void moe_decode_frag_order(const bf16n_weight & gate, const bf16n_weight & up, c
     a.ids = ids; a.ids_s0 = 4; a.ids_s1 = 4ll * n_used;
     a.rows_per_matrix = N; a.row0 = 0; a.nrows = N;
     a.y_tok = 4ll * n_used * N; a.y_slot = 4ll * N;
-    a.y = g; fo_gemv(gate, a, st);
-    a.y = u; fo_gemv(up, a, st);
+    a.y = g;
+    fo_gemv_two(gate, up, a, u, st);
     moe_swiglu(g, u, g, (int64_t) ncols * N, st);            // g := silu(g) * u
     bf16n_mmv_args d = a;
     d.x = g; d.x_bf16 = 0; d.x_per_slot = n_used; d.x_tok = 4ll * n_used * N; d.x_slot = 4ll * N;
