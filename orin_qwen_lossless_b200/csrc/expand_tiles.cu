@@ -54,6 +54,7 @@ __global__ void __launch_bounds__(EXPAND_WARPS * 32, 1) k_expand_tiles(const Exp
     const PairView w = blockIdx.y ? p.w[1] : p.w[0];
     const int row_offset = blockIdx.y ? IMG_ROWS / 2 : 0;
     for (int i = threadIdx.x; i < HP_MAX_PAIRS; i += blockDim.x) { const uint32_t e = __ldg(w.lut + i); ((uint4 *) lut)[i] = make_uint4(e, e, e, e); }
+    grid_dependency_wait(); // the routing is an earlier kernel's, and the images may still be read by one
     __syncthreads();
 
     const uint32_t piece = (uint32_t) (lane & 15) >> 1;
@@ -153,6 +154,7 @@ __global__ void __launch_bounds__(FO_EXPAND_WARPS * 32, 1) k_expand_tiles_fo(con
     const PairView w = blockIdx.y ? p.w[1] : p.w[0];
     const int row_offset = blockIdx.y ? IMG_ROWS / 2 : 0;
     for (int i = threadIdx.x; i < HP_MAX_PAIRS; i += blockDim.x) { const uint32_t e = __ldg(w.lut + i); ((uint4 *) lut)[i] = make_uint4(e, e, e, e); }
+    grid_dependency_wait(); // the routing is an earlier kernel's, and the images may still be read by one
     __syncthreads();
 
     const int KT = p.C * 8;
@@ -253,8 +255,7 @@ void expand_tiles(const bf16n_weight & w, const bf16n_weight * up, int n_experts
     const unsigned gx = (unsigned) std::min<int64_t>(std::max(1, device_info().sms / n_mats), (a.units + EXPAND_WARPS - 1) / EXPAND_WARPS);
     const dim3 grid(gx, (unsigned) n_mats);
     const Opaque k = {1u, 4u, ~0u, 32u, 16u};
-    if (w.K == 4 * CHUNK) { k_expand_tiles<4, 8, true><<<grid, EXPAND_WARPS * 32, EXPAND_SMEM, st>>>(a, k); }
-    else { k_expand_tiles<1, 16, false><<<grid, EXPAND_WARPS * 32, EXPAND_SMEM, st>>>(a, k); }
+    launch_chained(w.K == 4 * CHUNK ? k_expand_tiles<4, 8, true> : k_expand_tiles<1, 16, false>, grid, dim3(EXPAND_WARPS * 32), EXPAND_SMEM, st, a, k);
     check_launch();
 }
 
@@ -276,9 +277,19 @@ void expand_tiles_fo(const bf16n_weight & w, const bf16n_weight * up, int n_expe
     a.bands_per_block = rows_per_block / FO_BAND;
     a.blocks_per_expert = (int) (rows_per_expert / rows_per_block);
     const int n_mats = up ? 2 : 1;
-    const unsigned gx = (unsigned) std::min<int64_t>(std::max(1, device_info().sms / n_mats), (a.units + FO_EXPAND_WARPS - 1) / FO_EXPAND_WARPS);
+    // units are dealt round robin: of the last few warp counts, the one that leaves the last round fullest (256 experts of 512 x
+    // 2048: 17.03 rounds of 26 warps, 17.7 of 25)
+    const int64_t blocks = std::max(1, device_info().sms / n_mats);
+    int warps = FO_EXPAND_WARPS;
+    double best = 0.0;
+    for (int nw = FO_EXPAND_WARPS; nw >= FO_EXPAND_WARPS - 4; nw--) {
+        const int64_t slots = blocks * nw, rounds = (a.units + slots - 1) / slots;
+        const double full = (double) a.units / (double) (rounds * slots) * (1.0 - 0.005 * (FO_EXPAND_WARPS - nw));
+        if (full > best + 1e-9) { best = full; warps = nw; }
+    }
+    const dim3 grid((unsigned) std::min<int64_t>(blocks, (a.units + warps - 1) / warps), (unsigned) n_mats);
     const Opaque k = {1u, 4u, ~0u, 32u, 16u};
-    k_expand_tiles_fo<<<dim3(gx, (unsigned) n_mats), FO_EXPAND_WARPS * 32, FO_EXPAND_SMEM, st>>>(a, k);
+    launch_chained(k_expand_tiles_fo, grid, dim3(warps * 32), LUT_BYTES + (size_t) warps * (32 * RING_BYTES + FO_STAGE), st, a, k);
     check_launch();
 }
 

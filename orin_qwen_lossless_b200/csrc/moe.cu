@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(32) k_topk(const float * __restrict__ logits, 
 // ---------------------------------------------------------------- elementwise
 
 __global__ void k_swiglu(const float * __restrict__ g, const float * __restrict__ u, float * __restrict__ y, int64_t n) {
+    grid_dependency_wait();
     for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x) {
         y[i] = silu_f(ld_act_f32(g + i)) * ld_act_f32(u + i);
     }
@@ -84,17 +85,53 @@ __global__ void k_combine(const float * __restrict__ ys, const char * __restrict
     }
 }
 
+// The same for rows of whole 16-byte groups, four columns to a thread, the slots' loads in flight together. HBM bound: FP32
+// rows of every slot are read once.
+template <int S>
+__device__ __forceinline__ void combine4(const float * ys, const float * wk, int64_t n, float4 & acc) {
+    float4 v[S];
+#pragma unroll
+    for (int k = 0; k < S; k++) { v[k] = __ldcs((const float4 *) (ys + k * n)); }
+#pragma unroll
+    for (int k = 0; k < S; k++) {
+        acc.x = fmaf(wk[k], v[k].x, acc.x); acc.y = fmaf(wk[k], v[k].y, acc.y);
+        acc.z = fmaf(wk[k], v[k].z, acc.z); acc.w = fmaf(wk[k], v[k].w, acc.w);
+    }
+}
+__global__ void __launch_bounds__(256) k_combine4(const float * __restrict__ ys, const char * __restrict__ w, bool w_bf16, char * __restrict__ y, bool y_bf16,
+                                                  int n_used, int64_t n) {
+    __shared__ float ws[1024];
+    const int t = blockIdx.y;
+    for (int k = threadIdx.x; k < n_used; k += 256) {
+        const int64_t s = (int64_t) t * n_used + k;
+        ws[k] = w_bf16 ? to_f32(((const __nv_bfloat16 *) w)[s]) : ((const float *) w)[s];
+    }
+    __syncthreads();
+    for (int64_t i = (blockIdx.x * 256ll + threadIdx.x) * 4; i < n; i += gridDim.x * 1024ll) {
+        const float * p = ys + (int64_t) t * n_used * n + i;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        int k = 0;
+        for (; k + 8 <= n_used; k += 8) { combine4<8>(p + k * n, ws + k, n, acc); }
+        for (; k < n_used; k++) { combine4<1>(p + k * n, ws + k, n, acc); }
+        if (y_bf16) {
+            const __nv_bfloat162 a = __floats2bfloat162_rn(acc.x, acc.y), b = __floats2bfloat162_rn(acc.z, acc.w);
+            ((uint2 *) y)[(t * n + i) / 4] = make_uint2(*(const uint32_t *) &a, *(const uint32_t *) &b);
+        } else { ((float4 *) y)[(t * n + i) / 4] = acc; }
+    }
+}
+
 // ---------------------------------------------------------------- routing sort (prefill)
 
 // One block per expert. Pass 1 counts the routed pairs of lower-numbered experts (this expert's first output index);
-// pass 2 walks the tokens in order, 256 at a time, and compacts the tokens that use this expert with a block-wide
+// pass 2 walks the tokens in order, 1024 at a time (latency bound: a step is two block barriers and a trip to L2), and compacts the tokens that use this expert with a block-wide
 // exclusive scan, so the expert's pairs come out sorted by token.
+constexpr int ROUTE_THREADS = 1024, ROUTE_WARPS = ROUTE_THREADS / 32;
 template <typename TI>
-__global__ void __launch_bounds__(256) k_route(const TI * __restrict__ ids, int64_t row_stride, int32_t * __restrict__ ids_src1,
+__global__ void __launch_bounds__(ROUTE_THREADS) k_route(const TI * __restrict__ ids, int64_t row_stride, int32_t * __restrict__ ids_src1,
                                                int32_t * __restrict__ ids_dst, int32_t * __restrict__ bounds, int n_tok, int n_used,
                                                int nchannels_y, int sis1) {
     const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    __shared__ int warp_tot[8];
+    __shared__ int warp_tot[ROUTE_WARPS];
     __shared__ int s_base;
 
     // int32 ids in contiguous rows of a multiple of four: four ids per load (the common case: 8 slots per token)
@@ -102,12 +139,12 @@ __global__ void __launch_bounds__(256) k_route(const TI * __restrict__ ids, int6
     int lower = 0;
     if (vec) {
         const int4 * v = (const int4 *) ids;
-        for (int64_t i = tid; i < (int64_t) n_tok * n_used / 4; i += 256) {
+        for (int64_t i = tid; i < (int64_t) n_tok * n_used / 4; i += ROUTE_THREADS) {
             const int4 q = __ldg(v + i);
             lower += (q.x < e) + (q.y < e) + (q.z < e) + (q.w < e);
         }
     } else {
-        for (int64_t i = tid; i < (int64_t) n_tok * n_used; i += 256) {
+        for (int64_t i = tid; i < (int64_t) n_tok * n_used; i += ROUTE_THREADS) {
             const int t = (int) (i / n_used), s = (int) (i - (int64_t) t * n_used);
             lower += (int) ids[t * row_stride + s] < e;
         }
@@ -118,13 +155,13 @@ __global__ void __launch_bounds__(256) k_route(const TI * __restrict__ ids, int6
     __syncthreads();
     if (tid == 0) {
         int b = 0;
-        for (int i = 0; i < 8; i++) { b += warp_tot[i]; }
+        for (int i = 0; i < ROUTE_WARPS; i++) { b += warp_tot[i]; }
         s_base = b;
     }
     __syncthreads();
     const int base = s_base;
     int done = 0;
-    for (int t0 = 0; t0 < n_tok; t0 += 256) {
+    for (int t0 = 0; t0 < n_tok; t0 += ROUTE_THREADS) {
         const int t = t0 + tid;
         int slot = -1;
         if (t < n_tok) {
@@ -148,7 +185,7 @@ __global__ void __launch_bounds__(256) k_route(const TI * __restrict__ ids, int6
         if (lane == 0) { warp_tot[warp] = __popc(hit); }
         __syncthreads();
         int before = 0, total = 0;
-        for (int i = 0; i < 8; i++) {
+        for (int i = 0; i < ROUTE_WARPS; i++) {
             before += i < warp ? warp_tot[i] : 0;
             total += warp_tot[i];
         }
@@ -184,6 +221,12 @@ void moe_combine(const float * ys, const void * w, bool w_bf16, void * y, bool y
                  cudaStream_t st) {
     if (n_tok == 0 || n == 0) { return; }
     require(n_tok <= 65535, "moe_combine: too many tokens for one launch");
+    if (n % 4 == 0 && n_used <= 1024 && ((uintptr_t) ys | (uintptr_t) y) % 16 == 0) {
+        const dim3 grid4((unsigned) std::min<int64_t>((n + 1023) / 1024, 64), (unsigned) n_tok);
+        k_combine4<<<grid4, 256, 0, st>>>(ys, (const char *) w, w_bf16, (char *) y, y_bf16, n_used, n);
+        check_launch();
+        return;
+    }
     const dim3 grid((unsigned) std::min<int64_t>((n + 255) / 256, 64), (unsigned) n_tok);
     k_combine<<<grid, 256, 0, st>>>(ys, (const char *) w, w_bf16, (char *) y, y_bf16, n_used, n);
     check_launch();
@@ -202,10 +245,10 @@ void moe_route(const void * ids, bool ids_i64, int64_t ids_row_stride, int32_t *
     require(n_experts > 0, "routing needs at least one expert");
     require((int64_t) n_tok * ids_row_stride < INT32_MAX, "routing ids too large for 32-bit indexing");
     if (ids_i64) {
-        k_route<int64_t><<<n_experts, 256, 0, st>>>((const int64_t *) ids, ids_row_stride, ids_src1, ids_dst, bounds, n_tok, n_used,
+        k_route<int64_t><<<n_experts, ROUTE_THREADS, 0, st>>>((const int64_t *) ids, ids_row_stride, ids_src1, ids_dst, bounds, n_tok, n_used,
                                                     nchannels_y, sis1);
     } else {
-        k_route<int32_t><<<n_experts, 256, 0, st>>>((const int32_t *) ids, ids_row_stride, ids_src1, ids_dst, bounds, n_tok, n_used,
+        k_route<int32_t><<<n_experts, ROUTE_THREADS, 0, st>>>((const int32_t *) ids, ids_row_stride, ids_src1, ids_dst, bounds, n_tok, n_used,
                                                     nchannels_y, sis1);
     }
     check_launch();

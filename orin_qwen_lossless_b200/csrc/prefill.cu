@@ -436,8 +436,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_prefill(const PrefillArgs p) {
 //     them; tcgen05.commit hands activation slots and weight stages back and announces the finished accumulators;
 //   * warp 9, one thread: one 32 KB bulk copy per k-tile of the item's image into a ring of four weight stages
 //     (mbarrier expect_tx / complete_tx).
-// A work item is (expert, row block of 256 image rows); a pass covers up to TM_G x 128 of the expert's tokens, whose
-// accumulators (TM_G x 256 columns) fill tensor memory. The activations of a pass cross L2 -> shared memory once per
+// A pass is (expert, row block of 256 image rows, up to TM_G x 128 of the expert's tokens), whose
+// accumulators (TM_G x 256 columns) fill tensor memory. Passes are dealt round robin over the blocks, all first passes
+// before all second ones and so on (TileWalk): the first passes of a large batch are full and the last ones may hold a
+// few tokens, and dealt by row block one SM would get every short pass and another none. The activations of a pass cross L2 -> shared memory once per
 // 256 weight rows, and a weight k-tile is copied once per pass.
 constexpr int TM_N = 256, TM_G = 2, TM_WST = 4, TM_XSL = 6;
 constexpr int TM_GATHERERS = 256, TM_THREADS = 320, TM_MMA_WARP = 8, TM_W_WARP = 9;
@@ -446,6 +448,11 @@ constexpr int TM_STAGE_ROW = 256 + 16;       // epilogue staging: 256 output byt
 static_assert(TM_GATHERERS * TM_STAGE_ROW <= TM_XSL * X_SLOT_BYTES, "the epilogue stages its output rows in the activation ring");
 __host__ __device__ constexpr uint32_t tm_instr_desc() { return 1u << 4 | 1u << 7 | 1u << 10 | (uint32_t) (TM_N >> 3) << 17 | (uint32_t) (M_TOK >> 4) << 24; }
 static_assert(TM_G * TM_N <= TMEM_COLS, "accumulators of a pass must fit TMEM");
+
+// Which experts have more than l passes' worth of tokens, as bit masks, and their number, for l < TM_LEVELS (the last level
+// holds all the passes that are left of an expert). Lists experts without tokens nowhere, so no block draws an empty item.
+constexpr int TM_LEVELS = 8, TM_MASK_WORDS = 32, TM_MAX_EXPERTS = 32 * TM_MASK_WORDS;
+struct TileLevels { uint32_t mask[TM_LEVELS][TM_MASK_WORDS]; int count[TM_LEVELS]; };
 
 struct TileMmArgs {
     const unsigned char * images;       // [expert][row block][k-tile][256][128 bytes]
@@ -472,6 +479,38 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void tm_helper_bar() { asm volatile("bar.sync 1, %0;" ::"n"(TM_GATHERERS) : "memory"); }
 
+// the passes of this block, in the order that every role of it walks
+struct TileWalk {
+    const TileLevels & lv;
+    const int32_t * bounds;
+    int bpe, at, level;
+    int e, nb, jp, j1; // the pass: tokens [jp, min(jp + TM_G * M_TOK, j1)) of expert e, row block nb
+
+    __device__ __forceinline__ TileWalk(const TileLevels & l, const TileMmArgs & p) : lv(l), bounds(p.bounds), bpe(p.blocks_per_expert), at((int) blockIdx.x), level(0), e(0), nb(0), jp(0), j1(0) {}
+    __device__ __forceinline__ bool next() {
+        if (jp + TM_G * M_TOK < j1) { jp += TM_G * M_TOK; return true; } // the last level: the expert's remaining passes
+        for (; level < TM_LEVELS; level++) {
+            const int n = lv.count[level] * bpe;
+            if (at < n) { break; }
+            at -= n;
+        }
+        if (level == TM_LEVELS) { return false; }
+        int r = at / bpe;
+        nb = at - r * bpe;
+        const uint32_t * m = lv.mask[level];
+        int word = 0;
+        for (int c; r >= (c = __popc(m[word])); word++) { r -= c; }
+        uint32_t bits = m[word];
+        for (; r; r--) { bits &= bits - 1; }
+        e = 32 * word + __ffs(bits) - 1;
+        jp = __ldg(bounds + e) + level * TM_G * M_TOK;
+        j1 = __ldg(bounds + e + 1);
+        if (level + 1 < TM_LEVELS) { j1 = min(j1, jp + TM_G * M_TOK); }
+        at += gridDim.x;
+        return true;
+    }
+};
+
 template <bool GLU>
 __global__ void __launch_bounds__(TM_THREADS, 1) k_tile_mm(const TileMmArgs p) {
     extern __shared__ unsigned char smem_raw[];
@@ -483,8 +522,21 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_tile_mm(const TileMmArgs p) {
     uint64_t * acc_done = x_free + TM_XSL, * drained = acc_done + 1, * fin = drained + 1;
     uint32_t * tmem_slot = (uint32_t *) (fin + 1);
     volatile int * failed = (volatile int *) (tmem_slot + 1);
+    TileLevels & levels = *(TileLevels *) (smem + TM_WST * TM_W_STAGE + TM_XSL * X_SLOT_BYTES + 256);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    grid_dependency_wait(); // images, routing and activations all come from earlier launches
+    if (tid < TM_LEVELS) { levels.count[tid] = 0; }
+    __syncthreads();
+    for (int i = warp; i < TM_LEVELS * TM_MASK_WORDS; i += TM_THREADS / 32) {
+        const int l = i / TM_MASK_WORDS, word = i - l * TM_MASK_WORDS, e = 32 * word + lane;
+        const bool in = e < p.n_experts && __ldg(p.bounds + e + 1) - __ldg(p.bounds + e) > l * TM_G * M_TOK;
+        const uint32_t m = __ballot_sync(FULL, in);
+        if (lane == 0) {
+            levels.mask[l][word] = m;
+            if (m) { atomicAdd(&levels.count[l], __popc(m)); }
+        }
+    }
     if (tid == 0) {
         for (int i = 0; i < TM_WST; i++) { mbar_init(smem_u32(w_full + i), 1); mbar_init(smem_u32(w_empty + i), 1); }
         for (int i = 0; i < TM_XSL; i++) { mbar_init(smem_u32(x_full + i), TM_GATHERERS); mbar_init(smem_u32(x_free + i), 1); }
@@ -499,7 +551,8 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_tile_mm(const TileMmArgs p) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const int n_items = p.n_experts * p.blocks_per_expert, KT = p.ktiles;
+    const int KT = p.ktiles;
+    TileWalk walk(levels, p);
 
     if (warp == TM_W_WARP) {
         // ------------------------------------------------------------------ weight stages: one bulk copy per k-tile
@@ -507,19 +560,15 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_tile_mm(const TileMmArgs p) {
             uint32_t n = 0, issued = 0; // stages of the walk, copies actually started (equal until a wait fails)
             // (Asking each k-tile into L2 eight k-tiles before its bulk copy was measured and lost: 988 / 1631 us per layer
             // at 2048 / 8192 tokens against 952 / 1567 without.)
-            for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-                const int e = item / p.blocks_per_expert;
-                const int j0 = p.bounds[e], j1 = p.bounds[e + 1];
-                const unsigned char * img = p.images + (int64_t) item * KT * TM_W_STAGE;
-                for (int jp = j0; jp < j1; jp += TM_G * M_TOK) {
-                    for (int kt = 0; kt < KT; kt++, n++) {
-                        const uint32_t s = n % TM_WST, use = n / TM_WST;
-                        if (use >= 1) { wait_on(w_empty + s, (use - 1) & 1, failed); }
-                        if (*failed) { continue; }
-                        mbar_expect_tx(smem_u32(w_full + s), TM_W_STAGE);
-                        bulk_g2s(smem_u32(wbuf + s * TM_W_STAGE), img + (int64_t) kt * TM_W_STAGE, TM_W_STAGE, smem_u32(w_full + s));
-                        issued++;
-                    }
+            while (walk.next()) {
+                const unsigned char * img = p.images + ((int64_t) walk.e * p.blocks_per_expert + walk.nb) * KT * TM_W_STAGE;
+                for (int kt = 0; kt < KT; kt++, n++) {
+                    const uint32_t s = n % TM_WST, use = n / TM_WST;
+                    if (use >= 1) { wait_on(w_empty + s, (use - 1) & 1, failed); }
+                    if (*failed) { continue; }
+                    mbar_expect_tx(smem_u32(w_full + s), TM_W_STAGE);
+                    bulk_g2s(smem_u32(wbuf + s * TM_W_STAGE), img + (int64_t) kt * TM_W_STAGE, TM_W_STAGE, smem_u32(w_full + s));
+                    issued++;
                 }
             }
             if (*failed) { // copies may still be in flight: wait (bounded) for every stage's last one before the block ends
@@ -537,11 +586,10 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_tile_mm(const TileMmArgs p) {
         uint32_t n = 0;        // weight stages consumed
         uint32_t vv = 0;       // activation slots used
         uint32_t passes = 0;
-        for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-            const int e = item / p.blocks_per_expert, nb = item - e * p.blocks_per_expert;
-            const int j0 = p.bounds[e], j1 = p.bounds[e + 1];
-            for (int jp = j0; jp < j1; jp += TM_G * M_TOK) {
-                const int ntok = min(TM_G * M_TOK, j1 - jp), ng = (ntok + M_TOK - 1) / M_TOK;
+        {
+            while (walk.next()) {
+                const int nb = walk.nb, jp = walk.jp;
+                const int ntok = min(TM_G * M_TOK, walk.j1 - jp), ng = (ntok + M_TOK - 1) / M_TOK;
                 const int total = KT * ng;   // slots of the pass: for each k-tile, each token group
                 if (!mma_warp) {
                     int64_t my_dst[TM_G];    // output row of the token whose accumulators this thread reads
@@ -711,7 +759,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_tile_mm(const TileMmArgs p) {
     if (warp == 0) { tmem_free(tmem, TMEM_COLS); }
 }
 
-constexpr size_t TM_SMEM = (size_t) TM_WST * TM_W_STAGE + (size_t) TM_XSL * X_SLOT_BYTES + 256 + 1024;
+constexpr size_t TM_SMEM = (size_t) TM_WST * TM_W_STAGE + (size_t) TM_XSL * X_SLOT_BYTES + 256 + sizeof(TileLevels) + 1024;
 
 PairView view_of(const bf16n_weight & w) {
     return {w.plane, (const uint32_t *) (w.aux + w.off_a), (const uint32_t *) (w.aux + w.off_b),
@@ -784,8 +832,7 @@ void tile_mm(const void * images, const PrefillArgs & a, const int32_t * bounds,
     t.blocks_per_expert = (int) (a.rows_per_expert / rows_per_block);
     t.ktiles = (int) (K / 64);
     const unsigned grid = (unsigned) std::min<int64_t>(device_info().sms, (int64_t) n_experts * t.blocks_per_expert);
-    if (glu) { k_tile_mm<true><<<grid, TM_THREADS, TM_SMEM, st>>>(t); }
-    else { k_tile_mm<false><<<grid, TM_THREADS, TM_SMEM, st>>>(t); }
+    launch_chained(glu ? k_tile_mm<true> : k_tile_mm<false>, dim3(grid), dim3(TM_THREADS), TM_SMEM, st, t);
     check_launch();
 }
 
@@ -793,7 +840,7 @@ void tile_mm(const void * images, const PrefillArgs & a, const int32_t * bounds,
 bool two_pass(const bf16n_weight & w, const bf16n_weight * up, const PrefillArgs & a, int n_experts, cudaStream_t st) {
     const size_t need = prefill_workspace_bytes(w, up);
     const int rows_per_block = up ? TM_N / 2 : TM_N;
-    if (need == 0 || need > g_workspace_bytes || a.rows_per_expert % rows_per_block || ((uintptr_t) g_workspace % 1024)) { return false; }
+    if (need == 0 || need > g_workspace_bytes || a.rows_per_expert % rows_per_block || n_experts > TM_MAX_EXPERTS || ((uintptr_t) g_workspace % 1024)) { return false; }
     expand_tiles(w, up, n_experts, a.bounds, g_workspace, st);
     tile_mm(g_workspace, a, a.bounds, n_experts, w.K, up != nullptr, st);
     return true;
@@ -823,7 +870,7 @@ bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const 
                          void * scratch, size_t scratch_bytes, cudaStream_t st) {
     const size_t per_expert = (size_t) (w.rows / n_experts) * (size_t) w.K * 2 * (up ? 2 : 1);
     const int64_t rows_per_block = up ? TM_N / 2 : TM_N;
-    if (!scratch || (w.rows / n_experts) % rows_per_block || ((uintptr_t) scratch % 1024) || scratch_bytes < per_expert) { return false; }
+    if (!scratch || (w.rows / n_experts) % rows_per_block || n_experts > TM_MAX_EXPERTS || ((uintptr_t) scratch % 1024) || scratch_bytes < per_expert) { return false; }
     const PrefillArgs a = batch_args(w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16, dst_col, n_experts);
     const int fit = (int) std::min<size_t>((size_t) n_experts, scratch_bytes / per_expert);
     const int ranges = (n_experts + fit - 1) / fit, step = (n_experts + ranges - 1) / ranges; // ranges of equal size
