@@ -65,6 +65,9 @@ typedef struct bf16n_encoded bf16n_encoded;
  * Replaces bf16n::encode (encode.h:26, core/src/encode.cpp:443-526): same argument rules, same bytes. */
 int bf16n_encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order,
                  bf16n_encoded ** out);
+/* The same with the rows * K plane bytes written to the caller's buffer (null: kept in the result, as above). */
+int bf16n_encode_into(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order, uint8_t * plane,
+                      bf16n_encoded ** out);
 const uint8_t * bf16n_encoded_plane(const bf16n_encoded * e, size_t * nbytes);
 const uint8_t * bf16n_encoded_aux(const bf16n_encoded * e, size_t * nbytes);
 int bf16n_encoded_format(const bf16n_encoded * e);

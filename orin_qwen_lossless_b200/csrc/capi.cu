@@ -120,11 +120,16 @@ const char * bf16n_last_error(void) { return g_error.c_str(); }
 
 int bf16n_encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order,
                  bf16n_encoded ** out) {
+    return bf16n_encode_into(w, rows, K, format, R, chunk_major, frag_order, nullptr, out);
+}
+
+int bf16n_encode_into(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order, uint8_t * plane,
+                      bf16n_encoded ** out) {
     return guarded([&] {
         require(w != nullptr && out != nullptr, "encode: null argument");
         auto * r = new bf16n_encoded;
         try {
-            r->e = encode(w, rows, K, format, R, chunk_major != 0, frag_order != 0);
+            r->e = encode(w, rows, K, format, R, chunk_major != 0, frag_order != 0, plane);
         } catch (...) {
             delete r;
             throw;

@@ -19,6 +19,8 @@
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 namespace b16 {
 namespace {
 
@@ -159,12 +161,25 @@ __global__ void __launch_bounds__(256) k_int4_gemv(const bf16 * __restrict__ x, 
     }
 }
 
+// Two 2-bit fields moved to bits 8 and 9 of their halves, under the exponent of 4.0: (4 + a, 4 + b). Moving a field up is a
+// multiply (the pipe that the shifts, masks and merges leave idle), so the constants come in opaque.
+struct FieldShift { uint32_t up[4]; }; // 2^8, 2^6, 2^4, 2^2
+__device__ __forceinline__ __half2 field_half2(uint32_t moved) {
+    uint32_t p;
+    asm("lop3.b32 %0, %1, 0x03000300, 0x44004400, 0xEA;" : "=r"(p) : "r"(moved)); // (a & b) | c
+    return *(const __half2 *) &p;
+}
+template <int J> __device__ __forceinline__ __half2 field(uint32_t word, const FieldShift & k) { // field J of both halves
+    if constexpr (J < 4) { return field_half2(word * k.up[J]); }
+    else { return field_half2(word >> (2 * J - 8)); }
+}
+
 // 2 bit, K = 2048: a lane owns 16 contiguous bytes = 64 weights (half a scale group); a half2 pairs the fields at bits
 // 2 j and 2 j + 16 of a word (columns 16 wd + j and 16 wd + j + 8). sum_k (n_k - 1.5) x_k = sum_k n_k x_k - 1.5 sum_k x_k:
 // the second sum is a per-lane constant of the column. A row is only 512 bytes, so a warp keeps AHEAD rows in flight.
 template <int NC>
 __global__ void __launch_bounds__(256, NC == 1 ? 2 : 1) k_int2_gemv(const bf16 * __restrict__ x, const uint8_t * __restrict__ q,
-                                                                      const float * __restrict__ s, int64_t rows, float * __restrict__ y) {
+                                                                      const float * __restrict__ s, int64_t rows, float * __restrict__ y, const FieldShift k) {
     constexpr int K = 2048, AHEAD = 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     grid_launch_dependents();
@@ -202,7 +217,7 @@ __global__ void __launch_bounds__(256, NC == 1 ? 2 : 1) k_int2_gemv(const bf16 *
         }
         xsum[c] = sum;
     }
-    const __half2 bias = __float2half2_rn(1024.f);
+    const __half2 bias = __float2half2_rn(4.f);
     for (; r < rows; r += AHEAD * stride) {
 #pragma unroll
         for (int i = 0; i < AHEAD; i++) {
@@ -219,16 +234,17 @@ __global__ void __launch_bounds__(256, NC == 1 ? 2 : 1) k_int2_gemv(const bf16 *
                 __half2 h0[NC], h1[NC]; // two chains of four products: half the dependent latency
 #pragma unroll
                 for (int c = 0; c < NC; c++) { h0[c] = h1[c] = __float2half2_rn(0.f); }
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                    const __half2 w0 = __hsub2(magic_half2((words[wd] >> (2 * j)) & 0x00030003u), bias);
-                    const __half2 w1 = __hsub2(magic_half2((words[wd] >> (2 * j + 2)) & 0x00030003u), bias);
+                auto two = [&](auto jj) {
+                    constexpr int j = decltype(jj)::value;
+                    const __half2 w0 = __hsub2(field<j>(words[wd], k), bias), w1 = __hsub2(field<j + 1>(words[wd], k), bias);
 #pragma unroll
                     for (int c = 0; c < NC; c++) {
                         h0[c] = __hfma2(w0, xr[c][8 * wd + j], h0[c]);
                         h1[c] = __hfma2(w1, xr[c][8 * wd + j + 1], h1[c]);
                     }
-                }
+                };
+                two(std::integral_constant<int, 0>{}); two(std::integral_constant<int, 2>{});
+                two(std::integral_constant<int, 4>{}); two(std::integral_constant<int, 6>{});
 #pragma unroll
                 for (int c = 0; c < NC; c++) {
                     const float2 f = __half22float2(__hadd2(h0[c], h1[c]));
@@ -289,7 +305,21 @@ k_select(const float * __restrict__ scores, int rows, int n_cand, int32_t * __re
     const int lo = min(rows, rank * per), n = min(rows, lo + per) - lo;
     auto key = [&](int i) -> uint32_t { return keys_in_smem ? keys[i] : score_key(ld_act_f32(z + lo + i)); };
     if (keys_in_smem) {
-        for (int i = tid; i < n; i += SEL_THREADS) { keys[i] = score_key(ld_act_f32(z + lo + i)); }
+        int i = tid;
+        for (; i + 7 * SEL_THREADS < n; i += 8 * SEL_THREADS) { // eight loads in flight: one trip to L2, not eight
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) { v[j] = ld_act_f32(z + lo + i + j * SEL_THREADS); }
+#pragma unroll
+            for (int j = 0; j < 8; j++) { keys[i + j * SEL_THREADS] = score_key(v[j]); }
+        }
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 7; j++) { v[j] = i + j * SEL_THREADS < n ? ld_act_f32(z + lo + i + j * SEL_THREADS) : 0.f; }
+#pragma unroll
+        for (int j = 0; j < 7; j++) {
+            if (i + j * SEL_THREADS < n) { keys[i + j * SEL_THREADS] = score_key(v[j]); }
+        }
     }
     {   // this block's share of the logits
         const int64_t share = (vocab + SEL_BLOCKS - 1) / SEL_BLOCKS, first = rank * share, last = first + share < vocab ? first + share : vocab;
@@ -421,13 +451,14 @@ void draft_gemv(int bits, const void * x_bf16, int T, const uint8_t * q, const f
             default: int4_gemv_t<4>(x, q, s, rows, K, y, blocks, st); break;
         }
     } else {
+        const FieldShift fields = {{1u << 8, 1u << 6, 1u << 4, 1u << 2}};
         for (int t = 0; t < T; t += 2) { // two columns per launch, an odd last one alone
             if (T - t >= 2) {
                 const unsigned blocks = (unsigned) std::min<int64_t>((rows + 7) / 8, sms);
-                k_int2_gemv<2><<<blocks, 256, 0, st>>>(x + (int64_t) t * K, q, s, rows, y + (int64_t) t * rows);
+                k_int2_gemv<2><<<blocks, 256, 0, st>>>(x + (int64_t) t * K, q, s, rows, y + (int64_t) t * rows, fields);
             } else {
                 const unsigned blocks = (unsigned) std::min<int64_t>((rows + 7) / 8, sms * 2);
-                k_int2_gemv<1><<<blocks, 256, 0, st>>>(x + (int64_t) t * K, q, s, rows, y + (int64_t) t * rows);
+                k_int2_gemv<1><<<blocks, 256, 0, st>>>(x + (int64_t) t * K, q, s, rows, y + (int64_t) t * rows, fields);
             }
         }
     }

@@ -263,7 +263,7 @@ Bytes encode_nibble(const uint16_t * w, int64_t rows, int64_t K, uint8_t * plane
 
 } // namespace
 
-Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, bool chunk_major, bool frag_order) {
+Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, bool chunk_major, bool frag_order, uint8_t * plane) {
     if (K % CHUNK != 0 || K < CHUNK || K > K_MAX) { bad("K must be a multiple of 512 in [512, 4096], got " + std::to_string(K)); }
     if (rows <= 0) { bad("rows must be positive"); }
     if (format == FMT_NIBBLE) {
@@ -281,10 +281,13 @@ Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, b
     }
 
     Encoded out;
-    out.plane.resize((size_t) (rows * K));
+    if (!plane) {
+        out.plane.resize((size_t) (rows * K));
+        plane = out.plane.data();
+    }
     out.R = format == FMT_NIBBLE ? 0 : R;
     if (format == FMT_NIBBLE) {
-        out.aux = encode_nibble(w, rows, K, out.plane.data());
+        out.aux = encode_nibble(w, rows, K, plane);
         out.format = FMT_NIBBLE;
         return out;
     }
@@ -459,9 +462,9 @@ Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, b
     });
 
     if (h.flags & FLAG_FRAG_ORDER) {
-        write_plane_frag(w, rows, K, out.plane.data());
+        write_plane_frag(w, rows, K, plane);
     } else {
-        write_plane(w, rows, K, (h.flags & FLAG_CHUNK_MAJOR) ? R : 0, out.plane.data());
+        write_plane(w, rows, K, (h.flags & FLAG_CHUNK_MAJOR) ? R : 0, plane);
     }
     return out;
 }

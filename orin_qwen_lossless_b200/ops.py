@@ -97,7 +97,7 @@ def init() -> None:
 
 def fault_status() -> int:
     """Synchronises the current stream and returns (and clears) the bit mask of the kernels' bounded waits that ran out
-    since the last call: 1 staged GEMV, 2 MoE decode units, 4 fragment-order kernels, 8 batched kernel. 0: all outputs
+    since the last call: 1 staged GEMV, 2 MoE decode units, 4 fragment-order kernels, 8 batched kernel, 16 row gather. 0: all outputs
     complete; otherwise the outputs of the affected work items are NaN."""
     v = C.c_uint(0)
     check(lib().bf16n_fault_status(C.byref(v), _stream()))
@@ -119,8 +119,8 @@ def sm_count() -> int:
 # ------------------------------------------------------------------ host: encode, policy
 
 class _Encoded:
-    """The encoder's result, freed when the last tensor over its memory is (the tensors are the buffers the encoder wrote,
-    not copies of them)."""
+    """The encoder's result, freed when the last tensor over its memory is (the aux tensor is the buffer the encoder wrote, not
+    a copy of it)."""
 
     def __init__(self, handle):
         self.handle, self.free = handle, lib().bf16n_encoded_free
@@ -150,10 +150,9 @@ def encode(w: torch.Tensor, fmt: int, R: int, chunk_major: bool, frag_order: boo
     K = wc.shape[-1]
     rows = wc.numel() // max(K, 1)
     h = C.c_void_p()
-    check(lib().bf16n_encode(wc.data_ptr(), rows, K, fmt, R, int(chunk_major), int(frag_order), C.byref(h)))
-    owner = _Encoded(h)
-    plane = owner.tensor(lib().bf16n_encoded_plane).view(rows, K)
-    aux = owner.tensor(lib().bf16n_encoded_aux)
+    plane = torch.empty((rows, K), dtype=torch.uint8)     # the encoder writes into it
+    check(lib().bf16n_encode_into(wc.data_ptr(), rows, K, fmt, R, int(chunk_major), int(frag_order), plane.data_ptr(), C.byref(h)))
+    aux = _Encoded(h).tensor(lib().bf16n_encoded_aux)
     return plane, aux, parse_header(aux)
 
 
@@ -558,7 +557,8 @@ def draft_logits(h: torch.Tensor, w: Weight, head: DraftHead, vocab: int) -> tor
     h = h.contiguous()
     scores = head.scores(h)
     rows = scores.shape[1]
-    if rows <= min(w.meta.rows, vocab) and w.meta.K == K and w.plane.device == h.device and h.data_ptr() % 16 == 0:
+    graded = (h.requires_grad and torch.is_grad_enabled()) or torch.autograd.forward_ad.unpack_dual(h).tangent is not None
+    if rows <= min(w.meta.rows, vocab) and w.meta.K == K and w.plane.device == h.device and h.data_ptr() % 16 == 0 and not graded:
         cw = w.c()
         cand = torch.empty((n, head.candidates), dtype=torch.int32, device=h.device)
         cand_rows = torch.empty((n * head.candidates, K), dtype=torch.bfloat16, device=h.device)
@@ -567,7 +567,7 @@ def draft_logits(h: torch.Tensor, w: Weight, head: DraftHead, vocab: int) -> tor
             check(lib().bf16n_draft_logits(scores.data_ptr(), n, rows, head.candidates, C.byref(cw), h.data_ptr(), cand.data_ptr(),
                                            cand_rows.data_ptr(), out.data_ptr(), vocab, _stream()))
         return out
-    # a head with padding rows beyond the vocabulary (or an unaligned h)
+    # a head with padding rows beyond the vocabulary, an unaligned h, or one whose derivatives are wanted
     cand = scores.topk(head.candidates, dim=-1).indices                           # [n, C]
     rows = get_rows(cand.reshape(-1), w).view(n, head.candidates, K)              # exact BF16 rows
     exact = torch.einsum("nck,nk->nc", rows.float(), h.float())

@@ -1,4 +1,4 @@
-"""The tensors that encode() returns are the encoder's own buffers: either one stays valid without the other, views keep the
+"""The tensors that encode() returns are the buffers the encoder wrote: either one stays valid without the other, views keep the
 memory alive, and a second call does not touch the first call's result."""
 import gc
 

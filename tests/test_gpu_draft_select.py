@@ -82,3 +82,21 @@ def test_rows_of_every_position_in_a_unit(ops, K, R, n):
     ids = torch.from_numpy(np.random.default_rng(n).permutation(rows)[:n].astype(np.int32)).cuda()
     assert torch.equal(ops.get_rows(ids, w).view(torch.int16), src[ids.long()].view(torch.int16))
     assert torch.equal(ops.get_rows(ids.long(), w, torch.float32).view(torch.int32), src[ids.long()].float().view(torch.int32))
+
+
+def test_derivatives_keep_the_general_form(ops):
+    rows, K = 4096, 2048
+    bits = o.weights_like(rows, K, 8)
+    w = ops.upload(*ops.encode(to_bf16_tensor(bits), 3, 8, False), "cuda")
+    head = ops.DraftHead(2, *ops.int2_quantize(to_bf16_tensor(bits).cuda()), 32)
+    h = torch.from_numpy(np.random.default_rng(2).standard_normal((2, K)).astype(np.float32)).to(torch.bfloat16).cuda()
+    out = ops.draft_logits(h, w, head, rows)
+    assert out.grad_fn is None
+    hg = h.clone().requires_grad_()
+    og = ops.draft_logits(hg, w, head, rows)
+    finite = torch.isfinite(out)
+    assert torch.equal(torch.isfinite(og), finite) and torch.allclose(og[finite], out[finite], rtol=1e-4, atol=1e-4)
+    og[finite].sum().backward()
+    picked = finite.float() @ to_bf16_tensor(bits).cuda().float()
+    assert torch.allclose(hg.grad.float(), picked, rtol=2e-2, atol=2e-2)   # BF16 gradient of a sum of 32 rows
+    assert ops.draft_logits(h, w, head, rows + 100).shape == (2, rows + 100)
