@@ -40,4 +40,24 @@ static_assert(sizeof(AuxHeader) == 80, "aux header is 80 bytes");
 // Column (inside a 512-weight chunk) of slot s (0..15) of lane l (0..31); the slot is stored at plane byte 16*l + s.
 constexpr int chunk_col(int lane, int slot) { return 128 * (slot >> 2) + 4 * lane + (slot & 3); }
 
+#ifdef __CUDACC__
+#define B16_HOST_DEVICE __host__ __device__ __forceinline__
+#else
+#define B16_HOST_DEVICE inline
+#endif
+// The codes that end inside the HP_LMAX stream bits `window` (at most three) and their length: bits | codes << 8. A prefix
+// code: a code of at most the bits that are left is decided by them. The reader that skips by these entries advances by
+// them alone, so every entry names at least one code, whatever the table holds: a length that no table has (a damaged
+// aux buffer) counts as HP_LMAX bits.
+B16_HOST_DEVICE uint32_t codes_in_window(const uint32_t * lut, uint32_t window) {
+    uint32_t len = 0, count = 0;
+    for (; count < 3; count++) {
+        uint32_t l = lut[(window << len) & (HP_MAX_PAIRS - 1)] & 31u;
+        if (count == 0 && l > (uint32_t) HP_LMAX) { l = HP_LMAX; }
+        if (len + l > (uint32_t) HP_LMAX) { break; }
+        len += l;
+    }
+    return len | count << 8;
+}
+
 } // namespace b16

@@ -511,15 +511,7 @@ __global__ void __launch_bounds__(ROWS_THREADS) k_pair_rows_staged(const PairVie
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     stage_lut(lut, w.lut, HP_MAX_PAIRS);
     __syncthreads();
-    for (int i = threadIdx.x; i < HP_MAX_PAIRS; i += ROWS_THREADS) {
-        uint32_t len = 0, count = 0;
-        for (; count < 3; count++) { // a prefix code: a code of at most the bits that are left is decided by them
-            const uint32_t l = lut[(uint32_t) (i << len) & (HP_MAX_PAIRS - 1)] & 31u;
-            if (len + l > (uint32_t) HP_LMAX) { break; }
-            len += l;
-        }
-        many[i] = (uint16_t) (len | count << 8);
-    }
+    for (int i = threadIdx.x; i < HP_MAX_PAIRS; i += ROWS_THREADS) { many[i] = (uint16_t) codes_in_window(lut, (uint32_t) i); }
     grid_dependency_wait(); // the row ids may come from the kernel before this one; everything above is the matrix's own
     const int64_t i = (int64_t) blockIdx.x * rows_per_block + warp;
     const bool live = reads && i < n;

@@ -107,9 +107,9 @@ struct WindowReader {
             slide(o + e[q] + e[q + 1], k);
         }
     }
-    // passes over `n` codes; many: 16-bit entries, bits | codes << 8 of what ends inside 12 bits of stream
+    // passes over `n` codes; many: 16-bit entries of codes_in_window (format.h): each names one to three codes, so this ends
     __device__ __forceinline__ void skip(int n, uint32_t many, uint32_t lut, const Opaque & k) {
-        while (n >= 3) { // an entry holds one to three codes
+        while (n >= 3) {
             uint32_t m;
             asm("ld.shared.u16 %0, [%1];" : "=r"(m) : "r"(many + 2 * (shl_wrap_hi(lo, hi, o) >> (32 - HP_LMAX))));
             n -= (int) (m >> 8);
