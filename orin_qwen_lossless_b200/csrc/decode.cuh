@@ -61,8 +61,8 @@ __device__ __forceinline__ float silu_f(float v) { return __fdividef(v, 1.0f + _
 __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __uint_as_float((uint32_t) __bfloat16_as_ushort(v) << 16); }
 
-// Activations may have been written by the kernel right before this one on the stream, which can still be running when
-// this kernel starts (programmatic dependent launch). They are therefore read with ordinary coherent loads written as
+// Activations and routing data may have been written by the kernel right before this one on the stream, which can still be
+// running when this kernel starts (programmatic dependent launch). They are therefore read with ordinary coherent loads written as
 // volatile asm: such a load stays behind the grid dependency wait (the read-only ld.global.nc path may be moved above it
 // and may serve lines fetched before the producer's stores), and it still caches in L1 for the other rows of the block.
 __device__ __forceinline__ uint4 ld_act16(const void * p) {
@@ -78,6 +78,11 @@ __device__ __forceinline__ uint2 ld_act8(const void * p) {
 __device__ __forceinline__ float ld_act_f32(const float * p) {
     float v;
     asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ int32_t ld_act_s32(const int32_t * p) {
+    int32_t v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
 // x[i..i+3] as FP32 from global memory (i a multiple of 4; the caller guarantees 16-/8-byte alignment)

@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(EXPAND_WARPS * 32, 1) k_expand_tiles(const Exp
     for (int64_t u = (int64_t) blockIdx.x * nwarp + warp; u < p.units; u += (int64_t) gridDim.x * nwarp) {
         const int64_t row0 = u * R;
         const int e = (int) (row0 / p.rows_per_expert), ri = (int) (row0 - (int64_t) e * p.rows_per_expert);
-        if (p.bounds && __ldg(p.bounds + e + 1) == __ldg(p.bounds + e)) { continue; }
+        if (p.bounds && ld_act_s32(p.bounds + e + 1) == ld_act_s32(p.bounds + e)) { continue; }
         const int nb = ri / p.rows_per_block, img_row0 = ri - nb * p.rows_per_block + row_offset;
         unsigned char * img = p.images + ((int64_t) e * p.blocks_per_expert + nb) * ((int64_t) KT * IMG_KTILE_BYTES) + lane_part;
         RingReader rd;
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(FO_EXPAND_WARPS * 32, 1) k_expand_tiles_fo(con
     const int KT = p.C * 8;
     for (int64_t ur = (int64_t) blockIdx.x * nwarp + warp; ur < p.units; ur += (int64_t) gridDim.x * nwarp) {
         const int e = (int) (ur / p.units_per_expert), ue = (int) (ur - (int64_t) e * p.units_per_expert);
-        if (__ldg(p.bounds + e + 1) == __ldg(p.bounds + e)) { continue; }
+        if (ld_act_s32(p.bounds + e + 1) == ld_act_s32(p.bounds + e)) { continue; }
         const int64_t u = p.unit0 + ur;
         const int band = ue / p.C, slab = ue - band * p.C;
         const int nb = band / p.bands_per_block, img_row0 = (band - nb * p.bands_per_block) * FO_BAND + row_offset;

@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(32) k_topk(const float * __restrict__ logits, 
 #pragma unroll
     for (int i = 0; i < PER; i++) {
         const int e = i * 32 + lane;
-        v[i] = e < n_experts ? z[e] : -INFINITY;
+        v[i] = e < n_experts ? ld_act_f32(z + e) : -INFINITY;
     }
     float zmax = 0.f, denom = 0.f;
     for (int s = 0; s < k; s++) {

@@ -503,8 +503,8 @@ struct TileWalk {
         uint32_t bits = m[word];
         for (; r; r--) { bits &= bits - 1; }
         e = 32 * word + __ffs(bits) - 1;
-        jp = __ldg(bounds + e) + level * TM_G * M_TOK;
-        j1 = __ldg(bounds + e + 1);
+        jp = ld_act_s32(bounds + e) + level * TM_G * M_TOK;
+        j1 = ld_act_s32(bounds + e + 1);
         if (level + 1 < TM_LEVELS) { j1 = min(j1, jp + TM_G * M_TOK); }
         at += gridDim.x;
         return true;
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_tile_mm(const TileMmArgs p) {
     __syncthreads();
     for (int i = warp; i < TM_LEVELS * TM_MASK_WORDS; i += TM_THREADS / 32) {
         const int l = i / TM_MASK_WORDS, word = i - l * TM_MASK_WORDS, e = 32 * word + lane;
-        const bool in = e < p.n_experts && __ldg(p.bounds + e + 1) - __ldg(p.bounds + e) > l * TM_G * M_TOK;
+        const bool in = e < p.n_experts && ld_act_s32(p.bounds + e + 1) - ld_act_s32(p.bounds + e) > l * TM_G * M_TOK;
         const uint32_t m = __ballot_sync(FULL, in);
         if (lane == 0) {
             levels.mask[l][word] = m;
