@@ -38,6 +38,14 @@ typedef struct bf16n_weight {
     uint64_t off_a, off_b, off_c, off_d;
 } bf16n_weight;
 
+/* Matrices and the stream. Every call is ordered behind what was launched on its stream before it as far as activations, ids,
+ * routing, outputs and buffers go. A matrix is expected to stay as it is while products use it: the products of a decode step
+ * (bf16n_mmv, bf16n_mmv_group, bf16n_mmv_glu(_merged), bf16n_moe_decode) may begin to read it while kernels launched before
+ * them, several of this library's and the one in front of those, are still running. A caller that writes a matrix with a kernel
+ * of its own (an in-place swap) waits on the host until that kernel is complete before the next such product; a copy by
+ * cudaMemcpyAsync needs nothing. All other calls (bf16n_get_rows, bf16n_dequant, bf16n_verify, bf16n_draft_logits, bf16n_mm_ids and
+ * bf16n_mm_ids_scratch) read the matrix behind everything before them. */
+
 /* One matrix-vector product call: y[col] = W[rbase : rbase+nrows] x[col] for ncols columns.
  * Dense: column c = token c, rbase = row0.  With ids: column c = (token c / n_used, slot c % n_used), expert
  * e = ids[token, slot], rbase = row0 + e*rows_per_matrix; x of a column at x_tok*token + x_slot*(slot % x_per_slot),

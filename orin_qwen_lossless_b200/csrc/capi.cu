@@ -229,7 +229,7 @@ int bf16n_draft_logits(const float * scores, int T, int64_t rows, int n_cand, co
         draft_select(scores, T, rows, n_cand, cand, out, vocab, st);
         const int64_t n = (int64_t) T * n_cand;
         if (frag_order(*w)) { fo_gather_rows(*w, cand, 4, n, cand_rows, true, w->K * 2, 0, st); }
-        else { gather_rows(*w, cand, 4, n, cand_rows, true, w->K * 2, 0, st); }
+        else { gather_rows(*w, cand, 4, n, cand_rows, true, w->K * 2, 0, st, true); } // behind the selection
         draft_rescore(x_bf16, cand_rows, cand, T, n_cand, (int) w->K, out, vocab, st);
     });
 }
@@ -484,7 +484,7 @@ static void moe_decode_checked(const bf16n_weight * gate, const bf16n_weight * u
     if (router_logits) { moe_topk(router_logits, n_tok, n_experts, n_used, topk_ids, topk_weights, (cudaStream_t) stream); }
     if (frag) {
         moe_decode_frag_order(*gate, *up, *down, x, x_bf16 != 0, x_tok, topk_ids, topk_weights, n_tok, n_used, n_experts, scratch, y,
-                              y_bf16 != 0, (cudaStream_t) stream);
+                              y_bf16 != 0, (cudaStream_t) stream, router_logits != nullptr); // behind the router
         return;
     }
     moe_decode(*gate, *up, *down, x, x_bf16 != 0, x_tok, topk_ids, topk_weights, n_tok, n_used, n_experts_local, expert_lo,

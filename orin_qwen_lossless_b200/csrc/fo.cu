@@ -216,7 +216,7 @@ __device__ __forceinline__ float2 load_x2(const bf16 * p) {
 struct FoMat { PairView v; const AuxHeader * hdr; int64_t y_shift; }; // y_shift: bytes from the columns' outputs to this matrix's
 
 template <typename TX, bool MMA, int G = 1>
-__global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const FoMat m0, const FoMat m1, int C, Cols p, int nb, int ncols, const Opaque k) {
+__global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const FoMat m0, const FoMat m1, int C, Cols p, int nb, int ncols, bool lut_first, const Opaque k) {
     static_assert(!MMA || G == 1, "grouping is for the FMA form");
     extern __shared__ __align__(128) unsigned char smem[];
     const FoMat & mat = blockIdx.z ? m1 : m0;
@@ -236,8 +236,9 @@ __global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const FoMa
     if (lane == 0) { mbar_init(bar, 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncwarp();
-    stage_lut(lut, w.lut); // the matrix's own: while the kernel before this one drains
+    if (lut_first) { stage_lut(lut, w.lut); } // while the kernel before this one, which is this library's, drains (launch_behind)
     grid_dependency_wait(); // activations and expert ids may come from the kernel before this one
+    if (!lut_first) { stage_lut(lut, w.lut); }
     const TX * xg; OutVec out; int64_t rbase;
     column<TX>(p, MMA ? 0 : blockIdx.y, xg, out, rbase);
     out.p += mat.y_shift;
@@ -878,7 +879,7 @@ bool fo_split_applies(const bf16n_weight & w, const bf16n_mmv_args & a) {
 
 // one decode per column (two from four tokens on); with `up`, a second matrix of the shape whose outputs go to up_y
 template <typename TX>
-void fo_split(const bf16n_weight & w, const bf16n_weight * up, void * up_y, const bf16n_mmv_args & a, cudaStream_t st) {
+void fo_split(const bf16n_weight & w, const bf16n_weight * up, void * up_y, const bf16n_mmv_args & a, cudaStream_t st, bool behind_own) {
     const Cols p = make_cols(a);
     const int C = (int) (w.K / CHUNK), nb = std::max(1, 8 / C);
     const int64_t bands = p.nrows / BAND;
@@ -893,11 +894,11 @@ void fo_split(const bf16n_weight & w, const bf16n_weight * up, void * up_y, cons
     const int g = grouped ? FO_GROUP : 1;
     const size_t shm = 4 * HP_MAX_PAIRS + 128 + (size_t) w.K * 4 + (size_t) nb * C * 16 * g * 4 + (size_t) nb * C * FO_SPLIT_CAP;
     launch_chained(grouped ? k_fo_gemv_split<TX, false, FO_GROUP> : k_fo_gemv_split<TX, false>, grid, dim3(nb * C * 32), shm, st, m0, m1, C, p, nb,
-                   grouped ? a.ncols : 1, k);
+                   grouped ? a.ncols : 1, behind_own, k);
 }
 
 template <typename TX>
-void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st) {
+void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool behind_own) {
     Cols p = make_cols(a);
     // routed columns, and a single dense column of a small matrix: the kernels with one decode per column
     // From 16 bands per SM on, BF16 activations take the persistent kernel; below, it was measured level with or behind
@@ -905,7 +906,7 @@ void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st
     constexpr int64_t big_per_sm = 16;
     if (a.ids || (a.ncols == 1 && (p.nrows / BAND < (int64_t) device_info().sms * big_per_sm || !a.x_bf16))) {
         if (fo_split_applies(w, a)) {
-            fo_split<TX>(w, nullptr, nullptr, a, st);
+            fo_split<TX>(w, nullptr, nullptr, a, st, behind_own);
         } else {
             launch_fo<1, TX>(w, p, a.ids ? a.ncols : 1, st);
         }
@@ -946,7 +947,7 @@ void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st
                                        (size_t) nb * C * FO_SPLIT_CAP;
                     const Opaque k = {1u, 4u, ~0u, 32u};
                     launch_chained(k_fo_gemv_split<bf16, true>, dim3((unsigned) ((bands + nb - 1) / nb)), dim3(nb * C * 32), shm, st,
-                                   fo_mat(w), fo_mat(w), C, q, nb, nc, k);
+                                   fo_mat(w), fo_mat(w), C, q, nb, nc, behind_own || c0 > 0, k);
                 }
             } else {
                 const int warps = bands >= sms * 32 ? 8 : bands >= sms * 8 ? 4 : 2;
@@ -1050,13 +1051,13 @@ void fo_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_b
     check_launch();
 }
 
-void fo_gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st) {
-    if (a.x_bf16) { fo_gemv_t<bf16>(w, a, st); } else { fo_gemv_t<float>(w, a, st); }
+void fo_gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool behind_own) {
+    if (a.x_bf16) { fo_gemv_t<bf16>(w, a, st, behind_own); } else { fo_gemv_t<float>(w, a, st, behind_own); }
 }
 
-void fo_gemv_two(const bf16n_weight & w, const bf16n_weight & up, const bf16n_mmv_args & a, void * up_y, cudaStream_t st) {
+void fo_gemv_two(const bf16n_weight & w, const bf16n_weight & up, const bf16n_mmv_args & a, void * up_y, cudaStream_t st, bool behind_own) {
     if (fo_split_applies(w, a)) {
-        if (a.x_bf16) { fo_split<bf16>(w, &up, up_y, a, st); } else { fo_split<float>(w, &up, up_y, a, st); }
+        if (a.x_bf16) { fo_split<bf16>(w, &up, up_y, a, st, behind_own); } else { fo_split<float>(w, &up, up_y, a, st, behind_own); }
         return;
     }
     bf16n_mmv_args u = a;

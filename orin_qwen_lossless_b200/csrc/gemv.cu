@@ -886,7 +886,7 @@ void expand_compare(const bf16n_weight & w, int64_t row0, int64_t nrows, const u
 }
 
 void gather_rows(const bf16n_weight & w, const void * ids, int64_t ids_s0, int64_t n, void * dst, bool dst_bf16, int64_t dst_s1,
-                 int64_t row0, cudaStream_t st) {
+                 int64_t row0, cudaStream_t st, bool behind_own) {
     const int C = (int) (w.K / CHUNK);
     const unsigned gx = (unsigned) ((n + 7) / 8);
     const char * ip = (const char *) ids;
@@ -900,8 +900,8 @@ void gather_rows(const bf16n_weight & w, const void * ids, int64_t ids_s0, int64
         const uint32_t cap = (uint32_t) ((w.R * w.K * 3 / 8 + 64 + 15) & ~15ll);
         const size_t shm = 6 * HP_MAX_PAIRS + 128 + (size_t) per * cap;
         const Opaque k = {1u, 4u, ~0u, 32u};
-        launch_chained(dst_bf16 ? k_pair_rows_staged<true> : k_pair_rows_staged<false>, dim3((unsigned) ((n + per - 1) / per)), dim3(ROWS_THREADS), shm,
-                       st, pair_view(w), (const AuxHeader *) w.aux, C, w.R, ip, ids_s0, n, row0, dp, dst_s1, per, cap, k);
+        launch_behind(behind_own, dst_bf16 ? k_pair_rows_staged<true> : k_pair_rows_staged<false>, dim3((unsigned) ((n + per - 1) / per)), dim3(ROWS_THREADS),
+                      shm, st, pair_view(w), (const AuxHeader *) w.aux, C, w.R, ip, ids_s0, n, row0, dp, dst_s1, per, cap, k);
     } else {
         if (dst_bf16) { k_pair_rows<true><<<gx, 256, 0, st>>>(pair_view(w), C, w.R, ip, ids_s0, n, row0, dp, dst_s1); }
         else { k_pair_rows<false><<<gx, 256, 0, st>>>(pair_view(w), C, w.R, ip, ids_s0, n, row0, dp, dst_s1); }

@@ -35,16 +35,24 @@ inline void allow_dynamic_smem(const void * kernel, int bytes, int optin, const 
 #ifdef __CUDACC__
 // Launch of a kernel that may start while the kernel before it on the stream is still draining (programmatic dependent
 // launch): such a kernel calls grid_dependency_wait() before it touches anything an earlier kernel wrote or still reads,
-// and does only independent work (tables, barriers) above that line. Works under stream capture as well.
+// and does only independent work (barriers, a matrix's own tables) above that line. Works under stream capture as well.
+// A kernel that reads a matrix above the line is not ordered behind a kernel of the caller's that wrote the matrix. Where the
+// public interface says so (products of NIBBLE matrices, expert units of a decode step) the caller sees to that; all others
+// are launched with launch_behind, whose `own` says that the kernel in front is this library's, launched by the same call and
+// waiting for its own predecessors before it lets this one start: whatever wrote the matrix has then completed.
 template <typename... KArgs, typename... Args>
-void launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t shm, cudaStream_t st, Args &&... args) {
+void launch_behind(bool own, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t shm, cudaStream_t st, Args &&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = shm; cfg.stream = st;
     cudaLaunchAttribute attr = {};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+    attr.val.programmaticStreamSerializationAllowed = own ? 1 : 0;
     cfg.attrs = &attr; cfg.numAttrs = 1;
     cuda_ok(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...), "kernel launch");
+}
+template <typename... KArgs, typename... Args>
+void launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t shm, cudaStream_t st, Args &&... args) {
+    launch_behind(true, kernel, grid, block, shm, st, args...);
 }
 // Lets the next kernel on the stream begin its own prologue now. Only for kernels in which every block that has work also
 // waits (grid_dependency_wait) before it touches what earlier kernels wrote or read.
@@ -75,7 +83,7 @@ void expand_store(const bf16n_weight & w, int64_t row0, int64_t nrows, uint16_t 
 void expand_compare(const bf16n_weight & w, int64_t row0, int64_t nrows, const uint16_t * src, unsigned long long * total,
                     cudaStream_t st);
 void gather_rows(const bf16n_weight & w, const void * ids, int64_t ids_s0, int64_t n, void * dst, bool dst_bf16, int64_t dst_s1,
-                 int64_t row0, cudaStream_t st);
+                 int64_t row0, cudaStream_t st, bool behind_own = false);
 
 // device addresses of the words the kernels set when one of their bounded waits runs out (bf16n_fault_status)
 unsigned int * gemv_staged_fault_word();
@@ -98,8 +106,8 @@ void gemv_rings(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t s
 // fo.cu: fragment-order HUFPAIR tensors
 void fo_init();
 bool fo_supported(const bf16n_weight & w);
-void fo_gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st);
-void fo_gemv_two(const bf16n_weight & w, const bf16n_weight & up, const bf16n_mmv_args & a, void * up_y, cudaStream_t st); // routed columns
+void fo_gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool behind_own = false); // behind_own: see launch_behind
+void fo_gemv_two(const bf16n_weight & w, const bf16n_weight & up, const bf16n_mmv_args & a, void * up_y, cudaStream_t st, bool behind_own); // routed columns
 bool fo_mm_ids_supported(const bf16n_weight & w, const bf16n_weight * up);
 void fo_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
                const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
@@ -140,7 +148,7 @@ void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_
                 float * scratch, void * y, bool y_bf16, cudaStream_t st, const bf16n_peer_out * peers = nullptr);
 void moe_decode_frag_order(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_weight & down, const void * x, bool x_bf16,
                            int64_t x_tok, const int32_t * ids, const float * weights, int n_tok, int n_used, int n_experts,
-                           float * scratch, void * y, bool y_bf16, cudaStream_t st);
+                           float * scratch, void * y, bool y_bf16, cudaStream_t st, bool behind_own);
 void peer_sum(const float * parts, int n_parts, int64_t n, const float * extra, void * y, bool y_bf16, cudaStream_t st);
 
 size_t moe_decode_static_capacity_floats();
@@ -164,7 +172,7 @@ void expand_tiles_init();
 bool expand_tiles_supported(const bf16n_weight & w);
 void expand_tiles(const bf16n_weight & w, const bf16n_weight * up, int n_experts, const int32_t * bounds, void * images, cudaStream_t st);
 void expand_tiles_fo(const bf16n_weight & w, const bf16n_weight * up, int n_experts, int e0, int n, const int32_t * bounds, void * images,
-                     cudaStream_t st);
+                     cudaStream_t st, bool behind_own);
 bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
                          const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
                          void * scratch, size_t scratch_bytes, cudaStream_t st);

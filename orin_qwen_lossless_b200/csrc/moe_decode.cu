@@ -349,7 +349,7 @@ void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_
 // slot-order combine. All experts on this GPU (no expert slice). Same scratch layout as moe_decode.
 void moe_decode_frag_order(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_weight & down, const void * x, bool x_bf16,
                            int64_t x_tok, const int32_t * ids, const float * weights, int n_tok, int n_used, int n_experts,
-                           float * scratch, void * y, bool y_bf16, cudaStream_t st) {
+                           float * scratch, void * y, bool y_bf16, cudaStream_t st, bool behind_own) {
     const int64_t N = gate.rows / n_experts, H = down.rows / n_experts;
     const int ncols = n_tok * n_used;
     float * g = scratch, * u = g + (int64_t) ncols * N, * ys = u + (int64_t) ncols * N;
@@ -360,12 +360,12 @@ void moe_decode_frag_order(const bf16n_weight & gate, const bf16n_weight & up, c
     a.rows_per_matrix = N; a.row0 = 0; a.nrows = N;
     a.y_tok = 4ll * n_used * N; a.y_slot = 4ll * N;
     a.y = g;
-    fo_gemv_two(gate, up, a, u, st);
+    fo_gemv_two(gate, up, a, u, st, behind_own);
     moe_swiglu(g, u, g, (int64_t) ncols * N, st);            // g := silu(g) * u
     bf16n_mmv_args d = a;
     d.x = g; d.x_bf16 = 0; d.x_per_slot = n_used; d.x_tok = 4ll * n_used * N; d.x_slot = 4ll * N;
     d.rows_per_matrix = H; d.nrows = H; d.y = ys; d.y_tok = 4ll * n_used * H; d.y_slot = 4ll * H;
-    fo_gemv(down, d, st);
+    fo_gemv(down, d, st, true);                               // behind the SwiGLU
     const dim3 grid((unsigned) std::min<int64_t>((H + 255) / 256, 64), (unsigned) n_tok);
     launch_chained(k_combine_f32, grid, dim3(256), 0, st, ys, weights, (char *) y, y_bf16, n_used, H, PeerOut{});
     check_launch();

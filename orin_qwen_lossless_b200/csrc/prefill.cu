@@ -876,7 +876,7 @@ bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const 
     const int ranges = (n_experts + fit - 1) / fit, step = (n_experts + ranges - 1) / ranges; // ranges of equal size
     for (int e0 = 0; e0 < n_experts; e0 += step) {
         const int n = std::min(step, n_experts - e0);
-        expand_tiles_fo(w, up, n_experts, e0, n, bounds + e0, scratch, st);
+        expand_tiles_fo(w, up, n_experts, e0, n, bounds + e0, scratch, st, e0 > 0); // behind the range before
         tile_mm(scratch, a, bounds + e0, n, w.K, up != nullptr, st);
     }
     return true;

@@ -1,4 +1,4 @@
-"""Kernels launched with launch_chained may start before the kernel in front of them has finished: what that kernel writes
+"""Kernels launched with launch_chained or launch_behind may start before the kernel in front of them has finished: what that kernel writes
 (activations, routing) must be read behind the dependency wait with ordered loads, never through the read-only path
 (ld.global.nc), which the compiler may move above the wait and which may serve lines fetched before the stores. Checked on the
 sources: __ldg and ld_stream16 in such kernels read matrices only, and their read-only pointer parameters are read through
@@ -12,7 +12,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 SOURCES = {f: re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, f)).read()) for f in sorted(os.listdir(CSRC)) if f.endswith((".cu", ".cuh"))}
 # what a matrix's view gives: code table, unit and lane offsets, row tables, escapes, plane (pl, pw: pointers into it)
 MATRIX = re.compile(r"\b(lut|ubase|lrel|row_lut|esc_off|esc|plane|codes|pl|stream|pfirst|nrow)\b")
-CHAINED = sorted({k for s in SOURCES.values() for call in re.findall(r"launch_chained\(([^;]*?)dim3|launch_chained\(([^;]*?), grid", s)
+CHAINED = sorted({k for s in SOURCES.values() for call in re.findall(r"launch_(?:chained|behind)\(([^;]*?)dim3|launch_(?:chained|behind)\(([^;]*?), grid", s)
                   for k in re.findall(r"\bk_\w+", " ".join(call))})
 
 
