@@ -392,7 +392,8 @@ int bf16n_mm_ids(const bf16n_weight * w, const bf16n_weight * up, const void * x
 }
 
 size_t bf16n_mm_ids_scratch_bytes(const bf16n_weight * w, const bf16n_weight * up, int n_experts, int n_tok, int n_used) {
-    if (!w || !w->fo || (up && !up->fo) || n_experts <= 0 || w->rows % n_experts || n_tok <= 0 || n_used <= 0) { return 0; }
+    if (!w || !w->fo || n_experts <= 0 || w->rows < n_experts || w->rows % n_experts || n_tok <= 0 || n_used <= 0) { return 0; }
+    if (up && (!up->fo || up->rows != w->rows || up->K != w->K)) { return 0; }
     return fo_mm_ids_scratch_bytes(*w, up, n_experts, n_tok, n_used);
 }
 
@@ -401,6 +402,7 @@ int bf16n_mm_ids_scratch(const bf16n_weight * w, const bf16n_weight * up, const 
                          int n_tok, int n_used, void * scratch, size_t scratch_bytes, void * stream) {
     return guarded([&] {
         ensure_init();
+        require(w && x_bf16 && ids_src1 && ids_dst && bounds && dst, "mm_ids_scratch: null argument");
         check_weight(*w);
         if (up) { check_weight(*up); }
         require(n_experts > 0 && w->rows % n_experts == 0, "rows must split evenly into experts");

@@ -1026,6 +1026,9 @@ constexpr size_t FO_SCRATCH_MAX = (size_t) 1 << 30;
 size_t fo_mm_ids_scratch_bytes(const bf16n_weight & w, const bf16n_weight * up, int n_experts, int n_tok, int n_used) {
     const size_t per_expert = (size_t) (w.rows / n_experts) * (size_t) w.K * 2 * (up ? 2 : 1);
     if ((w.rows / n_experts) % (up ? 128 : 256) || per_expert > FO_SCRATCH_MAX) { return 0; }
+    // a call with more experts than the fused kernel lists is refused (fo_require_expert_count); 227 KB where no device is known
+    const int optin = device_info().smem_optin;
+    if (fo_mm_shm(up != nullptr, n_experts) > (size_t) (optin ? optin : 227 * 1024)) { return 0; }
     if ((int64_t) n_tok * n_used < (up ? FO_TWO_PASS_GLU : FO_TWO_PASS_ONE) * n_experts) { return 0; }
     return per_expert * std::min<size_t>((size_t) n_experts, FO_SCRATCH_MAX / per_expert);
 }

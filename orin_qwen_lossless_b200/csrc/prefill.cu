@@ -870,7 +870,7 @@ bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const 
                          void * scratch, size_t scratch_bytes, cudaStream_t st) {
     const size_t per_expert = (size_t) (w.rows / n_experts) * (size_t) w.K * 2 * (up ? 2 : 1);
     const int64_t rows_per_block = up ? TM_N / 2 : TM_N;
-    if (!scratch || (w.rows / n_experts) % rows_per_block || n_experts > TM_MAX_EXPERTS || ((uintptr_t) scratch % 1024) || scratch_bytes < per_expert) { return false; }
+    if (!scratch || per_expert == 0 || (w.rows / n_experts) % rows_per_block || n_experts > TM_MAX_EXPERTS || ((uintptr_t) scratch % 1024) || scratch_bytes < per_expert) { return false; }
     const PrefillArgs a = batch_args(w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16, dst_col, n_experts);
     const int fit = (int) std::min<size_t>((size_t) n_experts, scratch_bytes / per_expert);
     const int ranges = (n_experts + fit - 1) / fit, step = (n_experts + ranges - 1) / ranges; // ranges of equal size

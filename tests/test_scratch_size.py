@@ -1,0 +1,26 @@
+"""bf16n_mm_ids_scratch_bytes answers 0 for every call that has no use for scratch: an empty matrix, experts that do not split
+evenly or are more than a call takes, an up matrix of another shape or layout. Run in a process of its own: a wrong answer here
+was once an arithmetic trap."""
+import os
+import subprocess
+import sys
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SIZES = """
+import ctypes as C, sys
+from orin_qwen_lossless_b200 import _lib
+def w(rows, K=2048, fo=1, R=16, fmt=3):
+    return _lib.Weight(4096, 8192, fmt, R, K, rows, 0, fo, 256, 16640, 20000, 30000)
+def need(a, up, experts, tok=8192, used=8):
+    return _lib.lib().bf16n_mm_ids_scratch_bytes(C.byref(a), C.byref(up) if up is not None else None, experts, tok, used)
+print([need(w(0), None, 8), need(w(0), w(0), 1), need(w(100), None, 8), need(w(-4096), None, 8), need(w(8 * 512), w(8 * 256), 8),
+       need(w(8 * 512), w(8 * 512, K=512), 8), need(w(8 * 512), w(8 * 512, fo=0), 8), need(w(8 * 512, fo=0), None, 8),
+       need(w(2000 * 512), w(2000 * 512), 2000, 1 << 20), need(w(8 * 512), w(8 * 512), 8)])
+"""
+
+
+def test_sizes():
+    r = subprocess.run([sys.executable, "-c", SIZES], capture_output=True, text=True, timeout=120, cwd=ROOT)
+    assert r.returncode == 0, (r.returncode, r.stderr[-500:])
+    *none, some = eval(r.stdout)
+    assert none == [0] * 9 and some == 8 * 2 * 512 * 2048 * 2
