@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import struct
+import time
 from dataclasses import dataclass
 
 import torch
@@ -651,18 +652,25 @@ def moe_route(topk_ids: torch.Tensor, n_experts: int, per_slot: bool):
     return src1, dst, bounds
 
 
+# A refused request costs the process its allocator's cached blocks (freed with a synchronise before torch gives up), so a device
+# that had no memory for a call's tiles is not asked again for a while: device index -> when it last refused
+_scratch_refused: dict[int, float] = {}
+_SCRATCH_RETRY_S = 10.0
+
+
 def _mm_ids_scratch(cw, cu, n_experts: int, T: int, n_used: int, device) -> torch.Tensor | None:
-    """Memory for the decoded tiles of one batched call on fragment-order experts, from torch's allocator and back to it
-    when the call has been enqueued; None where the fused kernel is the faster one, under stream capture (a graph would
-    keep the memory) and when the memory is not to be had."""
+    """Memory (up to 1 GiB) for the decoded tiles of one batched call on fragment-order experts, from torch's allocator and
+    back to it when the call has been enqueued; None where the fused kernel is the faster one, under stream capture (a
+    graph would keep the memory) and when the memory is not to be had. Both forms give the same bits."""
     if torch.cuda.is_current_stream_capturing():
         return None
     need = lib().bf16n_mm_ids_scratch_bytes(C.byref(cw), C.byref(cu) if cu is not None else None, n_experts, T, n_used)
-    if need == 0:
+    if need == 0 or time.monotonic() - _scratch_refused.get(device.index, -_SCRATCH_RETRY_S) < _SCRATCH_RETRY_S:
         return None
     try:
         return torch.empty(need + 1024, dtype=torch.uint8, device=device)
     except torch.cuda.OutOfMemoryError:
+        _scratch_refused[device.index] = time.monotonic()
         return None
 
 

@@ -5,6 +5,8 @@ import os
 import subprocess
 import sys
 
+import torch
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SIZES = """
 import ctypes as C, sys
@@ -24,3 +26,23 @@ def test_sizes():
     assert r.returncode == 0, (r.returncode, r.stderr[-500:])
     *none, some = eval(r.stdout)
     assert none == [0] * 9 and some == 8 * 2 * 512 * 2048 * 2
+
+
+def test_a_refusal_is_not_repeated_for_every_call(monkeypatch):
+    """A device without memory for the tiles is asked once and then left alone for a while."""
+    from orin_qwen_lossless_b200 import _lib, ops
+    asked, now = [], [100.0]
+
+    def empty(n, **kw):
+        asked.append(kw["device"].index)
+        raise torch.cuda.OutOfMemoryError
+
+    monkeypatch.setattr(ops, "_scratch_refused", {})
+    monkeypatch.setattr(ops.torch, "empty", empty)
+    monkeypatch.setattr(ops.torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(ops.time, "monotonic", lambda: now[0])
+    w = _lib.Weight(4096, 8192, 3, 16, 2048, 8 * 512, 0, 1, 256, 16640, 20000, 30000)
+    for device, t in ((0, 100.0), (0, 100.1), (1, 101.0), (0, 109.0), (0, 111.0)):
+        now[0] = t
+        assert ops._mm_ids_scratch(w, w, 8, 8192, 8, torch.device("cuda", device)) is None
+    assert asked == [0, 1, 0]
