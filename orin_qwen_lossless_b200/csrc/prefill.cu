@@ -840,9 +840,12 @@ void tile_mm(const void * images, const PrefillArgs & a, const int32_t * bounds,
 bool two_pass(const bf16n_weight & w, const bf16n_weight * up, const PrefillArgs & a, int n_experts, cudaStream_t st) {
     const size_t need = prefill_workspace_bytes(w, up);
     const int rows_per_block = up ? TM_N / 2 : TM_N;
-    if (need == 0 || need > g_workspace_bytes || a.rows_per_expert % rows_per_block || n_experts > TM_MAX_EXPERTS || ((uintptr_t) g_workspace % 1024)) { return false; }
+    if (need == 0 || need > g_workspace_bytes || a.rows_per_expert % rows_per_block || ((uintptr_t) g_workspace % 1024)) { return false; }
     expand_tiles(w, up, n_experts, a.bounds, g_workspace, st);
-    tile_mm(g_workspace, a, a.bounds, n_experts, w.K, up != nullptr, st);
+    const size_t per_expert = need / (size_t) n_experts;
+    for (int e0 = 0; e0 < n_experts; e0 += TM_MAX_EXPERTS) { // the experts that a launch lists
+        tile_mm((const char *) g_workspace + e0 * per_expert, a, a.bounds + e0, std::min(TM_MAX_EXPERTS, n_experts - e0), w.K, up != nullptr, st);
+    }
     return true;
 }
 
@@ -870,9 +873,9 @@ bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const 
                          void * scratch, size_t scratch_bytes, cudaStream_t st) {
     const size_t per_expert = (size_t) (w.rows / n_experts) * (size_t) w.K * 2 * (up ? 2 : 1);
     const int64_t rows_per_block = up ? TM_N / 2 : TM_N;
-    if (!scratch || per_expert == 0 || (w.rows / n_experts) % rows_per_block || n_experts > TM_MAX_EXPERTS || ((uintptr_t) scratch % 1024) || scratch_bytes < per_expert) { return false; }
+    if (!scratch || per_expert == 0 || (w.rows / n_experts) % rows_per_block || ((uintptr_t) scratch % 1024) || scratch_bytes < per_expert) { return false; }
     const PrefillArgs a = batch_args(w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16, dst_col, n_experts);
-    const int fit = (int) std::min<size_t>((size_t) n_experts, scratch_bytes / per_expert);
+    const int fit = (int) std::min<size_t>((size_t) std::min(n_experts, TM_MAX_EXPERTS), scratch_bytes / per_expert);
     const int ranges = (n_experts + fit - 1) / fit, step = (n_experts + ranges - 1) / ranges; // ranges of equal size
     for (int e0 = 0; e0 < n_experts; e0 += step) {
         const int n = std::min(step, n_experts - e0);

@@ -179,3 +179,31 @@ def test_device_side_dispatch_on_one_rank(ops, layer):
         wts = torch.rand(T, TOPK, device="cuda")
         assert torch.equal(fmp(x, wts, ids), ops.moe_experts(x, enc_w["gate"], enc_w["up"], enc_w["down"], wts, ids, E))
     fmp.close()
+
+
+def test_more_experts_than_a_launch_lists(ops):
+    """1032 experts with a registered workspace: the two-pass form in two launches of the tensor-core pass."""
+    n, rows, T = 1032, 256, 64
+    bits = o.weights_like(rows * 8, 512, 5)
+    every = torch.from_numpy(bits.view(np.int16)).view(torch.bfloat16).repeat(n // 8, 1)   # expert e holds the rows of e % 8
+    w = ops.upload(*ops.encode(every, 3, 16, False), "cuda")
+    g = np.random.default_rng(3)
+    ids_np = np.stack([np.concatenate([[1031 - t % 8], g.choice(1020, 3, replace=False)]) for t in range(T)])
+    ids = torch.from_numpy(ids_np.astype(np.int32)).cuda()
+    a, a64 = act((T, 4, 512), 6)
+    need = ops.mm_ids_workspace_bytes(w)
+    buf = torch.zeros(need + 1024, dtype=torch.uint8, device="cuda")
+    ops.set_workspace(buf)
+    try:
+        y = ops.moe_mm_ids(a, ids, w, n).cpu().numpy()
+    finally:
+        ops.set_workspace(None)
+    off = (-buf.data_ptr()) % 1024
+    last = buf[off:off + need].view(n, -1)[1024:].any(dim=1).cpu().numpy()
+    assert last.all()      # the decode pass wrote the images of experts 1024 .. 1031: the call took the two-pass form
+    w64 = o.bf16_bits_to_f32(bits).astype(np.float64).reshape(8, rows, 512)
+    for t in range(T):
+        for s in range(4):
+            m = w64[ids_np[t, s] % 8]
+            assert (np.abs(y[t, s] - m @ a64[t, s]) <= MMA_REL * (np.abs(m) @ np.abs(a64[t, s]))).all(), (t, s)
+    assert ops.fault_status() == 0
