@@ -408,8 +408,8 @@ int bf16n_mm_ids_scratch(const bf16n_weight * w, const bf16n_weight * up, const 
         require(n_experts > 0 && w->rows % n_experts == 0, "rows must split evenly into experts");
         require(fo_mm_ids_supported(*w, up), "mm_ids_scratch: fragment-order experts only");
         fo_require_expert_count(up != nullptr, n_experts);
-        if (prefill_fo_two_pass(*w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16 != 0, dst_col, n_experts, scratch,
-                                scratch_bytes, (cudaStream_t) stream)) { return; }
+        if (prefill_fo_two_pass(*w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16 != 0, dst_col, n_experts,
+                                (int64_t) n_tok * n_used, scratch, scratch_bytes, (cudaStream_t) stream)) { return; }
         fo_mm_ids(*w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16 != 0, dst_col, n_experts, (cudaStream_t) stream);
     });
 }

@@ -175,7 +175,7 @@ void expand_tiles_fo(const bf16n_weight & w, const bf16n_weight * up, int n_expe
                      cudaStream_t st, bool behind_own);
 bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
                          const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
-                         void * scratch, size_t scratch_bytes, cudaStream_t st);
+                         int64_t n_pairs, void * scratch, size_t scratch_bytes, cudaStream_t st);
 void prefill_set_workspace(void * p, size_t bytes);
 size_t prefill_workspace_bytes(const bf16n_weight & w, const bf16n_weight * up);
 bool prefill_supported(const bf16n_weight & w, const bf16n_weight * up);

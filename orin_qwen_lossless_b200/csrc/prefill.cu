@@ -450,7 +450,8 @@ __host__ __device__ constexpr uint32_t tm_instr_desc() { return 1u << 4 | 1u << 
 static_assert(TM_G * TM_N <= TMEM_COLS, "accumulators of a pass must fit TMEM");
 
 // Which experts have more than l passes' worth of tokens, as bit masks, and their number, for l < TM_LEVELS (the last level
-// holds all the passes that are left of an expert). Lists experts without tokens nowhere, so no block draws an empty item.
+// holds all the passes that are left of an expert, dealt like the others). Lists experts without tokens nowhere, so no block
+// draws an empty item.
 constexpr int TM_LEVELS = 8, TM_MASK_WORDS = 32, TM_MAX_EXPERTS = 32 * TM_MASK_WORDS;
 struct TileLevels { uint32_t mask[TM_LEVELS][TM_MASK_WORDS]; int count[TM_LEVELS]; };
 
@@ -483,31 +484,51 @@ __device__ __forceinline__ void tm_helper_bar() { asm volatile("bar.sync 1, %0;"
 struct TileWalk {
     const TileLevels & lv;
     const int32_t * bounds;
-    int bpe, at, level;
-    int e, nb, jp, j1; // the pass: tokens [jp, min(jp + TM_G * M_TOK, j1)) of expert e, row block nb
+    int bpe, at, level, word;
+    uint32_t bits;     // last level: the experts of `word` not yet passed over
+    int e, nb, jp, j1; // the pass: tokens [jp, j1) of expert e, row block nb
 
-    __device__ __forceinline__ TileWalk(const TileLevels & l, const TileMmArgs & p) : lv(l), bounds(p.bounds), bpe(p.blocks_per_expert), at((int) blockIdx.x), level(0), e(0), nb(0), jp(0), j1(0) {}
+    __device__ __forceinline__ TileWalk(const TileLevels & l, const TileMmArgs & p)
+        : lv(l), bounds(p.bounds), bpe(p.blocks_per_expert), at((int) blockIdx.x), level(0), word(-1), bits(0u), e(0), nb(0), jp(0), j1(0) {}
+    __device__ __forceinline__ void pass(int l, int item_nb) {
+        nb = item_nb;
+        const int end = ld_act_s32(bounds + e + 1);
+        jp = ld_act_s32(bounds + e) + l * TM_G * M_TOK;
+        j1 = min(end, jp + TM_G * M_TOK);
+        at += gridDim.x;
+    }
     __device__ __forceinline__ bool next() {
-        if (jp + TM_G * M_TOK < j1) { jp += TM_G * M_TOK; return true; } // the last level: the expert's remaining passes
-        for (; level < TM_LEVELS; level++) {
+        for (; level < TM_LEVELS - 1; level++) {
             const int n = lv.count[level] * bpe;
-            if (at < n) { break; }
+            if (at < n) {
+                int r = at / bpe;
+                const int item_nb = at - r * bpe;
+                const uint32_t * m = lv.mask[level];
+                int w = 0;
+                for (int c; r >= (c = __popc(m[w])); w++) { r -= c; }
+                uint32_t b = m[w];
+                for (; r; r--) { b &= b - 1; }
+                e = 32 * w + __ffs(b) - 1;
+                pass(level, item_nb);
+                return true;
+            }
             at -= n;
         }
-        if (level == TM_LEVELS) { return false; }
-        int r = at / bpe;
-        nb = at - r * bpe;
-        const uint32_t * m = lv.mask[level];
-        int word = 0;
-        for (int c; r >= (c = __popc(m[word])); word++) { r -= c; }
-        uint32_t bits = m[word];
-        for (; r; r--) { bits &= bits - 1; }
-        e = 32 * word + __ffs(bits) - 1;
-        jp = ld_act_s32(bounds + e) + level * TM_G * M_TOK;
-        j1 = ld_act_s32(bounds + e + 1);
-        if (level + 1 < TM_LEVELS) { j1 = min(j1, jp + TM_G * M_TOK); }
-        at += gridDim.x;
-        return true;
+        if (lv.count[level] == 0) { return false; }
+        for (;; bits &= bits - 1) { // the last level: expert by expert, all the passes that are left of it
+            while (bits == 0u) {
+                if (++word == TM_MASK_WORDS) { word--; return false; }
+                bits = lv.mask[level][word];
+            }
+            e = 32 * word + __ffs(bits) - 1;
+            const int left = ld_act_s32(bounds + e + 1) - ld_act_s32(bounds + e) - level * TM_G * M_TOK;
+            const int n = (left + TM_G * M_TOK - 1) / (TM_G * M_TOK) * bpe;
+            if (at < n) {
+                pass(level + at / bpe, at % bpe);
+                return true;
+            }
+            at -= n;
+        }
     }
 };
 
@@ -528,13 +549,17 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_tile_mm(const TileMmArgs p) {
     grid_dependency_wait(); // images, routing and activations all come from earlier launches
     if (tid < TM_LEVELS) { levels.count[tid] = 0; }
     __syncthreads();
-    for (int i = warp; i < TM_LEVELS * TM_MASK_WORDS; i += TM_THREADS / 32) {
-        const int l = i / TM_MASK_WORDS, word = i - l * TM_MASK_WORDS, e = 32 * word + lane;
-        const bool in = e < p.n_experts && ld_act_s32(p.bounds + e + 1) - ld_act_s32(p.bounds + e) > l * TM_G * M_TOK;
-        const uint32_t m = __ballot_sync(FULL, in);
-        if (lane == 0) {
-            levels.mask[l][word] = m;
-            if (m) { atomicAdd(&levels.count[l], __popc(m)); }
+    for (int word = warp; word < TM_MASK_WORDS; word += TM_THREADS / 32) {
+        const int e = 32 * word + lane;
+        int n = 0;
+        if (e < p.n_experts) { n = ld_act_s32(p.bounds + e + 1) - ld_act_s32(p.bounds + e); }
+#pragma unroll
+        for (int l = 0; l < TM_LEVELS; l++) {
+            const uint32_t m = __ballot_sync(FULL, n > l * TM_G * M_TOK);
+            if (lane == 0) {
+                levels.mask[l][word] = m;
+                if (m) { atomicAdd(&levels.count[l], __popc(m)); }
+            }
         }
     }
     if (tid == 0) {
@@ -819,7 +844,7 @@ size_t prefill_workspace_bytes(const bf16n_weight & w, const bf16n_weight * up) 
 namespace {
 
 // tensor-core pass over decoded tiles: experts [0, n_experts) of `bounds` and `images`
-void tile_mm(const void * images, const PrefillArgs & a, const int32_t * bounds, int n_experts, int64_t K, bool glu, cudaStream_t st) {
+void tile_mm(const void * images, const PrefillArgs & a, const int32_t * bounds, int n_experts, int64_t K, bool glu, int64_t n_pairs, cudaStream_t st) {
     const int rows_per_block = glu ? TM_N / 2 : TM_N;
     TileMmArgs t = {};
     t.images = (const unsigned char *) images;
@@ -831,20 +856,23 @@ void tile_mm(const void * images, const PrefillArgs & a, const int32_t * bounds,
     t.n_experts = n_experts;
     t.blocks_per_expert = (int) (a.rows_per_expert / rows_per_block);
     t.ktiles = (int) (K / 64);
-    const unsigned grid = (unsigned) std::min<int64_t>(device_info().sms, (int64_t) n_experts * t.blocks_per_expert);
+    // a block for every pass that the call's pairs can make: a few experts with many pairs each still fill the machine
+    const int64_t passes = std::min<int64_t>(n_experts, n_pairs) + n_pairs / (TM_G * M_TOK);
+    const unsigned grid = (unsigned) std::min<int64_t>(device_info().sms, std::max<int64_t>(1, passes * t.blocks_per_expert));
     launch_chained(glu ? k_tile_mm<true> : k_tile_mm<false>, dim3(grid), dim3(TM_THREADS), TM_SMEM, st, t);
     check_launch();
 }
 
 // decode pass (expand_tiles.cu) + tensor-core pass over the decoded tiles
-bool two_pass(const bf16n_weight & w, const bf16n_weight * up, const PrefillArgs & a, int n_experts, cudaStream_t st) {
+bool two_pass(const bf16n_weight & w, const bf16n_weight * up, const PrefillArgs & a, int n_experts, int64_t n_pairs, cudaStream_t st) {
     const size_t need = prefill_workspace_bytes(w, up);
     const int rows_per_block = up ? TM_N / 2 : TM_N;
     if (need == 0 || need > g_workspace_bytes || a.rows_per_expert % rows_per_block || ((uintptr_t) g_workspace % 1024)) { return false; }
     expand_tiles(w, up, n_experts, a.bounds, g_workspace, st);
     const size_t per_expert = need / (size_t) n_experts;
     for (int e0 = 0; e0 < n_experts; e0 += TM_MAX_EXPERTS) { // the experts that a launch lists
-        tile_mm((const char *) g_workspace + e0 * per_expert, a, a.bounds + e0, std::min(TM_MAX_EXPERTS, n_experts - e0), w.K, up != nullptr, st);
+        tile_mm((const char *) g_workspace + e0 * per_expert, a, a.bounds + e0, std::min(TM_MAX_EXPERTS, n_experts - e0), w.K, up != nullptr,
+                n_pairs, st);
     }
     return true;
 }
@@ -870,7 +898,7 @@ PrefillArgs batch_args(const bf16n_weight & w, const bf16n_weight * up, const vo
 // scratch holds. False: the scratch holds no expert, or the rows are not whole row blocks (the fused kernel serves both).
 bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
                          const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
-                         void * scratch, size_t scratch_bytes, cudaStream_t st) {
+                         int64_t n_pairs, void * scratch, size_t scratch_bytes, cudaStream_t st) {
     const size_t per_expert = (size_t) (w.rows / n_experts) * (size_t) w.K * 2 * (up ? 2 : 1);
     const int64_t rows_per_block = up ? TM_N / 2 : TM_N;
     if (!scratch || per_expert == 0 || (w.rows / n_experts) % rows_per_block || ((uintptr_t) scratch % 1024) || scratch_bytes < per_expert) { return false; }
@@ -880,7 +908,7 @@ bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const 
     for (int e0 = 0; e0 < n_experts; e0 += step) {
         const int n = std::min(step, n_experts - e0);
         expand_tiles_fo(w, up, n_experts, e0, n, bounds + e0, scratch, st, e0 > 0); // behind the range before
-        tile_mm(scratch, a, bounds + e0, n, w.K, up != nullptr, st);
+        tile_mm(scratch, a, bounds + e0, n, w.K, up != nullptr, n_pairs, st);
     }
     return true;
 }
@@ -888,11 +916,10 @@ bool prefill_fo_two_pass(const bf16n_weight & w, const bf16n_weight * up, const 
 void prefill_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
                     const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,
                     int n_tok, int n_used, cudaStream_t st) {
-    (void) n_tok; (void) n_used;
     const PrefillArgs a = batch_args(w, up, x_bf16, x_row, ids_src1, ids_dst, bounds, dst, dst_bf16, dst_col, n_experts);
     const int rows_out = (up ? DEC_WARPS / 2 : DEC_WARPS) * w.R;
     require(a.rows_per_expert % rows_out == 0, "rows per expert must be a multiple of the batched kernel's row block");
-    if (g_workspace && two_pass(w, up, a, n_experts, st)) { return; }
+    if (g_workspace && two_pass(w, up, a, n_experts, (int64_t) n_tok * n_used, st)) { return; }
     const unsigned grid = (unsigned) std::min<int64_t>(device_info().sms, (int64_t) n_experts * (a.rows_per_expert / rows_out));
     if (up) {
         k_prefill<4, 8, true, true, G_TOK, SLOTS_GLU><<<grid, NTHREADS, smem_bytes<true, SLOTS_GLU>(), st>>>(a);
