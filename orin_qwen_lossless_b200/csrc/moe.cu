@@ -123,15 +123,18 @@ __global__ void __launch_bounds__(256) k_combine4(const float * __restrict__ ys,
 // ---------------------------------------------------------------- routing sort (prefill)
 
 // One block per expert. Pass 1 counts the routed pairs of lower-numbered experts (this expert's first output index);
-// pass 2 walks the tokens in order, 1024 at a time (latency bound: a step is two block barriers and a trip to L2), and compacts the tokens that use this expert with a block-wide
-// exclusive scan, so the expert's pairs come out sorted by token.
-constexpr int ROUTE_THREADS = 1024, ROUTE_WARPS = ROUTE_THREADS / 32;
-template <typename TI>
-__global__ void __launch_bounds__(ROUTE_THREADS) k_route(const TI * __restrict__ ids, int64_t row_stride, int32_t * __restrict__ ids_src1,
-                                               int32_t * __restrict__ ids_dst, int32_t * __restrict__ bounds, int n_tok, int n_used,
-                                               int nchannels_y, int sis1) {
+// pass 2 walks the tokens in order, THREADS at a time (latency bound: a step is two block barriers and a trip to L2), and
+// compacts the tokens that use this expert with a block-wide exclusive scan, so the expert's pairs come out sorted by token.
+// Blocks of 1024 threads take fewer steps where every block has an SM to itself and the tokens are many; otherwise they only
+// start later and share SMs. 256 / 1024 threads in us, eight slots per token: 64 experts 2.4 / 3.4 at 64 tokens, 4.1 / 4.1 at
+// 1024, 25.1 / 17.0 at 8192; 160 experts 4.7 / 5.8 at 1024, 27.0 / 28.7 at 8192; 512 experts 33.9 / 52.3 at 8192.
+template <int THREADS, typename TI>
+__global__ void __launch_bounds__(THREADS) k_route(const TI * __restrict__ ids, int64_t row_stride, int32_t * __restrict__ ids_src1,
+                                                   int32_t * __restrict__ ids_dst, int32_t * __restrict__ bounds, int n_tok, int n_used,
+                                                   int nchannels_y, int sis1) {
+    constexpr int WARPS = THREADS / 32;
     const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    __shared__ int warp_tot[ROUTE_WARPS];
+    __shared__ int warp_tot[WARPS];
     __shared__ int s_base;
 
     // int32 ids in contiguous rows of a multiple of four: four ids per load (the common case: 8 slots per token)
@@ -139,12 +142,12 @@ __global__ void __launch_bounds__(ROUTE_THREADS) k_route(const TI * __restrict__
     int lower = 0;
     if (vec) {
         const int4 * v = (const int4 *) ids;
-        for (int64_t i = tid; i < (int64_t) n_tok * n_used / 4; i += ROUTE_THREADS) {
+        for (int64_t i = tid; i < (int64_t) n_tok * n_used / 4; i += THREADS) {
             const int4 q = __ldg(v + i);
             lower += (q.x < e) + (q.y < e) + (q.z < e) + (q.w < e);
         }
     } else {
-        for (int64_t i = tid; i < (int64_t) n_tok * n_used; i += ROUTE_THREADS) {
+        for (int64_t i = tid; i < (int64_t) n_tok * n_used; i += THREADS) {
             const int t = (int) (i / n_used), s = (int) (i - (int64_t) t * n_used);
             lower += (int) ids[t * row_stride + s] < e;
         }
@@ -155,13 +158,13 @@ __global__ void __launch_bounds__(ROUTE_THREADS) k_route(const TI * __restrict__
     __syncthreads();
     if (tid == 0) {
         int b = 0;
-        for (int i = 0; i < ROUTE_WARPS; i++) { b += warp_tot[i]; }
+        for (int i = 0; i < WARPS; i++) { b += warp_tot[i]; }
         s_base = b;
     }
     __syncthreads();
     const int base = s_base;
     int done = 0;
-    for (int t0 = 0; t0 < n_tok; t0 += ROUTE_THREADS) {
+    for (int t0 = 0; t0 < n_tok; t0 += THREADS) {
         const int t = t0 + tid;
         int slot = -1;
         if (t < n_tok) {
@@ -185,7 +188,7 @@ __global__ void __launch_bounds__(ROUTE_THREADS) k_route(const TI * __restrict__
         if (lane == 0) { warp_tot[warp] = __popc(hit); }
         __syncthreads();
         int before = 0, total = 0;
-        for (int i = 0; i < ROUTE_WARPS; i++) {
+        for (int i = 0; i < WARPS; i++) {
             before += i < warp ? warp_tot[i] : 0;
             total += warp_tot[i];
         }
@@ -244,12 +247,13 @@ void moe_route(const void * ids, bool ids_i64, int64_t ids_row_stride, int32_t *
     require(n_tok > 0 && n_tok < (1 << 22) && n_used > 0 && n_used < (1 << 10), "routing sizes out of range");
     require(n_experts > 0, "routing needs at least one expert");
     require((int64_t) n_tok * ids_row_stride < INT32_MAX, "routing ids too large for 32-bit indexing");
+    const bool wide = n_experts <= device_info().sms && n_tok >= 1024;
     if (ids_i64) {
-        k_route<int64_t><<<n_experts, ROUTE_THREADS, 0, st>>>((const int64_t *) ids, ids_row_stride, ids_src1, ids_dst, bounds, n_tok, n_used,
-                                                    nchannels_y, sis1);
+        const auto kernel = wide ? k_route<1024, int64_t> : k_route<256, int64_t>;
+        kernel<<<n_experts, wide ? 1024 : 256, 0, st>>>((const int64_t *) ids, ids_row_stride, ids_src1, ids_dst, bounds, n_tok, n_used, nchannels_y, sis1);
     } else {
-        k_route<int32_t><<<n_experts, ROUTE_THREADS, 0, st>>>((const int32_t *) ids, ids_row_stride, ids_src1, ids_dst, bounds, n_tok, n_used,
-                                                    nchannels_y, sis1);
+        const auto kernel = wide ? k_route<1024, int32_t> : k_route<256, int32_t>;
+        kernel<<<n_experts, wide ? 1024 : 256, 0, st>>>((const int32_t *) ids, ids_row_stride, ids_src1, ids_dst, bounds, n_tok, n_used, nchannels_y, sis1);
     }
     check_launch();
 }
