@@ -894,8 +894,10 @@ void gather_rows(const bf16n_weight & w, const void * ids, int64_t ids_s0, int64
     if (w.format == FMT_NIBBLE) {
         if (dst_bf16) { k_nib_rows<true><<<gx, 256, 0, st>>>(nib_view(w), C, ip, ids_s0, n, row0, dp, dst_s1); }
         else { k_nib_rows<false><<<gx, 256, 0, st>>>(nib_view(w), C, ip, ids_s0, n, row0, dp, dst_s1); }
-    } else if (n <= (int64_t) device_info().sms * 4) {
-        // few rows: spread over the SMs, at most two to a block (k_pair_rows: eight)
+    } else if (n <= (int64_t) device_info().sms * 4 && w.R * C >= 32) {
+        // Few rows: spread over the SMs, at most two to a block (k_pair_rows: eight). Units of fewer than 32 chunks have little to
+        // pass over, and the skip table costs more than it saves. General / staged in us, 64 rows: R * C = 1: 2.9 / 6.0,
+        // 4: 4.1 / 6.8, 8: 6.2 / 8.0, 16: 10.3 / 9.5 (256 rows: 10.5 / 11.4), 32: 19.4 / 13.3.
         const int per = n > device_info().sms * 2 ? 2 : 1;
         const uint32_t cap = (uint32_t) ((w.R * w.K * 3 / 8 + 64 + 15) & ~15ll);
         const size_t shm = 6 * HP_MAX_PAIRS + 128 + (size_t) per * cap;

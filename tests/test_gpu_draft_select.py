@@ -69,7 +69,7 @@ def test_candidates_and_scores(ops, rows, T, n_cand):
             assert (np.abs(out[t, want] - wr @ x64) <= GEMV_REL * (np.abs(wr) @ np.abs(x64))).all(), (kind, t)
 
 
-@pytest.mark.parametrize("K, R", [(512, 1), (512, 16), (1024, 2), (2048, 16), (4096, 16)])
+@pytest.mark.parametrize("K, R", [(512, 1), (512, 16), (1024, 2), (1024, 16), (2048, 4), (2048, 8), (2048, 16), (4096, 16)])
 @pytest.mark.parametrize("n", [1, 300])
 def test_rows_of_every_position_in_a_unit(ops, K, R, n):
     rows = 16 * 20
