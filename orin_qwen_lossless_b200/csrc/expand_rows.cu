@@ -2,7 +2,8 @@
 // reader of the large-matrix decode GEMV: one unit per warp, streams through per-lane cp.async rings, plane bytes four
 // steps ahead. What bounds it depends on the matrix: one with a few hundred units (8192 x 2048, R = 16: 512) is one chain
 // of R K / 64 dependent table lookups per lane, and reading the streams and the plane lane by lane from global memory
-// inside that chain (k_pair_expand) more than doubled it (8192 x 2048: 78 us, here 30); a matrix with many units is bound by HBM and the table's bank conflicts.
+// inside that chain (k_pair_expand) more than doubled it (8192 x 2048: 71 us, here 26, warm); a matrix with many units is bound by
+// HBM and the table's bank conflicts.
 // Units are dealt over the blocks first and the warps of a block second, so that few units reach every SM.
 #include "launch.h"
 #include "rings.cuh"
@@ -89,7 +90,17 @@ void expand_rows_init() {
     allow_dynamic_smem((const void *) k_expand_rows<CompareBF16>, (int) ROW_SMEM, optin, "expand rows");
 }
 
-bool expand_rows_applies(const bf16n_weight & w) { return w.format == FMT_HUFPAIR && !w.fo && (w.R * (w.K / CHUNK)) % AHEAD == 0; }
+// Opening a unit costs the rings a trip to memory that only the unit's own steps hide, and 28 warps per SM hide less of it than
+// the general kernel's 64; so short units take the rings only while the call has few of them. General / rings in us by steps
+// of 512 weights to a unit and units of the call: 4 steps: 4.8 / 4.5 for 256 units, 5.8 / 5.6 for 1024, 5.9 / 6.9 for 2048,
+// 44 / 63 for 32768; 8 steps: 12.4 / 9.1 for 2048, 14.7 / 14.1 for 4096, 23.2 / 24.3 for 8192, 84.5 / 95.7 for 32768; 16 steps: 20.9 / 12.7
+// for 2048, 46.3 / 48.0 for 8192, 95.1 / 90.7 for 16384; 32 steps: 27.8 / 16.1 for 1024, 58.5 / 44.6 for 4096, 218 / 177 for 16384.
+bool expand_rows_applies(const bf16n_weight & w, int64_t nrows) {
+    const int64_t steps = w.R * (w.K / CHUNK);
+    if (w.format != FMT_HUFPAIR || w.fo || steps % AHEAD) { return false; }
+    const int64_t units = nrows / w.R, round = (int64_t) ROW_WARPS * device_info().sms;
+    return steps >= 32 || units <= (steps == 4 ? round / 4 : round) || (steps == 16 && units >= 3 * round);
+}
 
 void expand_rows(const bf16n_weight & w, int64_t row0, int64_t nrows, const StoreBF16 & sink, cudaStream_t st) { launch(w, row0, nrows, sink, st); }
 void expand_rows(const bf16n_weight & w, int64_t row0, int64_t nrows, const CompareBF16 & sink, cudaStream_t st) { launch(w, row0, nrows, sink, st); }

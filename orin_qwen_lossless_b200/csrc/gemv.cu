@@ -733,9 +733,9 @@ void launch_expand(const bf16n_weight & w, int64_t row0, int64_t nrows, const Si
     const unsigned gx = (unsigned) std::max<int64_t>(1, std::min<int64_t>((work + 7) / 8, (int64_t) device_info().sms * 16));
     if (w.format == FMT_NIBBLE) {
         k_nib_expand<Sink><<<gx, 256, 0, st>>>(nib_view(w), C, row0, nrows, sink);
-    } else if (expand_rows_applies(w)) {
+    } else if (expand_rows_applies(w, nrows)) {
         expand_rows(w, row0, nrows, sink, st);
-    } else if (w.format == FMT_HUFPAIR) { // fewer than four steps of 512 weights to a unit (R = 1 or 2, short rows)
+    } else if (w.format == FMT_HUFPAIR) { // short units, or fewer than four steps of 512 weights to one
         k_pair_expand<Sink><<<gx, 256, 0, st>>>(pair_view(w), C, w.R, w.cm != 0, row0, nrows, sink);
     } else {
         k_huf_expand<Sink><<<gx, 256, 0, st>>>(huf_view(w), C, w.R, row0, nrows, sink);

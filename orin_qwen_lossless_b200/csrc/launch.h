@@ -68,7 +68,7 @@ __device__ __forceinline__ void grid_dependency_wait() {
 // expand_rows.cu: exact reconstruction of lane-major HUFPAIR matrices
 namespace dev { struct StoreBF16; struct CompareBF16; }
 void expand_rows_init();
-bool expand_rows_applies(const bf16n_weight & w);
+bool expand_rows_applies(const bf16n_weight & w, int64_t nrows);
 void expand_rows(const bf16n_weight & w, int64_t row0, int64_t nrows, const dev::StoreBF16 & sink, cudaStream_t st);
 void expand_rows(const bf16n_weight & w, int64_t row0, int64_t nrows, const dev::CompareBF16 & sink, cudaStream_t st);
 

@@ -13,6 +13,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("rows, K, R, cm", [
     (16, 512, 16, False), (3, 512, 1, False), (8, 512, 4, False), (6, 1024, 2, False), (5, 2048, 1, False), (34, 2048, 2, False),
     (640, 2048, 16, False), (48, 4096, 16, False), (40, 2048, 8, True), (24, 1024, 4, True), (32768, 512, 4, False),
+    (33200, 512, 8, False), (66560, 1024, 16, False), (8320, 1024, 2, False),
 ])
 def test_reconstruction_is_exact(rows, K, R, cm):
     from orin_qwen_lossless_b200 import ops
