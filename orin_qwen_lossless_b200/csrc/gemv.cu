@@ -273,20 +273,31 @@ __device__ __forceinline__ void nib_load(NibRow<C> & d, const NibView & w, int64
     d.rec = d.e0 + lane < d.e1 ? __ldg(w.esc + d.e0 + lane) : 0u;
 }
 
-// the row's BF16 pairs (escaped slots decode to +0), ready before the activations are
-template <int C>
-struct NibWords { uint32_t w[C][8]; uint32_t e0, e1, rec; };
-
-template <int C>
-__device__ __forceinline__ void nib_decode(const NibRow<C> & r, NibWords<C> & d) {
+// the row's BF16 pairs (escaped slots decode to +0), ready before the activations are. Rows of 4096 columns stay as loaded and are
+// decoded chunk by chunk as they are used: 64 registers of words would cost a block per SM (three products of 2048 rows, one
+// token: 10.8 us, decoded ahead 13.2).
+template <int C, bool AHEAD = (C < 8)>
+struct NibWords {
+    uint32_t w[C][8]; uint32_t e0, e1, rec;
+    __device__ __forceinline__ void set(const NibRow<C> & r) {
 #pragma unroll
-    for (int c = 0; c < C; c++) {
-        nib_assemble8(r.sm[c], r.cd[c], r.L, d.w[c]);
+        for (int c = 0; c < C; c++) {
+            nib_assemble8(r.sm[c], r.cd[c], r.L, w[c]);
 #pragma unroll
-        for (int q = 0; q < 8; q++) { asm volatile("" : "+r"(d.w[c][q])); } // decoded here, not where they are used
+            for (int q = 0; q < 8; q++) { asm volatile("" : "+r"(w[c][q])); } // decoded here, not where they are used
+        }
+        e0 = r.e0; e1 = r.e1; rec = r.rec;
     }
-    d.e0 = r.e0; d.e1 = r.e1; d.rec = r.rec;
-}
+    __device__ __forceinline__ void chunk(int c, uint32_t (&out)[8]) const {
+#pragma unroll
+        for (int q = 0; q < 8; q++) { out[q] = w[c][q]; }
+    }
+};
+template <int C>
+struct NibWords<C, false> : NibRow<C> {
+    __device__ __forceinline__ void set(const NibRow<C> & r) { (NibRow<C> &) *this = r; }
+    __device__ __forceinline__ void chunk(int c, uint32_t (&out)[8]) const { nib_assemble8(this->sm[c], this->cd[c], this->L, out); }
+};
 
 // four activations as they lie in memory
 template <typename TX> struct RawX4;
@@ -305,7 +316,7 @@ template <> struct RawX4<bf16> {
 // chunks are requested before the first of them is used: one trip to L2, not one per chunk.
 template <int C, int M, typename TX>
 __device__ __forceinline__ void nib_dots(const NibWords<C> (&d)[M], const NibView * const (&w)[M], const TX * x, int lane, float (&sum)[M]) {
-    constexpr int G = C < 4 ? C : 4;
+    constexpr int G = C < 4 ? C : C == 4 ? 4 : 1;
     float a[M][4];
 #pragma unroll
     for (int m = 0; m < M; m++) { a[m][0] = a[m][1] = a[m][2] = a[m][3] = 0.f; }
@@ -318,7 +329,11 @@ __device__ __forceinline__ void nib_dots(const NibWords<C> (&d)[M], const NibVie
         for (int c = 0; c < G; c++) {
             const float4 xq[4] = {q[4 * c].f(), q[4 * c + 1].f(), q[4 * c + 2].f(), q[4 * c + 3].f()};
 #pragma unroll
-            for (int m = 0; m < M; m++) { fma_chunk(d[m].w[c0 + c], xq, a[m]); }
+            for (int m = 0; m < M; m++) {
+                uint32_t wv[8];
+                d[m].chunk(c0 + c, wv);
+                fma_chunk(wv, xq, a[m]);
+            }
         }
     }
 #pragma unroll
@@ -343,9 +358,11 @@ __device__ __forceinline__ void nib_dots(const NibWords<C> (&d)[M], const NibVie
 // Behind the wait are one trip to L2 for the activations (one per chunk, and two for a gate/up pair, before), the products and the
 // sums. 48 layers of three launches each: 460 -> 349 us; 20 layers at 2 / 4 tokens: 237 / 337 -> 188 / 256 us. Measured and left:
 // activations staged in shared memory once per block, its rows multiplied with up to four columns (359 us; 225 / 360).
-constexpr int nib_blocks(int C, bool glu) { return glu ? (C <= 2 ? 3 : C == 4 ? 2 : 1) : C == 8 ? 2 : C == 4 ? 3 : 4; } // per SM: room for the launches behind
+constexpr int nib_blocks(int C, bool glu, int x_bytes) { // per SM: room for the launches behind, and as many as the registers of a row allow
+    return glu ? (C == 1 ? 4 : C == 2 ? 3 : C == 4 ? 2 : 1) : C == 8 ? (x_bytes == 2 ? 3 : 2) : C == 4 ? 3 : C == 2 ? 5 : 6;
+}
 template <int C, typename TX, bool GLU>
-__global__ void __launch_bounds__(256, nib_blocks(C, GLU)) k_nib_gemv(const NibView g, const NibView v, Cols p) {
+__global__ void __launch_bounds__(256, nib_blocks(C, GLU, sizeof(TX))) k_nib_gemv(const NibView g, const NibView v, Cols p) {
     constexpr int M = GLU ? 2 : 1;
     bool waited = p.ids != nullptr; // expert ids, when there are any, belong to an earlier kernel too
     if (waited) { grid_dependency_wait(); } else { grid_launch_dependents(); }
@@ -362,7 +379,7 @@ __global__ void __launch_bounds__(256, nib_blocks(C, GLU)) k_nib_gemv(const NibV
 #pragma unroll
             for (int m = 0; m < M; m++) { nib_load<C>(row[m], *w[m], rbase + r, lane); }
 #pragma unroll
-            for (int m = 0; m < M; m++) { nib_decode<C>(row[m], d[m]); }
+            for (int m = 0; m < M; m++) { d[m].set(row[m]); }
         }
         if (!waited) { grid_dependency_wait(); waited = true; }
         float s[M];
@@ -799,7 +816,7 @@ __device__ __forceinline__ void nib_item_rows(const NibItem & it, int block, int
         {
             NibRow<C> row;
             nib_load<C>(row, it.v, it.row0 + r, lane);
-            nib_decode<C>(row, d[0]);
+            d[0].set(row);
         }
         if (!waited) { grid_dependency_wait(); waited = true; } // weights first, then the activations an earlier kernel may have written
         float s[1];
@@ -811,10 +828,9 @@ __device__ __forceinline__ void nib_item_rows(const NibItem & it, int block, int
 
 // Every block belongs to one item of the group (a prefix table of block ranges); within its item it is a block of the
 // single-product kernel: same loads, same order of operations, so the results are the same bits. WIDE adds rows of 4096
-// columns and the registers for them; without, three blocks fit an SM and the 352 blocks of a layer's three products are
-// resident at once (two left a second wave).
+// columns. Three blocks fit an SM, and the 352 blocks of a layer's three products are resident at once (two left a second wave).
 template <bool WIDE>
-__global__ void __launch_bounds__(256, WIDE ? 1 : 3) k_nib_gemv_group(const NibGroup g) {
+__global__ void __launch_bounds__(256, 3) k_nib_gemv_group(const NibGroup g) {
     grid_launch_dependents(); // as in k_nib_gemv
     int m = 0;
     while (m + 1 < g.n && (int) blockIdx.x >= g.item[m + 1].first_block) { m++; }
