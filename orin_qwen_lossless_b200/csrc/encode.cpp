@@ -199,7 +199,12 @@ Bytes encode_nibble(const uint16_t * w, int64_t rows, int64_t K, uint8_t * plane
     h.off_b = h.off_a + (uint64_t) rows * K / 2;
     h.off_c = h.off_b + (uint64_t) rows * 16;
     h.off_d = h.off_c + (uint64_t) (rows + 1) * 4;
-    std::vector<uint8_t> head(h.off_d, 0); // everything but the escape list, whose size is known last
+    // Everything is written in place. The escape list's size is known last: there is room behind for one weight in 64 (more,
+    // and the buffer moves once).
+    Bytes aux;
+    aux.reserve(h.off_d + (uint64_t) rows * K / 16 + 4);
+    aux.resize(h.off_d);
+    memset(aux.data(), 0, HEADER_BYTES);
     parallel_ranges(nblk, 1, [&](int64_t b0, int64_t b1, int) {
         for (int64_t b = b0; b < b1; b++) {
             for (int64_t r = b * BLK; r < std::min(rows, (b + 1) * BLK); r++) {
@@ -213,14 +218,15 @@ Bytes encode_nibble(const uint16_t * w, int64_t rows, int64_t K, uint8_t * plane
                 int code_of[256];
                 std::fill(code_of, code_of + 256, -1);
                 code_of[0] = 0;
-                uint8_t * tab = head.data() + h.off_b + r * 16;
+                uint8_t * tab = aux.data() + h.off_b + r * 16;
+                memset(tab, 0, 16);
                 for (int i = 0, n = 1; i < 127 && n < 16 && hist[order[i]] > 0; i++, n++) {
                     tab[n] = (uint8_t) order[i];
                     code_of[order[i]] = n;
                 }
                 uint32_t n_esc = 0;
                 for (int64_t c = 0; c < C; c++) {
-                    uint8_t * codes = head.data() + h.off_a + (r * C + c) * 256;
+                    uint8_t * codes = aux.data() + h.off_a + (r * C + c) * 256;
                     uint8_t * pl = plane + r * K + c * CHUNK;
                     for (int l = 0; l < 32; l++) {
                         uint64_t packed = 0;
@@ -247,8 +253,8 @@ Bytes encode_nibble(const uint16_t * w, int64_t rows, int64_t K, uint8_t * plane
     });
     for (int64_t r = 0; r < rows; r++) { esc_off[r + 1] += esc_off[r]; }
     h.n_a = esc_off[rows];
-    Bytes aux(h.off_d + std::max<uint64_t>(h.n_a, 1) * 4, 0);
-    memcpy(aux.data(), head.data(), head.size());
+    aux.resize(h.off_d + std::max<uint64_t>(h.n_a, 1) * 4);
+    if (h.n_a == 0) { memset(aux.data() + h.off_d, 0, 4); }
     memcpy(aux.data(), &h, sizeof h);
     put_at(aux, h.off_c, esc_off.data(), esc_off.size());
     uint64_t o = h.off_d;
