@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(256) k_int4_gemv(const bf16 * __restrict__ x, 
                                                    int64_t rows, float * __restrict__ y) {
     constexpr int K = NIT * 1024;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    grid_launch_dependents();
+    grid_dependency_wait(); // at once: launched behind everything older
     __half2 xr[T][NIT][16];
 #pragma unroll
     for (int t = 0; t < T; t++) {
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(256, NC == 1 ? 2 : 1) k_int2_gemv(const bf16 *
                                                                       const float * __restrict__ s, int64_t rows, float * __restrict__ y, const FieldShift k) {
     constexpr int K = 2048, AHEAD = 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    grid_launch_dependents();
+    grid_dependency_wait(); // at once: launched behind everything older
     const int64_t stride = (int64_t) gridDim.x * 8;
     int64_t r = blockIdx.x * 8 + warp;
     uint4 v[AHEAD]; float sc[AHEAD];

@@ -51,3 +51,12 @@ def test_ordered_loads(name):
 def test_pass_walk_of_the_tile_product():
     s = SOURCES["prefill.cu"]
     assert "__ldg" not in _block(s, s.index("struct TileWalk"))
+
+
+def test_kernels_that_let_their_successor_start_wait_themselves():
+    for f, s in SOURCES.items():
+        for m in re.finditer(r"__global__[^;{]*?\b(k_\w+)\([^{;]*\)\s*\{", s):
+            body = _block(s, m.end() - 1)
+            if "grid_launch_dependents()" in body:
+                waits = "grid_dependency_wait()" in body or any("grid_dependency_wait()" in _block(s, s.index(h)) for h in ("nib_item_rows(",) if h in body)
+                assert waits, f"{m.group(1)} in {f}"
