@@ -662,10 +662,10 @@ def _mm_ids_scratch(cw, cu, n_experts: int, T: int, n_used: int, device) -> torc
     """Memory (up to 1 GiB) for the decoded tiles of one batched call on fragment-order experts, from torch's allocator and
     back to it when the call has been enqueued; None where the fused kernel is the faster one, under stream capture (a
     graph would keep the memory) and when the memory is not to be had. Both forms give the same bits."""
-    if torch.cuda.is_current_stream_capturing():
-        return None
     need = lib().bf16n_mm_ids_scratch_bytes(C.byref(cw), C.byref(cu) if cu is not None else None, n_experts, T, n_used)
-    if need == 0 or time.monotonic() - _scratch_refused.get(device.index, -_SCRATCH_RETRY_S) < _SCRATCH_RETRY_S:
+    if need == 0 or torch.cuda.is_current_stream_capturing():
+        return None
+    if time.monotonic() - _scratch_refused.get(device.index, -_SCRATCH_RETRY_S) < _SCRATCH_RETRY_S:
         return None
     try:
         return torch.empty(need + 1024, dtype=torch.uint8, device=device)
