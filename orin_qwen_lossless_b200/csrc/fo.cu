@@ -17,6 +17,8 @@
 #include <type_traits>
 #include "launch.h"
 
+#include <cmath>
+
 namespace b16 {
 namespace {
 
@@ -1011,26 +1013,46 @@ void fo_require_expert_count(bool glu, int n_experts) {
 
 // Scratch of the two-pass form (prefill_fo_two_pass), 0 where the fused kernel is taken. The fused kernel decodes an
 // expert once per 96 of its tokens on 16 warps per SM, the two-pass form once on 26, but sends the weights through memory as
-// BF16 (two bytes written and read per weight). Measured, fused / two-pass in us, at 16, 64, 80, 96 and 256 pairs per expert:
-//   gate/up + SwiGLU (512 x 2048), 256 experts: 609 / 593, 643 / 602, 743 / 602, 1017 / 605, 1950 / 959
-//                                   16 experts:  93 / 72,   97 / 73,   99 / 72,   99 / 74,  184 / 123
-//   down (2048 x 512), 256 experts:             304 / 309, 357 / 330, 395 / 334, 548 / 336, 1119 / 529
-//                       16 experts:              28 / 37,   32 / 40,   33 / 39,   56 / 39,   83 / 57
-// hence the two lines; a call with few pairs per expert is left alone although a pair of matrices would gain a little.
+// BF16 (two bytes written and read per weight) in two launches. Which is faster depends on how many waves of work items either
+// makes on the machine, so the rule estimates both, in us: a wave of the fused kernel (an item is 256 rows, or 128 of a gate/up
+// pair, by 96 tokens) takes 7 + 20.5 per 512 columns; a round of the decode pass (one unit per warp) 20; a wave of the tensor-core
+// pass (256 rows by up to 256 tokens) 3 + 5 per 512 columns while an expert's tokens fit one group of 128, else 8 + 9; 3 for the
+// second launch. Tokens of an expert are taken as spread by a binomial deviation around the mean. Fitted to 750 measured pairs
+// (10 shapes of K 512 .. 4096 and 256 .. 2048 rows per expert, 1 .. 256 experts, 16 .. 8192 pairs per expert): where the rule
+// takes one form, the other is never more than 3% faster. Some of them, fused / two-pass:
+//   gate/up 512 x 2048, 256 experts, 16 / 64 / 256 pairs each: 609 / 593, 643 / 602, 1950 / 959; 16 experts, 16: 93 / 72
+//   2048 x 512, 256 experts, 16 / 80 / 256: 304 / 309, 395 / 334, 1119 / 529; 1 expert, 256: 27 / 40; 4 experts, 4096: 258 / 105
+//   512 x 512, 64 experts, 16 (gate/up): 50 / 57; 1024 x 256 (K = 1024), 1 expert, 1024: 46 / 50
+// A call with few pairs per expert is left alone although a long row would gain.
 // At most 1 GiB (256 experts of the gate/up pair at a time, twice the call's own FP32 outputs at 8192 tokens): every range
 // ends with partly empty waves of both passes (gate/up of 256 experts in 1, 2, 4, 16 ranges: 541 / 602 / 664 / 1156 us at
 // 64 pairs per expert, 855 / 957 / 1041 / 1939 at 256), which images that stay in L2 do not make up for.
 constexpr int64_t FO_TWO_PASS_GLU = 16, FO_TWO_PASS_ONE = 80; // routed pairs per expert
 constexpr size_t FO_SCRATCH_MAX = (size_t) 1 << 30;
 
+static bool fo_two_pass_pays(int64_t rows_per_expert, int64_t K, bool glu, int n_experts, int n_range, int n_tok, int n_used) {
+    const double sms = device_info().sms ? device_info().sms : 148, C = (double) (K / CHUNK);
+    const double per = (double) n_tok * n_used / n_experts, dev = std::sqrt(per * std::max(0.0, 1.0 - (double) n_used / n_experts));
+    const double blocks = (double) rows_per_expert / (glu ? 128 : 256); // row blocks of an expert, in both forms
+    auto tiles = [&](double tokens) { return 0.5 * (std::ceil(std::max(per - dev, 1.0) / tokens) + std::ceil((per + dev) / tokens)); };
+    auto waves = [&](double items, double slots) { return std::max(1.0, std::ceil(items / slots)); };
+    const double fused = (7.0 + 20.5 * C) * waves(n_experts * blocks * tiles(96.0), sms);
+    const double decode = 20.0 * waves((double) n_range * (rows_per_expert / BAND) * C, std::floor(sms / (glu ? 2 : 1)) * 26.0);
+    const double multiply = (per + dev <= 128.0 ? 3.0 + 5.0 * C : 8.0 + 9.0 * C) * waves(n_range * blocks * tiles(256.0), sms);
+    return (decode + multiply + 3.0) * std::ceil((double) n_experts / n_range) < fused;
+}
+
 size_t fo_mm_ids_scratch_bytes(const bf16n_weight & w, const bf16n_weight * up, int n_experts, int n_tok, int n_used) {
-    const size_t per_expert = (size_t) (w.rows / n_experts) * (size_t) w.K * 2 * (up ? 2 : 1);
-    if ((w.rows / n_experts) % (up ? 128 : 256) || per_expert > FO_SCRATCH_MAX) { return 0; }
+    const int64_t rows_per_expert = w.rows / n_experts;
+    const size_t per_expert = (size_t) rows_per_expert * (size_t) w.K * 2 * (up ? 2 : 1);
+    if (rows_per_expert % (up ? 128 : 256) || per_expert > FO_SCRATCH_MAX) { return 0; }
     // a call with more experts than the fused kernel lists is refused (fo_require_expert_count); 227 KB where no device is known
     const int optin = device_info().smem_optin;
     if (fo_mm_shm(up != nullptr, n_experts) > (size_t) (optin ? optin : 227 * 1024)) { return 0; }
     if ((int64_t) n_tok * n_used < (up ? FO_TWO_PASS_GLU : FO_TWO_PASS_ONE) * n_experts) { return 0; }
-    return per_expert * std::min<size_t>((size_t) n_experts, FO_SCRATCH_MAX / per_expert);
+    const int n_range = (int) std::min<size_t>((size_t) n_experts, FO_SCRATCH_MAX / per_expert);
+    if (!fo_two_pass_pays(rows_per_expert, w.K, up != nullptr, n_experts, n_range, n_tok, n_used)) { return 0; }
+    return per_expert * (size_t) n_range;
 }
 
 void fo_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,

@@ -1,10 +1,12 @@
 """bf16n_mm_ids_scratch_bytes answers 0 for every call that has no use for scratch: an empty matrix, experts that do not split
 evenly or are more than a call takes, an up matrix of another shape or layout. Run in a process of its own: a wrong answer here
 was once an arithmetic trap."""
+import ctypes as C
 import os
 import subprocess
 import sys
 
+import pytest
 import torch
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -46,3 +48,18 @@ def test_a_refusal_is_not_repeated_for_every_call(monkeypatch):
         now[0] = t
         assert ops._mm_ids_scratch(w, w, 8, 8192, 8, torch.device("cuda", device)) is None
     assert asked == [0, 1, 0]
+
+
+@pytest.mark.parametrize("glu, K, rows, experts, pairs, two_pass", [
+    (True, 2048, 512, 256, 16, True), (True, 2048, 512, 256, 256, True), (True, 2048, 512, 16, 16, True), (True, 2048, 512, 1, 4096, True),
+    (False, 512, 2048, 256, 80, True), (False, 512, 2048, 256, 64, False), (False, 512, 2048, 4, 4096, True),
+    (False, 512, 2048, 1, 256, False), (False, 512, 512, 128, 80, False), (True, 512, 512, 64, 16, False),
+    (True, 1024, 1024, 16, 32, False), (False, 1024, 256, 1, 1024, False), (True, 3072, 256, 64, 64, True),
+])
+def test_the_form_that_was_measured_faster(glu, K, rows, experts, pairs, two_pass):
+    """Shapes on both sides of the rule between the fused kernel and the two-pass form (which alone asks for scratch)."""
+    from orin_qwen_lossless_b200 import _lib
+    w = _lib.Weight(4096, 8192, 3, 16, K, experts * rows, 0, 1, 256, 16640, 20000, 30000)
+    used = min(8, experts)
+    need = _lib.lib().bf16n_mm_ids_scratch_bytes(C.byref(w), C.byref(w) if glu else None, experts, experts * pairs // used, used)
+    assert (need > 0) == two_pass
