@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(256) k_huf_gemv(const HufView g, const HufView
 template <int C>
 struct NibRow { uint4 sm[C]; uint2 cd[C]; uint4 L; uint32_t e0, e1, rec; }; // rec: this lane's first escape record
 
-template <int C>
+template <int C, bool RECORDS>
 __device__ __forceinline__ void nib_load(NibRow<C> & d, const NibView & w, int64_t row, int lane) {
     constexpr int K = C * CHUNK;
 #pragma unroll
@@ -270,34 +270,23 @@ __device__ __forceinline__ void nib_load(NibRow<C> & d, const NibView & w, int64
     d.L = __ldg(w.row_lut + row);
     d.e0 = __ldg(w.esc_off + row);
     d.e1 = __ldg(w.esc_off + row + 1);
-    d.rec = d.e0 + lane < d.e1 ? __ldg(w.esc + d.e0 + lane) : 0u;
+    if (RECORDS) { d.rec = d.e0 + lane < d.e1 ? __ldg(w.esc + d.e0 + lane) : 0u; }
 }
 
-// the row's BF16 pairs (escaped slots decode to +0), ready before the activations are. Rows of 4096 columns stay as loaded and are
-// decoded chunk by chunk as they are used: 64 registers of words would cost a block per SM (three products of 2048 rows, one
-// token: 10.8 us, decoded ahead 13.2).
-template <int C, bool AHEAD = (C < 8)>
-struct NibWords {
-    uint32_t w[C][8]; uint32_t e0, e1, rec;
-    __device__ __forceinline__ void set(const NibRow<C> & r) {
-#pragma unroll
-        for (int c = 0; c < C; c++) {
-            nib_assemble8(r.sm[c], r.cd[c], r.L, w[c]);
-#pragma unroll
-            for (int q = 0; q < 8; q++) { asm volatile("" : "+r"(w[c][q])); } // decoded here, not where they are used
-        }
-        e0 = r.e0; e1 = r.e1; rec = r.rec;
-    }
-    __device__ __forceinline__ void chunk(int c, uint32_t (&out)[8]) const {
-#pragma unroll
-        for (int q = 0; q < 8; q++) { out[q] = w[c][q]; }
-    }
-};
+// the row's BF16 pairs (escaped slots decode to +0), ready before the activations are
 template <int C>
-struct NibWords<C, false> : NibRow<C> {
-    __device__ __forceinline__ void set(const NibRow<C> & r) { (NibRow<C> &) *this = r; }
-    __device__ __forceinline__ void chunk(int c, uint32_t (&out)[8]) const { nib_assemble8(this->sm[c], this->cd[c], this->L, out); }
-};
+struct NibWords { uint32_t w[C][8]; uint32_t e0, e1, rec; };
+
+template <int C>
+__device__ __forceinline__ void nib_decode(const NibRow<C> & r, NibWords<C> & d) {
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        nib_assemble8(r.sm[c], r.cd[c], r.L, d.w[c]);
+#pragma unroll
+        for (int q = 0; q < 8; q++) { asm volatile("" : "+r"(d.w[c][q])); } // decoded here, not where they are used
+    }
+    d.e0 = r.e0; d.e1 = r.e1; d.rec = r.rec;
+}
 
 // four activations as they lie in memory
 template <typename TX> struct RawX4;
@@ -316,7 +305,7 @@ template <> struct RawX4<bf16> {
 // chunks are requested before the first of them is used: one trip to L2, not one per chunk.
 template <int C, int M, typename TX>
 __device__ __forceinline__ void nib_dots(const NibWords<C> (&d)[M], const NibView * const (&w)[M], const TX * x, int lane, float (&sum)[M]) {
-    constexpr int G = C < 4 ? C : C == 4 ? 4 : 1;
+    constexpr int G = C < 4 ? C : 4;
     float a[M][4];
 #pragma unroll
     for (int m = 0; m < M; m++) { a[m][0] = a[m][1] = a[m][2] = a[m][3] = 0.f; }
@@ -329,11 +318,7 @@ __device__ __forceinline__ void nib_dots(const NibWords<C> (&d)[M], const NibVie
         for (int c = 0; c < G; c++) {
             const float4 xq[4] = {q[4 * c].f(), q[4 * c + 1].f(), q[4 * c + 2].f(), q[4 * c + 3].f()};
 #pragma unroll
-            for (int m = 0; m < M; m++) {
-                uint32_t wv[8];
-                d[m].chunk(c0 + c, wv);
-                fma_chunk(wv, xq, a[m]);
-            }
+            for (int m = 0; m < M; m++) { fma_chunk(d[m].w[c0 + c], xq, a[m]); }
         }
     }
 #pragma unroll
@@ -349,6 +334,46 @@ __device__ __forceinline__ void nib_dots(const NibWords<C> (&d)[M], const NibVie
     }
 }
 
+// the same for one row as loaded, decoded chunk by chunk as it is multiplied: the same operations in the same order
+template <int C, typename TX>
+__device__ __forceinline__ float nib_dot(const NibRow<C> & d, const NibView & w, const TX * x, int lane) {
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        uint32_t wv[8];
+        nib_assemble8(d.sm[c], d.cd[c], d.L, wv);
+        float4 xq[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) { xq[j] = ldg_x4(x, c * CHUNK + 128 * j + 4 * lane); }
+        fma_chunk(wv, xq, a);
+    }
+    float acc = (a[0] + a[1]) + (a[2] + a[3]);
+    for (uint32_t i = d.e0 + lane; i < d.e1; i += 32) {
+        const uint32_t rec = __ldg(w.esc + i);
+        acc = fmaf(__uint_as_float(esc_bits(rec) << 16), ldg_x1(x, rec & 0xFFF), acc);
+    }
+    return warp_sum(acc);
+}
+
+// sums of M rows, AHEAD or as they come; `waited`: this warp has waited for the kernel before this one
+template <int C, bool AHEAD, int M, typename TX>
+__device__ __forceinline__ void nib_rows(const NibView * const (&w)[M], int64_t row, const TX * x, int lane, bool & waited, float (&sum)[M]) {
+    NibRow<C> raw[M];
+#pragma unroll
+    for (int m = 0; m < M; m++) { nib_load<C, AHEAD>(raw[m], *w[m], row, lane); }
+    if constexpr (AHEAD) {
+        NibWords<C> d[M];
+#pragma unroll
+        for (int m = 0; m < M; m++) { nib_decode<C>(raw[m], d[m]); }
+        if (!waited) { grid_dependency_wait(); waited = true; }
+        nib_dots<C, M, TX>(d, w, x, lane, sum);
+    } else {
+        if (!waited) { grid_dependency_wait(); waited = true; }
+#pragma unroll
+        for (int m = 0; m < M; m++) { sum[m] = nib_dot<C, TX>(raw[m], *w[m], x, lane); }
+    }
+}
+
 // GLU: g rows are the gate, v rows the up half (separate matrices, or the same matrix shifted by nrows rows)
 //
 // What bounds it: a decode step is a row of launches that depend on each other, each of a few microseconds. So everything
@@ -358,14 +383,16 @@ __device__ __forceinline__ void nib_dots(const NibWords<C> (&d)[M], const NibVie
 // Behind the wait are one trip to L2 for the activations (one per chunk, and two for a gate/up pair, before), the products and the
 // sums. 48 layers of three launches each: 460 -> 349 us; 20 layers at 2 / 4 tokens: 237 / 337 -> 188 / 256 us. Measured and left:
 // activations staged in shared memory once per block, its rows multiplied with up to four columns (359 us; 225 / 360).
-constexpr int nib_blocks(int C, bool glu, int x_bytes) { // per SM: room for the launches behind, and as many as the registers of a row allow
-    return glu ? (C == 1 ? 4 : C == 2 ? 3 : C == 4 ? 2 : 1) : C == 8 ? (x_bytes == 2 ? 3 : 2) : C == 4 ? 3 : C == 2 ? 5 : 6;
-}
-template <int C, typename TX, bool GLU>
-__global__ void __launch_bounds__(256, nib_blocks(C, GLU, sizeof(TX))) k_nib_gemv(const NibView g, const NibView v, Cols p) {
+// Blocks of later waves find the kernel before long complete, and there decoding ahead only puts the trip for the row in front of the
+// trip for the activations, in registers that cost resident blocks: launches of more than three waves request both
+// together and decode as they multiply (AHEAD = false / true, us: 2048 x 512, eight tokens 4.5 / 5.2; 8192 x 512, two tokens
+// 4.6 / 5.0; 8192 x 4096, one token 10.4 / 11.1; up to three waves AHEAD is level or faster: 2048 x 512, one token 2.0 / 1.8).
+constexpr int nib_blocks(int C, bool glu) { return glu ? (C <= 2 ? 3 : C == 4 ? 2 : 1) : C == 8 ? 2 : C == 4 ? 3 : 4; } // AHEAD, per SM: room for the launches behind (otherwise 0: the compiler's own choice)
+template <int C, typename TX, bool GLU, bool AHEAD>
+__global__ void __launch_bounds__(256, AHEAD ? nib_blocks(C, GLU) : 0) k_nib_gemv(const NibView g, const NibView v, Cols p) {
     constexpr int M = GLU ? 2 : 1;
     bool waited = p.ids != nullptr; // expert ids, when there are any, belong to an earlier kernel too
-    if (waited) { grid_dependency_wait(); } else { grid_launch_dependents(); }
+    if (waited) { grid_dependency_wait(); } else if (AHEAD) { grid_launch_dependents(); }
     const TX * xg; OutVec out; int64_t rbase;
     column<TX>(p, blockIdx.y, xg, out, rbase);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -373,17 +400,8 @@ __global__ void __launch_bounds__(256, nib_blocks(C, GLU, sizeof(TX))) k_nib_gem
     w[0] = &g;
     if constexpr (GLU) { w[1] = &v; }
     for (int64_t r = (int64_t) blockIdx.x * 8 + warp; r < p.nrows; r += (int64_t) gridDim.x * 8) {
-        NibWords<C> d[M];
-        {
-            NibRow<C> row[M];
-#pragma unroll
-            for (int m = 0; m < M; m++) { nib_load<C>(row[m], *w[m], rbase + r, lane); }
-#pragma unroll
-            for (int m = 0; m < M; m++) { d[m].set(row[m]); }
-        }
-        if (!waited) { grid_dependency_wait(); waited = true; }
         float s[M];
-        nib_dots<C, M, TX>(d, w, xg, lane, s);
+        nib_rows<C, AHEAD, M, TX>(w, rbase + r, xg, lane, waited, s);
         if (lane == 0) {
             if constexpr (GLU) { out.put(r, s[1] * silu_f(s[0])); } else { out.put(r, s[0]); }
         }
@@ -623,14 +641,19 @@ dim3 row_geometry(int64_t work, int ncols) { // 8 warps per block, one work item
     return dim3((unsigned) std::max<int64_t>(1, std::min<int64_t>((work + 7) / 8, cap)), (unsigned) ncols);
 }
 
+template <int C, typename TX, bool GLU>
+void launch_nib_c(const NibView & g, const NibView & v, const Cols & p, int ncols, cudaStream_t st) {
+    const dim3 grid = row_geometry(p.nrows, ncols);
+    const bool few = (int64_t) grid.x * grid.y <= 3 * (int64_t) device_info().sms * nib_blocks(C, GLU);
+    launch_chained(few ? k_nib_gemv<C, TX, GLU, true> : k_nib_gemv<C, TX, GLU, false>, grid, dim3(256), 0, st, g, v, p);
+}
 template <typename TX, bool GLU>
 void launch_nib(const NibView & g, const NibView & v, const Cols & p, int64_t K, int ncols, cudaStream_t st) {
-    const dim3 grid = row_geometry(p.nrows, ncols);
     switch (K / CHUNK) {
-        case 1: launch_chained(k_nib_gemv<1, TX, GLU>, grid, dim3(256), 0, st, g, v, p); break;
-        case 2: launch_chained(k_nib_gemv<2, TX, GLU>, grid, dim3(256), 0, st, g, v, p); break;
-        case 4: launch_chained(k_nib_gemv<4, TX, GLU>, grid, dim3(256), 0, st, g, v, p); break;
-        case 8: launch_chained(k_nib_gemv<8, TX, GLU>, grid, dim3(256), 0, st, g, v, p); break;
+        case 1: launch_nib_c<1, TX, GLU>(g, v, p, ncols, st); break;
+        case 2: launch_nib_c<2, TX, GLU>(g, v, p, ncols, st); break;
+        case 4: launch_nib_c<4, TX, GLU>(g, v, p, ncols, st); break;
+        case 8: launch_nib_c<8, TX, GLU>(g, v, p, ncols, st); break;
         default: fail_invalid("unsupported K");
     }
 }
@@ -804,7 +827,7 @@ struct NibItem { // one dense NIBBLE product of a group
 };
 struct NibGroup { int n; NibItem item[GROUP_MAX]; };
 
-template <int C, typename TX>
+template <int C, bool AHEAD, typename TX>
 __device__ __forceinline__ void nib_item_rows(const NibItem & it, int block, int col) {
     const TX * xg = (const TX *) (it.x + col * it.x_tok);
     const OutVec out = {it.y + col * it.y_tok, it.y_bf16};
@@ -812,39 +835,34 @@ __device__ __forceinline__ void nib_item_rows(const NibItem & it, int block, int
     const NibView * w[1] = {&it.v};
     bool waited = false;
     for (int64_t r = (int64_t) block * 8 + warp; r < it.nrows; r += (int64_t) it.blocks * 8) {
-        NibWords<C> d[1];
-        {
-            NibRow<C> row;
-            nib_load<C>(row, it.v, it.row0 + r, lane);
-            d[0].set(row);
-        }
-        if (!waited) { grid_dependency_wait(); waited = true; } // weights first, then the activations an earlier kernel may have written
         float s[1];
-        nib_dots<C, 1, TX>(d, w, xg, lane, s);
+        nib_rows<C, AHEAD, 1, TX>(w, it.row0 + r, xg, lane, waited, s); // weights first, then the activations an earlier kernel may have written
         if (lane == 0) { out.put(r, s[0]); }
     }
     if (!waited) { grid_dependency_wait(); }
 }
 
 // Every block belongs to one item of the group (a prefix table of block ranges); within its item it is a block of the
-// single-product kernel: same loads, same order of operations, so the results are the same bits. WIDE adds rows of 4096
-// columns. Three blocks fit an SM, and the 352 blocks of a layer's three products are resident at once (two left a second wave).
+// single-product kernel: same loads, same order of operations, so the results are the same bits. Three blocks fit an SM, and the
+// 352 blocks of a layer's three products are resident at once (two left a second wave). WIDE adds rows of 4096 columns and
+// decodes every item as it multiplies: ahead, such a row's registers left one block per SM (three products of 2048 x 4096: 13.2
+// against 10.8 us).
 template <bool WIDE>
-__global__ void __launch_bounds__(256, 3) k_nib_gemv_group(const NibGroup g) {
-    grid_launch_dependents(); // as in k_nib_gemv
+__global__ void __launch_bounds__(256, WIDE ? 0 : 3) k_nib_gemv_group(const NibGroup g) {
+    if (!WIDE) { grid_launch_dependents(); } // as in k_nib_gemv
     int m = 0;
     while (m + 1 < g.n && (int) blockIdx.x >= g.item[m + 1].first_block) { m++; }
     const NibItem & it = g.item[m];
     const int local = (int) blockIdx.x - it.first_block, col = local / it.blocks, block = local % it.blocks;
     switch (it.chunks * 2 + (it.x_bf16 ? 1 : 0)) {
-        case 2: nib_item_rows<1, float>(it, block, col); break;
-        case 3: nib_item_rows<1, bf16>(it, block, col); break;
-        case 4: nib_item_rows<2, float>(it, block, col); break;
-        case 5: nib_item_rows<2, bf16>(it, block, col); break;
-        case 8: nib_item_rows<4, float>(it, block, col); break;
-        case 9: nib_item_rows<4, bf16>(it, block, col); break;
-        case 16: if constexpr (WIDE) { nib_item_rows<8, float>(it, block, col); } break;
-        case 17: if constexpr (WIDE) { nib_item_rows<8, bf16>(it, block, col); } break;
+        case 2: nib_item_rows<1, !WIDE, float>(it, block, col); break;
+        case 3: nib_item_rows<1, !WIDE, bf16>(it, block, col); break;
+        case 4: nib_item_rows<2, !WIDE, float>(it, block, col); break;
+        case 5: nib_item_rows<2, !WIDE, bf16>(it, block, col); break;
+        case 8: nib_item_rows<4, !WIDE, float>(it, block, col); break;
+        case 9: nib_item_rows<4, !WIDE, bf16>(it, block, col); break;
+        case 16: if constexpr (WIDE) { nib_item_rows<8, false, float>(it, block, col); } break;
+        case 17: if constexpr (WIDE) { nib_item_rows<8, false, bf16>(it, block, col); } break;
         default: grid_dependency_wait(); break;
     }
 }

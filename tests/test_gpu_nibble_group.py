@@ -38,11 +38,10 @@ def test_group_equals_single_products(shapes, T, fp32):
 
 
 @pytest.mark.parametrize("K", [512, 1024, 2048, 4096])
-@pytest.mark.parametrize("T, fp32", [(1, True), (3, False)])
-def test_glu(K, T, fp32):
+@pytest.mark.parametrize("T, fp32, rows", [(1, True, 21), (3, False, 21), (3, True, 4001), (4, False, 4001)])   # 4001: more than three waves
+def test_glu(K, T, fp32, rows):
     from orin_qwen_lossless_b200 import ops
     ops.init()
-    rows = 21
     bits = _bits(2 * rows, K, K)
     w = ops.upload(*ops.encode(to_bf16_tensor(bits), 1, 0, False), "cuda")
     x = torch.from_numpy(np.random.default_rng(K).standard_normal((T, K)).astype(np.float32)).to(torch.bfloat16).cuda()
