@@ -77,7 +77,7 @@ def test_expert_parallel_partials_add_up(ops, layer, ranks):
     assert torch.allclose(total, full.double(), rtol=0, atol=2.0 ** -18 * float(full.abs().max()) * K_TOP)
 
 
-@pytest.mark.parametrize("T", [1, 2, 4])
+@pytest.mark.parametrize("T", [1, 2, 4, 9, 48])   # 9: more than 64 routed columns; 48: gate and up in two launches
 def test_step_over_fragment_order_experts(ops, layer, T):
     """The vLLM layout (16-row fragment-order bands for gate, up and down) through the same entry point: equal to the
     operator chain over the same weights (bitwise) and within the bound of the FP64 layer; an expert slice is refused."""

@@ -81,3 +81,72 @@ def test_scratch_rule():
     assert need(C.byref(w), None, 32, 4096, TOPK) == 0     # 128 rows per expert: no whole row block of 256
     lane_major = ops.encode(to_bf16_tensor(o.weights_like(E * N, H, 31)), 3, 8, True)
     assert need(C.byref(ops.upload(*lane_major, "cuda").c()), None, E, 4096, TOPK) == 0
+
+
+def _public(ops, K, rows, n, T, used, glu, seed):
+    """A product through ops.moe_mm_ids as a program calls it, and what the scratch rule says about it."""
+    import ctypes as C
+    from orin_qwen_lossless_b200 import _lib
+    w, u = (ops.upload(*ops.encode(to_bf16_tensor(o.weights_like(n * rows, K, seed + i)), 3, 16, False, True), "cuda") for i in range(2))
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(T, K, device="cuda", generator=g).to(torch.bfloat16)
+    ids = torch.rand(T, n, device="cuda", generator=g).topk(used, dim=1).indices.to(torch.int32).contiguous()
+    cw, cu = w.c(), u.c()
+    need = _lib.lib().bf16n_mm_ids_scratch_bytes(C.byref(cw), C.byref(cu) if glu else None, n, T, used)
+    return (lambda: ops.moe_mm_ids(x, ids, w, n, up=u if glu else None, out_dtype=torch.bfloat16 if glu else torch.float32)), need
+
+
+@pytest.mark.parametrize("K, rows, n, T, used, glu", [
+    (512, 512, 8, 4000, 8, False), (512, 512, 64, 4096, 8, True), (1024, 256, 8, 4000, 2, True), (1536, 768, 4, 700, 2, False),
+    (2048, 512, 1, 1000, 1, True), (3072, 256, 16, 300, 8, True), (4096, 256, 4, 600, 4, False), (4096, 1024, 3, 129, 3, True),
+])
+def test_both_forms_give_the_same_bits(layer, monkeypatch, K, rows, n, T, used, glu):
+    """The public call takes the two-pass form here; without scratch it runs the fused kernel: not a bit differs, so memory and
+    capture, which decide between them, do not show in results."""
+    ops = layer[0]
+    run, need = _public(ops, K, rows, n, T, used, glu, K + n)
+    assert need > 0
+    taken = []
+    real = ops._mm_ids_scratch
+    monkeypatch.setattr(ops, "_mm_ids_scratch", lambda *a: taken.append(real(*a)) or taken[-1])
+    two = run()
+    assert taken[0] is not None and taken[0].numel() >= need
+    monkeypatch.setattr(ops, "_mm_ids_scratch", lambda *a: None)
+    assert torch.equal(two, run())
+
+
+def test_capture_and_a_full_device_run_the_fused_kernel(layer, monkeypatch):
+    ops = layer[0]
+    monkeypatch.setattr(ops, "_scratch_refused", {})
+    run, need = _public(ops, 2048, 512, 48, 600, 8, True, 9)
+    assert need == 48 * 2 * 512 * 2048 * 2
+    want = run()
+
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        g = torch.cuda.CUDAGraph()
+        before = torch.cuda.memory_allocated()
+        with torch.cuda.graph(g, stream=s):
+            got = run()
+        assert torch.cuda.memory_allocated() - before < need      # no tiles in the graph's memory
+        got.zero_()
+        g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    del g
+
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction(min(1.0, (torch.cuda.memory_reserved() + need // 2) / total))
+    try:
+        assert torch.equal(run(), want)
+        assert list(ops._scratch_refused) == [torch.cuda.current_device()]
+        with monkeypatch.context() as m:      # not asked again while the refusal is fresh
+            m.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+            empty = torch.empty
+            m.setattr(ops.torch, "empty", lambda *a, **k: pytest.fail("asked again") if a and a[0] == need + 1024 else empty(*a, **k))
+            assert torch.equal(run(), want)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    ops._scratch_refused.clear()
+    assert torch.equal(run(), want)
