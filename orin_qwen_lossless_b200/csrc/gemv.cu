@@ -383,10 +383,10 @@ __device__ __forceinline__ void nib_rows(const NibView * const (&w)[M], int64_t 
 // Behind the wait are one trip to L2 for the activations (one per chunk, and two for a gate/up pair, before), the products and the
 // sums. 48 layers of three launches each: 460 -> 349 us; 20 layers at 2 / 4 tokens: 237 / 337 -> 188 / 256 us. Measured and left:
 // activations staged in shared memory once per block, its rows multiplied with up to four columns (359 us; 225 / 360).
-// Blocks of later waves find the kernel before long complete, and there decoding ahead only puts the trip for the row in front of the
-// trip for the activations, in registers that cost resident blocks: launches of more than three waves request both
+// A warp's later rows find the kernel before long complete, and there decoding ahead only puts the trip for the row in front of the
+// trip for the activations, in registers that cost resident blocks: launches of more than three rows per resident warp request both
 // together and decode as they multiply (AHEAD = false / true, us: 2048 x 512, eight tokens 4.5 / 5.2; 8192 x 512, two tokens
-// 4.6 / 5.0; 8192 x 4096, one token 10.4 / 11.1; up to three waves AHEAD is level or faster: 2048 x 512, one token 2.0 / 1.8).
+// 4.6 / 5.0; 8192 x 4096, one token 10.4 / 11.1).
 constexpr int nib_blocks(int C, bool glu) { return glu ? (C <= 2 ? 3 : C == 4 ? 2 : 1) : C == 8 ? 2 : C == 4 ? 3 : 4; } // AHEAD, per SM: room for the launches behind (otherwise 0: the compiler's own choice)
 template <int C, typename TX, bool GLU, bool AHEAD>
 __global__ void __launch_bounds__(256, AHEAD ? nib_blocks(C, GLU) : 0) k_nib_gemv(const NibView g, const NibView v, Cols p) {
@@ -644,7 +644,7 @@ dim3 row_geometry(int64_t work, int ncols) { // 8 warps per block, one work item
 template <int C, typename TX, bool GLU>
 void launch_nib_c(const NibView & g, const NibView & v, const Cols & p, int ncols, cudaStream_t st) {
     const dim3 grid = row_geometry(p.nrows, ncols);
-    const bool few = (int64_t) grid.x * grid.y <= 3 * (int64_t) device_info().sms * nib_blocks(C, GLU);
+    const bool few = p.nrows * ncols <= 3 * (int64_t) device_info().sms * nib_blocks(C, GLU) * 8; // rows against resident warps
     launch_chained(few ? k_nib_gemv<C, TX, GLU, true> : k_nib_gemv<C, TX, GLU, false>, grid, dim3(256), 0, st, g, v, p);
 }
 template <typename TX, bool GLU>

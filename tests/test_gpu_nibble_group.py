@@ -38,7 +38,7 @@ def test_group_equals_single_products(shapes, T, fp32):
 
 
 @pytest.mark.parametrize("K", [512, 1024, 2048, 4096])
-@pytest.mark.parametrize("T, fp32, rows", [(1, True, 21), (3, False, 21), (3, True, 4001), (4, False, 4001)])   # 4001: more than three waves
+@pytest.mark.parametrize("T, fp32, rows", [(1, True, 21), (3, False, 21), (3, True, 4001), (4, False, 4001)])   # 4001: more than three rows to a warp
 def test_glu(K, T, fp32, rows):
     from orin_qwen_lossless_b200 import ops
     ops.init()
