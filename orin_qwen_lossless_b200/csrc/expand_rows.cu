@@ -76,7 +76,7 @@ void launch(const bf16n_weight & w, int64_t row0, int64_t nrows, const Sink & si
     if (units == 0) { return; }
     const int warps = (int) std::min<int64_t>(ROW_WARPS, std::max<int64_t>((units + sms - 1) / sms, 8)); // eight stage the tables
     const unsigned blocks = (unsigned) std::min(sms, units);
-    const ring::Opaque k = {1u, 4u, ~0u, 32u, 16u};
+    const ring::Opaque k = {1u, 4u, ~0u, 16u};
     k_expand_rows<Sink><<<blocks, warps * 32, LUT_BYTES + (size_t) warps * 32 * RING_BYTES, st>>>(pair_view(w), (int) (w.K / CHUNK), w.R, w.cm != 0, row0,
                                                                                                 units, sink, k);
     check_launch();

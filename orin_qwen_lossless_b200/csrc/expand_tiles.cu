@@ -254,7 +254,7 @@ void expand_tiles(const bf16n_weight & w, const bf16n_weight * up, int n_experts
     const int n_mats = up ? 2 : 1;
     const unsigned gx = (unsigned) std::min<int64_t>(std::max(1, device_info().sms / n_mats), (a.units + EXPAND_WARPS - 1) / EXPAND_WARPS);
     const dim3 grid(gx, (unsigned) n_mats);
-    const Opaque k = {1u, 4u, ~0u, 32u, 16u};
+    const Opaque k = {1u, 4u, ~0u, 16u};
     // the first kernel of its call: behind whatever the caller launched (launch_behind)
     launch_behind(false, w.K == 4 * CHUNK ? k_expand_tiles<4, 8, true> : k_expand_tiles<1, 16, false>, grid, dim3(EXPAND_WARPS * 32), EXPAND_SMEM, st, a, k);
     check_launch();
@@ -289,7 +289,7 @@ void expand_tiles_fo(const bf16n_weight & w, const bf16n_weight * up, int n_expe
         if (full > best + 1e-9) { best = full; warps = nw; }
     }
     const dim3 grid((unsigned) std::min<int64_t>(blocks, (a.units + warps - 1) / warps), (unsigned) n_mats);
-    const Opaque k = {1u, 4u, ~0u, 32u, 16u};
+    const Opaque k = {1u, 4u, ~0u, 16u};
     launch_behind(behind_own, k_expand_tiles_fo, grid, dim3(warps * 32), LUT_BYTES + (size_t) warps * (32 * RING_BYTES + FO_STAGE), st, a, k);
     check_launch();
 }

@@ -885,7 +885,7 @@ void fo_split(const bf16n_weight & w, const bf16n_weight * up, void * up_y, cons
     const Cols p = make_cols(a);
     const int C = (int) (w.K / CHUNK), nb = std::max(1, 8 / C);
     const int64_t bands = p.nrows / BAND;
-    const Opaque k = {1u, 4u, ~0u, 32u};
+    const Opaque k = {1u, 4u};
     const dim3 grid((unsigned) ((bands + nb - 1) / nb), (unsigned) a.ncols, up ? 2 : 1);
     const FoMat m0 = fo_mat(w), m1 = up ? fo_mat(*up, (char *) up_y - (char *) a.y) : m0;
     // routed columns of 4..8 whole tokens: columns with the same expert share one decode (same bits per column).
@@ -939,7 +939,7 @@ void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st
             q.y += c0 * p.y_tok;
             const int nc = std::min(8, a.ncols - c0);
             if (big) {
-                const Opaque k = {1u, 4u, ~0u, 32u};
+                const Opaque k = {1u, 4u};
                 launch_chained(k_fo_gemv_staged, dim3((unsigned) sms), dim3(staged_warps * 32), shm_staged, st, pair_view(w),
                                (const AuxHeader *) w.aux, C, q, nc, k);
             } else if (C <= 8) { // small and mid-size matrices: a band's slabs on separate warps, streams staged
@@ -947,7 +947,7 @@ void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st
                     const int nb = std::max(1, 8 / C);
                     const size_t shm = 4 * HP_MAX_PAIRS + 128 + (size_t) 8 * (w.K + FO_SPLIT_XPAD) * 2 + (size_t) nb * C * 128 * 4 +
                                        (size_t) nb * C * FO_SPLIT_CAP;
-                    const Opaque k = {1u, 4u, ~0u, 32u};
+                    const Opaque k = {1u, 4u};
                     launch_chained(k_fo_gemv_split<bf16, true>, dim3((unsigned) ((bands + nb - 1) / nb)), dim3(nb * C * 32), shm, st,
                                    fo_mat(w), fo_mat(w), C, q, nb, nc, behind_own || c0 > 0, k);
                 }

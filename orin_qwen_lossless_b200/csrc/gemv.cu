@@ -804,6 +804,7 @@ void gemv_init() {
     ATTR((k_pair_glu<4, bf16>), 8 * HP_MAX_PAIRS + 4 * CHUNK * 4);
     ATTR(k_pair_rows_staged<true>, 6 * HP_MAX_PAIRS + 128 + 2 * (16 * K_MAX * 3 / 8 + 80));
     ATTR(k_pair_rows_staged<false>, 6 * HP_MAX_PAIRS + 128 + 2 * (16 * K_MAX * 3 / 8 + 80));
+#undef ATTR
     expand_rows_init();
     gemv_staged_init();
     gemv_rings_init();
@@ -935,7 +936,7 @@ void gather_rows(const bf16n_weight & w, const void * ids, int64_t ids_s0, int64
         const int per = n > device_info().sms * 2 ? 2 : 1;
         const uint32_t cap = (uint32_t) ((w.R * w.K * 3 / 8 + 64 + 15) & ~15ll);
         const size_t shm = 6 * HP_MAX_PAIRS + 128 + (size_t) per * cap;
-        const Opaque k = {1u, 4u, ~0u, 32u};
+        const Opaque k = {1u, 4u};
         launch_behind(behind_own, dst_bf16 ? k_pair_rows_staged<true> : k_pair_rows_staged<false>, dim3((unsigned) ((n + per - 1) / per)), dim3(ROWS_THREADS),
                       shm, st, pair_view(w), (const AuxHeader *) w.aux, C, w.R, ip, ids_s0, n, row0, dp, dst_s1, per, cap, k);
     } else {

@@ -260,7 +260,7 @@ void launch_rings(const bf16n_weight & w, const Cols & p, int nc, int ncols_grid
     }
     const dim3 grid((unsigned) sms, (unsigned) ncols_grid);
     const size_t shm = fixed_smem(w.K, nc) + (size_t) best * RING_SET;
-    const Opaque k = {1u, 4u, ~0u, 32u, 16u};
+    const Opaque k = {1u, 4u, ~0u, 16u};
     const PairView v = pair_view(w);
 #define GO(CC, NT, NC) if (p.peers.n) { k_pair_gemv_rings<CC, NT, NC, true><<<grid, best * 32, shm, st>>>(v, w.R, p, k); } \
                        else { k_pair_gemv_rings<CC, NT, NC, false><<<grid, best * 32, shm, st>>>(v, w.R, p, k); }

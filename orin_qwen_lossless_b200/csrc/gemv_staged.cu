@@ -196,7 +196,7 @@ void gemv_staged(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t 
     const size_t shm = FIXED_SMEM + (size_t) best * cap;
     const AuxHeader * hdr = (const AuxHeader *) w.aux;
     const PairView v = pair_view(w);
-    const Opaque k = {1u, 4u, ~0u, 32u};
+    const Opaque k = {1u, 4u};
 #define GO(CC, TX) if (p.peers.n) { k_pair_gemv_staged<CC, TX, true><<<grid, best * 32, shm, st>>>(v, hdr, w.R, p, cap, k); } \
                    else { k_pair_gemv_staged<CC, TX, false><<<grid, best * 32, shm, st>>>(v, hdr, w.R, p, cap, k); }
     if (a.x_bf16) {

@@ -242,7 +242,7 @@ void launch_units(const ExpertMat & m0, const ExpertMat & m1, int n_mats, const 
     const bool plane = all_warps <= (int64_t) device_info().sms * g_plane_staged_warps_per_sm;
     const dim3 grid((unsigned) ((units + warps - 1) / warps), (unsigned) ncols, (unsigned) n_mats);
     const size_t shm = 4 * HP_MAX_PAIRS + 128 + (size_t) warps * (p.cap_bytes + (plane ? R * C * CHUNK : 0));
-    const Opaque k = {1u, 4u, ~0u, 32u};
+    const Opaque k = {1u, 4u};
     static bool attr_done = false; // set once per instantiation, during bf16n_init's warm-up call (before any capture)
     if (!attr_done) {
         cuda_ok(cudaFuncSetAttribute(k_expert_units<C, R, CM, TX, GLU_IN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024),

@@ -18,7 +18,7 @@ namespace ring {
 
 using namespace dev;
 
-struct Opaque { uint32_t one, four, minus_one, thirty_two, sixteen; }; // see gemv_staged.cu: keeps adds on the multiply pipe
+struct Opaque { uint32_t one, four, minus_one, sixteen; }; // see gemv_staged.cu: keeps adds on the multiply pipe
 
 constexpr int RING_BYTES = 128;
 constexpr uint32_t RING_TARGET = 96; // fetch while at most this many bytes are ahead of the read pointer
@@ -116,8 +116,8 @@ struct RingReader {
         e1 = lds32_ro(imad(v2 >> (32 - HP_LMAX), k.sixteen, lut));
         const uint32_t o2 = o + e0 + e1;
         // The window slides when the offset passes a word. Predicated, so that lookups and the assembly and products of earlier
-        // codes can be scheduled across it (as a branch: 171 against 168 us for one column of 248320 x 2048, 88 against 82 for
-        // four of 62080 x 2048). The top-up's three tests per 32 codes are better left to branch (170 and 83 predicated).
+        // codes can be scheduled across it (as a branch: 88 against 82 us for four columns of 62080 x 2048; one column of 248320 x
+        // 2048 is level within the runs' spread). The top-up's three tests per 32 codes are better left to branch (83 predicated).
         const uint32_t at = ring_addr(next, key);
         asm("{\n\t.reg .pred p;\n\t.reg .u32 t;\n\txor.b32 t, %5, %6;\n\tand.b32 t, t, 32;\n\tsetp.ne.u32 p, t, 0;\n\t"
             "@p mov.u32 %0, %1;\n\t@p mov.u32 %1, %2;\n\t@p ld.shared.u32 %2, [%9];\n\t@p mad.lo.u32 %3, %7, %8, %3;\n\t}"

@@ -62,7 +62,7 @@ __device__ __forceinline__ uint32_t shl_wrap_hi(uint32_t lo, uint32_t hi, uint32
 // multiply-add. On sm_100a shifts, logic ops and byte permutes issue at half rate on one pipe and integer multiply-adds
 // at half rate on another; the decoder is bound by the first, so every add that can be phrased as a multiply-add by one
 // of these constants runs on the second instead.
-struct Opaque { uint32_t one, four, minus_one, thirty_two; };
+struct Opaque { uint32_t one, four; };
 
 __device__ __forceinline__ uint32_t imad(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
@@ -80,8 +80,8 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr, uint32_t token = 0) {
 // Lane stream reader over words in shared memory (addresses are 32-bit shared-window addresses). The stream is seen through
 // a window of three consecutive words and a bit offset, as in rings.cuh: a view is one funnel shift and nothing is shifted
 // per code. Against a 64-bit buffer that is shifted and refilled (its predecessor here) the chain of a code is two
-// instructions shorter: 238 -> 222 us for eight one-token steps of 256 routed experts, 287 -> 264 us for four four-token steps of 128,
-// 71 -> 62 us for FP32 activations on 62080 x 2048.
+// instructions shorter: 238 -> 222 us for eight one-token steps of 256 routed experts (212 with the slide predicated, below),
+// 287 -> 264 us for four four-token steps of 128, 71 -> 62 us for FP32 activations on 62080 x 2048.
 struct WindowReader {
     uint32_t next, hi, lo, ahead, o, token;
 
