@@ -656,6 +656,7 @@ def moe_route(topk_ids: torch.Tensor, n_experts: int, per_slot: bool):
 # that had no memory for a call's tiles is not asked again for a while: device index -> when it last refused
 _scratch_refused: dict[int, float] = {}
 _SCRATCH_RETRY_S = 10.0
+_SCRATCH_PAIRS = (16, 80)   # routed pairs per expert below which bf16n_mm_ids_scratch_bytes is 0 anyway (gate/up, one matrix): not asked
 
 
 def _mm_ids_scratch(cw, cu, n_experts: int, T: int, n_used: int, device) -> torch.Tensor | None:
@@ -702,7 +703,8 @@ def moe_mm_ids(x: torch.Tensor, topk_ids: torch.Tensor, w: Weight, n_experts: in
     args = (C.byref(cw), C.byref(cu) if cu is not None else None, x.data_ptr(), w.meta.K, src1.data_ptr(), dst.data_ptr(),
             bounds.data_ptr(), y.data_ptr(), int(out_dtype == torch.bfloat16), N, n_experts, T, n_used)
     with torch.cuda.device(x.device):
-        scratch = _mm_ids_scratch(cw, cu, n_experts, T, n_used, x.device) if w.meta.frag_order else None
+        wants = w.meta.frag_order and T * n_used >= _SCRATCH_PAIRS[up is None] * n_experts
+        scratch = _mm_ids_scratch(cw, cu, n_experts, T, n_used, x.device) if wants else None
         if scratch is None:
             check(lib().bf16n_mm_ids(*args, _stream()))
         else:

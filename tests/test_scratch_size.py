@@ -63,3 +63,12 @@ def test_the_form_that_was_measured_faster(glu, K, rows, experts, pairs, two_pas
     used = min(8, experts)
     need = _lib.lib().bf16n_mm_ids_scratch_bytes(C.byref(w), C.byref(w) if glu else None, experts, experts * pairs // used, used)
     assert (need > 0) == two_pass
+
+
+@pytest.mark.parametrize("K, rows, experts", [(512, 2048, 256), (2048, 512, 256), (4096, 1024, 1), (4096, 256, 64), (1536, 768, 8)])
+def test_calls_that_are_not_asked_about_would_get_none(K, rows, experts):
+    from orin_qwen_lossless_b200 import _lib, ops
+    w = _lib.Weight(4096, 8192, 3, 16, K, experts * rows, 0, 1, 256, 16640, 20000, 30000)
+    for one, pairs in enumerate(ops._SCRATCH_PAIRS):
+        tokens = pairs * experts - 1          # one slot each: just below the line
+        assert _lib.lib().bf16n_mm_ids_scratch_bytes(C.byref(w), None if one else C.byref(w), experts, tokens, 1) == 0
