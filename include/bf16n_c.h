@@ -76,6 +76,11 @@ int bf16n_encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R,
 /* The same with the rows * K plane bytes written to the caller's buffer (null: kept in the result, as above). */
 int bf16n_encode_into(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order, uint8_t * plane,
                       bf16n_encoded ** out);
+/* The same with the aux bytes in the caller's memory too: aux_memory(context, n) is called once, on this thread, for n bytes (at
+ * least 16-byte aligned; null fails the call); the result then holds the format and R only. Null: as bf16n_encode_into. */
+typedef void * (*bf16n_aux_memory)(void * context, size_t nbytes);
+int bf16n_encode_with(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order, uint8_t * plane,
+                      bf16n_aux_memory aux_memory, void * context, bf16n_encoded ** out);
 const uint8_t * bf16n_encoded_plane(const bf16n_encoded * e, size_t * nbytes);
 const uint8_t * bf16n_encoded_aux(const bf16n_encoded * e, size_t * nbytes);
 int bf16n_encoded_format(const bf16n_encoded * e);

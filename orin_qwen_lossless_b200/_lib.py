@@ -43,10 +43,13 @@ class PeerOut(C.Structure):
 
 
 # name -> (restype, argtypes); every symbol include/bf16n_c.h declares
+AuxMemory = C.CFUNCTYPE(C.c_void_p, C.c_void_p, C.c_size_t)   # (context, bytes) -> address
+
 SIGNATURES = {
     "bf16n_last_error": (C.c_char_p, []),
     "bf16n_encode": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_void_p)]),
     "bf16n_encode_into": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.POINTER(C.c_void_p)]),
+    "bf16n_encode_with": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, AuxMemory, C.c_void_p, C.POINTER(C.c_void_p)]),
     "bf16n_encoded_plane": (C.c_void_p, [C.c_void_p, C.POINTER(C.c_size_t)]),
     "bf16n_encoded_aux": (C.c_void_p, [C.c_void_p, C.POINTER(C.c_size_t)]),
     "bf16n_encoded_format": (C.c_int, [C.c_void_p]),

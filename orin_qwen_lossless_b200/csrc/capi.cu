@@ -118,24 +118,36 @@ extern "C" {
 
 const char * bf16n_last_error(void) { return g_error.c_str(); }
 
-int bf16n_encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order,
-                 bf16n_encoded ** out) {
-    return bf16n_encode_into(w, rows, K, format, R, chunk_major, frag_order, nullptr, out);
-}
-
-int bf16n_encode_into(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order, uint8_t * plane,
-                      bf16n_encoded ** out) {
+static int encode_to(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order, uint8_t * plane,
+                     const AuxMemory & aux_memory, bf16n_encoded ** out) {
     return guarded([&] {
         require(w != nullptr && out != nullptr, "encode: null argument");
         auto * r = new bf16n_encoded;
         try {
-            r->e = encode(w, rows, K, format, R, chunk_major != 0, frag_order != 0, plane);
+            r->e = encode(w, rows, K, format, R, chunk_major != 0, frag_order != 0, plane, aux_memory);
         } catch (...) {
             delete r;
             throw;
         }
         *out = r;
     });
+}
+
+int bf16n_encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order,
+                 bf16n_encoded ** out) {
+    return encode_to(w, rows, K, format, R, chunk_major, frag_order, nullptr, {}, out);
+}
+
+int bf16n_encode_into(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order, uint8_t * plane,
+                      bf16n_encoded ** out) {
+    return encode_to(w, rows, K, format, R, chunk_major, frag_order, plane, {}, out);
+}
+
+int bf16n_encode_with(const uint16_t * w, int64_t rows, int64_t K, int format, int R, int chunk_major, int frag_order, uint8_t * plane,
+                      bf16n_aux_memory aux_memory, void * context, bf16n_encoded ** out) {
+    AuxMemory memory;
+    if (aux_memory) { memory = [=](size_t n) { return (uint8_t *) aux_memory(context, n); }; }
+    return encode_to(w, rows, K, format, R, chunk_major, frag_order, plane, memory, out);
 }
 const uint8_t * bf16n_encoded_plane(const bf16n_encoded * e, size_t * n) { if (n) { *n = e->e.plane.size(); } return e->e.plane.data(); }
 const uint8_t * bf16n_encoded_aux(const bf16n_encoded * e, size_t * n) { if (n) { *n = e->e.aux.size(); } return e->e.aux.data(); }

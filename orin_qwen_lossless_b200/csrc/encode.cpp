@@ -181,95 +181,88 @@ struct bit_sink {
     inline void finish() { if (nb) { *out++ = (uint32_t) (acc << (32 - nb)); } }
 };
 
-template <typename B, typename T> void put_at(B & buf, uint64_t off, const T * src, size_t n) {
-    if (n) { memcpy(buf.data() + off, src, n * sizeof(T)); }
+template <typename T> void put_at(uint8_t * buf, uint64_t off, const T * src, size_t n) {
+    if (n) { memcpy(buf + off, src, n * sizeof(T)); }
 }
 
 // ------------------------------------------------------------------ NIBBLE
 
-Bytes encode_nibble(const uint16_t * w, int64_t rows, int64_t K, uint8_t * plane) {
+void encode_nibble(const uint16_t * w, int64_t rows, int64_t K, uint8_t * plane, const AuxMemory & memory) {
     const int64_t C = K / CHUNK;
-    constexpr int64_t BLK = 256;
-    const int64_t nblk = (rows + BLK - 1) / BLK;
-    std::vector<std::vector<uint32_t>> esc_blk(nblk);
-    std::vector<uint32_t> esc_off(rows + 1, 0);
     AuxHeader h = {};
     h.magic = MAGIC; h.format = FMT_NIBBLE; h.K = (uint32_t) K; h.rows = (uint64_t) rows;
     h.off_a = HEADER_BYTES;
     h.off_b = h.off_a + (uint64_t) rows * K / 2;
     h.off_c = h.off_b + (uint64_t) rows * 16;
     h.off_d = h.off_c + (uint64_t) (rows + 1) * 4;
-    // Everything is written in place. The escape list's size is known last: there is room behind for one weight in 64 (more,
-    // and the buffer moves once).
-    Bytes aux;
-    aux.reserve(h.off_d + (uint64_t) rows * K / 16 + 4);
-    aux.resize(h.off_d);
-    memset(aux.data(), 0, HEADER_BYTES);
-    parallel_ranges(nblk, 1, [&](int64_t b0, int64_t b1, int) {
-        for (int64_t b = b0; b < b1; b++) {
-            for (int64_t r = b * BLK; r < std::min(rows, (b + 1) * BLK); r++) {
-                const uint16_t * row = w + r * K;
-                int hist[256] = {0};
-                for (int64_t k = 0; k < K; k++) { hist[expo(row[k])]++; }
-                // table: entry 0 = exponent 0, then the 15 most frequent exponents in 1..127 (ties: smaller first)
-                int order[127];
-                for (int i = 0; i < 127; i++) { order[i] = i + 1; }
-                std::stable_sort(order, order + 127, [&](int a, int c) { return hist[a] > hist[c]; });
-                int code_of[256];
-                std::fill(code_of, code_of + 256, -1);
-                code_of[0] = 0;
-                uint8_t * tab = aux.data() + h.off_b + r * 16;
-                memset(tab, 0, 16);
-                for (int i = 0, n = 1; i < 127 && n < 16 && hist[order[i]] > 0; i++, n++) {
-                    tab[n] = (uint8_t) order[i];
-                    code_of[order[i]] = n;
-                }
-                uint32_t n_esc = 0;
-                for (int64_t c = 0; c < C; c++) {
-                    uint8_t * codes = aux.data() + h.off_a + (r * C + c) * 256;
-                    uint8_t * pl = plane + r * K + c * CHUNK;
-                    for (int l = 0; l < 32; l++) {
-                        uint64_t packed = 0;
-                        for (int s = 0; s < 16; s++) {
-                            const int col = (int) (c * CHUNK) + chunk_col(l, s);
-                            const uint16_t v = row[col];
-                            int code = code_of[expo(v)];
-                            uint8_t sm = sign_mant(v);
-                            if (code < 0) { // escape: exact value in the list, slot reads as +0
-                                esc_blk[b].push_back((uint32_t) col | ((uint32_t) sm << 12) | (expo(v) << 20));
-                                n_esc++;
-                                code = 0;
-                                sm = 0;
-                            }
-                            packed |= (uint64_t) code << (4 * s);
-                            pl[16 * l + s] = sm;
-                        }
-                        memcpy(codes + 8 * l, &packed, 8);
-                    }
-                }
-                esc_off[r + 1] = n_esc; // per-row count; prefix-summed below
+    // tables first, and with them the escapes of every row: then the size is known and the rest is written in place
+    std::vector<uint8_t> tables((size_t) rows * 16);
+    std::vector<uint32_t> esc_off(rows + 1, 0);
+    parallel_ranges(rows, 64, [&](int64_t r0, int64_t r1, int) {
+        for (int64_t r = r0; r < r1; r++) {
+            const uint16_t * row = w + r * K;
+            int hist[256] = {0};
+            for (int64_t k = 0; k < K; k++) { hist[expo(row[k])]++; }
+            // table: entry 0 = exponent 0, then the 15 most frequent exponents in 1..127 (ties: smaller first)
+            int order[127];
+            for (int i = 0; i < 127; i++) { order[i] = i + 1; }
+            std::stable_sort(order, order + 127, [&](int a, int c) { return hist[a] > hist[c]; });
+            int64_t coded = hist[0];
+            for (int i = 0, n = 1; i < 127 && n < 16 && hist[order[i]] > 0; i++, n++) {
+                tables[r * 16 + n] = (uint8_t) order[i];
+                coded += hist[order[i]];
             }
+            esc_off[r + 1] = (uint32_t) (K - coded); // per-row count; prefix-summed below
         }
     });
     for (int64_t r = 0; r < rows; r++) { esc_off[r + 1] += esc_off[r]; }
     h.n_a = esc_off[rows];
-    aux.resize(h.off_d + std::max<uint64_t>(h.n_a, 1) * 4);
-    if (h.n_a == 0) { memset(aux.data() + h.off_d, 0, 4); }
-    memcpy(aux.data(), &h, sizeof h);
+    uint8_t * aux = memory(h.off_d + std::max<uint64_t>(h.n_a, 1) * 4);
+    memset(aux, 0, HEADER_BYTES);
+    memcpy(aux, &h, sizeof h);
+    put_at(aux, h.off_b, tables.data(), tables.size());
     put_at(aux, h.off_c, esc_off.data(), esc_off.size());
-    uint64_t o = h.off_d;
-    for (auto & v : esc_blk) {
-        put_at(aux, o, v.data(), v.size());
-        o += v.size() * 4;
-    }
-    return aux;
+    uint32_t * esc = (uint32_t *) (aux + h.off_d);
+    if (h.n_a == 0) { esc[0] = 0; }
+    parallel_ranges(rows, 64, [&](int64_t r0, int64_t r1, int) {
+        for (int64_t r = r0; r < r1; r++) {
+            const uint16_t * row = w + r * K;
+            int code_of[256];
+            std::fill(code_of, code_of + 256, -1);
+            code_of[0] = 0;
+            for (int n = 1; n < 16 && tables[r * 16 + n]; n++) { code_of[tables[r * 16 + n]] = n; }
+            uint32_t * out = esc + esc_off[r];
+            for (int64_t c = 0; c < C; c++) {
+                uint8_t * codes = aux + h.off_a + (r * C + c) * 256;
+                uint8_t * pl = plane + r * K + c * CHUNK;
+                for (int l = 0; l < 32; l++) {
+                    uint64_t packed = 0;
+                    for (int s = 0; s < 16; s++) {
+                        const int col = (int) (c * CHUNK) + chunk_col(l, s);
+                        const uint16_t v = row[col];
+                        int code = code_of[expo(v)];
+                        uint8_t sm = sign_mant(v);
+                        if (code < 0) { // escape: exact value in the list, slot reads as +0
+                            *out++ = (uint32_t) col | ((uint32_t) sm << 12) | (expo(v) << 20);
+                            code = 0;
+                            sm = 0;
+                        }
+                        packed |= (uint64_t) code << (4 * s);
+                        pl[16 * l + s] = sm;
+                    }
+                    memcpy(codes + 8 * l, &packed, 8);
+                }
+            }
+        }
+    });
 }
 
 // ------------------------------------------------------------------ HUFFMAN / HUFPAIR streams
 
 } // namespace
 
-Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, bool chunk_major, bool frag_order, uint8_t * plane) {
+Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, bool chunk_major, bool frag_order, uint8_t * plane,
+               const AuxMemory & aux_memory) {
     if (K % CHUNK != 0 || K < CHUNK || K > K_MAX) { bad("K must be a multiple of 512 in [512, 4096], got " + std::to_string(K)); }
     if (rows <= 0) { bad("rows must be positive"); }
     if (format == FMT_NIBBLE) {
@@ -291,9 +284,18 @@ Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, b
         out.plane.resize((size_t) (rows * K));
         plane = out.plane.data();
     }
+    const AuxMemory memory = [&](size_t n) -> uint8_t * {
+        if (!aux_memory) {
+            out.aux.resize(n);
+            return out.aux.data();
+        }
+        uint8_t * p = aux_memory(n);
+        if (!p) { throw std::bad_alloc(); }
+        return p;
+    };
     out.R = format == FMT_NIBBLE ? 0 : R;
     if (format == FMT_NIBBLE) {
-        out.aux = encode_nibble(w, rows, K, plane);
+        encode_nibble(w, rows, K, plane, memory);
         out.format = FMT_NIBBLE;
         return out;
     }
@@ -418,17 +420,17 @@ Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, b
         stream_off = h.off_c;
     }
     h.n_a = (uint64_t) units; h.n_b = n_words;
-    out.aux.resize(stream_off + (n_words + tail) * 4);
-    memset(out.aux.data(), 0, HEADER_BYTES);
-    if (pair) { memset(out.aux.data() + h.off_c + (uint64_t) units * 32 * 2, 0, h.off_d - h.off_c - (uint64_t) units * 32 * 2); }
-    memset(out.aux.data() + stream_off + n_words * 4, 0, (size_t) tail * 4);
-    memcpy(out.aux.data(), &h, sizeof h);
-    put_at(out.aux, h.off_a, lut.data(), lut.size());
+    uint8_t * aux = memory(stream_off + (n_words + tail) * 4);
+    memset(aux, 0, HEADER_BYTES);
+    if (pair) { memset(aux + h.off_c + (uint64_t) units * 32 * 2, 0, h.off_d - h.off_c - (uint64_t) units * 32 * 2); }
+    memset(aux + stream_off + n_words * 4, 0, (size_t) tail * 4);
+    memcpy(aux, &h, sizeof h);
+    put_at(aux, h.off_a, lut.data(), lut.size());
 
     // offsets
     if (pair) {
-        uint32_t * ub = (uint32_t *) (out.aux.data() + h.off_b);
-        uint16_t * lr = (uint16_t *) (out.aux.data() + h.off_c);
+        uint32_t * ub = (uint32_t *) (aux + h.off_b);
+        uint16_t * lr = (uint16_t *) (aux + h.off_c);
         for (int64_t u = 0; u < units; u++) {
             ub[u] = (uint32_t) unit_start[u];
             uint32_t rel = 0;
@@ -439,7 +441,7 @@ Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, b
             }
         }
     } else {
-        uint32_t * lo = (uint32_t *) (out.aux.data() + h.off_b);
+        uint32_t * lo = (uint32_t *) (aux + h.off_b);
         for (int64_t u = 0; u < units; u++) {
             uint64_t at = unit_start[u];
             for (int l = 0; l < 32; l++) {
@@ -450,7 +452,7 @@ Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, b
     }
 
     // pass 2: the bits, in place
-    uint32_t * stream = (uint32_t *) (out.aux.data() + stream_off);
+    uint32_t * stream = (uint32_t *) (aux + stream_off);
     parallel_ranges(units, 8, [&](int64_t u0, int64_t u1, int) {
         for (int64_t u = u0; u < u1; u++) {
             uint32_t * at = stream + unit_start[u];

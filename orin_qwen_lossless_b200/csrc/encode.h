@@ -4,6 +4,7 @@
 #include "format.h"
 
 #include <cstdint>
+#include <functional>
 #include <memory>
 #include <utility>
 #include <vector>
@@ -29,8 +30,10 @@ struct Encoded {
 // rows x K BF16 bit patterns, row-major. Argument rules and std::invalid_argument behaviour as the reference:
 //   NIBBLE: R = 0, no layout flags; HUFFMAN/HUFPAIR: R in {1,2,4,8,16}, rows % R == 0;
 //   chunk_major: HUFPAIR, K > 512, R in {4,8,16}; frag_order: HUFPAIR, R = 16, not chunk-major; 512 <= K <= 4096, K % 512 == 0.
-// plane: where the rows * K plane bytes go (null: into Encoded::plane).
+// plane: where the rows * K plane bytes go (null: into Encoded::plane). aux_memory: called once, with the number of aux bytes, for
+// the memory they go to (empty: into Encoded::aux).
+using AuxMemory = std::function<uint8_t *(size_t)>;
 Encoded encode(const uint16_t * w, int64_t rows, int64_t K, int format, int R, bool chunk_major, bool frag_order = false,
-               uint8_t * plane = nullptr);
+               uint8_t * plane = nullptr, const AuxMemory & aux_memory = {});
 
 } // namespace b16

@@ -119,24 +119,6 @@ def sm_count() -> int:
 
 # ------------------------------------------------------------------ host: encode, policy
 
-class _Encoded:
-    """The encoder's result, freed when the last tensor over its memory is (the aux tensor is the buffer the encoder wrote, not
-    a copy of it)."""
-
-    def __init__(self, handle):
-        self.handle, self.free = handle, lib().bf16n_encoded_free
-
-    def tensor(self, part) -> torch.Tensor:
-        n = C.c_size_t(0)
-        p = part(self.handle, C.byref(n))
-        buf = (C.c_uint8 * n.value).from_address(C.cast(p, C.c_void_p).value)
-        buf.owner = self      # torch.frombuffer keeps buf alive
-        return torch.frombuffer(buf, dtype=torch.uint8)
-
-    def __del__(self):
-        self.free(self.handle)
-
-
 def encode(w: torch.Tensor, fmt: int, R: int, chunk_major: bool, frag_order: bool = False
            ) -> tuple[torch.Tensor, torch.Tensor, Meta]:
     """Encode a BF16 CPU tensor (..., K) on all host cores: (plane uint8 [rows, K], aux uint8 [n], Meta). FMT_HUFPAIR
@@ -150,10 +132,25 @@ def encode(w: torch.Tensor, fmt: int, R: int, chunk_major: bool, frag_order: boo
     wc = w.contiguous()
     K = wc.shape[-1]
     rows = wc.numel() // max(K, 1)
+    plane = torch.empty((rows, K), dtype=torch.uint8)     # the encoder writes into both tensors
+    made = []
+
+    def aux_memory(_, n):
+        try:
+            made.append(torch.empty(n, dtype=torch.uint8))
+            return made[0].data_ptr()
+        except Exception as e:      # raised below; the encoder ends when it gets no memory
+            made.append(e)
+            return None
+
     h = C.c_void_p()
-    plane = torch.empty((rows, K), dtype=torch.uint8)     # the encoder writes into it
-    check(lib().bf16n_encode_into(wc.data_ptr(), rows, K, fmt, R, int(chunk_major), int(frag_order), plane.data_ptr(), C.byref(h)))
-    aux = _Encoded(h).tensor(lib().bf16n_encoded_aux)
+    rc = lib().bf16n_encode_with(wc.data_ptr(), rows, K, fmt, R, int(chunk_major), int(frag_order), plane.data_ptr(), _lib.AuxMemory(aux_memory),
+                                 None, C.byref(h))
+    if made and isinstance(made[0], Exception):
+        raise made[0]
+    check(rc)
+    lib().bf16n_encoded_free(h)
+    aux = made[0]
     return plane, aux, parse_header(aux)
 
 

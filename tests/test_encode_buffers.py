@@ -1,5 +1,5 @@
-"""The tensors that encode() returns are the buffers the encoder wrote: either one stays valid without the other, views keep the
-memory alive, and a second call does not touch the first call's result."""
+"""The tensors that encode() returns are the buffers the encoder wrote, in torch's memory: either one stays valid without the other,
+views keep the memory alive, a second call does not touch the first call's result, and both can be resized like any tensor."""
 import gc
 
 import numpy as np
@@ -37,3 +37,34 @@ def test_nibble_bytes_in_a_used_heap():
         plane, aux, _ = ops.encode(to_bf16_tensor(bits), 1, 0, False)
         p0, a0, _ = o.encode(bits, 1, 0)
         assert np.array_equal(plane.numpy().ravel(), p0.ravel()) and np.array_equal(aux.numpy(), a0)
+
+
+def test_results_are_ordinary_tensors():
+    from orin_qwen_lossless_b200 import ops
+    bits = o.weights_like(32, 512, 1)
+    for fmt, R in ((1, 0), (2, 4), (3, 4)):
+        plane, aux, _ = ops.encode(to_bf16_tensor(bits), fmt, R, False)
+        want, n = aux.clone(), aux.numel()
+        assert aux.data_ptr() % 16 == 0 and aux.untyped_storage().nbytes() == n
+        aux.resize_(n + 4096)
+        assert torch.equal(aux[:n], want)
+        plane.resize_(64, 512)
+
+
+def test_no_memory_for_the_result(monkeypatch):
+    import pytest
+    from orin_qwen_lossless_b200 import ops
+    real, calls = torch.empty, []
+
+    def empty(*a, **k):
+        calls.append(a)
+        if len(calls) == 2:      # the plane is there, the aux buffer is not to be had
+            raise MemoryError("no memory")
+        return real(*a, **k)
+
+    w = to_bf16_tensor(o.weights_like(32, 512, 1))
+    monkeypatch.setattr(ops.torch, "empty", empty)
+    with pytest.raises(MemoryError):
+        ops.encode(w, 3, 4, False)
+    monkeypatch.undo()
+    ops.encode(w, 3, 4, False)
