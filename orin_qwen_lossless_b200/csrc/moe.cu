@@ -24,7 +24,11 @@ __global__ void __launch_bounds__(32) k_topk(const float * __restrict__ logits, 
 #pragma unroll
     for (int i = 0; i < PER; i++) {
         const int e = i * 32 + lane;
-        v[i] = e < n_experts ? ld_act_f32(z + e) : -INFINITY;
+        v[i] = ld_act_f32(z + min(e, n_experts - 1)); // all in flight together: no branch around a load
+    }
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        if (i * 32 + lane >= n_experts) { v[i] = -INFINITY; }
     }
     float zmax = 0.f, denom = 0.f;
     for (int s = 0; s < k; s++) {

@@ -202,9 +202,11 @@ __global__ void k_combine_f32(const float * __restrict__ ys, const float * __res
     const OutVec out = {y + (int64_t) t * n * (y_bf16 ? 2 : 4), y_bf16};
     for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x) {
         float acc = 0.f;
-        for (int kx = 0; kx < n_used; kx++) { // the slot outputs come from the launch right before this one: ordered loads
+        // the slot outputs come from the launch right before this one: ordered loads. The weights are older than that launch, whose
+        // blocks waited for everything before it, and may be read ahead.
+        for (int kx = 0; kx < n_used; kx++) {
             const int64_t s = (int64_t) t * n_used + kx;
-            acc = fmaf(ld_act_f32(w + s), ld_act_f32(ys + s * n + i), acc);
+            acc = fmaf(w[s], ld_act_f32(ys + s * n + i), acc);
         }
         out.put(i, acc);
         peers_put(peers, (int64_t) t * n * (y_bf16 ? 2 : 4), y_bf16, i, acc);

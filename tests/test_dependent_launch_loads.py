@@ -16,6 +16,10 @@ CHAINED = sorted({k for s in SOURCES.values() for call in re.findall(r"launch_(?
                   for k in re.findall(r"\bk_\w+", " ".join(call))})
 
 
+# read-only parameters that are older than the kernel in front, which itself waited for everything before it
+OLDER = {("k_combine_f32", "w")}
+
+
 def _block(s, start):
     depth, i = 0, s.index("{", start)
     for j in range(i, len(s)):
@@ -43,6 +47,8 @@ def test_ordered_loads(name):
     for arg in re.findall(r"(?:__ldg|ld_stream16)\(((?:[^()]|\([^()]*\))*)\)", body):
         assert MATRIX.search(arg), f"{name} reads {arg} through the read-only path"
     for p in re.findall(r"const [\w:]+ \*\s*__restrict__ (\w+)", params):
+        if (name, p) in OLDER:
+            continue
         assert not re.search(rf"\b{p}\s*\[", body), f"{name} reads {p} without an ordered load"
         for alias in re.findall(rf"(\w+) = {p} \+", body):
             assert not re.search(rf"\b{alias}\s*\[", body), f"{name} reads {p} (as {alias}) without an ordered load"
