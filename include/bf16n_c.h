@@ -130,6 +130,16 @@ int bf16n_fault_status(unsigned int * flags, void * stream);
 /* GEMV (<= a few columns), dense or routed by expert ids. multi_col != 0: dense batches of 2..4 columns decode the
  * matrix once per group of 4. Replaces bf16n::mmv (launch.h:50, launch.cu:313-325). */
 int bf16n_mmv(const bf16n_weight * w, const bf16n_mmv_args * a, void * stream, int multi_col);
+/* Marks of a lane-major HUFPAIR matrix: where every 64th code of every lane stream begins, bf16n_marks_bytes(w) bytes of device
+ * memory (about 1.2 % of the matrix; 0: this layout has none) that the caller owns and bf16n_marks_build fills on the stream, once
+ * per matrix. With them a product or a reconstruction of few units walks a lane stream from several places at once. They are hints:
+ * every place is checked against where the codes before it ended, and where one does not agree (a matrix written since, marks not
+ * written yet, any bytes at all) the unit is decoded from its start. Results never depend on them, and marks = NULL is the call
+ * without them. They have no counterpart in the reference. */
+size_t bf16n_marks_bytes(const bf16n_weight * w);
+int bf16n_marks_build(const bf16n_weight * w, void * marks, void * stream);
+int bf16n_mmv_marked(const bf16n_weight * w, const void * marks, const bf16n_mmv_args * a, void * stream, int multi_col);
+int bf16n_dequant_marked(const bf16n_weight * w, const void * marks, int64_t row0, int64_t nrows, uint16_t * out, void * stream);
 /* n independent products on one stream, w[i] with a[i]: the small dense NIBBLE products among them (K 512..4096, up to
  * 8 columns; the per-layer projections and routers that are each too small to fill the GPU) share one grid, eight
  * products per launch, instead of one launch each; everything else is launched as bf16n_mmv would launch it. Results

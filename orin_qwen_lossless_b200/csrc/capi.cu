@@ -17,7 +17,10 @@ std::once_flag g_once;
 int g_init_status = BF16N_OK;
 std::string g_init_error;
 int g_device = -1;                         // the device bf16n_init ran on: the only one this process may launch on
-unsigned int * g_fault_words[5] = {};      // bit i of bf16n_fault_status: gemv_staged, moe_decode, fragment order, prefill, row gather
+constexpr int FAULT_WORDS = 6;
+unsigned int * g_fault_words[FAULT_WORDS] = {};
+constexpr unsigned int FAULT_BITS[FAULT_WORDS] = {BF16N_FAULT_GEMV_STAGED, BF16N_FAULT_MOE_DECODE, BF16N_FAULT_FRAG_ORDER, BF16N_FAULT_PREFILL,
+                                                  BF16N_FAULT_ROW_GATHER, BF16N_FAULT_GEMV_STAGED};
 std::atomic<uint64_t> g_peer_wait_ns{2000000000ull};
 
 template <typename F>
@@ -56,6 +59,7 @@ void ensure_init() {
             g_fault_words[2] = fo_fault_word();
             g_fault_words[3] = prefill_fault_word();
             g_fault_words[4] = row_gather_fault_word();
+            g_fault_words[5] = gemv_parts_fault_word();
         } catch (const std::exception & e) {
             g_init_status = BF16N_ECUDA;
             g_init_error = e.what();
@@ -202,14 +206,14 @@ int bf16n_fault_status(unsigned int * flags, void * stream) {
         require(flags != nullptr, "fault_status: null argument");
         ensure_init();
         cudaStream_t st = (cudaStream_t) stream;
-        unsigned int seen[5] = {0, 0, 0, 0, 0};
-        for (int i = 0; i < 5; i++) {
+        unsigned int seen[FAULT_WORDS] = {};
+        for (int i = 0; i < FAULT_WORDS; i++) {
             cuda_ok(cudaMemcpyAsync(&seen[i], g_fault_words[i], sizeof(unsigned int), cudaMemcpyDeviceToHost, st), "fault word read");
             cuda_ok(cudaMemsetAsync(g_fault_words[i], 0, sizeof(unsigned int), st), "fault word clear");
         }
         cuda_ok(cudaStreamSynchronize(st), "fault word read");
         *flags = 0;
-        for (int i = 0; i < 5; i++) { if (seen[i]) { *flags |= 1u << i; } }
+        for (int i = 0; i < FAULT_WORDS; i++) { if (seen[i]) { *flags |= FAULT_BITS[i]; } }
     });
 }
 
@@ -254,7 +258,7 @@ int bf16n_set_peer_wait_limit_ms(unsigned int ms) {
 }
 int bf16n_sm_count(int * out) { return guarded([&] { ensure_init(); *out = g_info.sms; }); }
 
-int bf16n_mmv(const bf16n_weight * w, const bf16n_mmv_args * a, void * stream, int multi_col) {
+int bf16n_mmv_marked(const bf16n_weight * w, const void * marks, const bf16n_mmv_args * a, void * stream, int multi_col) {
     return guarded([&] {
         ensure_init();
         check_weight(*w);
@@ -264,7 +268,21 @@ int bf16n_mmv(const bf16n_weight * w, const bf16n_mmv_args * a, void * stream, i
         if (a->nrows == 0) { return; }
         if (frag_order(*w)) { fo_gemv(*w, *a, (cudaStream_t) stream); return; }
         if (expert_units_applies(*w, *a)) { expert_units_mmv(*w, *a, (cudaStream_t) stream); return; }
-        gemv(*w, *a, (cudaStream_t) stream, multi_col != 0);
+        gemv(*w, *a, (cudaStream_t) stream, multi_col != 0, nullptr, (const uint16_t *) marks);
+    });
+}
+int bf16n_mmv(const bf16n_weight * w, const bf16n_mmv_args * a, void * stream, int multi_col) {
+    return bf16n_mmv_marked(w, nullptr, a, stream, multi_col);
+}
+
+size_t bf16n_marks_bytes(const bf16n_weight * w) { return w ? marks_bytes(*w) : 0; }
+int bf16n_marks_build(const bf16n_weight * w, void * marks, void * stream) {
+    return guarded([&] {
+        ensure_init();
+        require(w && marks, "marks_build: null argument");
+        check_weight(*w);
+        require(marks_bytes(*w) > 0, "marks_build: this layout has no marks");
+        marks_build(*w, (uint16_t *) marks, (cudaStream_t) stream);
     });
 }
 
@@ -325,7 +343,7 @@ int bf16n_mmv_glu(const bf16n_weight * g, const bf16n_weight * u, const bf16n_mm
     });
 }
 
-int bf16n_dequant(const bf16n_weight * w, int64_t row0, int64_t nrows, uint16_t * out, void * stream) {
+int bf16n_dequant_marked(const bf16n_weight * w, const void * marks, int64_t row0, int64_t nrows, uint16_t * out, void * stream) {
     return guarded([&] {
         ensure_init();
         check_weight(*w);
@@ -333,8 +351,11 @@ int bf16n_dequant(const bf16n_weight * w, int64_t row0, int64_t nrows, uint16_t 
         require(row0 >= 0 && nrows > 0 && row0 + nrows <= w->rows, "dequant rows out of range");
         require(w->format == FMT_NIBBLE || (nrows % w->R == 0 && row0 % w->R == 0), "dequant rows must be whole units");
         if (frag_order(*w)) { fo_expand_store(*w, row0, nrows, out, (cudaStream_t) stream); return; }
-        expand_store(*w, row0, nrows, out, (cudaStream_t) stream);
+        expand_store(*w, row0, nrows, out, (cudaStream_t) stream, (const uint16_t *) marks);
     });
+}
+int bf16n_dequant(const bf16n_weight * w, int64_t row0, int64_t nrows, uint16_t * out, void * stream) {
+    return bf16n_dequant_marked(w, nullptr, row0, nrows, out, stream);
 }
 
 int bf16n_verify(const bf16n_weight * w, int64_t row0, int64_t nrows, const uint16_t * src, unsigned long long * mismatches,

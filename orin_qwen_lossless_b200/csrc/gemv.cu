@@ -808,9 +808,11 @@ void gemv_init() {
     expand_rows_init();
     gemv_staged_init();
     gemv_rings_init();
+    gemv_parts_init();
 }
 
-void gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers) {
+void gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers, const uint16_t * marks) {
+    if (!(peers && peers->n_peers > 0) && (multi_col || a.ncols == 1) && gemv_parts_applies(w, marks, a)) { gemv_parts(w, marks, a, st); return; }
     if (a.x_bf16) { launch_gemv<bf16>(w, a, st, multi_col, peers); } else { launch_gemv<float>(w, a, st, multi_col, peers); }
 }
 
@@ -911,7 +913,8 @@ void gemv_glu(const bf16n_weight & g, const bf16n_weight & u, const bf16n_mmv_ar
     if (a.x_bf16) { launch_glu<bf16>(g, nullptr, &u, a, st); } else { launch_glu<float>(g, nullptr, &u, a, st); }
 }
 
-void expand_store(const bf16n_weight & w, int64_t row0, int64_t nrows, uint16_t * out, cudaStream_t st) {
+void expand_store(const bf16n_weight & w, int64_t row0, int64_t nrows, uint16_t * out, cudaStream_t st, const uint16_t * marks) {
+    if (expand_parts_applies(w, marks, nrows)) { expand_parts(w, marks, row0, nrows, StoreBF16{out, w.K}, st); return; }
     launch_expand(w, row0, nrows, StoreBF16{out, w.K}, st);
 }
 

@@ -1,0 +1,247 @@
+// Matrices of few lane-major pair-Huffman units with marks (parts.cuh): the decode GEMV of 1 to 8 dense columns and the exact
+// reconstruction. One warp per part, so that a chain is 64 lookups long whatever the unit's size, and all parts of a unit in
+// one block.
+//
+// What bounds them is latency: the code table, the unit's streams (one bulk copy) and the part's first plane bytes (straight into
+// registers, the others into L2) are one trip to memory together, then come 64 dependent lookups. 8192 x 2048, one token: 20.2 us
+// with a warp to each of the 512 units, 9.1 with 4096 parts (2.4 TB/s of stored bytes; 0.37 of what HBM gives). Activations lie in
+// shared memory as they are given; a quad of a column is read where it is multiplied, off the chain. Four blocks fit an SM at 64
+// registers, so 512 units of eight parts are one wave. Two and four columns take units in turn (16384 x 2048, 2 columns: 23.7 us
+// with a block to each unit, 20.4 so); one and eight do not, whose registers that overflows (9.1 against 10.1, 42 against 44).
+#include "parts.cuh"
+#include "sinks.cuh"
+
+namespace b16 {
+namespace {
+
+using namespace dev;
+
+constexpr int PART_WARPS = 8;                 // of a block; 16 where a unit has sixteen parts
+static_assert(PART_WARPS / 2 <= PART_UNITS, "units of two parts");
+
+// a quad of a column's activations: products in the format's order
+template <typename TX> struct Quad;
+template <> struct Quad<bf16> {
+    uint2 v;
+    __device__ __forceinline__ void load(uint32_t xs, int col) { asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(xs + col * 2)); }
+    __device__ __forceinline__ void fma(uint32_t w0, uint32_t w1, float (&a)[4]) const {
+        LaneX<1, bf16>::fma2(w0, v.x, a[0], a[1]);
+        LaneX<1, bf16>::fma2(w1, v.y, a[2], a[3]);
+    }
+};
+template <> struct Quad<float> {
+    float4 v;
+    __device__ __forceinline__ void load(uint32_t xs, int col) {
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(xs + col * 4));
+    }
+    __device__ __forceinline__ void fma(uint32_t w0, uint32_t w1, float (&a)[4]) const {
+        a[0] = fmaf(bf16lo_f32(w0), v.x, a[0]);
+        a[1] = fmaf(bf16hi_f32(w0), v.y, a[1]);
+        a[2] = fmaf(bf16lo_f32(w1), v.z, a[2]);
+        a[3] = fmaf(bf16hi_f32(w1), v.w, a[3]);
+    }
+};
+
+// NC dense columns (those from ncols on are computed and not stored) of row-major units. A part is 8 / C whole rows, so parts
+// share nothing but the check of their starts.
+__host__ __device__ constexpr int parts_resident(int C, int NC) { return C == 8 ? (NC == 1 ? 2 : 1) : NC == 1 ? 4 : NC <= 4 ? 3 : 2; } // blocks of an SM, by registers
+__host__ __device__ constexpr bool parts_loop(int NC) { return NC == 2 || NC == 4; }
+template <int C, int NC, typename TX>
+__global__ void __launch_bounds__(C == 8 ? 512 : 256, parts_resident(C, NC)) k_gemv_parts(const Parts p, const Cols q, int R, int ncols, const Opaque k) {
+    constexpr int K = C * CHUNK, ROWS = PART_STEPS / C;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int lane = threadIdx.x & 31;
+    unsigned char * xs = smem + part_smem(blockDim.x >> 5, (blockDim.x >> 5) / p.parts, p.cap).end;
+    const uint32_t xa = smem_u32(xs);
+    float mine[NC]; // lane r: row r of the part
+    auto prologue = [&] {
+        grid_dependency_wait(); // the activations may be the kernel's before this one
+        constexpr int VEC = 8 / (int) sizeof(TX); // eight bytes a load: what the interface asks of x and its strides
+        for (int i = threadIdx.x; i < NC * (K / VEC); i += blockDim.x) {
+            const int n = i / (K / VEC), c = i - n * (K / VEC);
+            ((uint2 *) xs)[i] = ld_act8(q.x + min(n, ncols - 1) * q.x_tok + c * 8);
+        }
+    };
+    auto rows = [&](auto & rd, uint32_t lut, PartPlane & pl, int64_t, int) {
+        float a[NC][4];
+#pragma unroll 1
+        for (int h = 0; h < PART_STEPS; h += PART_AHEAD) { // four steps as straight code: eight spill
+#pragma unroll
+            for (int i = 0; i < PART_AHEAD; i++) {
+                const int c = C == 8 ? h + i : i % C;
+                if (C == 8 ? h + i == 0 : c == 0) {
+#pragma unroll
+                    for (int n = 0; n < NC; n++) { a[n][0] = a[n][1] = a[n][2] = a[n][3] = 0.f; }
+                }
+                uint32_t e[8], wv[8];
+                rd.take8(lut, k, e);
+                assemble8(pl.template step<parts_loop(NC)>(h, i), e, wv);
+#pragma unroll
+                for (int n = 0; n < NC; n++) {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        Quad<TX> x;
+                        x.load(xa + n * K * (int) sizeof(TX), c * CHUNK + 128 * j + 4 * lane);
+                        x.fma(wv[2 * j], wv[2 * j + 1], a[n]);
+                    }
+                }
+                if (C == 8 ? h + i == C - 1 : c == C - 1) {
+#pragma unroll
+                    for (int n = 0; n < NC; n++) {
+                        const float sum = warp_sum((a[n][0] + a[n][1]) + (a[n][2] + a[n][3]));
+                        if (lane == (h + i) / C) { mine[n] = sum; }
+                    }
+                    if (C < 4) { __syncwarp(); } // keeps the next row's activation loads, and their registers, behind this row
+                }
+            }
+        }
+    };
+    auto put = [&](int64_t u, int s) {
+        if (lane < ROWS) {
+#pragma unroll
+            for (int n = 0; n < NC; n++) {
+                const OutVec out = {q.y + n * q.y_tok, q.y_bf16};
+                if (n < ncols) { out.put(u * R + s * ROWS + lane, mine[n]); }
+            }
+        }
+    };
+    walk_parts<parts_loop(NC)>(p, q.row0 / R, q.nrows / R, R * K, smem, prologue, rows, put);
+}
+
+template <typename Sink, int THREADS> // 512: units of more than eight parts
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_expand_parts(const Parts p, int C, int R, bool cm, int64_t unit0, int64_t units, const Sink sink_in, const Opaque k) {
+    Sink sink = sink_in;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int lane = threadIdx.x & 31;
+    auto chunks = [&](auto & rd, uint32_t lut, PartPlane & pl, int64_t u, int s) {
+        int rr = cm ? s * PART_STEPS % R : s * PART_STEPS / C, c = cm ? s * PART_STEPS / R : s * PART_STEPS % C;
+#pragma unroll 1
+        for (int h = 0; h < PART_STEPS; h += PART_AHEAD) {
+#pragma unroll
+            for (int i = 0; i < PART_AHEAD; i++) {
+                uint32_t e[8], wv[8];
+                rd.take8(lut, k, e);
+                assemble8(pl.template step<false>(h, i), e, wv);
+                sink.chunk(u * R + rr, c, lane, wv);
+                if (cm) { if (++rr == R) { rr = 0; c++; } } else { if (++c == C) { c = 0; rr++; } }
+            }
+        }
+    };
+    walk_parts<false>(p, unit0, units, R * C * CHUNK, smem, [] {}, chunks, [](int64_t, int) {});
+}
+
+// One warp per unit, once per matrix: where every 64 codes of a lane begin.
+__global__ void __launch_bounds__(256) k_marks(const PairView w, int parts, int64_t units, uint16_t * marks) {
+    __shared__ uint32_t lut[HP_MAX_PAIRS];
+    for (int i = threadIdx.x; i < HP_MAX_PAIRS; i += 256) { lut[i] = __ldg(w.lut + i); }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int64_t u = (int64_t) blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += (int64_t) gridDim.x * 8) {
+        PairReader rd;
+        rd.open(w, u, lane);
+        uint32_t bits = 0;
+        for (int s = 1; s < parts; s++) {
+#pragma unroll 1
+            for (int i = 0; i < PART_STEPS; i++) {
+                uint32_t e[8];
+                rd.take8(lut, e);
+#pragma unroll
+                for (int q = 0; q < 8; q++) { bits += e[q] & 31u; }
+            }
+            marks[(u * (parts - 1) + s - 1) * 32 + lane] = (uint16_t) bits;
+        }
+    }
+}
+
+// units of a block: as many as eight warps take
+int units_per_block(int parts) { return std::max(1, PART_WARPS / parts); }
+
+template <int C, int NC, typename TX>
+void launch_gemv_parts(const bf16n_weight & w, const uint16_t * marks, const Cols & q, int ncols, cudaStream_t st) {
+    const Parts p = make_parts(w, marks);
+    const int per = units_per_block(p.parts), warps = per * p.parts;
+    const int64_t units = q.nrows / w.R, blocks = (units + per - 1) / per;
+    const size_t shm = part_smem(warps, per, p.cap).end + (size_t) NC * w.K * sizeof(TX);
+    const Opaque k = {1u, 4u};
+    launch_chained(k_gemv_parts<C, NC, TX>, dim3((unsigned) (parts_loop(NC) ? std::min(blocks, (int64_t) device_info().sms * parts_resident(C, NC)) : blocks)), dim3(warps * 32), shm, st, p, q, w.R, ncols, k);
+}
+template <int C, typename TX>
+void gemv_parts_c(const bf16n_weight & w, const uint16_t * marks, const Cols & q, int ncols, cudaStream_t st) {
+    switch (ncols) {
+        case 1: launch_gemv_parts<C, 1, TX>(w, marks, q, ncols, st); break;
+        case 2: launch_gemv_parts<C, 2, TX>(w, marks, q, ncols, st); break;
+        case 3: case 4: launch_gemv_parts<C, 4, TX>(w, marks, q, ncols, st); break;
+        default: launch_gemv_parts<C, 8, TX>(w, marks, q, ncols, st); break;
+    }
+}
+
+} // namespace
+
+BF16N_DEFINE_FAULT_WORD(gemv_parts_fault_word)
+
+void gemv_parts_init() {
+    const int optin = device_info().smem_optin;
+#define ATTR(C, N, TX) allow_dynamic_smem((const void *) k_gemv_parts<C, N, TX>, optin, optin, "parts");
+#define ATTR_C(C, TX) ATTR(C, 1, TX) ATTR(C, 2, TX) ATTR(C, 4, TX) ATTR(C, 8, TX)
+    ATTR_C(1, bf16) ATTR_C(2, bf16) ATTR_C(4, bf16) ATTR_C(8, bf16) ATTR_C(1, float) ATTR_C(2, float) ATTR_C(4, float) ATTR_C(8, float)
+#undef ATTR_C
+#undef ATTR
+    allow_dynamic_smem((const void *) k_expand_parts<StoreBF16, 256>, optin, optin, "parts");
+    allow_dynamic_smem((const void *) k_expand_parts<StoreBF16, 512>, optin, optin, "parts");
+}
+
+size_t marks_bytes(const bf16n_weight & w) {
+    const int parts = unit_parts(w);
+    return parts ? (size_t) (w.rows / w.R) * (parts - 1) * 32 * sizeof(uint16_t) : 0;
+}
+
+void marks_build(const bf16n_weight & w, uint16_t * marks, cudaStream_t st) {
+    const int64_t units = w.rows / w.R;
+    k_marks<<<(unsigned) std::min<int64_t>((units + 7) / 8, (int64_t) device_info().sms * 8), 256, 0, st>>>(pair_view(w), unit_parts(w), units, marks);
+    check_launch();
+}
+
+// Where the parts are the faster form, by units of the product. Whole units / parts in us (16 rows to a unit):
+//   1 column:  8192 x 2048 20.2 / 9.1, 16384 x 2048 22.1 / 17.0, 24576 x 2048 25.3 / 25.9; 16384 x 1024 12.7 / 9.0, 32768 x 1024
+//              15.7 / 16.6: up to 1024 units. FP32 activations the same: 23.3 / 20.5 and 26.8 / 30.9 for 1024 and 1536 units.
+//   2:         24576 x 2048 32.0 / 28.4, 32768 x 2048 35.6 / 35.2, 62080 x 2048 68.6 / 63.0; 65536 x 1024 45.5 / 37.8
+//   4:         16384 x 2048 32.3 / 25.2, 24576 x 2048 36.5 / 36.2, 32768 x 2048 41.2 / 44.8 (3 columns: decoded twice without parts)
+//   8:         8192 x 2048 55 / 20.8, 62080 x 2048 156.7 / 126.9 (two decodes of four columns without parts)
+//   4096 columns of weights have no other form that stages streams: 8192 x 4096 82 / 18, 16384 x 4096 89 / 34.
+bool gemv_parts_applies(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a) {
+    const int C = (int) (w.K / CHUNK), parts = unit_parts(w);
+    if (!marks || !parts || parts > (C == 8 ? 2 : 1) * PART_WARPS || w.cm || a.ids || a.ncols > 8 || !(C == 1 || C == 2 || C == 4 || C == 8)) { return false; }
+    return a.nrows / w.R <= (C < 8 && (a.ncols == 1 || a.ncols == 4) ? 1024 : 4096);
+}
+
+void gemv_parts(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a, cudaStream_t st) {
+    const Cols q = make_cols(a);
+#define GO(C) case C: if (a.x_bf16) { gemv_parts_c<C, bf16>(w, marks, q, a.ncols, st); } else { gemv_parts_c<C, float>(w, marks, q, a.ncols, st); } break;
+    switch (w.K / CHUNK) { GO(1) GO(2) GO(4) GO(8) default: fail_invalid("unsupported K"); }
+#undef GO
+}
+
+// Rings or general kernel / parts in us: 8192 x 2048 24.5 / 10.6, 16384 x 2048 31.0 / 21.1, 62080 x 2048 87.5 / 73.5, 16384 x 4096 64.7 /
+// 46.1, 65536 x 1024 43.5 / 43.2; units of two parts: 16384 x 512 9.4 / 6.6, 65536 x 512 20.7 / 22.4.
+bool expand_parts_applies(const bf16n_weight & w, const uint16_t * marks, int64_t nrows) {
+    const int parts = unit_parts(w);
+    return marks && parts && nrows / w.R <= (parts > 2 ? 4096 : 2048);
+}
+
+template <typename Sink>
+static void expand_parts_to(const bf16n_weight & w, const uint16_t * marks, int64_t row0, int64_t nrows, const Sink & sink, cudaStream_t st) {
+    const Parts p = make_parts(w, marks);
+    const int per = units_per_block(p.parts), warps = per * p.parts;
+    const int64_t units = nrows / w.R;
+    if (units == 0) { return; }
+    const Opaque k = {1u, 4u};
+    auto * kernel = warps > 8 ? k_expand_parts<Sink, 512> : k_expand_parts<Sink, 256>;
+    kernel<<<(unsigned) ((units + per - 1) / per), warps * 32, part_smem(warps, per, p.cap).end, st>>>(p, (int) (w.K / CHUNK), w.R, w.cm != 0, row0 / w.R, units,
+                                                                                                      sink, k);
+    check_launch();
+}
+void expand_parts(const bf16n_weight & w, const uint16_t * marks, int64_t row0, int64_t nrows, const StoreBF16 & sink, cudaStream_t st) {
+    expand_parts_to(w, marks, row0, nrows, sink, st);
+}
+
+} // namespace b16

@@ -72,14 +72,24 @@ bool expand_rows_applies(const bf16n_weight & w, int64_t nrows);
 void expand_rows(const bf16n_weight & w, int64_t row0, int64_t nrows, const dev::StoreBF16 & sink, cudaStream_t st);
 void expand_rows(const bf16n_weight & w, int64_t row0, int64_t nrows, const dev::CompareBF16 & sink, cudaStream_t st);
 
+// gemv_parts.cu: few units, whose marks cut the lane streams (marks: null, or marks_bytes(w) bytes that marks_build wrote)
+void gemv_parts_init();
+size_t marks_bytes(const bf16n_weight & w); // 0: this layout has none
+void marks_build(const bf16n_weight & w, uint16_t * marks, cudaStream_t st);
+bool gemv_parts_applies(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a);
+void gemv_parts(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a, cudaStream_t st);
+bool expand_parts_applies(const bf16n_weight & w, const uint16_t * marks, int64_t nrows);
+void expand_parts(const bf16n_weight & w, const uint16_t * marks, int64_t row0, int64_t nrows, const dev::StoreBF16 & sink, cudaStream_t st);
+
 // gemv.cu
 void gemv_init();
-void gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers = nullptr);
+void gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers = nullptr,
+          const uint16_t * marks = nullptr);
 bool gemv_groupable(const bf16n_weight & w, const bf16n_mmv_args & a);
 void gemv_group(const bf16n_weight * w, const bf16n_mmv_args * a, int n, cudaStream_t st);
 void gemv_glu_merged(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st);
 void gemv_glu(const bf16n_weight & g, const bf16n_weight & u, const bf16n_mmv_args & a, cudaStream_t st);
-void expand_store(const bf16n_weight & w, int64_t row0, int64_t nrows, uint16_t * out, cudaStream_t st);
+void expand_store(const bf16n_weight & w, int64_t row0, int64_t nrows, uint16_t * out, cudaStream_t st, const uint16_t * marks = nullptr);
 void expand_compare(const bf16n_weight & w, int64_t row0, int64_t nrows, const uint16_t * src, unsigned long long * total,
                     cudaStream_t st);
 void gather_rows(const bf16n_weight & w, const void * ids, int64_t ids_s0, int64_t n, void * dst, bool dst_bf16, int64_t dst_s1,
@@ -91,6 +101,7 @@ unsigned int * moe_decode_fault_word();
 unsigned int * fo_fault_word();
 unsigned int * prefill_fault_word();
 unsigned int * row_gather_fault_word();
+unsigned int * gemv_parts_fault_word();
 
 // gemv_staged.cu
 void gemv_staged_init();

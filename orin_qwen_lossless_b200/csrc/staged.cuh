@@ -89,6 +89,9 @@ struct WindowReader {
         token = wait_token;
         hi = lds32(addr, token); lo = lds32(addr + 4, token); ahead = lds32(addr + 8, token); next = addr + 12; o = 0;
     }
+    // the same at bit `bit` (0..31) of the word at `addr`; position(): bits from the word at `start` to the next code
+    __device__ __forceinline__ void open_at(uint32_t addr, uint32_t bit, uint32_t wait_token) { open(addr, wait_token); o = bit; }
+    __device__ __forceinline__ uint32_t position(uint32_t start) const { return (next - 12u - start) * 8u + (o & 31u); }
     // at most one word on; predicated, so that lookups and products are scheduled across it (a branch: 223 against 212 us for
     // the eight one-token steps above)
     __device__ __forceinline__ void slide(uint32_t o2, const Opaque & k) {

@@ -62,6 +62,7 @@ class Weight:
     plane: torch.Tensor
     aux: torch.Tensor
     meta: Meta
+    marks: torch.Tensor | None = None    # where the lane streams can be entered (bf16n_marks_build): a hint, checked on the device
 
     @property
     def m(self) -> list[int]:
@@ -70,6 +71,9 @@ class Weight:
     @property
     def nbytes(self) -> int:
         return self.plane.numel() + self.aux.numel()
+
+    def marks_ptr(self) -> int | None:
+        return None if self.marks is None or self.marks.device != self.plane.device else self.marks.data_ptr()
 
     def c(self) -> CWeight:
         m = self.meta
@@ -166,7 +170,22 @@ def choose(rows: int, K: int, n_matrices: int = 1, *, engine: str = "vllm", mode
 
 
 def upload(plane: torch.Tensor, aux: torch.Tensor, meta: Meta, device: torch.device | str) -> Weight:
-    return Weight(plane.to(device), aux.to(device), meta)
+    w = Weight(plane.to(device), aux.to(device), meta)
+    w.marks = _make_marks(w)
+    return w
+
+
+def _make_marks(w: Weight) -> torch.Tensor | None:
+    """The marks of a matrix that was just uploaded; None for layouts without them, off the process's GPU and under capture."""
+    if w.meta.format != FMT_HUFPAIR or w.meta.frag_order or not w.plane.is_cuda or torch.cuda.is_current_stream_capturing():
+        return None
+    cw = w.c()
+    n = lib().bf16n_marks_bytes(C.byref(cw))
+    if n == 0:
+        return None
+    with torch.cuda.device(w.plane.device):
+        marks = torch.empty(n, dtype=torch.uint8, device=w.plane.device)
+        return marks if lib().bf16n_marks_build(C.byref(cw), marks.data_ptr(), _stream()) == _lib.OK else None
 
 
 # ------------------------------------------------------------------ device: dequant / verify
@@ -178,7 +197,7 @@ def dequant(w: Weight, row0: int = 0, nrows: int | None = None) -> torch.Tensor:
     cw = w.c()
     out = torch.empty((nrows, w.meta.K), dtype=torch.bfloat16, device=w.plane.device)
     with torch.cuda.device(w.plane.device):
-        check(lib().bf16n_dequant(C.byref(cw), row0, nrows, out.data_ptr(), _stream()))
+        check(lib().bf16n_dequant_marked(C.byref(cw), w.marks_ptr(), row0, nrows, out.data_ptr(), _stream()))
     return out
 
 
@@ -313,7 +332,7 @@ def _mmv_common(x, w: Weight, ids, rows_per_matrix: int, out_bf16: bool, glu: bo
         if glu:
             check(lib().bf16n_mmv_glu_merged(C.byref(cw), C.byref(a), _stream()))
         else:
-            check(lib().bf16n_mmv(C.byref(cw), C.byref(a), _stream(), int(multi_col)))
+            check(lib().bf16n_mmv_marked(C.byref(cw), w.marks_ptr(), C.byref(a), _stream(), int(multi_col)))
     return y
 
 
