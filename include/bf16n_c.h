@@ -241,6 +241,13 @@ int bf16n_moe_decode(const bf16n_weight * gate, const bf16n_weight * up, const b
                      int n_used, int expert_lo, int n_experts_local, float * scratch, size_t scratch_bytes, void * y, int y_bf16,
                      void * stream);
 
+/* bf16n_moe_decode (peers = NULL) or bf16n_moe_decode_peers with the matrices' marks (bf16n_marks_build; any may be NULL). */
+struct bf16n_peer_out;
+int bf16n_moe_decode_marked(const bf16n_weight * gate, const bf16n_weight * up, const bf16n_weight * down, const void * gate_marks,
+                            const void * up_marks, const void * down_marks, const void * x, int x_bf16, int64_t x_tok, const float * router_logits,
+                            int n_experts, int32_t * topk_ids, float * topk_weights, int n_tok, int n_used, int expert_lo, int n_experts_local,
+                            float * scratch, size_t scratch_bytes, void * y, int y_bf16, const struct bf16n_peer_out * peers, void * stream);
+
 /* bf16n_moe_decode for callers that cannot allocate device memory. It has no counterpart in the reference.
  *
  * Who needs it: code that runs a decode step at a point where cudaMalloc is not an option - an engine whose device

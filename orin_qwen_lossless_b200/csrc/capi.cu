@@ -267,7 +267,7 @@ int bf16n_mmv_marked(const bf16n_weight * w, const void * marks, const bf16n_mmv
         check_x(*w, *a);
         if (a->nrows == 0) { return; }
         if (frag_order(*w)) { fo_gemv(*w, *a, (cudaStream_t) stream); return; }
-        if (expert_units_applies(*w, *a)) { expert_units_mmv(*w, *a, (cudaStream_t) stream); return; }
+        if (expert_units_applies(*w, *a)) { expert_units_mmv(*w, *a, (cudaStream_t) stream, (const uint16_t *) marks); return; }
         gemv(*w, *a, (cudaStream_t) stream, multi_col != 0, nullptr, (const uint16_t *) marks);
     });
 }
@@ -487,7 +487,7 @@ size_t bf16n_moe_decode_scratch_bytes(int n_tok, int n_used, int64_t rows_gate, 
 static void moe_decode_checked(const bf16n_weight * gate, const bf16n_weight * up, const bf16n_weight * down, const void * x, int x_bf16,
                                int64_t x_tok, const float * router_logits, int n_experts, int32_t * topk_ids, float * topk_weights,
                                int n_tok, int n_used, int expert_lo, int n_experts_local, float * scratch, size_t scratch_bytes,
-                               void * y, int y_bf16, void * stream, const bf16n_peer_out * peers) {
+                               void * y, int y_bf16, void * stream, const bf16n_peer_out * peers, const ExpertMarks & marks = {}) {
     ensure_init();
     require(gate && up && down, "moe_decode: null weight");
     require(n_tok <= 0 || (x && y && topk_ids && topk_weights && scratch), "moe_decode: null argument");
@@ -523,9 +523,19 @@ static void moe_decode_checked(const bf16n_weight * gate, const bf16n_weight * u
         return;
     }
     moe_decode(*gate, *up, *down, x, x_bf16 != 0, x_tok, topk_ids, topk_weights, n_tok, n_used, n_experts_local, expert_lo,
-               scratch, y, y_bf16 != 0, (cudaStream_t) stream, peers);
+               scratch, y, y_bf16 != 0, (cudaStream_t) stream, peers, marks);
 }
 
+int bf16n_moe_decode_marked(const bf16n_weight * gate, const bf16n_weight * up, const bf16n_weight * down, const void * gate_marks,
+                            const void * up_marks, const void * down_marks, const void * x, int x_bf16, int64_t x_tok, const float * router_logits,
+                            int n_experts, int32_t * topk_ids, float * topk_weights, int n_tok, int n_used, int expert_lo, int n_experts_local,
+                            float * scratch, size_t scratch_bytes, void * y, int y_bf16, const bf16n_peer_out * peers, void * stream) {
+    return guarded([&] {
+        moe_decode_checked(gate, up, down, x, x_bf16, x_tok, router_logits, n_experts, topk_ids, topk_weights, n_tok, n_used, expert_lo,
+                           n_experts_local, scratch, scratch_bytes, y, y_bf16, stream, peers,
+                           {(const uint16_t *) gate_marks, (const uint16_t *) up_marks, (const uint16_t *) down_marks});
+    });
+}
 int bf16n_moe_decode(const bf16n_weight * gate, const bf16n_weight * up, const bf16n_weight * down, const void * x, int x_bf16,
                      int64_t x_tok, const float * router_logits, int n_experts, int32_t * topk_ids, float * topk_weights, int n_tok,
                      int n_used, int expert_lo, int n_experts_local, float * scratch, size_t scratch_bytes, void * y, int y_bf16,

@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(C == 8 ? 512 : 256, parts_resident(C, NC)) k_g
     const uint32_t xa = smem_u32(xs);
     float mine[NC]; // lane r: row r of the part
     auto prologue = [&] {
+        stage_table(smem, p.w.lut);
         grid_dependency_wait(); // the activations may be the kernel's before this one
         constexpr int VEC = 8 / (int) sizeof(TX); // eight bytes a load: what the interface asks of x and its strides
         for (int i = threadIdx.x; i < NC * (K / VEC); i += blockDim.x) {
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(C == 8 ? 512 : 256, parts_resident(C, NC)) k_g
             }
         }
     };
-    auto put = [&](int64_t u, int s) {
+    auto put = [&](int64_t u, int s, bool) {
         if (lane < ROWS) {
 #pragma unroll
             for (int n = 0; n < NC; n++) {
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(C == 8 ? 512 : 256, parts_resident(C, NC)) k_g
             }
         }
     };
-    walk_parts<parts_loop(NC)>(p, q.row0 / R, q.nrows / R, R * K, smem, prologue, rows, put);
+    walk_parts<parts_loop(NC)>(p, first_unit(p), q.nrows / R, q.row0 / R, R * K, smem, prologue, rows, put);
 }
 
 template <typename Sink, int THREADS> // 512: units of more than eight parts
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_expand_parts(const 
             }
         }
     };
-    walk_parts<false>(p, unit0, units, R * C * CHUNK, smem, [] {}, chunks, [](int64_t, int) {});
+    walk_parts<false>(p, first_unit(p), units, unit0, R * C * CHUNK, smem, [&] { stage_table(smem, p.w.lut); }, chunks, [](int64_t, int, bool) {});
 }
 
 // One warp per unit, once per matrix: where every 64 codes of a lane begin.

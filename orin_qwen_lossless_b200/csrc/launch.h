@@ -151,12 +151,13 @@ void moe_route(const void * ids, bool ids_i64, int64_t ids_row_stride, int32_t *
 
 // moe_decode.cu
 void moe_decode_init();
+struct ExpertMarks { const uint16_t * gate = nullptr, * up = nullptr, * down = nullptr; };
 bool expert_units_applies(const bf16n_weight & w, const bf16n_mmv_args & a);
-void expert_units_mmv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st);
+void expert_units_mmv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, const uint16_t * marks = nullptr);
 bool moe_decode_supported(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_weight & down);
 void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_weight & down, const void * x, bool x_bf16,
                 int64_t x_tok, const int32_t * ids, const float * weights, int n_tok, int n_used, int n_experts_local, int e_lo,
-                float * scratch, void * y, bool y_bf16, cudaStream_t st, const bf16n_peer_out * peers = nullptr);
+                float * scratch, void * y, bool y_bf16, cudaStream_t st, const bf16n_peer_out * peers = nullptr, const ExpertMarks & marks = {});
 void moe_decode_frag_order(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_weight & down, const void * x, bool x_bf16,
                            int64_t x_tok, const int32_t * ids, const float * weights, int n_tok, int n_used, int n_experts,
                            float * scratch, void * y, bool y_bf16, cudaStream_t st, bool behind_own);

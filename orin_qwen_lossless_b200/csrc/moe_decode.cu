@@ -12,8 +12,7 @@
 // Columns whose expert lies outside [e_lo, e_lo + e_n) (expert-parallel ranks own a slice of the experts) write zeros.
 // Summation order per row is the format's (chunk sums per row, then the xor butterfly), identical to the general
 // kernels, so results are bit-identical to bf16n_mmv on the same expert.
-#include "staged.cuh"
-#include "launch.h"
+#include "parts.cuh"
 
 #include <cstdlib>
 #include <mutex>
@@ -27,6 +26,7 @@ struct ExpertMat { // one stacked expert matrix (n_experts * rows_per_expert row
     PairView v;
     const AuxHeader * hdr;
     char * y;          // FP32 output [n_tok, n_used, rows_per_expert]
+    const uint16_t * marks; // null: none
 };
 
 struct ExpertCols {
@@ -194,6 +194,151 @@ __global__ void __launch_bounds__(256) k_expert_units(const ExpertMat m0, const 
     if (lane < R) { y[u * R + lane] = mine; }
 }
 
+// this lane's products of one chunk, in the format's order
+__device__ __forceinline__ float dot16(const uint32_t (&wv)[8], const float4 (&x)[4]) {
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        a[0] = fmaf(bf16lo_f32(wv[2 * j]), x[j].x, a[0]);
+        a[1] = fmaf(bf16hi_f32(wv[2 * j]), x[j].y, a[1]);
+        a[2] = fmaf(bf16lo_f32(wv[2 * j + 1]), x[j].z, a[2]);
+        a[3] = fmaf(bf16hi_f32(wv[2 * j + 1]), x[j].w, a[3]);
+    }
+    return (a[0] + a[1]) + (a[2] + a[3]);
+}
+
+// The same with the units cut into parts (parts.cuh), a warp to each: a chain is 64 lookups instead of 256 (gate / up) or 128 (down).
+// A part of a chunk-major unit is one chunk of its eight rows: the lanes' chunk sums meet in shared memory and are added in chunk
+// order before the butterfly, which is the order above. A part of a row-major unit is eight whole rows.
+template <int C, int R, bool CM, typename TX, bool GLU_IN>
+__global__ void __launch_bounds__(256, 4) k_expert_parts(const ExpertMat m0, const ExpertMat m1, const ExpertCols p, const Opaque k) {
+    static_assert(CM ? R == PART_STEPS : C == 1, "a part is a chunk of all rows, or whole rows of one chunk");
+    constexpr int PARTS = R * C / PART_STEPS, PER = 8 / PARTS;   // parts of a unit, units of a block
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const ExpertMat & m = blockIdx.z ? m1 : m0;
+    stage_table(smem, m.v.lut);
+    if (!p.early_ids) { grid_dependency_wait(); } // as above
+    const int col = blockIdx.y, t = col / p.n_used, s = col - t * p.n_used;
+    const int e = *(const int32_t *) (p.ids + t * p.ids_s1 + s * p.ids_s0) - p.e_lo;
+    const int64_t units = p.rows_per_expert / R;
+    float * y = (float *) m.y + ((int64_t) t * p.n_used + s) * p.rows_per_expert;
+    if (e < 0 || e >= p.e_n) { // not this rank's expert: the combine adds exact zeros
+        const int64_t r = (int64_t) blockIdx.x * PER * R + threadIdx.x;
+        if (threadIdx.x < PER * R && r < p.rows_per_expert) { y[r] = 0.f; }
+        return;
+    }
+    const Parts parts = {m.v, m.hdr, m.marks, PARTS, p.cap_bytes};
+    float * sums = (float *) (smem + part_smem(8, PER, p.cap_bytes).end) + (warp / PARTS) * (PARTS * R * 32) + lane; // CM: [part][row][lane]
+    float4 x[4];     // the lane's activations of one chunk: of the part's (CM), or all there are
+    auto load_x = [&](int c) {
+        const char * xp = p.x + t * p.x_tok + s * p.x_slot;
+        const float * x2 = GLU_IN ? p.x2 + (xp - p.x) / 4 : nullptr;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int at = c * CHUNK + 128 * j + 4 * lane;
+            x[j] = ldg_x4((const TX *) xp, at); // an ordered load: stays behind the dependency wait
+            if (GLU_IN) {
+                const float4 g = x[j], w2 = ldg_x4(x2, at);
+                x[j] = make_float4(silu_f(g.x) * w2.x, silu_f(g.y) * w2.y, silu_f(g.z) * w2.z, silu_f(g.w) * w2.w);
+            }
+        }
+    };
+    float mine = 0.f; // row-major: lane r holds row r of the part
+    auto rows = [&](auto & rd, uint32_t lut, PartPlane & pl, int64_t, int part) {
+        if (CM && part != warp % PARTS) { load_x(part); } // a warp that decodes the whole unit
+#pragma unroll 1
+        for (int h = 0; h < PART_STEPS; h += PART_AHEAD) {
+#pragma unroll
+            for (int i = 0; i < PART_AHEAD; i++) {
+                uint32_t en[8], wv[8];
+                rd.take8(lut, k, en);
+                assemble8(pl.template step<false>(h, i), en, wv);
+                const float v = dot16(wv, x);
+                if (CM) {
+                    sums[(part * R + h + i) * 32] = v;
+                } else {
+                    const float sum = warp_sum(v);
+                    if (lane == h + i) { mine = sum; }
+                }
+            }
+        }
+    };
+    auto put = [&](int64_t u, int part, bool alone) {
+        if (!CM) {
+            if (lane < PART_STEPS) { y[u * R + part * PART_STEPS + lane] = mine; }
+            return;
+        }
+        if (alone && part + 1 < PARTS) { return; }
+        const int first = alone ? 0 : part * (R / PARTS), last = alone ? R : first + R / PARTS;
+        for (int r = first; r < last; r++) {
+            float acc = 0.f;
+#pragma unroll
+            for (int c = 0; c < C; c++) { acc += sums[(c * R + r) * 32]; }
+            acc = warp_sum(acc);
+            if (lane == 0) { y[u * R + r] = acc; }
+        }
+    };
+    walk_parts<false>(parts, first_unit(parts), units, (int64_t) e * units, R * C * CHUNK, smem, [&] {
+        if (p.early_ids) { grid_dependency_wait(); }
+        load_x(CM ? warp % PARTS : 0);
+    }, rows, put);
+}
+
+// The down product and the weighted sum over the slots in one launch: a block takes one unit's rows in every slot's expert (two
+// warps each), so the slots' outputs of these rows meet in shared memory and are added in slot order, as k_combine_f32 adds them.
+// One token of 8 slots: 25.0 us a step with a launch of its own for the sum, 23.0 so.
+constexpr int COMBINE_SLOTS = PART_UNITS;
+__global__ void __launch_bounds__(512, 2) k_down_combine(const ExpertMat m, const ExpertCols p, const float * weights, char * out, bool out_bf16, const Opaque k) {
+    constexpr int R = 16, PARTS = 2;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ float ys[COMBINE_SLOTS][R];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = warp / PARTS, t = blockIdx.y;
+    stage_table(smem, m.v.lut);
+    // the ids and weights are older than the kernel in front (early_ids)
+    const int e = *(const int32_t *) (p.ids + t * p.ids_s1 + s * p.ids_s0) - p.e_lo;
+    const bool held = e >= 0 && e < p.e_n;
+    const int64_t units = p.rows_per_expert / R;
+    const Parts parts = {m.v, m.hdr, m.marks, PARTS, p.cap_bytes};
+    if (lane < PART_STEPS) { ys[s][(warp % PARTS) * PART_STEPS + lane] = 0.f; } // another rank's expert adds exact zeros
+    float4 x[4];
+    float mine = 0.f;
+    auto prologue = [&] {
+        grid_dependency_wait();
+        const char * xp = p.x + t * p.x_tok + s * p.x_slot;
+        const float * x2 = p.x2 + (xp - p.x) / 4;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float4 g = ldg_x4((const float *) xp, 128 * j + 4 * lane), u = ldg_x4(x2, 128 * j + 4 * lane);
+            x[j] = make_float4(silu_f(g.x) * u.x, silu_f(g.y) * u.y, silu_f(g.z) * u.z, silu_f(g.w) * u.w);
+        }
+    };
+    auto rows = [&](auto & rd, uint32_t lut, PartPlane & pl, int64_t, int) {
+#pragma unroll 1
+        for (int h = 0; h < PART_STEPS; h += PART_AHEAD) {
+#pragma unroll
+            for (int i = 0; i < PART_AHEAD; i++) {
+                uint32_t en[8], wv[8];
+                rd.take8(lut, k, en);
+                assemble8(pl.template step<false>(h, i), en, wv);
+                const float sum = warp_sum(dot16(wv, x));
+                if (lane == h + i) { mine = sum; }
+            }
+        }
+    };
+    auto put = [&](int64_t, int part, bool) {
+        if (lane < PART_STEPS) { ys[s][part * PART_STEPS + lane] = mine; }
+    };
+    walk_parts<false>(parts, blockIdx.x, held ? units : 0, (int64_t) e * units, R * CHUNK, smem, prologue, rows, put);
+    __syncthreads();
+    if (threadIdx.x < R) {
+        float acc = 0.f;
+        for (int kx = 0; kx < p.n_used; kx++) { acc = fmaf(weights[(int64_t) t * p.n_used + kx], ys[kx][threadIdx.x], acc); }
+        const OutVec o = {out + (int64_t) t * p.rows_per_expert * (out_bf16 ? 2 : 4), out_bf16};
+        o.put((int64_t) blockIdx.x * R + threadIdx.x, acc);
+    }
+}
+
 // y[t, i] = sum over slots, in slot order, of w[t, k] * ys[t, k, i]
 __global__ void k_combine_f32(const float * __restrict__ ys, const float * __restrict__ w, char * __restrict__ y, bool y_bf16, int n_used,
                               int64_t n, const PeerOut peers) {
@@ -227,10 +372,13 @@ __global__ void k_peer_sum(const float * __restrict__ parts, int n_parts, int64_
     }
 }
 
-ExpertMat expert_mat(const bf16n_weight & w, float * y) { return {pair_view(w), (const AuxHeader *) w.aux, (char *) y}; }
+ExpertMat expert_mat(const bf16n_weight & w, float * y, const uint16_t * marks = nullptr) { return {pair_view(w), (const AuxHeader *) w.aux, (char *) y, marks}; }
 
 uint32_t unit_cap(const bf16n_weight & w) { return (uint32_t) ((w.R * w.K * 3 / 8 + 64 + 15) & ~15ll); }
 
+// Parts while a launch has few columns: a step of 1 / 2 / 3 / 4 / 6 / 8 tokens of 8 slots takes 26.6 / 42.0 / 61 / 64 / 86 / 105.7 us a warp to
+// a unit and 23.0 / 32.7 / 45.7 / 57.1 / 80.8 / 100.7 a warp to a part; 16 and 32 tokens 179 and 336 against 190 and 358 (the blocks' openings).
+constexpr int g_parts_max_cols = 64;
 int g_plane_staged_warps_per_sm = 8; // stage the plane too while the launch has at most this many warps per SM
 
 template <int C, int R, bool CM, typename TX, bool GLU_IN>
@@ -251,9 +399,18 @@ void launch_units(const ExpertMat & m0, const ExpertMat & m1, int n_mats, const 
                 "k_expert_units attribute");
         cuda_ok(cudaFuncSetAttribute(k_expert_units<C, R, CM, TX, GLU_IN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024),
                 "k_expert_units attribute");
+        cuda_ok(cudaFuncSetAttribute(k_expert_parts<C, R, CM, TX, GLU_IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024), "k_expert_parts attribute");
         attr_done = true;
     }
     if (ncols == 0) { return; }
+    if (m0.marks && m1.marks && ncols <= g_parts_max_cols) {
+        constexpr int PARTS = R * C / PART_STEPS, PER = 8 / PARTS;
+        const size_t shm = part_smem(8, PER, p.cap_bytes).end + (CM ? PER * PARTS * R * 32 * sizeof(float) : 0);
+        launch_chained(k_expert_parts<C, R, CM, TX, GLU_IN>, dim3((unsigned) ((units + PER - 1) / PER), (unsigned) ncols, (unsigned) n_mats), dim3(256), shm, st, m0, m1, p,
+                       Opaque{1u, 4u});
+        check_launch();
+        return;
+    }
     if (plane && shm <= 128 * 1024) {
         launch_chained(k_expert_units<C, R, CM, TX, GLU_IN, true>, grid, dim3(warps * 32), shm, st, m0, m1, p, k);
     } else {
@@ -290,6 +447,7 @@ void moe_decode_init() {
     launch_units<1, 16, false, float, true>(none, none, 1, p, 0, nullptr);
     launch_units<1, 16, false, float, false>(none, none, 1, p, 0, nullptr);
     launch_units<1, 16, false, bf16, false>(none, none, 1, p, 0, nullptr);
+    allow_dynamic_smem((const void *) k_down_combine, 128 * 1024, device_info().smem_optin, "down and combine");
 }
 
 // bf16n_mmv with expert ids on the expert shapes of the decode step takes the unit kernel too (one warp per unit, bulk-copy
@@ -303,13 +461,13 @@ bool expert_units_applies(const bf16n_weight & w, const bf16n_mmv_args & a) {
     return whole && dense_y && x_ok && a.ncols <= 65535;
 }
 
-void expert_units_mmv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st) {
+void expert_units_mmv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, const uint16_t * marks) {
     ExpertCols p = {};
     p.x = (const char *) a.x; p.x_tok = a.x_tok; p.x_slot = a.x_per_slot == 1 ? 0 : a.x_slot;
     p.ids = (const char *) a.ids; p.ids_s0 = a.ids_s0; p.ids_s1 = a.ids_s1;
     p.n_used = a.n_used; p.rows_per_expert = a.rows_per_matrix; p.e_lo = 0; p.e_n = (int) (w.rows / a.rows_per_matrix);
     p.cap_bytes = unit_cap(w);
-    const ExpertMat m = expert_mat(w, (float *) a.y);
+    const ExpertMat m = expert_mat(w, (float *) a.y, marks);
     if (w.cm) {
         if (a.x_bf16) { launch_units<4, 8, true, bf16, false>(m, m, 1, p, a.ncols, st); }
         else { launch_units<4, 8, true, float, false>(m, m, 1, p, a.ncols, st); }
@@ -323,7 +481,7 @@ void expert_units_mmv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStre
 // scratch: FP32 [2 * n_tok * n_used * N + n_tok * n_used * H] (N, H = rows per expert of gate and down).
 void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_weight & down, const void * x, bool x_bf16,
                 int64_t x_tok, const int32_t * ids, const float * weights, int n_tok, int n_used, int n_experts_local, int e_lo,
-                float * scratch, void * y, bool y_bf16, cudaStream_t st, const bf16n_peer_out * peers) {
+                float * scratch, void * y, bool y_bf16, cudaStream_t st, const bf16n_peer_out * peers, const ExpertMarks & marks) {
     const int64_t N = gate.rows / n_experts_local, H = down.rows / n_experts_local;
     const int ncols = n_tok * n_used;
     float * g = scratch, * u = g + (int64_t) ncols * N, * ys = u + (int64_t) ncols * N;
@@ -333,15 +491,21 @@ void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_
     p.n_used = n_used; p.rows_per_expert = N; p.e_lo = e_lo; p.e_n = n_experts_local;
     p.cap_bytes = unit_cap(gate);
     if (x_bf16) {
-        launch_units<4, 8, true, bf16, false>(expert_mat(gate, g), expert_mat(up, u), 2, p, ncols, st);
+        launch_units<4, 8, true, bf16, false>(expert_mat(gate, g, marks.gate), expert_mat(up, u, marks.up), 2, p, ncols, st);
     } else {
-        launch_units<4, 8, true, float, false>(expert_mat(gate, g), expert_mat(up, u), 2, p, ncols, st);
+        launch_units<4, 8, true, float, false>(expert_mat(gate, g, marks.gate), expert_mat(up, u, marks.up), 2, p, ncols, st);
     }
     ExpertCols q = p;
     q.x = (const char *) g; q.x2 = u; q.x_tok = 4ll * n_used * N; q.x_slot = 4ll * N;
     q.rows_per_expert = H; q.cap_bytes = unit_cap(down);
     q.early_ids = true; // the ids precede the gate / up launch, whose outputs are the only thing this launch waits for
-    launch_units<1, 16, false, float, true>(expert_mat(down, ys), expert_mat(down, ys), 1, q, ncols, st);
+    if (marks.down && n_used <= COMBINE_SLOTS && ncols <= g_parts_max_cols && !(peers && peers->n_peers > 0)) {
+        launch_chained(k_down_combine, dim3((unsigned) (H / down.R), (unsigned) n_tok), dim3((unsigned) n_used * 64), part_smem(2 * n_used, n_used, q.cap_bytes).end,
+                       st, expert_mat(down, nullptr, marks.down), q, weights, (char *) y, y_bf16, Opaque{1u, 4u});
+        check_launch();
+        return;
+    }
+    launch_units<1, 16, false, float, true>(expert_mat(down, ys, marks.down), expert_mat(down, ys, marks.down), 1, q, ncols, st);
     const dim3 grid((unsigned) std::min<int64_t>((H + 255) / 256, 64), (unsigned) n_tok);
     launch_chained(k_combine_f32, grid, dim3(256), 0, st, ys, weights, (char *) y, y_bf16, n_used, H, make_peer_out(peers));
 }

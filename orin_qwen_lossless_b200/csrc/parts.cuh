@@ -37,12 +37,12 @@ struct PartSmem { uint32_t bars, starts, streams, end; };
 __host__ __device__ inline PartSmem part_smem(int warps, int units, uint32_t cap) {
     PartSmem s;
     s.bars = 4 * HP_MAX_PAIRS;
-    s.starts = s.bars + 64;
+    s.starts = s.bars + 16 * 8;
     s.streams = s.starts + 2 * warps * 128;
     s.end = s.streams + 2 * units * (cap + PART_SLACK);
     return s;
 }
-constexpr int PART_UNITS = 4;                 // units of a block at a time, at most
+constexpr int PART_UNITS = 8;                 // units of a block at a time, at most
 
 // Where one warp's part of a unit begins.
 struct PartStart {
@@ -76,15 +76,27 @@ struct PartPlane {
     }
 };
 
+__device__ __forceinline__ void stage_table(unsigned char * smem, const uint32_t * lut) {
+    for (int i = threadIdx.x; i < HP_MAX_PAIRS / 4; i += blockDim.x) { ((uint4 *) smem)[i] = __ldg((const uint4 *) lut + i); }
+}
+
+// the unit, of those that a block takes at a time, that this warp works on
+__device__ __forceinline__ int64_t first_unit(const Parts & p) {
+    const int per_block = (int) (blockDim.x >> 5) / p.parts;
+    return (int64_t) blockIdx.x * per_block + (int) (threadIdx.x >> 5) / p.parts;
+}
+
 // Every block takes units in turn, one warp to a part, all parts of a unit at once; the next unit's streams are copied, its plane
 // asked for and its start looked up while this one is decoded, and one block barrier a unit carries the check of its marks.
-//   prologue()                  what else the block needs, and the wait for the kernel in front; the barrier behind it is here
+//   u, units, unit0             this warp's (first) unit, where units end, and the matrix's unit that is unit 0
+//   prologue()                  what else the block needs, and the wait for the kernel in front; the barrier behind it is here. The
+//                               code table (stage_table) is at the front of the shared memory before that barrier
 //   decode(rd, lut, pl, u, s)   the 64 codes of part s
-//   store(u, s)                 after the check: results that decode() kept
+//   store(u, s, alone)          after the check: results that decode() kept; alone: this warp decodes all parts, s is the last so far
 // LOOP = false: a block has one turn (as many blocks as it takes), and nothing of a next one is kept in registers.
 template <bool LOOP, typename Prologue, typename Decode, typename Store>
-__device__ __forceinline__ void walk_parts(const Parts & p, int64_t unit0, int64_t units, int unit_bytes, unsigned char * smem, Prologue && prologue,
-                                           Decode && decode, Store && store) {
+__device__ __forceinline__ void walk_parts(const Parts & p, int64_t u, int64_t units, int64_t unit0, int unit_bytes, unsigned char * smem,
+                                           Prologue && prologue, Decode && decode, Store && store) {
     __shared__ int broken[3][PART_UNITS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5, per_block = nwarp / p.parts;
     const int ul = warp / p.parts, part = warp - ul * p.parts;
@@ -92,8 +104,7 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t unit0, int64
     const uint32_t base = smem_u32(smem), bar = base + lay.bars + 16 * ul, buf0 = base + lay.streams + 2 * ul * (p.cap + PART_SLACK);
     const uint32_t starts0 = base + lay.starts + warp * 128 + lane * 4;
     const int64_t stride = (int64_t) gridDim.x * per_block;
-    int64_t u = (int64_t) blockIdx.x * per_block + ul;
-    const int rounds = !LOOP ? 1 : (int) ((units - (int64_t) blockIdx.x * per_block + stride - 1) / stride); // the same for every warp of the block
+    const int rounds = !LOOP ? 1 : (int) ((units - (u - ul) + stride - 1) / stride); // the same for every warp of the block
     const uint8_t * plane = p.w.plane + part * (PART_STEPS * CHUNK) + 16 * lane;
 
     bool dead = false; // a copy never arrived (reported): this warp's units are decoded from global memory from then on
@@ -113,12 +124,11 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t unit0, int64
     PartStart cur = {};
     PartPlane pl = {};
     if (u < units) {
+        pl.load(plane + (unit0 + u) * unit_bytes); // ahead of the start, whose trip to memory the streams' copy waits for
         cur.load(p, unit0 + u, part, lane);
         announce(cur, 0);
-        pl.load(plane + (unit0 + u) * unit_bytes);
         if (lane == 0) { bulk_prefetch_l2(pl.cur - 16 * lane + PART_AHEAD * CHUNK, (PART_STEPS - PART_AHEAD) * CHUNK); }
     }
-    for (int i = threadIdx.x; i < HP_MAX_PAIRS / 4; i += blockDim.x) { ((uint4 *) smem)[i] = __ldg((const uint4 *) p.w.lut + i); }
     if (threadIdx.x < 3 * PART_UNITS) { ((int *) broken)[threadIdx.x] = 0; }
     prologue();
     __syncthreads();
@@ -155,7 +165,7 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t unit0, int64
         __syncthreads();
         if (threadIdx.x < PART_UNITS) { broken[slot == 0 ? 2 : slot - 1][threadIdx.x] = 0; } // read before this barrier, used after the next
         if (active && staged && !broken[slot][ul]) {
-            store(u, part);
+            store(u, part, false);
         } else if (active && part == 0) { // streams longer than the buffer, or marks that are not this matrix's: the unit from its start
             GlobalReader rd;
             rd.lut = (const uint32_t *) smem;
@@ -165,7 +175,7 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t unit0, int64
                 pl.load(plane + (unit0 + u) * unit_bytes + s * (PART_STEPS * CHUNK));
                 pl.next = pl.cur;
                 decode(rd, 0u, pl, u, s);
-                store(u, s);
+                store(u, s, true);
             }
             if (LOOP) { pl.load(next); }
         } else if (LOOP && !staged) {

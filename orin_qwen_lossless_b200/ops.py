@@ -838,12 +838,9 @@ def moe_decode(x: torch.Tensor, gate: Weight, up: Weight, down: Weight, n_expert
             raise RuntimeError("bf16n.moe_decode: out must be contiguous")
         if out.dtype not in (torch.float32, torch.bfloat16) or out.device.type != "cuda":
             raise RuntimeError("bf16n.moe_decode: out must be an f32 or bf16 CUDA tensor")
-    args = (C.byref(cg), C.byref(cu), C.byref(cd), x.data_ptr(), int(x.dtype == torch.bfloat16), x.stride(0) * x.element_size(),
+    args = (C.byref(cg), C.byref(cu), C.byref(cd), gate.marks_ptr(), up.marks_ptr(), down.marks_ptr(), x.data_ptr(), int(x.dtype == torch.bfloat16), x.stride(0) * x.element_size(),
             router_logits.data_ptr() if router_logits is not None else None, n_experts, topk_ids.data_ptr(), topk_weights.data_ptr(),
             T, top_k, expert_lo, n_local, scratch.data_ptr(), scratch.numel() * 4, y.data_ptr(), int(y.dtype == torch.bfloat16))
     with torch.cuda.device(dev):
-        if peers is None:
-            check(lib().bf16n_moe_decode(*args, _stream()))
-        else:
-            check(lib().bf16n_moe_decode_peers(*args, C.byref(peers), _stream()))
+        check(lib().bf16n_moe_decode_marked(*args, None if peers is None else C.byref(peers), _stream()))
     return y, topk_weights, topk_ids

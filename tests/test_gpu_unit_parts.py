@@ -62,6 +62,28 @@ def test_marks_change_nothing(ops, rows, K, R, cm, wide):
     assert ops.fault_status() == 0
 
 
+@pytest.mark.parametrize("T", [1, 3, 8])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_decode_step_of_experts(ops, T, dtype):
+    E, k, lo, n = 12, 4, 3, 7       # a slice of the experts: slots routed elsewhere are zeros
+    ws = [_made(ops, n * r, K, R, cm)[1] for r, K, R, cm in ((512, 2048, 8, True), (512, 2048, 8, True), (2048 - 16, 512, 16, False))]
+    x = torch.randn(T, 2048, device="cuda").to(dtype)
+    ids = torch.stack([torch.randperm(E, device="cuda")[:k] for _ in range(T)]).to(torch.int32)
+    weights = torch.rand(T, k, device="cuda")
+    routed = (ids - lo).clamp(0, n - 1)
+
+    def call():
+        step = ops.moe_decode(x, *ws, E, k, topk_weights=weights, topk_ids=ids, expert_lo=lo, n_experts_local=n)[0]
+        return [step, ops.mmv(x, ws[0], routed, 512), ops.mmv(torch.randn(T, k, 512, generator=torch.Generator().manual_seed(1)).cuda().to(dtype), ws[2], routed, 2032)]
+
+    good, ws = ws, [ops.Weight(w.plane, w.aux, w.meta) for w in ws]
+    want = call()
+    for marks in zip(*(_marks(ops, w) for w in good)):
+        ws = [ops.Weight(w.plane, w.aux, w.meta, m.view(torch.uint8)) for w, m in zip(good, marks)]
+        assert all(torch.equal(a, b) for a, b in zip(call(), want))
+    assert ops.fault_status() == 0
+
+
 def test_a_swapped_matrix_needs_no_new_marks(ops):
     rows, K = 1024, 2048
     _, a = _made(ops, rows, K, 16, False)
