@@ -669,7 +669,7 @@ static bool mid_size_by_column(const bf16n_weight & w, const bf16n_mmv_args & a,
 }
 
 template <typename TX>
-void launch_gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers) {
+void launch_gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers, const uint16_t * marks) {
     const Cols p = make_cols(a, peers);
     if (peers && peers->n_peers > 0) {
         require(w.format == FMT_HUFPAIR && !w.cm && !a.ids, "peer outputs need a dense row-major HUFPAIR product");
@@ -689,7 +689,7 @@ void launch_gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t 
             }
 #undef CM
         } else if (gemv_rings_enabled() && gemv_rings_applies(w, a)) {
-            gemv_rings(w, a, st, multi_col, peers); // large matrices, BF16 activations: 1, 2 or 4 columns per decode
+            gemv_rings(w, a, st, multi_col, peers, marks); // large matrices, BF16 activations: 1, 2 or 4 columns per decode
             return;
         } else if (!a.ids && a.ncols > 1 && multi_col && !mid_size_by_column(w, a, units)) {
             unit_geometry(units, 1, 16, grid, threads);
@@ -813,7 +813,7 @@ void gemv_init() {
 
 void gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers, const uint16_t * marks) {
     if (!(peers && peers->n_peers > 0) && (multi_col || a.ncols == 1) && gemv_parts_applies(w, marks, a)) { gemv_parts(w, marks, a, st); return; }
-    if (a.x_bf16) { launch_gemv<bf16>(w, a, st, multi_col, peers); } else { launch_gemv<float>(w, a, st, multi_col, peers); }
+    if (a.x_bf16) { launch_gemv<bf16>(w, a, st, multi_col, peers, marks); } else { launch_gemv<float>(w, a, st, multi_col, peers, marks); }
 }
 
 // ---------------------------------------------------------------- several independent small products in one launch

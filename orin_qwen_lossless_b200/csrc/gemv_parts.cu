@@ -191,6 +191,11 @@ void gemv_parts_init() {
     allow_dynamic_smem((const void *) k_expand_parts<StoreBF16, 512>, optin, optin, "parts");
 }
 
+int unit_parts(const bf16n_weight & w) {
+    const int64_t steps = w.R * (w.K / CHUNK);
+    return w.format == FMT_HUFPAIR && !w.fo && steps % PART_STEPS == 0 && steps >= 2 * PART_STEPS && steps <= 16 * PART_STEPS ? (int) (steps / PART_STEPS) : 0;
+}
+
 size_t marks_bytes(const bf16n_weight & w) {
     const int parts = unit_parts(w);
     return parts ? (size_t) (w.rows / w.R) * (parts - 1) * 32 * sizeof(uint16_t) : 0;
@@ -205,14 +210,17 @@ void marks_build(const bf16n_weight & w, uint16_t * marks, cudaStream_t st) {
 // Where the parts are the faster form, by units of the product. Whole units / parts in us (16 rows to a unit):
 //   1 column:  8192 x 2048 20.2 / 9.1, 16384 x 2048 22.1 / 17.0, 24576 x 2048 25.3 / 25.9; 16384 x 1024 12.7 / 9.0, 32768 x 1024
 //              15.7 / 16.6: up to 1024 units. FP32 activations the same: 23.3 / 20.5 and 26.8 / 30.9 for 1024 and 1536 units.
-//   2:         24576 x 2048 32.0 / 28.4, 32768 x 2048 35.6 / 35.2, 62080 x 2048 68.6 / 63.0; 65536 x 1024 45.5 / 37.8
+//   2:         24576 x 2048 32.0 / 28.4, 32768 x 2048 35.6 / 35.2, 47360 x 2048 42.0 / 50.2; 65536 x 1024 45.5 / 37.8 (36.5 with the last
+//              round of whole units in parts), 65536 x 512 28.7 / 23.2
 //   4:         16384 x 2048 32.3 / 25.2, 24576 x 2048 36.5 / 36.2, 32768 x 2048 41.2 / 44.8 (3 columns: decoded twice without parts)
 //   8:         8192 x 2048 55 / 20.8, 62080 x 2048 156.7 / 126.9 (two decodes of four columns without parts)
 //   4096 columns of weights have no other form that stages streams: 8192 x 4096 82 / 18, 16384 x 4096 89 / 34.
 bool gemv_parts_applies(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a) {
     const int C = (int) (w.K / CHUNK), parts = unit_parts(w);
     if (!marks || !parts || parts > (C == 8 ? 2 : 1) * PART_WARPS || w.cm || a.ids || a.ncols > 8 || !(C == 1 || C == 2 || C == 4 || C == 8)) { return false; }
-    return a.nrows / w.R <= (C < 8 && (a.ncols == 1 || a.ncols == 4) ? 1024 : 4096);
+    const int64_t units = a.nrows / w.R;
+    if (C < 8 && a.ncols == 2) { return units <= 4096 && units * C <= 6144; }
+    return units <= (C < 8 && (a.ncols == 1 || a.ncols == 4) ? 1024 : 4096);
 }
 
 void gemv_parts(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a, cudaStream_t st) {

@@ -66,6 +66,8 @@ __device__ __forceinline__ void fma_bf16x2(uint32_t w, uint32_t x, float & lo, f
         : "+f"(lo), "+f"(hi) : "r"(w), "r"(x));
 }
 
+__device__ __forceinline__ void group_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
 // Measured alternatives that lost (248320 x 2048, one column, 174 us as built): activations widened to FP32 in tensor
 // memory with plain fma 183 us (three more instructions per pair of weights); 32 warps of 64 registers 192 us; plane
 // bytes prefetched two chunks ahead instead of a row 179 us; activations read from shared memory 184 us; one table 178 us.
@@ -76,14 +78,17 @@ __host__ __device__ constexpr int tmem_cols(int C, int NC) { // per lane: 8 C wo
 }
 
 // One unit per warp. NC dense columns share the decode (NC = 1 also serves routed columns: blockIdx.y picks the column).
-template <int C, int NT, int NC, bool PEERS = false> // PEERS: the output also goes to the other GPUs (a separate instantiation: the plain kernel carries none of it)
-__global__ void __launch_bounds__(NT, 1) k_pair_gemv_rings(const PairView w, int R, Cols p, const Opaque k) {
+// PEERS: the output also goes to the other GPUs; CUT: the last round's units in parts (separate instantiations: the plain kernel carries none of it)
+template <int C, int NT, int NC, bool PEERS = false, bool CUT = false>
+__global__ void __launch_bounds__(NT, 1) k_pair_gemv_rings(const PairView w, const AuxHeader * hdr, int R, Cols p, const uint16_t * marks, int parts, int mark_stride, const Opaque k) {
     constexpr int K = C * CHUNK;
     constexpr int XW = C * 8;           // TMEM words per column and lane
     constexpr int STEPS = 2 * C * NC;   // four-word TMEM loads per row: one per (half chunk, column)
     constexpr uint32_t TCOLS = tmem_cols(C, NC);
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint32_t tmem_slot;
+    __shared__ uint16_t starts[CUT ? NT : 1]; // the mark that a warp's part started from, per lane
+    __shared__ int broken[2][CUT ? NT / 64 : 1];
     uint32_t * lut = (uint32_t *) smem; // four interleaved tables | NC x K BF16 activations | one 4 KB ring set per warp
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const uint32_t lut_s = smem_u32(lut);
@@ -126,27 +131,46 @@ __global__ void __launch_bounds__(NT, 1) k_pair_gemv_rings(const PairView w, int
     uint4 xa, xb = make_uint4(0, 0, 0, 0);
     tmem_ld4(x_addr(0), xa);
 
-    const int64_t units = p.nrows / R;
-    // warp w of block b takes units w * blocks + b, + blocks * warps, ...: a matrix with few units still reaches every SM
-    for (int64_t u = (int64_t) warp * gridDim.x + blockIdx.x; u < units; u += (int64_t) gridDim.x * nwarp) {
-        const int64_t g = rbase / R + u;
+    // Unit i of block b is unit i * blocks + b of the product, so that a matrix with few units still reaches every SM. Warps take whole
+    // units in rounds; with marks (parts.cuh), the units that would leave the last round partly empty go to groups of `parts` warps, a
+    // warp to a part of whole rows.
+    const int64_t units = p.nrows / R, own = (units - blockIdx.x + gridDim.x - 1) / gridDim.x, whole = CUT ? own / nwarp * nwarp : own;
+    const int groups = CUT ? nwarp / parts : 0, group = CUT ? warp / parts : 0, part = warp - group * parts, part_rows = CUT ? R / parts : R;
+    int64_t i = warp;
+    bool again = false; // the unit of a broken group once more, by its first warp alone
+    for (int turn = 0;;) {
+        const bool cut = CUT && i >= whole;
+        if (!CUT && i >= own) { break; }
+        if (cut && !again) {
+            if (turn == 0) { i = whole + group; }
+            if (group >= groups || i >= own) { break; }
+        }
+        const int64_t u = i * gridDim.x + blockIdx.x, g = rbase / R + u;
+        const int r0 = cut && !again ? part * part_rows : 0, r1 = cut && !again ? r0 + part_rows : R;
+        const uint32_t at = cut && part && !again ? __ldg(marks + (g * (mark_stride * parts - 1) + part * mark_stride - 1) * 32 + lane) : 0u;
+        if (cut) { starts[warp * 32 + lane] = (uint16_t) at; }
         RingReader rd;
+        uint32_t first;
         {
             const uint32_t w0 = __ldg(w.ubase + g), l0 = __ldg(w.lrel + g * 32 + lane);
-            rd.open((const uint8_t *) (w.stream + (w0 & ~3u)), ((w0 & 3u) + l0) * 4u, key, k);
+            first = ((w0 & 3u) + l0) * 4u;
+            // a wrong mark: no granule behind the stream's padding is copied (bytes from the unit's base)
+            const uint32_t last = cut ? (min((uint32_t) hdr->n_b + HP_TAIL_WORDS - 4u - (w0 & ~3u), 1u << 28) * 4u) & ~15u : ~15u;
+            rd.open((const uint8_t *) (w.stream + (w0 & ~3u)), first + (at >> 5) * 4u, key, k, last);
         }
         cp_async_commit();
-        const uint8_t * pl = w.plane + g * R * K + 16 * lane;
+        const uint8_t * pl = w.plane + (g * R + r0) * K + 16 * lane;
         uint4 nx[C]; // plane bytes one row ahead of the decode
 #pragma unroll
         for (int c = 0; c < C; c++) { nx[c] = ld_stream16(pl + c * CHUNK); }
         rd.token = cp_async_wait_all();
         rd.first_words();
+        rd.o = at & 31u;
         float mine[NC];
 #pragma unroll
         for (int n = 0; n < NC; n++) { mine[n] = 0.f; }
-        for (int rr = 0; rr < R; rr++) {
-            if (rr) {
+        for (int rr = r0; rr < r1; rr++) {
+            if (rr != r0) {
                 rd.token = cp_async_wait_all(); // copies issued one row ago
                 rd.template top_up<3>(k);
                 cp_async_commit();
@@ -154,7 +178,7 @@ __global__ void __launch_bounds__(NT, 1) k_pair_gemv_rings(const PairView w, int
             float a[NC][4];
 #pragma unroll
             for (int n = 0; n < NC; n++) { a[n][0] = a[n][1] = a[n][2] = a[n][3] = 0.f; }
-            const uint8_t * nrow = pl + (rr + 1 < R ? rr + 1 : rr) * K;
+            const uint8_t * nrow = pl + (rr + 1 < r1 ? rr + 1 - r0 : rr - r0) * K;
 #pragma unroll
             for (int c = 0; c < C; c++) {
                 const uint4 sm = nx[c];
@@ -191,7 +215,19 @@ __global__ void __launch_bounds__(NT, 1) k_pair_gemv_rings(const PairView w, int
                 if (lane == rr) { mine[n] = s; }
             }
         }
-        if (lane < R) {
+        if (CUT && cut && !again) { // did every part end where the next one began?
+            int & bad = broken[turn & 1][group];
+            if (part == 0 && lane == 0) { bad = 0; } // last read before the barriers of the turn before
+            group_sync(1 + group, parts * 32);
+            if (part + 1 < parts && !__all_sync(FULL, (uint16_t) rd.position(first) == starts[(warp + 1) * 32 + lane]) && lane == 0) { bad = 1; }
+            group_sync(1 + group, parts * 32);
+            if (bad) {
+                if (part == 0) { again = true; continue; }
+                i += groups; turn++;
+                continue;
+            }
+        }
+        if (lane >= r0 && lane < r1) {
 #pragma unroll
             for (int n = 0; n < NC; n++) {
                 const OutVec o = {out.p + n * p.y_tok, out.bf16};
@@ -199,6 +235,9 @@ __global__ void __launch_bounds__(NT, 1) k_pair_gemv_rings(const PairView w, int
                 if (PEERS) { peers_put(p, (NC == 1 ? (int) blockIdx.y : 0) + n, u * R + lane, mine[n]); }
             }
         }
+        i += cut ? groups : nwarp;
+        turn += cut;
+        again = false;
     }
     tmem_ld_wait(xa);
     tmem_fence_before();
@@ -220,7 +259,8 @@ constexpr int g_warps = 28; // most warps per block (72 registers per thread)
 void gemv_rings_init() {
     const int optin = device_info().smem_optin;
 #define ATTR(CC, NT, NC) allow_dynamic_smem((const void *) k_pair_gemv_rings<CC, NT, NC>, optin, optin, "rings"); \
-                         allow_dynamic_smem((const void *) k_pair_gemv_rings<CC, NT, NC, true>, optin, optin, "rings");
+                         allow_dynamic_smem((const void *) k_pair_gemv_rings<CC, NT, NC, true>, optin, optin, "rings"); \
+                         allow_dynamic_smem((const void *) k_pair_gemv_rings<CC, NT, NC, false, true>, optin, optin, "rings");
     RINGS_FOR_EACH(ATTR)
 #undef ATTR
 }
@@ -243,7 +283,7 @@ bool gemv_rings_applies(const bf16n_weight & w, const bf16n_mmv_args & a) {
 namespace {
 
 // nc dense columns starting at p.x / p.y (nc = 1: also `ncols_grid` routed or dense columns, one decode each)
-void launch_rings(const bf16n_weight & w, const Cols & p, int nc, int ncols_grid, cudaStream_t st) {
+void launch_rings(const bf16n_weight & w, const Cols & p, int nc, int ncols_grid, cudaStream_t st, const uint16_t * marks) {
     const int64_t units = p.nrows / w.R, sms = device_info().sms;
     const int cap = nc == 1 ? (w.K == 2048 ? g_warps : std::min(g_warps, 28)) : nc == 2 ? std::min(g_warps, 24) : std::min(g_warps, 20);
     const int max_warps = std::max(4, cap);
@@ -258,12 +298,32 @@ void launch_rings(const bf16n_weight & w, const Cols & p, int nc, int ncols_grid
         const double eff = (double) units / (double) (rounds * slots) * (1.0 - 0.01 * (max_warps - nw));
         if (eff > best_eff + 1e-9) { best_eff = eff; best = nw; }
     }
+    // In rounds of a full block: a round of n units costs about 0.4 + 0.6 n / max_warps (its chain's length, whatever shares the SM); cut
+    // into four parts each, as many units at a time as there are groups of four warps, a turn costs 0.28 / 0.26 / 0.22 for one, two
+    // and four columns. A gain of less than 4.5 % is not sure. Measured, whole units / parts in us by units of 16 x 2048 per SM: one column, 28 warps: 29: 67.8 / 55.8, 34:
+    // 70.2 / 60.4, 57: 107.6 / 97.6, but 47 (three turns): 79.3 / 85.4; two columns, 24 warps: 29: 71.1 / 57.9, 37 (three turns): 76.2 /
+    // 78.9; four columns, 20 warps: 23: 76.8 / 59.9, 27 (two turns): 80.6 / 71.0, 37 (four turns): 91.3 / 100.6. Units of two parts gain nothing.
+    const int all_parts = marks && ncols_grid == 1 && !p.ids && !p.peers.n ? unit_parts(w) : 0, mark_stride = all_parts / 4;
+    int parts = 0;
+    if (all_parts >= 4 && all_parts % 4 == 0 && w.R % 4 == 0) {
+        const double turn = nc == 1 ? 0.28 : nc == 2 ? 0.26 : 0.22;
+        const int64_t own = (units + sms - 1) / sms;
+        auto round = [&](int64_t n) { return n ? 0.4 + 0.6 * (double) n / max_warps : 0.0; };
+        double least = 0.955 * ((double) (own / best) * round(best) + round(own % best));
+        for (int nw = max_warps; nw >= std::max(4, max_warps - 3); nw--) {
+            const int64_t rest = own % nw, groups = nw / 4;
+            const double cost = (double) (own / nw) * round(nw) + turn * (double) ((rest + groups - 1) / groups);
+            if (own >= nw && rest && cost < least) { least = cost; best = nw; parts = 4; }
+        }
+    }
     const dim3 grid((unsigned) sms, (unsigned) ncols_grid);
     const size_t shm = fixed_smem(w.K, nc) + (size_t) best * RING_SET;
     const Opaque k = {1u, 4u, ~0u, 16u};
     const PairView v = pair_view(w);
-#define GO(CC, NT, NC) if (p.peers.n) { k_pair_gemv_rings<CC, NT, NC, true><<<grid, best * 32, shm, st>>>(v, w.R, p, k); } \
-                       else { k_pair_gemv_rings<CC, NT, NC, false><<<grid, best * 32, shm, st>>>(v, w.R, p, k); }
+    const AuxHeader * hdr = (const AuxHeader *) w.aux;
+#define GO(CC, NT, NC) if (p.peers.n) { k_pair_gemv_rings<CC, NT, NC, true><<<grid, best * 32, shm, st>>>(v, hdr, w.R, p, marks, parts, mark_stride, k); } \
+                       else if (parts > 1) { k_pair_gemv_rings<CC, NT, NC, false, true><<<grid, best * 32, shm, st>>>(v, hdr, w.R, p, marks, parts, mark_stride, k); } \
+                       else { k_pair_gemv_rings<CC, NT, NC, false><<<grid, best * 32, shm, st>>>(v, hdr, w.R, p, marks, parts, mark_stride, k); }
     const int C = (int) (w.K / CHUNK);
     if (nc == 4) { switch (C) { case 1: GO(1, 640, 4); break; case 2: GO(2, 640, 4); break; default: GO(4, 640, 4); break; } }
     else if (nc == 2) { switch (C) { case 1: GO(1, 768, 2); break; case 2: GO(2, 768, 2); break; default: GO(4, 768, 2); break; } }
@@ -275,10 +335,10 @@ void launch_rings(const bf16n_weight & w, const Cols & p, int nc, int ncols_grid
 
 } // namespace
 
-void gemv_rings(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers) {
+void gemv_rings(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers, const uint16_t * marks) {
     const Cols p = make_cols(a, peers);
     if (a.ids || a.ncols == 1 || !multi_col || (peers && peers->n_peers > 0)) { // one decode per column
-        launch_rings(w, p, 1, a.ncols, st);
+        launch_rings(w, p, 1, a.ncols, st, marks);
         return;
     }
     for (int c0 = 0; c0 < a.ncols;) { // dense columns: four, two or one per decode
@@ -286,7 +346,7 @@ void gemv_rings(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t s
         Cols q = p;
         q.x += c0 * p.x_tok;
         q.y += c0 * p.y_tok;
-        launch_rings(w, q, nc, 1, st);
+        launch_rings(w, q, nc, 1, st, marks);
         c0 += nc;
     }
 }

@@ -74,6 +74,7 @@ void expand_rows(const bf16n_weight & w, int64_t row0, int64_t nrows, const dev:
 
 // gemv_parts.cu: few units, whose marks cut the lane streams (marks: null, or marks_bytes(w) bytes that marks_build wrote)
 void gemv_parts_init();
+int unit_parts(const bf16n_weight & w);    // parts of a unit, 0 when this layout is not cut
 size_t marks_bytes(const bf16n_weight & w); // 0: this layout has none
 void marks_build(const bf16n_weight & w, uint16_t * marks, cudaStream_t st);
 bool gemv_parts_applies(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a);
@@ -112,7 +113,7 @@ void gemv_staged(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t 
 void gemv_rings_init();
 bool gemv_rings_enabled();
 bool gemv_rings_applies(const bf16n_weight & w, const bf16n_mmv_args & a);
-void gemv_rings(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers = nullptr);
+void gemv_rings(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool multi_col, const bf16n_peer_out * peers = nullptr, const uint16_t * marks = nullptr);
 
 // fo.cu: fragment-order HUFPAIR tensors
 void fo_init();

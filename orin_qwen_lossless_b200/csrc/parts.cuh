@@ -177,7 +177,7 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t u, int64_t u
                 decode(rd, 0u, pl, u, s);
                 store(u, s, true);
             }
-            if (LOOP) { pl.load(next); }
+            if (LOOP) { pl.load(next); pl.next = next; }
         } else if (LOOP && !staged) {
             pl.load(pl.next);
         }
@@ -188,12 +188,6 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t u, int64_t u
 
 } // namespace dev
 
-// Host: parts of a unit, 0 when this layout is not cut
-inline int unit_parts(const bf16n_weight & w) {
-    const int64_t steps = w.R * (w.K / CHUNK);
-    return w.format == FMT_HUFPAIR && !w.fo && steps % dev::PART_STEPS == 0 && steps >= 2 * dev::PART_STEPS && steps <= 16 * dev::PART_STEPS
-               ? (int) (steps / dev::PART_STEPS) : 0;
-}
 inline dev::Parts make_parts(const bf16n_weight & w, const uint16_t * marks) {
     return {dev::pair_view(w), (const AuxHeader *) w.aux, marks, unit_parts(w), (uint32_t) ((w.R * w.K * 3 / 8 + 64 + 15) & ~15ll)};
 }

@@ -78,6 +78,7 @@ struct RingReader {
     const uint8_t * base; // global
     uint32_t key;         // ring base | lane swizzle
     uint32_t fetched;     // offset of the next granule to copy
+    uint32_t limit;       // offset of the last granule that the aux buffer holds: a reader started by a wrong mark stays below it
     uint32_t next;        // offset of the next word to read
     uint32_t hi, lo, ahead, o;
     uint32_t token;       // from the last cp.async wait
@@ -89,15 +90,15 @@ struct RingReader {
 #pragma unroll
         for (int i = 0; i < ROUNDS; i++) {
             if (avail <= (int32_t) RING_TARGET) {
-                cp_async16(ring_addr(fetched, key), base + fetched);
+                cp_async16(ring_addr(fetched, key), base + min(fetched, limit));
                 fetched = imad(k.sixteen, k.one, fetched);
                 avail = (int32_t) imad(k.sixteen, k.one, (uint32_t) avail);
             }
         }
     }
     // start of a unit: offset of this lane's first word; the caller commits, waits and then calls first_words()
-    __device__ __forceinline__ void open(const uint8_t * unit_base, uint32_t first, uint32_t ring_key, const Opaque & k) {
-        base = unit_base; key = ring_key;
+    __device__ __forceinline__ void open(const uint8_t * unit_base, uint32_t first, uint32_t ring_key, const Opaque & k, uint32_t last = ~15u) {
+        base = unit_base; key = ring_key; limit = last;
         fetched = first & ~15u;
         next = first;
         top_up<7>(k);
@@ -108,6 +109,8 @@ struct RingReader {
         ahead = lds32(ring_addr(next + 8, key), token);
         next += 12; o = 0;
     }
+    // bits from the word at offset `first` to the next code
+    __device__ __forceinline__ uint32_t position(uint32_t first) const { return (next - 12u - first) * 8u + (o & 31u); }
     // two codes: their table entries. `lut`: this lane's copy of the table (entries 16 bytes apart)
     __device__ __forceinline__ void take2(uint32_t lut, const Opaque & k, uint32_t & e0, uint32_t & e1) {
         const uint32_t v1 = shl_wrap_hi(lo, hi, o);          // 32 valid bits from the offset on: two codes are at most 24

@@ -84,6 +84,18 @@ def test_decode_step_of_experts(ops, T, dtype):
     assert ops.fault_status() == 0
 
 
+@pytest.mark.parametrize("rows,K,R", [(148 * 28 * 16 + 16 * 333, 512, 16), (148 * 20 * 16 + 16 * 700, 1024, 16), (148 * 24 * 8 + 8 * 149, 2048, 8),
+                                      (62080, 2048, 16)])
+def test_last_round_of_a_large_product(ops, rows, K, R):
+    _, w = _made(ops, rows, K, R, False)
+    plain = ops.Weight(w.plane, w.aux, w.meta)
+    xs = [torch.randn(T, K, device="cuda").to(torch.bfloat16) for T in (1, 2, 4)]
+    want = [ops.mmv(x, plain) for x in xs]
+    for marks in _marks(ops, w):
+        w.marks = marks.view(torch.uint8)
+        assert all(torch.equal(ops.mmv(x, w), y) for x, y in zip(xs, want))
+
+
 def test_a_swapped_matrix_needs_no_new_marks(ops):
     rows, K = 1024, 2048
     _, a = _made(ops, rows, K, 16, False)
