@@ -130,7 +130,7 @@ def lib():
     global _lib
     if _lib is None:
         path = _build.LIB
-        if not os.path.exists(path):
+        if not (os.path.exists(path) and os.path.exists(_build.CALLS)):
             _build.build()
         _lib = C.CDLL(path)
         for name, (res, args) in SIGNATURES.items():
@@ -138,6 +138,13 @@ def lib():
             fn.restype = res
             fn.argtypes = args
     return _lib
+
+
+def calls():
+    """The extension module of the calls that the host bounds (csrc/host_calls.cpp)."""
+    lib()
+    from . import _calls
+    return _calls
 
 
 def check(rc: int) -> None:

@@ -91,6 +91,19 @@ class Weight:
                        int(m.frag_order), m.off_a, m.off_b, m.off_c, m.off_d)
 
 
+_calls = None
+
+
+def _native():
+    """mmv, linear and draft_logits in native code; they return None for calls that the Python functions are to see."""
+    global _calls
+    if _calls is None:
+        m = _lib.calls()
+        m.register(Weight, Meta)
+        _calls = m
+    return _calls
+
+
 def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
@@ -338,6 +351,10 @@ def _mmv_common(x, w: Weight, ids, rows_per_matrix: int, out_bf16: bool, glu: bo
 
 def mmv(x: torch.Tensor, w: Weight, ids: torch.Tensor | None = None, rows_per_matrix: int = 0,
         out_dtype: torch.dtype = torch.float32, multi_col: bool = True, out: torch.Tensor | None = None) -> torch.Tensor:
+    if ids is None and out is None and not rows_per_matrix:
+        y = (_calls or _native()).mmv(x, w, out_dtype == torch.bfloat16, bool(multi_col))
+        if y is not None:
+            return y
     return _mmv_common(x, w, ids, rows_per_matrix, out_dtype == torch.bfloat16, False, multi_col, out)
 
 
@@ -407,6 +424,9 @@ def mmv_glu2(x: torch.Tensor, gate: Weight, up: Weight, out_dtype: torch.dtype =
 def linear(x: torch.Tensor, w: Weight, bias: torch.Tensor | None = None) -> torch.Tensor:
     """y = x W^T (+ bias) in BF16: up to 8 tokens through the decode GEMV (FP32 accumulation; the bias is added in FP32
     before the single rounding), more through exact dequantisation in 64 MiB row chunks + a BF16 GEMM."""
+    y = (_calls or _native()).linear(x, w, bias, GEMV_MAX_TOKENS, DEQUANT_CHUNK_BYTES)
+    if y is not None:
+        return y
     m = w.meta
     if x.dtype != torch.bfloat16:
         raise RuntimeError("bf16n.linear: x must be bf16")
@@ -570,6 +590,10 @@ def make_draft_head(w: torch.Tensor, bits: int) -> DraftHead:
 def draft_logits(h: torch.Tensor, w: Weight, head: DraftHead, vocab: int) -> torch.Tensor:
     """Draft-token logits: the k-bit head selects candidates, the gathered lossless rows are re-scored in FP32, every
     other entry is -inf. A proposal path: candidate coverage does not guarantee the exact head's argmax."""
+    if type(head) is DraftHead:
+        y = (_calls or _native()).draft_logits(h, w, head.bits, head.q, head.s, head.candidates, vocab)
+        if y is not None:
+            return y
     n, K = h.shape
     h = h.contiguous()
     scores = head.scores(h)
