@@ -140,6 +140,10 @@ size_t bf16n_marks_bytes(const bf16n_weight * w);
 int bf16n_marks_build(const bf16n_weight * w, void * marks, void * stream);
 int bf16n_mmv_marked(const bf16n_weight * w, const void * marks, const bf16n_mmv_args * a, void * stream, int multi_col);
 int bf16n_dequant_marked(const bf16n_weight * w, const void * marks, int64_t row0, int64_t nrows, uint16_t * out, void * stream);
+int bf16n_get_rows_marked(const bf16n_weight * w, const void * marks, const void * ids, int64_t ids_s0, int64_t n, void * dst, int dst_bf16,
+                          int64_t dst_s1, void * stream, int64_t row0);
+int bf16n_draft_logits_marked(const float * scores, int T, int64_t rows, int n_cand, const bf16n_weight * w, const void * marks, const void * x_bf16,
+                              int32_t * cand, void * cand_rows, float * out, int64_t vocab, void * stream);
 /* n independent products on one stream, w[i] with a[i]: the small dense NIBBLE products among them (K 512..4096, up to
  * 8 columns; the per-layer projections and routers that are each too small to fill the GPU) share one grid, eight
  * products per launch, instead of one launch each; everything else is launched as bf16n_mmv would launch it. Results

@@ -66,6 +66,8 @@ SIGNATURES = {
     "bf16n_marks_build": (C.c_int, [C.POINTER(Weight), C.c_void_p, C.c_void_p]),
     "bf16n_mmv_marked": (C.c_int, [C.POINTER(Weight), C.c_void_p, C.POINTER(MmvArgs), C.c_void_p, C.c_int]),
     "bf16n_dequant_marked": (C.c_int, [C.POINTER(Weight), C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
+    "bf16n_get_rows_marked": (C.c_int, [C.POINTER(Weight), C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_int, C.c_int64, C.c_void_p, C.c_int64]),
+    "bf16n_draft_logits_marked": (C.c_int, [C.c_void_p, C.c_int, C.c_int64, C.c_int, C.POINTER(Weight), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]),
     "bf16n_mmv_group": (C.c_int, [C.POINTER(Weight), C.POINTER(MmvArgs), C.c_int, C.c_void_p]),
     "bf16n_mmv_glu_merged": (C.c_int, [C.POINTER(Weight), C.POINTER(MmvArgs), C.c_void_p]),
     "bf16n_mmv_glu": (C.c_int, [C.POINTER(Weight), C.POINTER(Weight), C.POINTER(MmvArgs), C.c_void_p]),

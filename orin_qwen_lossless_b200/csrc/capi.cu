@@ -230,8 +230,8 @@ int bf16n_int2_gemv(const void * x_bf16, int T, const uint8_t * q, const float *
     return guarded([&] { ensure_init(); draft_gemv(2, x_bf16, T, q, s, rows, K, y, (cudaStream_t) stream); });
 }
 
-int bf16n_draft_logits(const float * scores, int T, int64_t rows, int n_cand, const bf16n_weight * w, const void * x_bf16, int32_t * cand,
-                       void * cand_rows, float * out, int64_t vocab, void * stream) {
+int bf16n_draft_logits_marked(const float * scores, int T, int64_t rows, int n_cand, const bf16n_weight * w, const void * marks, const void * x_bf16,
+                              int32_t * cand, void * cand_rows, float * out, int64_t vocab, void * stream) {
     return guarded([&] {
         ensure_init();
         require(scores && w && x_bf16 && cand && cand_rows && out, "draft_logits: null argument");
@@ -244,10 +244,20 @@ int bf16n_draft_logits(const float * scores, int T, int64_t rows, int n_cand, co
         cudaStream_t st = (cudaStream_t) stream;
         draft_select(scores, T, rows, n_cand, cand, out, vocab, st);
         const int64_t n = (int64_t) T * n_cand;
+        if (rows_parts_applies(*w, (const uint16_t *) marks, n)) { // gathered and multiplied in one launch
+            const RowScores s = {x_bf16, n_cand, out, vocab};
+            rows_parts(*w, (const uint16_t *) marks, cand, 4, n, cand_rows, true, w->K * 2, 0, &s, st, true);
+            return;
+        }
         if (frag_order(*w)) { fo_gather_rows(*w, cand, 4, n, cand_rows, true, w->K * 2, 0, st); }
         else { gather_rows(*w, cand, 4, n, cand_rows, true, w->K * 2, 0, st, true); } // behind the selection
         draft_rescore(x_bf16, cand_rows, cand, T, n_cand, (int) w->K, out, vocab, st);
     });
+}
+
+int bf16n_draft_logits(const float * scores, int T, int64_t rows, int n_cand, const bf16n_weight * w, const void * x_bf16, int32_t * cand,
+                       void * cand_rows, float * out, int64_t vocab, void * stream) {
+    return bf16n_draft_logits_marked(scores, T, rows, n_cand, w, nullptr, x_bf16, cand, cand_rows, out, vocab, stream);
 }
 
 int bf16n_set_peer_wait_limit_ms(unsigned int ms) {
@@ -372,8 +382,8 @@ int bf16n_verify(const bf16n_weight * w, int64_t row0, int64_t nrows, const uint
     });
 }
 
-int bf16n_get_rows(const bf16n_weight * w, const void * ids, int64_t ids_s0, int64_t n, void * dst, int dst_bf16, int64_t dst_s1,
-                   void * stream, int64_t row0) {
+int bf16n_get_rows_marked(const bf16n_weight * w, const void * marks, const void * ids, int64_t ids_s0, int64_t n, void * dst, int dst_bf16,
+                          int64_t dst_s1, void * stream, int64_t row0) {
     return guarded([&] {
         ensure_init();
         check_weight(*w);
@@ -383,8 +393,12 @@ int bf16n_get_rows(const bf16n_weight * w, const void * ids, int64_t ids_s0, int
         require(w->format != FMT_HUFFMAN, "get_rows is not implemented for the single-symbol Huffman format");
         if (n == 0) { return; }
         if (frag_order(*w)) { fo_gather_rows(*w, ids, ids_s0, n, dst, dst_bf16 != 0, dst_s1, row0, (cudaStream_t) stream); return; }
-        gather_rows(*w, ids, ids_s0, n, dst, dst_bf16 != 0, dst_s1, row0, (cudaStream_t) stream);
+        gather_rows(*w, ids, ids_s0, n, dst, dst_bf16 != 0, dst_s1, row0, (cudaStream_t) stream, false, (const uint16_t *) marks);
     });
+}
+int bf16n_get_rows(const bf16n_weight * w, const void * ids, int64_t ids_s0, int64_t n, void * dst, int dst_bf16, int64_t dst_s1,
+                   void * stream, int64_t row0) {
+    return bf16n_get_rows_marked(w, nullptr, ids, ids_s0, n, dst, dst_bf16, dst_s1, stream, row0);
 }
 
 int bf16n_mm_ids_supported(const bf16n_weight * w, const bf16n_weight * up) {

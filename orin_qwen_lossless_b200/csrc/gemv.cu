@@ -485,19 +485,6 @@ __global__ void __launch_bounds__(256) k_nib_expand(const NibView w, int C, int6
 
 // gather: dst[i] = W[row0 + ids[i]], FP32 or BF16. A Huffman-coded row is reached by decoding its unit from the start.
 template <bool BF>
-__device__ __forceinline__ void put_row_chunk(char * o, int c, int lane, const uint32_t (&w)[8]) {
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int i = c * CHUNK + 128 * j + 4 * lane;
-        if (BF) {
-            *(uint2 *) (o + 2 * i) = make_uint2(w[2 * j], w[2 * j + 1]);
-        } else {
-            *(float4 *) (o + 4 * i) = make_float4(bf16lo_f32(w[2 * j]), bf16hi_f32(w[2 * j]), bf16lo_f32(w[2 * j + 1]), bf16hi_f32(w[2 * j + 1]));
-        }
-    }
-}
-
-template <bool BF>
 __global__ void __launch_bounds__(256) k_pair_rows(const PairView w, int C, int R, const char * ids, int64_t ids_s0, int64_t n,
                                                     int64_t row0, char * dst, int64_t dst_s1) {
     __shared__ uint32_t lut[HP_MAX_PAIRS];
@@ -924,7 +911,11 @@ void expand_compare(const bf16n_weight & w, int64_t row0, int64_t nrows, const u
 }
 
 void gather_rows(const bf16n_weight & w, const void * ids, int64_t ids_s0, int64_t n, void * dst, bool dst_bf16, int64_t dst_s1,
-                 int64_t row0, cudaStream_t st, bool behind_own) {
+                 int64_t row0, cudaStream_t st, bool behind_own, const uint16_t * marks) {
+    if (rows_parts_applies(w, marks, n)) {
+        rows_parts(w, marks, ids, ids_s0, n, dst, dst_bf16, dst_s1, row0, nullptr, st, behind_own);
+        return;
+    }
     const int C = (int) (w.K / CHUNK);
     const unsigned gx = (unsigned) ((n + 7) / 8);
     const char * ip = (const char *) ids;

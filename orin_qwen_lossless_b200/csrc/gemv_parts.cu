@@ -109,6 +109,21 @@ __global__ void __launch_bounds__(C == 8 ? 512 : 256, parts_resident(C, NC)) k_g
     walk_parts<parts_loop(NC)>(p, first_unit(p), q.nrows / R, q.row0 / R, R * K, smem, prologue, rows, put);
 }
 
+// a BF16 row in shared memory times a token's activations: FP32 sums, as k_rescore of draft.cu adds them
+template <int K>
+__device__ __forceinline__ float row_product(const bf16 * a, const bf16 * b, int lane) {
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int k = lane * 8; k < K; k += 256) {
+        const uint4 p = *(const uint4 *) (a + k), q = ld_act16(b + k);
+        acc[0] = fmaf(bf16lo_f32(p.x), bf16lo_f32(q.x), acc[0]); acc[1] = fmaf(bf16hi_f32(p.x), bf16hi_f32(q.x), acc[1]);
+        acc[2] = fmaf(bf16lo_f32(p.y), bf16lo_f32(q.y), acc[2]); acc[3] = fmaf(bf16hi_f32(p.y), bf16hi_f32(q.y), acc[3]);
+        acc[0] = fmaf(bf16lo_f32(p.z), bf16lo_f32(q.z), acc[0]); acc[1] = fmaf(bf16hi_f32(p.z), bf16hi_f32(q.z), acc[1]);
+        acc[2] = fmaf(bf16lo_f32(p.w), bf16lo_f32(q.w), acc[2]); acc[3] = fmaf(bf16hi_f32(p.w), bf16hi_f32(q.w), acc[3]);
+    }
+    return warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
+}
+
 template <typename Sink, int THREADS> // 512: units of more than eight parts
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_expand_parts(const Parts p, int C, int R, bool cm, int64_t unit0, int64_t units, const Sink sink_in, const Opaque k) {
     Sink sink = sink_in;
@@ -129,6 +144,93 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_expand_parts(const 
         }
     };
     walk_parts<false>(p, first_unit(p), units, unit0, R * C * CHUNK, smem, [&] { stage_table(smem, p.w.lut); }, chunks, [](int64_t, int, bool) {});
+}
+
+// Few rows (a draft step's candidates, the tokens of a decode batch), one block each: the warp of the part that the row lies in
+// passes over the rows before it there and decodes it, the warps of the parts before that only walk their codes, so that the row's
+// start is known to be right when the block meets. 128 candidates of 62080 x 2048: 19.7 us by a walk of up to 15 rows from the unit's
+// start (with a table of the codes that end in 12 bits of stream), 4.7 so. SCORED: the row is multiplied with its token's activations as well.
+template <int C, bool BF, bool SCORED>
+__global__ void __launch_bounds__(512) k_rows_parts(const Parts p, int R, const char * ids, int64_t ids_s0, int64_t row0, char * dst, int64_t dst_s1,
+                                                    const RowScores scores, const Opaque k) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ int broken;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    const PartSmem lay = part_smem(nwarp, 1, p.cap);
+    const uint32_t base = smem_u32(smem), bar = base + lay.bars, words = base + lay.streams, starts = base + lay.starts + warp * 128 + lane * 4;
+    if (threadIdx.x == 0) {
+        broken = 0;
+        mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    stage_table(smem, p.w.lut);
+    grid_dependency_wait(); // the row ids may come from the kernel before this one; everything above is the matrix's own
+    const int64_t gr = row0 + *(const volatile int32_t *) (ids + blockIdx.x * ids_s0), unit = gr / R;
+    const int t0 = (int) (gr - unit * R) * C, part = t0 / PART_STEPS;
+    const uint8_t * pl = p.w.plane + gr * (C * CHUNK) + 16 * lane;
+    PartStart cur = {};
+    uint4 sm[C];
+    if (warp <= part) {
+        if (warp == part) {
+#pragma unroll
+            for (int c = 0; c < C; c++) { sm[c] = ld_stream16(pl + c * CHUNK); }
+        }
+        cur.load(p, unit, warp, lane);
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(starts), "r"(cur.at) : "memory");
+        if (threadIdx.x == 0 && cur.bytes <= p.cap) {
+            mbar_expect_tx(bar, cur.bytes);
+            bulk_g2s(words, p.w.stream + cur.first, cur.bytes, bar);
+        }
+    }
+    __syncthreads();
+    char * o = dst + blockIdx.x * dst_s1;
+    unsigned char * row_s = smem + lay.end; // SCORED: the row as BF16
+    auto row = [&](auto & rd, uint32_t lut, int before) { // `before` steps, then the row
+        for (int i = 0; i < before; i++) { uint32_t e[8]; rd.take8(lut, k, e); }
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            uint32_t e[8], wv[8];
+            rd.take8(lut, k, e);
+            assemble8(sm[c], e, wv);
+            put_row_chunk<BF>(o, c, lane, wv);
+            if (SCORED) { put_row_chunk<true>((char *) row_s, c, lane, wv); }
+        }
+    };
+    if (warp <= part) {
+        bool good = false;
+        if (cur.bytes <= p.cap) {
+            const uint32_t landed = mbar_wait(bar, 0u);
+            if (landed) {
+                WindowReader rd;
+                rd.open_at(words + 4 * min(cur.my + (cur.at >> 5), cur.bytes / 4), cur.at & 31u, landed);
+                if (warp == part) {
+                    row(rd, base, t0 - part * PART_STEPS);
+                    good = true;
+                } else {
+                    for (int i = 0; i < PART_STEPS; i++) { uint32_t e[8]; rd.take8(base, k, e); }
+                    good = __all_sync(FULL, rd.position(words + 4 * cur.my) == lds32(starts + 128, rd.next));
+                }
+            } else if (lane == 0) {
+                atomicOr(&g_wait_expired, 1u);
+            }
+        }
+        if (!good && lane == 0) { broken = 1; }
+    }
+    __syncthreads();
+    if (warp != part) { return; }
+    if (broken) {
+        GlobalReader rd;
+        rd.lut = (const uint32_t *) smem;
+        rd.rd.open(p.w, unit, lane);
+        row(rd, 0u, t0);
+    }
+    if (SCORED) {
+        __syncwarp();
+        const int t = (int) blockIdx.x / scores.n_cand;
+        const bf16 * a = (const bf16 *) row_s, * b = (const bf16 *) scores.x_bf16 + (int64_t) t * (C * CHUNK);
+        const float v = row_product<C * CHUNK>(a, b, lane);
+        if (lane == 0) { scores.out[t * scores.vocab + (gr - row0)] = v; }
+    }
 }
 
 // One warp per unit, once per matrix: where every 64 codes of a lane begin.
@@ -187,6 +289,10 @@ void gemv_parts_init() {
     ATTR_C(1, bf16) ATTR_C(2, bf16) ATTR_C(4, bf16) ATTR_C(8, bf16) ATTR_C(1, float) ATTR_C(2, float) ATTR_C(4, float) ATTR_C(8, float)
 #undef ATTR_C
 #undef ATTR
+#define ATTR(C) allow_dynamic_smem((const void *) k_rows_parts<C, true, true>, optin, optin, "rows"); allow_dynamic_smem((const void *) k_rows_parts<C, true, false>, optin, optin, "rows"); \
+                allow_dynamic_smem((const void *) k_rows_parts<C, false, false>, optin, optin, "rows");
+    ATTR(1) ATTR(2) ATTR(4) ATTR(8)
+#undef ATTR
     allow_dynamic_smem((const void *) k_expand_parts<StoreBF16, 256>, optin, optin, "parts");
     allow_dynamic_smem((const void *) k_expand_parts<StoreBF16, 512>, optin, optin, "parts");
 }
@@ -194,6 +300,27 @@ void gemv_parts_init() {
 int unit_parts(const bf16n_weight & w) {
     const int64_t steps = w.R * (w.K / CHUNK);
     return w.format == FMT_HUFPAIR && !w.fo && steps % PART_STEPS == 0 && steps >= 2 * PART_STEPS && steps <= 16 * PART_STEPS ? (int) (steps / PART_STEPS) : 0;
+}
+
+// Walk from the unit's start (a warp to a row) / parts in us: 592 rows of 2048 columns 21.9 / 7.4, 9472 101 / 68; 592 rows of 512 columns (two
+// parts) 10.0 / 5.2, 2368 11.1 / 10.3, 4736 15.4 / 17.4.
+bool rows_parts_applies(const bf16n_weight & w, const uint16_t * marks, int64_t n) {
+    const int64_t C = w.K / CHUNK;
+    return marks && unit_parts(w) && !w.cm && n <= (int64_t) device_info().sms * (unit_parts(w) > 2 ? 64 : 16) && (C == 1 || C == 2 || C == 4 || C == 8);
+}
+
+void rows_parts(const bf16n_weight & w, const uint16_t * marks, const void * ids, int64_t ids_s0, int64_t n, void * dst, bool dst_bf16, int64_t dst_s1,
+                int64_t row0, const RowScores * scores, cudaStream_t st, bool behind_own) {
+    const Parts p = make_parts(w, marks);
+    const size_t shm = part_smem(p.parts, 1, p.cap).end + (scores ? (size_t) w.K * 2 : 0);
+    auto go = [&](auto * kernel) {
+        launch_behind(behind_own, kernel, dim3((unsigned) n), dim3(p.parts * 32), shm, st, p, w.R, (const char *) ids, ids_s0, row0, (char *) dst, dst_s1,
+                      scores ? *scores : RowScores{}, Opaque{1u, 4u});
+        check_launch();
+    };
+#define GO(C) case C: if (scores) { go(k_rows_parts<C, true, true>); } else if (dst_bf16) { go(k_rows_parts<C, true, false>); } else { go(k_rows_parts<C, false, false>); } break;
+    switch (w.K / CHUNK) { GO(1) GO(2) GO(4) GO(8) default: fail_invalid("unsupported K"); }
+#undef GO
 }
 
 size_t marks_bytes(const bf16n_weight & w) {

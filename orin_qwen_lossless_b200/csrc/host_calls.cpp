@@ -198,8 +198,8 @@ PyObject * call_draft(PyObject *, PyObject * const * args, Py_ssize_t n) {
                                                                 rows, (int) K, (float *) scores.mutable_data_ptr(), st));
             at::Tensor cand = at::empty({T, cands}, f32.dtype(at::kInt)), cand_rows = at::empty({T * cands, K}, f32.dtype(at::kBFloat16));
             out = at::empty({T, vocab}, f32);
-            ok(bf16n_draft_logits((const float *) scores.const_data_ptr(), (int) T, rows, (int) cands, &m.c, h.const_data_ptr(), (int32_t *) cand.mutable_data_ptr(),
-                                  cand_rows.mutable_data_ptr(), (float *) out.mutable_data_ptr(), vocab, st));
+            ok(bf16n_draft_logits_marked((const float *) scores.const_data_ptr(), (int) T, rows, (int) cands, &m.c, m.marks, h.const_data_ptr(),
+                                         (int32_t *) cand.mutable_data_ptr(), cand_rows.mutable_data_ptr(), (float *) out.mutable_data_ptr(), vocab, st));
         }
         return THPVariable_Wrap(std::move(out));
     });

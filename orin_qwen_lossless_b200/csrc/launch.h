@@ -81,6 +81,11 @@ bool gemv_parts_applies(const bf16n_weight & w, const uint16_t * marks, const bf
 void gemv_parts(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a, cudaStream_t st);
 bool expand_parts_applies(const bf16n_weight & w, const uint16_t * marks, int64_t nrows);
 void expand_parts(const bf16n_weight & w, const uint16_t * marks, int64_t row0, int64_t nrows, const dev::StoreBF16 & sink, cudaStream_t st);
+// Rows of a matrix with marks; scores: the rows are multiplied too (a draft step's candidates)
+struct RowScores { const void * x_bf16; int n_cand; float * out; int64_t vocab; }; // out[t, ids[i]] = row i . x_t, t = i / n_cand
+bool rows_parts_applies(const bf16n_weight & w, const uint16_t * marks, int64_t n);
+void rows_parts(const bf16n_weight & w, const uint16_t * marks, const void * ids, int64_t ids_s0, int64_t n, void * dst, bool dst_bf16, int64_t dst_s1,
+                int64_t row0, const RowScores * scores, cudaStream_t st, bool behind_own);
 
 // gemv.cu
 void gemv_init();
@@ -94,7 +99,7 @@ void expand_store(const bf16n_weight & w, int64_t row0, int64_t nrows, uint16_t 
 void expand_compare(const bf16n_weight & w, int64_t row0, int64_t nrows, const uint16_t * src, unsigned long long * total,
                     cudaStream_t st);
 void gather_rows(const bf16n_weight & w, const void * ids, int64_t ids_s0, int64_t n, void * dst, bool dst_bf16, int64_t dst_s1,
-                 int64_t row0, cudaStream_t st, bool behind_own = false);
+                 int64_t row0, cudaStream_t st, bool behind_own = false, const uint16_t * marks = nullptr);
 
 // device addresses of the words the kernels set when one of their bounded waits runs out (bf16n_fault_status)
 unsigned int * gemv_staged_fault_word();

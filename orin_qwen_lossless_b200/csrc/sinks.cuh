@@ -7,6 +7,20 @@
 namespace b16 {
 namespace dev {
 
+// chunk c of a gathered row
+template <bool BF>
+__device__ __forceinline__ void put_row_chunk(char * o, int c, int lane, const uint32_t (&w)[8]) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int i = c * CHUNK + 128 * j + 4 * lane;
+        if (BF) {
+            *(uint2 *) (o + 2 * i) = make_uint2(w[2 * j], w[2 * j + 1]);
+        } else {
+            *(float4 *) (o + 4 * i) = make_float4(bf16lo_f32(w[2 * j]), bf16hi_f32(w[2 * j]), bf16lo_f32(w[2 * j + 1]), bf16hi_f32(w[2 * j + 1]));
+        }
+    }
+}
+
 struct StoreBF16 { // row-major BF16 output
     uint16_t * out;
     int64_t K;

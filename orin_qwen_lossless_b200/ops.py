@@ -481,7 +481,7 @@ def get_rows(ids: torch.Tensor, w: Weight, out_dtype: torch.dtype = torch.bfloat
     n = ids.shape[0]
     out = torch.empty((n, w.meta.K), dtype=out_dtype, device=w.plane.device)
     with torch.cuda.device(w.plane.device):
-        check(lib().bf16n_get_rows(C.byref(cw), ids.data_ptr(), ids.stride(0) * ids.element_size(), n, out.data_ptr(),
+        check(lib().bf16n_get_rows_marked(C.byref(cw), w.marks_ptr(), ids.data_ptr(), ids.stride(0) * ids.element_size(), n, out.data_ptr(),
                                    int(out_dtype == torch.bfloat16), w.meta.K * out.element_size(), _stream(), 0))
     return out
 
@@ -605,8 +605,8 @@ def draft_logits(h: torch.Tensor, w: Weight, head: DraftHead, vocab: int) -> tor
         cand_rows = torch.empty((n * head.candidates, K), dtype=torch.bfloat16, device=h.device)
         out = torch.empty((n, vocab), dtype=torch.float32, device=h.device)
         with torch.cuda.device(h.device):
-            check(lib().bf16n_draft_logits(scores.data_ptr(), n, rows, head.candidates, C.byref(cw), h.data_ptr(), cand.data_ptr(),
-                                           cand_rows.data_ptr(), out.data_ptr(), vocab, _stream()))
+            check(lib().bf16n_draft_logits_marked(scores.data_ptr(), n, rows, head.candidates, C.byref(cw), w.marks_ptr(), h.data_ptr(), cand.data_ptr(),
+                                                  cand_rows.data_ptr(), out.data_ptr(), vocab, _stream()))
         return out
     # a head with padding rows beyond the vocabulary, an unaligned h, or one whose derivatives are wanted
     cand = scores.topk(head.candidates, dim=-1).indices                           # [n, C]

@@ -53,8 +53,12 @@ def test_marks_change_nothing(ops, rows, K, R, cm, wide):
     if K == 1536:
         xs = []         # reconstruction only: no product has this width
     want = [ops.mmv(x, plain) for x in xs]
+    ids = torch.randperm(rows)[:300]
     for marks in _marks(ops, w):
         w.marks = marks.view(torch.uint8)
+        if not cm:
+            assert torch.equal(ops.get_rows(ids.cuda(), w).cpu().view(torch.int16), src[ids].view(torch.int16))
+            assert torch.equal(ops.get_rows(ids.int().cuda(), w, torch.float32).cpu(), src[ids].float())
         assert torch.equal(ops.dequant(w).cpu().view(torch.int16), src.view(torch.int16))
         assert torch.equal(ops.dequant(w, R, rows - 2 * R).cpu().view(torch.int16), src[R:rows - R].view(torch.int16))
         for x, y in zip(xs, want):
@@ -94,6 +98,18 @@ def test_last_round_of_a_large_product(ops, rows, K, R):
     for marks in _marks(ops, w):
         w.marks = marks.view(torch.uint8)
         assert all(torch.equal(ops.mmv(x, w), y) for x, y in zip(xs, want))
+
+
+@pytest.mark.parametrize("T", [1, 3])
+def test_candidates_of_a_draft_step(ops, T):
+    src, w = _made(ops, 4096, 2048, 16, False)
+    plain = ops.Weight(w.plane, w.aux, w.meta)
+    head = ops.DraftHead(2, *ops.int2_quantize(src.cuda()), 128)
+    h = torch.randn(T, 2048, device="cuda").to(torch.bfloat16)
+    want = ops.draft_logits(h, plain, head, 4100)
+    for marks in _marks(ops, w):
+        w.marks = marks.view(torch.uint8)
+        assert torch.equal(ops.draft_logits(h, w, head, 4100), want)
 
 
 def test_a_swapped_matrix_needs_no_new_marks(ops):
