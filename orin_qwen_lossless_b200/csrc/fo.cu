@@ -433,6 +433,7 @@ __global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const FoMa
 // Shared memory holds the 8 activation rows as BF16, each padded by 8 elements so that the B-fragment reads of a warp
 // fall into 32 different banks; columns beyond ncols are zero.
 constexpr int XPAD = 8;
+constexpr int STAGED_WARPS = 28;
 constexpr int FO_BARS = 512; // room for two mbarriers per warp of the staged kernel (up to 32 warps)
 __global__ void __launch_bounds__(512) k_fo_gemv_mma(const PairView w, int C, Cols p, int ncols, int64_t n_units) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -743,23 +744,25 @@ __global__ void __launch_bounds__(FO_WARPS * 32, 1) k_fo_mm_ids(const FoBatch p)
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-// The same product with the streams staged: one persistent block per SM of up to 32 warps, a warp walks bands and copies each slab's
-// stream block into its own shared-memory buffer with one bulk async copy (two buffers in turn, so the next slab's copy
-// runs under the current slab's decoding; bounded wait, as in gemv_staged.cu), reads it with the staged reader and
-// prefetches the plane bytes one tile pair ahead. Serves 1..8 dense BF16 columns. A slab whose streams do not fit the
-// buffer (more than 3 bits per weight) is read straight from global memory.
+// The same product with the streams staged: one persistent block per SM of up to 28 warps, a warp walks bands and copies each slab's
+// stream block into its shared-memory buffer with one bulk async copy (bounded wait, as in gemv_staged.cu; the next slab's streams and
+// plane are asked into L2 meanwhile), reads it with the staged reader and the plane four tile pairs ahead. What bounded it was the
+// shared-memory pipe (72 % of its cycles, a lookup in one table costing 3.3 wavefronts, against 41 % of the issue slots), so the
+// table is spread over copies without conflicts, at two more instructions a code; now the ALU pipe (65 %). The spread table takes the room of
+// a second stream buffer per warp. 124160 x 2048, eight columns: 106 -> 99 us, 65536 x 4096: 132 -> 102. Serves 1..8 dense
+// BF16 columns. A slab whose streams do not fit the buffer (more than 3 bits per weight) is read straight from global memory.
 constexpr uint32_t FO_CAP = (BAND * CHUNK * 3 / 8 + 64 + 15) & ~15u;
 
-__global__ void __launch_bounds__(1024) k_fo_gemv_staged(const PairView w, const AuxHeader * hdr, int C, Cols p, int ncols, const Opaque k) {
+__global__ void __launch_bounds__(STAGED_WARPS * 32, 1) k_fo_gemv_staged(const PairView w, const AuxHeader * hdr, int C, Cols p, int ncols, const Opaque k) {
     extern __shared__ __align__(128) unsigned char smem[];
-    uint32_t * lut = (uint32_t *) smem;
-    uint64_t * bars = (uint64_t *) (smem + 4 * HP_MAX_PAIRS);            // two per warp
+    uint64_t * bars = (uint64_t *) (smem + SPREAD_BYTES);                // one per warp
     const int K = C * CHUNK, XS = K + XPAD;
-    bf16 * xs = (bf16 *) (smem + 4 * HP_MAX_PAIRS + FO_BARS);
+    bf16 * xs = (bf16 *) (smem + SPREAD_BYTES + FO_BARS);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    unsigned char * buf = smem + 4 * HP_MAX_PAIRS + FO_BARS + (size_t) 8 * XS * 2 + (size_t) warp * 2 * FO_CAP;
-    stage_lut(lut, w.lut);
-    if (lane == 0) { mbar_init(smem_u32(bars + 2 * warp), 1); mbar_init(smem_u32(bars + 2 * warp + 1), 1); }
+    unsigned char * buf = smem + SPREAD_BYTES + FO_BARS + (size_t) 8 * XS * 2 + (size_t) warp * FO_CAP;
+    const SpreadTable codes = stage_spread(smem, w.lut);
+    const uint32_t bar = smem_u32(bars + warp);
+    if (lane == 0) { mbar_init(bar, 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     grid_dependency_wait();
     for (int i = threadIdx.x; i < 8 * (K / 8); i += blockDim.x) { // 16-byte pieces; columns beyond ncols are zero
@@ -779,74 +782,83 @@ __global__ void __launch_bounds__(1024) k_fo_gemv_staged(const PairView w, const
         g.my = w0 - g.start + __ldg(w.lrel + gu * 32 + lane);
         return g;
     };
-    auto stage = [&](const Geo & g, int b) { // one lane starts the copy of a slab's streams into buffer b
+    auto stage = [&](const Geo & g) { // one lane starts the copy of a slab's streams
         if (g.bytes <= FO_CAP && lane == 0) {
-            const uint32_t bar = smem_u32(bars + 2 * warp + b);
             mbar_expect_tx(bar, g.bytes);
-            bulk_g2s(smem_u32(buf + b * FO_CAP), w.stream + g.start, g.bytes, bar);
+            bulk_g2s(smem_u32(buf), w.stream + g.start, g.bytes, bar);
         }
     };
     const int g8 = lane >> 2, t4 = lane & 3;
     const bf16 * xl = xs + g8 * XS + 2 * t4;
-    uint32_t parity = 0u; // bit b: phase of buffer b's barrier
+    uint32_t parity = 0u; // of the barrier
     bool dead = false;    // a bulk copy of this warp never arrived: no further copies, NaN outputs
     const int64_t bands = p.nrows / BAND;
-    for (int64_t b = (int64_t) blockIdx.x * nwarp + warp; b < bands; b += (int64_t) gridDim.x * nwarp) {
+    const int64_t band_step = (int64_t) gridDim.x * nwarp;
+    Geo cur = {};
+    if ((int64_t) blockIdx.x * nwarp + warp < bands) { cur = geometry((p.row0 / BAND + (int64_t) blockIdx.x * nwarp + warp) * C); }
+    for (int64_t b = (int64_t) blockIdx.x * nwarp + warp; b < bands; b += band_step) {
         const int64_t gband = p.row0 / BAND + b;
-        float d[4] = {0.f, 0.f, 0.f, 0.f};
-        Geo cur = geometry(gband * C);
-        __syncwarp(); // every lane is done with both buffers (previous band)
-        if (!dead) { stage(cur, 0); }
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
         for (int slab = 0; slab < C && !dead; slab++) {
-            Geo nxt = {0, 0, 0};
-            if (slab + 1 < C) {
-                nxt = geometry(gband * C + slab + 1);
-                __syncwarp(); // the buffer about to be refilled was read two slabs ago by every lane
-                stage(nxt, (slab + 1) & 1);
-            }
+            __syncwarp(); // every lane is done with the buffer (previous slab)
+            stage(cur);
             const uint8_t * pl = w.plane + gband * BAND * (int64_t) K + (int64_t) slab * (16 * 512) + 16 * lane;
-            if (lane == 0) { // the next unit's plane bytes into L2 (the next slab, or the first slab of this warp's next band)
-                const int64_t nb = b + (int64_t) gridDim.x * nwarp;
-                if (slab + 1 < C) { bulk_prefetch_l2(pl + 16 * 512, 16 * 512); }
-                else if (nb < bands) { bulk_prefetch_l2(w.plane + (p.row0 / BAND + nb) * BAND * (int64_t) K, 16 * 512); }
+            // the next unit (the next slab, or the first slab of this warp's next band): its start, and its streams and plane into L2
+            const int64_t next = slab + 1 < C ? gband * C + slab + 1 : b + band_step < bands ? (gband + band_step) * C : -1;
+            Geo nxt = {};
+            if (next >= 0) {
+                nxt = geometry(next);
+                if (lane == 0) {
+                    bulk_prefetch_l2(w.plane + next * (16 * 512), 16 * 512);
+                    bulk_prefetch_l2(w.stream + nxt.start, nxt.bytes);
+                }
             }
-            auto body = [&](auto & rd, uint32_t lut_arg) {
-                uint4 nx = ld_stream16(pl);
-                for (int pp = 0; pp < 16; pp++) {
-                    const uint4 cu = nx;
-                    if (pp + 1 < 16) { nx = ld_stream16(pl + (pp + 1) * 512); }
-                    uint32_t e[8], a[8];
-                    rd.take8(lut_arg, k, e);
-                    assemble8(cu, e, a);
+            float d[4] = {0.f, 0.f, 0.f, 0.f}; // the slab's sums; slabs are added in order, in FP32, as k_fo_gemv_split adds them
+            auto body = [&](auto & rd) {
+                uint4 nx[4];
 #pragma unroll
-                    for (int kk = 0; kk < 2; kk++) {
-                        const int col = (slab * 32 + 2 * pp + kk) * 16;
-                        const uint32_t b0 = *(const uint32_t *) (xl + col), b1 = *(const uint32_t *) (xl + col + 8);
-                        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-                                     "{%0, %1, %2, %3};"
-                                     : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                                     : "r"(a[4 * kk]), "r"(a[4 * kk + 1]), "r"(a[4 * kk + 2]), "r"(a[4 * kk + 3]), "r"(b0), "r"(b1));
+                for (int i = 0; i < 4; i++) { nx[i] = ld_stream16(pl + i * 512); }
+#pragma unroll 1
+                for (int pp4 = 0; pp4 < 16; pp4 += 4) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const int pp = pp4 + i;
+                        const uint4 cu = nx[i];
+                        if (pp4 + 4 < 16) { nx[i] = ld_stream16(pl + (pp + 4) * 512); }
+                        uint32_t e[8], a[8];
+                        rd.take8(codes, k, e);
+                        assemble8(cu, e, a);
+#pragma unroll
+                        for (int kk = 0; kk < 2; kk++) {
+                            const int col = (slab * 32 + 2 * pp + kk) * 16;
+                            const uint32_t b0 = *(const uint32_t *) (xl + col), b1 = *(const uint32_t *) (xl + col + 8);
+                            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                                         "{%0, %1, %2, %3};"
+                                         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                                         : "r"(a[4 * kk]), "r"(a[4 * kk + 1]), "r"(a[4 * kk + 2]), "r"(a[4 * kk + 3]), "r"(b0), "r"(b1));
+                        }
                     }
                 }
             };
             if (cur.bytes <= FO_CAP) {
-                const int bi = slab & 1;
-                const uint32_t landed = mbar_wait(smem_u32(bars + 2 * warp + bi), (parity >> bi) & 1u);
+                const uint32_t landed = mbar_wait(bar, parity);
                 if (!landed) { // the copy never arrived: this band and the warp's later bands are written as NaN
                     if (lane == 0) { atomicOr(&g_wait_expired, 1u); }
                     dead = true;
                     break;
                 }
-                parity ^= 1u << bi;
+                parity ^= 1u;
                 WindowReader rd;
-                rd.open(smem_u32(buf + bi * FO_CAP) + 4 * cur.my, landed);
-                body(rd, smem_u32(lut));
+                rd.open(smem_u32(buf) + 4 * cur.my, landed);
+                body(rd);
             } else {
                 GlobalReader rd;
-                rd.lut = lut;
+                rd.lut = w.lut;
                 rd.rd.open(w, gband * C + slab, lane);
-                body(rd, 0u);
+                body(rd);
             }
+#pragma unroll
+            for (int i = 0; i < 4; i++) { sum[i] = slab ? sum[i] + d[i] : d[i]; }
             cur = nxt;
         }
 #pragma unroll
@@ -854,7 +866,7 @@ __global__ void __launch_bounds__(1024) k_fo_gemv_staged(const PairView w, const
             const int n = 2 * t4 + (i & 1);
             if (n < ncols) {
                 const OutVec o = {p.y + n * p.y_tok, p.y_bf16};
-                o.put(b * BAND + g8 + 8 * (i >> 1), dead ? __int_as_float(0x7fc00000) : d[i]);
+                o.put(b * BAND + g8 + 8 * (i >> 1), dead ? __int_as_float(0x7fc00000) : sum[i]);
             }
         }
     }
@@ -903,8 +915,10 @@ template <typename TX>
 void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool behind_own) {
     Cols p = make_cols(a);
     // routed columns, and a single dense column of a small matrix: the kernels with one decode per column
-    // From 16 bands per SM on, BF16 activations take the persistent kernel; below, it was measured level with or behind
-    // the split kernels (16384 x 2048: 34.6 against 22.4 us at one token, 35.9 against 35.6 at eight).
+    // Two and more columns take the persistent kernel from 6 bands per SM on: split / staged in us, eight columns, 12288 x 2048 (5.2
+    // bands) 29.3 / 27.6, 16384 x 2048 33.2 / 28.8, 32768 x 2048 57.4 / 33.8, 32768 x 4096 164 / 67, 16384 x 512 9.1 / 8.2, but 8192 x 2048 17.6 /
+    // 25.6. Both add the slabs in order: the same bits. A single column stays with the FMAs of the split kernel up to 16 bands per SM, whose
+    // sums the tensor core's are not as near to (16384 x 2048: 21.8 us there, 27.7 staged).
     constexpr int64_t big_per_sm = 16;
     if (a.ids || (a.ncols == 1 && (p.nrows / BAND < (int64_t) device_info().sms * big_per_sm || !a.x_bf16))) {
         if (fo_split_applies(w, a)) {
@@ -923,15 +937,15 @@ void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st
         // One persistent block per SM with as many warps as the shared memory holds stream buffers for (28 with K = 2048;
         // the decode chains need the occupancy), then the fewest warps that still finish in the same number of bands
         // per warp, so that no warp slows the others down for nothing.
-        const size_t shm_fixed = 4 * HP_MAX_PAIRS + FO_BARS + x_bytes;
+        const size_t shm_fixed = SPREAD_BYTES + FO_BARS + x_bytes;
         const size_t optin = (size_t) device_info().smem_optin;
-        int staged_warps = optin > shm_fixed ? (int) std::min<size_t>(32, (optin - shm_fixed) / (2 * FO_CAP)) : 0;
+        int staged_warps = optin > shm_fixed ? (int) std::min<size_t>(STAGED_WARPS, (optin - shm_fixed) / FO_CAP) : 0;
         if (staged_warps > 0) {
             const int64_t rounds = (bands + sms * staged_warps - 1) / (sms * staged_warps);
             staged_warps = (int) ((bands + sms * rounds - 1) / (sms * rounds));
         }
-        const size_t shm_staged = shm_fixed + (size_t) staged_warps * 2 * FO_CAP;
-        const bool big = bands >= sms * big_per_sm && (uintptr_t) p.x % 16 == 0 && p.x_tok % 16 == 0 && staged_warps >= 1 &&
+        const size_t shm_staged = shm_fixed + (size_t) staged_warps * FO_CAP;
+        const bool big = bands >= sms * (a.ncols >= 2 ? 6 : big_per_sm) && (uintptr_t) p.x % 16 == 0 && p.x_tok % 16 == 0 && staged_warps >= 1 &&
                          shm_staged <= optin;
         for (int c0 = 0; c0 < a.ncols; c0 += 8) {
             Cols q = p;
@@ -986,7 +1000,7 @@ void fo_init() {
     ATTR(k_fo_gemv_mma);
     ATTR((k_fo_gemv_split<float, false>)); ATTR((k_fo_gemv_split<bf16, false>)); ATTR((k_fo_gemv_split<bf16, true>));
     ATTR((k_fo_gemv_split<float, false, FO_GROUP>)); ATTR((k_fo_gemv_split<bf16, false, FO_GROUP>));
-    ATTR(k_fo_gemv_staged);
+    allow_dynamic_smem((const void *) k_fo_gemv_staged, optin, optin, "k_fo_gemv_staged");
     ATTR(k_fo_mm_ids<false>); ATTR(k_fo_mm_ids<true>);
 #undef ATTR
 }

@@ -77,6 +77,40 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr, uint32_t token = 0) {
     return v;
 }
 
+// The code table without bank conflicts. Codes are canonical, so the long ones are the numerically largest: a view of 12 bits that
+// starts with a code of at most 8 bits needs its first 8 bits only, and the entries are q (those views by 8 bits) and 4096 - 16 q (the
+// others by all 12); on the weights of the benchmark 466 instead of 4096. So many fit a copy for every lane (or every second one,
+// and so on for flatter tables), and lanes that share no copy cannot collide. Entry of a view: max(view >> 8, view - 15 q).
+constexpr int SPREAD_BYTES = 64 << 10;
+struct SpreadTable {
+    uint32_t base, stride; // address of this lane's copy of entry 0, bytes from entry to entry
+    int32_t shift;         // -15 q
+    __device__ __forceinline__ uint32_t look(uint32_t view) const { // view: the stream from the code on, at the top
+        return lds32(imad((uint32_t) __viaddmax_s32((int32_t) (view >> (32 - HP_LMAX)), shift, (int32_t) (view >> 24)), stride, base));
+    }
+};
+// Every thread of the block; the caller's next block barrier completes the table. Whatever the table holds, entries stay below
+// SPREAD_BYTES: the largest view is entry 4095 - 15 q of 4096 - 15 q.
+__device__ __forceinline__ SpreadTable stage_spread(unsigned char * table, const uint32_t * lut) {
+    constexpr int SHORT = HP_MAX_PAIRS / 16;
+    __shared__ int first_long;
+    if (threadIdx.x == 0) { first_long = SHORT; }
+    __syncthreads();
+    for (int i = threadIdx.x; i < SHORT; i += blockDim.x) {
+        if ((__ldg(lut + 16 * i) & 31u) > 8u) { atomicMin(&first_long, i); }
+    }
+    __syncthreads();
+    int q = first_long, entries = HP_MAX_PAIRS - 15 * q;
+    const int log_copies = entries <= SPREAD_BYTES / 128 ? 5 : entries <= SPREAD_BYTES / 64 ? 4 : entries <= SPREAD_BYTES / 32 ? 3 : 2;
+    if (log_copies == 2) { q = 0; entries = HP_MAX_PAIRS; }
+    for (int i = threadIdx.x; i < entries << (log_copies - 2); i += blockDim.x) {
+        const int at = i >> (log_copies - 2);
+        const uint32_t e = __ldg(lut + (at < q ? 16 * at : at + 15 * q));
+        ((uint4 *) table)[i] = make_uint4(e, e, e, e);
+    }
+    return {smem_u32(table) + (threadIdx.x & ((1u << log_copies) - 1u)) * 4u, 4u << log_copies, -15 * q};
+}
+
 // Lane stream reader over words in shared memory (addresses are 32-bit shared-window addresses). The stream is seen through
 // a window of three consecutive words and a bit offset, as in rings.cuh: a view is one funnel shift and nothing is shifted
 // per code. Against a 64-bit buffer that is shifted and refilled (its predecessor here) the chain of a code is two
@@ -110,6 +144,15 @@ struct WindowReader {
             slide(o + e[q] + e[q + 1], k);
         }
     }
+    __device__ __forceinline__ void take8(const SpreadTable & t, const Opaque & k, uint32_t (&e)[8]) {
+#pragma unroll
+        for (int q = 0; q < 8; q += 2) {
+            const uint32_t v1 = shl_wrap_hi(lo, hi, o);
+            e[q] = t.look(v1);
+            e[q + 1] = t.look(shl_wrap_hi(0u, v1, e[q]));
+            slide(o + e[q] + e[q + 1], k);
+        }
+    }
     // passes over `n` codes; many: 16-bit entries of codes_in_window (format.h): each names one to three codes, so this ends
     __device__ __forceinline__ void skip(int n, uint32_t many, uint32_t lut, const Opaque & k) {
         while (n >= 3) {
@@ -126,7 +169,7 @@ struct WindowReader {
 struct GlobalReader {
     PairReader rd;
     const uint32_t * lut;
-    __device__ __forceinline__ void take8(uint32_t, const Opaque &, uint32_t (&e)[8]) { rd.take8(lut, e); }
+    template <typename Table> __device__ __forceinline__ void take8(const Table &, const Opaque &, uint32_t (&e)[8]) { rd.take8(lut, e); }
 };
 
 // this lane's activations of a K-column row, in registers
