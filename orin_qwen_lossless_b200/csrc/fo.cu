@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const FoMa
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncwarp();
     if (lut_first) { stage_lut(lut, w.lut); } // while the kernel before this one, which is this library's, drains (launch_behind)
-    grid_dependency_wait(); // activations and expert ids may come from the kernel before this one
+    grid_wait(); // activations and expert ids may come from the kernel before this one
     if (!lut_first) { stage_lut(lut, w.lut); }
     const TX * xg; OutVec out; int64_t rbase;
     column<TX>(p, MMA ? 0 : blockIdx.y, xg, out, rbase);
@@ -366,6 +366,7 @@ __global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const FoMa
         };
         if (bytes <= FO_SPLIT_CAP) {
             const uint32_t landed = mbar_wait(bar, 0u);
+            grid_launch_dependents();
             if (landed) {
                 WindowReader rd;
                 rd.open(smem_u32(buf) + 4 * (w0 - (w0 & ~3u) + my), landed);
@@ -424,6 +425,107 @@ __global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const FoMa
                 }
             }
         }
+    }
+}
+
+// The down product of a decode step, the SwiGLU in front of it and the weighted sum over the slots behind it in one launch: a block
+// takes one band of every slot's expert (one slab: K = 512), a warp to a slot, so the slots' outputs of these rows meet in shared memory
+// and are added in slot order, as k_combine_f32 adds them. Products, sums and SwiGLU are those of k_fo_gemv_split and k_swiglu, bit for bit.
+constexpr int FO_COMBINE_SLOTS = 16;
+__global__ void __launch_bounds__(FO_COMBINE_SLOTS * 32) k_fo_down_combine(const FoMat m, const float * g, const float * u, const int32_t * ids, const float * weights,
+                                                                           int n_used, int64_t rows_per_expert, char * y, bool y_bf16, const Opaque k) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ float ys[FO_COMBINE_SLOTS][BAND], ws[FO_COMBINE_SLOTS];
+    __shared__ uint64_t bars[FO_COMBINE_SLOTS];
+    const PairView & w = m.v;
+    uint32_t * lut = (uint32_t *) smem;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.y;
+    float * xs = (float *) (smem + 4 * HP_MAX_PAIRS) + warp * CHUNK;
+    unsigned char * buf = smem + 4 * HP_MAX_PAIRS + (size_t) n_used * CHUNK * 4 + (size_t) warp * FO_SPLIT_CAP;
+    const uint32_t bar = smem_u32(bars + warp);
+    if (lane == 0) { mbar_init(bar, 1); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncwarp();
+    // The ids and weights are older than the kernel in front, which waited for them; its outputs are waited for below.
+    const int64_t col = (int64_t) t * n_used + warp, unit = (int64_t) ids[col] * (rows_per_expert / BAND) + blockIdx.x;
+    const uint8_t * pl = w.plane + unit * (BAND * CHUNK) + 16 * lane;
+    uint4 ring[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) { ring[i] = ld_stream16(pl + i * 512); }
+    const uint32_t w0 = __ldg(w.ubase + unit), w1 = unit + 1 < (int64_t) m.hdr->n_a ? __ldg(w.ubase + unit + 1) : (uint32_t) m.hdr->n_b;
+    const uint32_t start = w0 & ~3u, bytes = ((w1 - start + 4u + 3u) & ~3u) * 4u, my = w0 - start + __ldg(w.lrel + unit * 32 + lane);
+    if (lane == 0) {
+        if (bytes <= FO_SPLIT_CAP) {
+            mbar_expect_tx(bar, bytes);
+            bulk_g2s(smem_u32(buf), w.stream + start, bytes, bar);
+        }
+        bulk_prefetch_l2(w.plane + unit * (BAND * CHUNK), BAND * CHUNK);
+        ws[warp] = weights[col];
+    }
+    stage_lut(lut, w.lut);
+    grid_dependency_wait();
+    {
+        float4 gv[4], uv[4]; // in flight together
+#pragma unroll
+        for (int i = 0; i < 4; i++) { gv[i] = ldg_x4(g + col * CHUNK, 4 * lane + 128 * i); uv[i] = ldg_x4(u + col * CHUNK, 4 * lane + 128 * i); }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            *(float4 *) (xs + 4 * lane + 128 * i) = make_float4(silu_f(gv[i].x) * uv[i].x, silu_f(gv[i].y) * uv[i].y, silu_f(gv[i].z) * uv[i].z,
+                                                               silu_f(gv[i].w) * uv[i].w);
+        }
+    }
+    __syncthreads();
+    const int cq = 2 * (lane & 3);
+    float acc[2] = {0.f, 0.f};
+    auto body = [&](auto & rd, uint32_t lut_arg) {
+#pragma unroll 1
+        for (int pp4 = 0; pp4 < 16; pp4 += 4) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int pp = pp4 + i;
+                const uint4 cur = ring[i];
+                if (pp4 + 4 < 16) { ring[i] = ld_stream16(pl + (pp + 4) * 512); }
+                uint32_t e[8], wv[8];
+                rd.take8(lut_arg, k, e);
+                assemble8(cur, e, wv);
+#pragma unroll
+                for (int q8 = 0; q8 < 8; q8++) {
+                    const int q = q8 & 3;
+                    const float2 x0 = *(const float2 *) (xs + (2 * pp + (q8 >> 2)) * 16 + cq + 8 * (q >> 1));
+                    acc[q & 1] = fmaf(bf16hi_f32(wv[q8]), x0.y, fmaf(bf16lo_f32(wv[q8]), x0.x, acc[q & 1]));
+                }
+            }
+        }
+    };
+    if (bytes <= FO_SPLIT_CAP) {
+        const uint32_t landed = mbar_wait(bar, 0u);
+        if (landed) {
+            WindowReader rd;
+            rd.open(smem_u32(buf) + 4 * my, landed);
+            body(rd, smem_u32(lut));
+        } else { // the copy never arrived: the flag reports it and the rows become NaN
+            if (lane == 0) { atomicOr(&g_wait_expired, 1u); }
+            acc[0] = acc[1] = __int_as_float(0x7fc00000);
+        }
+    } else {
+        GlobalReader rd;
+        rd.lut = lut;
+        rd.rd.open(w, unit, lane);
+        body(rd, 0u);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        float v = acc[h];
+        v += __shfl_xor_sync(FULL, v, 1);
+        v += __shfl_xor_sync(FULL, v, 2);
+        if ((lane & 3) == 0) { ys[warp][(lane >> 2) + 8 * h] = v; }
+    }
+    __syncthreads();
+    if (threadIdx.x < BAND) {
+        float sum = 0.f;
+        for (int s = 0; s < n_used; s++) { sum = fmaf(ws[s], ys[s][threadIdx.x], sum); }
+        const OutVec out = {y + (int64_t) t * rows_per_expert * (y_bf16 ? 2 : 4), y_bf16};
+        out.put((int64_t) blockIdx.x * BAND + threadIdx.x, sum);
     }
 }
 
@@ -1001,8 +1103,25 @@ void fo_init() {
     ATTR((k_fo_gemv_split<float, false>)); ATTR((k_fo_gemv_split<bf16, false>)); ATTR((k_fo_gemv_split<bf16, true>));
     ATTR((k_fo_gemv_split<float, false, FO_GROUP>)); ATTR((k_fo_gemv_split<bf16, false, FO_GROUP>));
     allow_dynamic_smem((const void *) k_fo_gemv_staged, optin, optin, "k_fo_gemv_staged");
+    allow_dynamic_smem((const void *) k_fo_down_combine, optin, optin, "k_fo_down_combine");
     ATTR(k_fo_mm_ids<false>); ATTR(k_fo_mm_ids<true>);
 #undef ATTR
+}
+
+// From four tokens on the launches of their own decode an expert once for two columns that picked it, which is worth more than the
+// launches saved where slots are many for the experts. Own launches / one, us a step of 8 slots: 128 experts, 1 / 2 / 3 / 4 / 8 tokens 26.5 / 43.8 /
+// 61.7 / 70.4 / 107.6 and 23.1 / 38.3 / 52.0 / 68.9 / 107.4; 32 experts, 4 / 8 tokens 61.8 / 87.1 and 62.7 / 91.1; 16 experts, 8 tokens 75.8 and 82.5.
+bool fo_down_combine_applies(const bf16n_weight & down, int n_tok, int n_used, int n_experts) {
+    return down.K == CHUNK && n_used <= FO_COMBINE_SLOTS && (n_tok < 4 || 2 * n_tok * n_used <= n_experts);
+}
+// y[t] = sum over slots of weights[t, s] * down[ids[t, s]] (silu(g) * u)[t, s]; g and u are the outputs of the launch in front
+void fo_down_combine(const bf16n_weight & down, const float * g, const float * u, const int32_t * ids, const float * weights, int n_tok, int n_used,
+                     int n_experts, void * y, bool y_bf16, cudaStream_t st) {
+    const int64_t H = down.rows / n_experts;
+    const size_t shm = even_smem(4 * HP_MAX_PAIRS + (size_t) n_used * (CHUNK * 4 + FO_SPLIT_CAP), H / BAND * n_tok);
+    launch_chained(k_fo_down_combine, dim3((unsigned) (H / BAND), (unsigned) n_tok), dim3((unsigned) n_used * 32), shm, st, fo_mat(down), g, u, ids, weights,
+                   n_used, H, (char *) y, y_bf16, Opaque{1u, 4u});
+    check_launch();
 }
 
 // K up to 4096 columns with 8 activation columns staged as FP32 beside the table

@@ -32,6 +32,14 @@ inline void allow_dynamic_smem(const void * kernel, int bytes, int optin, const 
     cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, std::min(bytes, optin - (int) fa.sharedSizeBytes)), what);
 }
 
+// Shared memory that keeps a launch of a few blocks per SM spread evenly: blocks of a dependent launch are placed while the kernel in front
+// still holds some SMs, and would crowd on the others (the down launch of a one-token decode step: 13 us with up to four blocks on an
+// SM, 9 with one on each). `bytes` at least, and more than lets one block beyond the even share on an SM.
+inline size_t even_smem(size_t bytes, int64_t blocks) {
+    const int64_t share = (blocks + device_info().sms - 1) / device_info().sms;
+    return std::max(bytes, share <= 3 ? (size_t) device_info().smem_optin / (share + 1) : 0);
+}
+
 #ifdef __CUDACC__
 // Launch of a kernel that may start while the kernel before it on the stream is still draining (programmatic dependent
 // launch): such a kernel calls grid_dependency_wait() before it touches anything an earlier kernel wrote or still reads,
@@ -57,6 +65,9 @@ void launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t shm,
 // Lets the next kernel on the stream begin its own prologue now. Only for kernels in which every block that has work also
 // waits (grid_dependency_wait) before it touches what earlier kernels wrote or read.
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The wait alone, for a kernel that lets its successor begin later: a successor's prologue asks for its own streams and planes, and
+// while this kernel's are still on their way they are in each other's way.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Blocks until every kernel this one depends on has completed and its writes are visible; then lets the next kernel on
 // the stream begin its own prologue.
 __device__ __forceinline__ void grid_dependency_wait() {
@@ -125,6 +136,9 @@ void fo_init();
 bool fo_supported(const bf16n_weight & w);
 void fo_gemv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st, bool behind_own = false); // behind_own: see launch_behind
 void fo_gemv_two(const bf16n_weight & w, const bf16n_weight & up, const bf16n_mmv_args & a, void * up_y, cudaStream_t st, bool behind_own); // routed columns
+bool fo_down_combine_applies(const bf16n_weight & down, int n_tok, int n_used, int n_experts);
+void fo_down_combine(const bf16n_weight & down, const float * g, const float * u, const int32_t * ids, const float * weights, int n_tok, int n_used,
+                     int n_experts, void * y, bool y_bf16, cudaStream_t st);
 bool fo_mm_ids_supported(const bf16n_weight & w, const bf16n_weight * up);
 void fo_mm_ids(const bf16n_weight & w, const bf16n_weight * up, const void * x_bf16, int64_t x_row, const int32_t * ids_src1,
                const int32_t * ids_dst, const int32_t * bounds, void * dst, bool dst_bf16, int64_t dst_col, int n_experts,

@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(256, 4) k_expert_parts(const ExpertMat m0, con
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const ExpertMat & m = blockIdx.z ? m1 : m0;
     stage_table(smem, m.v.lut);
-    if (!p.early_ids) { grid_dependency_wait(); } // as above
+    if (!p.early_ids) { grid_wait(); } // as above
     const int col = blockIdx.y, t = col / p.n_used, s = col - t * p.n_used;
     const int e = *(const int32_t *) (p.ids + t * p.ids_s1 + s * p.ids_s0) - p.e_lo;
     const int64_t units = p.rows_per_expert / R;
@@ -280,23 +280,24 @@ __global__ void __launch_bounds__(256, 4) k_expert_parts(const ExpertMat m0, con
         }
     };
     walk_parts<false>(parts, first_unit(parts), units, (int64_t) e * units, R * C * CHUNK, smem, [&] {
-        if (p.early_ids) { grid_dependency_wait(); }
+        if (p.early_ids) { grid_wait(); }
         load_x(CM ? warp % PARTS : 0);
     }, rows, put);
 }
 
 // The down product and the weighted sum over the slots in one launch: a block takes one unit's rows in every slot's expert (two
 // warps each), so the slots' outputs of these rows meet in shared memory and are added in slot order, as k_combine_f32 adds them.
-// One token of 8 slots: 25.0 us a step with a launch of its own for the sum, 23.0 so.
+// One token of 8 slots: 25.0 us a step with a launch of its own for the sum, 20.0 so.
 constexpr int COMBINE_SLOTS = PART_UNITS;
 __global__ void __launch_bounds__(512, 2) k_down_combine(const ExpertMat m, const ExpertCols p, const float * weights, char * out, bool out_bf16, const Opaque k) {
     constexpr int R = 16, PARTS = 2;
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ float ys[COMBINE_SLOTS][R];
+    __shared__ float ys[COMBINE_SLOTS][R], ws[COMBINE_SLOTS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, s = warp / PARTS, t = blockIdx.y;
     stage_table(smem, m.v.lut);
     // the ids and weights are older than the kernel in front (early_ids)
     const int e = *(const int32_t *) (p.ids + t * p.ids_s1 + s * p.ids_s0) - p.e_lo;
+    if (warp % PARTS == 0 && lane == 0) { ws[s] = weights[(int64_t) t * p.n_used + s]; }
     const bool held = e >= 0 && e < p.e_n;
     const int64_t units = p.rows_per_expert / R;
     const Parts parts = {m.v, m.hdr, m.marks, PARTS, p.cap_bytes};
@@ -304,7 +305,7 @@ __global__ void __launch_bounds__(512, 2) k_down_combine(const ExpertMat m, cons
     float4 x[4];
     float mine = 0.f;
     auto prologue = [&] {
-        grid_dependency_wait();
+        grid_wait();
         const char * xp = p.x + t * p.x_tok + s * p.x_slot;
         const float * x2 = p.x2 + (xp - p.x) / 4;
 #pragma unroll
@@ -333,7 +334,7 @@ __global__ void __launch_bounds__(512, 2) k_down_combine(const ExpertMat m, cons
     __syncthreads();
     if (threadIdx.x < R) {
         float acc = 0.f;
-        for (int kx = 0; kx < p.n_used; kx++) { acc = fmaf(weights[(int64_t) t * p.n_used + kx], ys[kx][threadIdx.x], acc); }
+        for (int kx = 0; kx < p.n_used; kx++) { acc = fmaf(ws[kx], ys[kx][threadIdx.x], acc); }
         const OutVec o = {out + (int64_t) t * p.rows_per_expert * (out_bf16 ? 2 : 4), out_bf16};
         o.put((int64_t) blockIdx.x * R + threadIdx.x, acc);
     }
@@ -377,7 +378,7 @@ ExpertMat expert_mat(const bf16n_weight & w, float * y, const uint16_t * marks =
 uint32_t unit_cap(const bf16n_weight & w) { return (uint32_t) ((w.R * w.K * 3 / 8 + 64 + 15) & ~15ll); }
 
 // Parts while a launch has few columns: a step of 1 / 2 / 3 / 4 / 6 / 8 tokens of 8 slots takes 26.6 / 42.0 / 61 / 64 / 86 / 105.7 us a warp to
-// a unit and 23.0 / 32.7 / 45.7 / 57.1 / 80.8 / 100.7 a warp to a part; 16 and 32 tokens 179 and 336 against 190 and 358 (the blocks' openings).
+// a unit and 20.0 / 32.4 / 45.6 / 56.8 / 81.0 / 100.7 a warp to a part; 16 and 32 tokens 179 and 336 against 190 and 358 (the blocks' openings).
 constexpr int g_parts_max_cols = 64;
 int g_plane_staged_warps_per_sm = 8; // stage the plane too while the launch has at most this many warps per SM
 
@@ -500,8 +501,8 @@ void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_
     q.rows_per_expert = H; q.cap_bytes = unit_cap(down);
     q.early_ids = true; // the ids precede the gate / up launch, whose outputs are the only thing this launch waits for
     if (marks.down && n_used <= COMBINE_SLOTS && ncols <= g_parts_max_cols && !(peers && peers->n_peers > 0)) {
-        launch_chained(k_down_combine, dim3((unsigned) (H / down.R), (unsigned) n_tok), dim3((unsigned) n_used * 64), part_smem(2 * n_used, n_used, q.cap_bytes).end,
-                       st, expert_mat(down, nullptr, marks.down), q, weights, (char *) y, y_bf16, Opaque{1u, 4u});
+        launch_chained(k_down_combine, dim3((unsigned) (H / down.R), (unsigned) n_tok), dim3((unsigned) n_used * 64),
+                       even_smem(part_smem(2 * n_used, n_used, q.cap_bytes).end, H / down.R * n_tok), st, expert_mat(down, nullptr, marks.down), q, weights, (char *) y, y_bf16, Opaque{1u, 4u});
         check_launch();
         return;
     }
@@ -527,6 +528,10 @@ void moe_decode_frag_order(const bf16n_weight & gate, const bf16n_weight & up, c
     a.y_tok = 4ll * n_used * N; a.y_slot = 4ll * N;
     a.y = g;
     fo_gemv_two(gate, up, a, u, st, behind_own);
+    if (fo_down_combine_applies(down, n_tok, n_used, n_experts)) {
+        fo_down_combine(down, g, u, ids, weights, n_tok, n_used, n_experts, y, y_bf16, st);
+        return;
+    }
     moe_swiglu(g, u, g, (int64_t) ncols * N, st);            // g := silu(g) * u
     bf16n_mmv_args d = a;
     d.x = g; d.x_bf16 = 0; d.x_per_slot = n_used; d.x_tok = 4ll * n_used * N; d.x_slot = 4ll * N;

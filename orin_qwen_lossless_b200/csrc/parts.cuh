@@ -146,6 +146,7 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t u, int64_t u
         }
         if (active && staged) {
             const uint32_t landed = dead ? 0u : mbar_wait(bar + 8 * b, (phases >> b) & 1u), words = buf0 + b * (p.cap + PART_SLACK);
+            if (!LOOP) { grid_launch_dependents(); }
             phases ^= 1u << b;
             bool joined = false;
             if (landed) {
