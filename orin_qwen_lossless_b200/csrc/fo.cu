@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256, G > 1 ? 4 : 1) k_fo_gemv_split(const FoMa
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncwarp();
     if (lut_first) { stage_lut(lut, w.lut); } // while the kernel before this one, which is this library's, drains (launch_behind)
-    grid_wait(); // activations and expert ids may come from the kernel before this one
+    bare_grid_dependency_wait(); // activations and expert ids may come from the kernel before this one
     if (!lut_first) { stage_lut(lut, w.lut); }
     const TX * xg; OutVec out; int64_t rbase;
     column<TX>(p, MMA ? 0 : blockIdx.y, xg, out, rbase);

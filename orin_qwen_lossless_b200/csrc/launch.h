@@ -67,7 +67,7 @@ void launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t shm,
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // The wait alone, for a kernel that lets its successor begin later: a successor's prologue asks for its own streams and planes, and
 // while this kernel's are still on their way they are in each other's way.
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void bare_grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Blocks until every kernel this one depends on has completed and its writes are visible; then lets the next kernel on
 // the stream begin its own prologue.
 __device__ __forceinline__ void grid_dependency_wait() {

@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(256, 4) k_expert_parts(const ExpertMat m0, con
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const ExpertMat & m = blockIdx.z ? m1 : m0;
     stage_table(smem, m.v.lut);
-    if (!p.early_ids) { grid_wait(); } // as above
+    if (!p.early_ids) { bare_grid_dependency_wait(); } // as above
     const int col = blockIdx.y, t = col / p.n_used, s = col - t * p.n_used;
     const int e = *(const int32_t *) (p.ids + t * p.ids_s1 + s * p.ids_s0) - p.e_lo;
     const int64_t units = p.rows_per_expert / R;
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(256, 4) k_expert_parts(const ExpertMat m0, con
         }
     };
     walk_parts<false>(parts, first_unit(parts), units, (int64_t) e * units, R * C * CHUNK, smem, [&] {
-        if (p.early_ids) { grid_wait(); }
+        if (p.early_ids) { bare_grid_dependency_wait(); }
         load_x(CM ? warp % PARTS : 0);
     }, rows, put);
 }
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(512, 2) k_down_combine(const ExpertMat m, cons
     float4 x[4];
     float mine = 0.f;
     auto prologue = [&] {
-        grid_wait();
+        bare_grid_dependency_wait();
         const char * xp = p.x + t * p.x_tok + s * p.x_slot;
         const float * x2 = p.x2 + (xp - p.x) / 4;
 #pragma unroll
