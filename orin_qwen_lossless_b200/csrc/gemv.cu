@@ -632,7 +632,9 @@ template <int C, typename TX, bool GLU>
 void launch_nib_c(const NibView & g, const NibView & v, const Cols & p, int ncols, cudaStream_t st) {
     const dim3 grid = row_geometry(p.nrows, ncols);
     const bool few = p.nrows * ncols <= 3 * (int64_t) device_info().sms * nib_blocks(C, GLU) * 8; // rows against resident warps
-    launch_chained(few ? k_nib_gemv<C, TX, GLU, true> : k_nib_gemv<C, TX, GLU, false>, grid, dim3(256), 0, st, g, v, p);
+    // spread evenly (even_smem): chains of products of 1024 x 2048, 2048 x 2048, 1024 x 4096, one column: 2.49 / 2.90 / 3.26 us a launch with blocks
+    // crowded where the launch in front had ended, 1.75 / 2.29 / 2.31 so; two tokens through 24 layers of small matrices 227 and 201 us
+    launch_chained(few ? k_nib_gemv<C, TX, GLU, true> : k_nib_gemv<C, TX, GLU, false>, grid, dim3(256), even_smem(0, (int64_t) grid.x * grid.y), st, g, v, p);
 }
 template <typename TX, bool GLU>
 void launch_nib(const NibView & g, const NibView & v, const Cols & p, int64_t K, int ncols, cudaStream_t st) {
@@ -776,6 +778,7 @@ void launch_expand(const bf16n_weight & w, int64_t row0, int64_t nrows, const Si
 
 BF16N_DEFINE_FAULT_WORD(row_gather_fault_word)
 
+static void gemv_group_init();
 void gemv_init() {
     const int optin = device_info().smem_optin;
 #define ATTR(KERNEL, BYTES) allow_dynamic_smem((const void *) KERNEL, (int) (BYTES), optin, #KERNEL)
@@ -792,6 +795,12 @@ void gemv_init() {
     ATTR(k_pair_rows_staged<true>, 6 * HP_MAX_PAIRS + 128 + 2 * (16 * K_MAX * 3 / 8 + 80));
     ATTR(k_pair_rows_staged<false>, 6 * HP_MAX_PAIRS + 128 + 2 * (16 * K_MAX * 3 / 8 + 80));
 #undef ATTR
+#define NIB_ATTR(C, TX, GLU) allow_dynamic_smem((const void *) k_nib_gemv<C, TX, GLU, true>, optin, optin, "nib"); allow_dynamic_smem((const void *) k_nib_gemv<C, TX, GLU, false>, optin, optin, "nib");
+#define NIB_ATTR_C(C) NIB_ATTR(C, float, false) NIB_ATTR(C, bf16, false) NIB_ATTR(C, float, true) NIB_ATTR(C, bf16, true)
+    NIB_ATTR_C(1) NIB_ATTR_C(2) NIB_ATTR_C(4) NIB_ATTR_C(8)
+#undef NIB_ATTR_C
+#undef NIB_ATTR
+    gemv_group_init();
     expand_rows_init();
     gemv_staged_init();
     gemv_rings_init();
@@ -859,6 +868,11 @@ __global__ void __launch_bounds__(256, WIDE ? 0 : 3) k_nib_gemv_group(const NibG
 
 } // namespace
 
+static void gemv_group_init() {
+    allow_dynamic_smem((const void *) k_nib_gemv_group<false>, device_info().smem_optin, device_info().smem_optin, "nib group");
+    allow_dynamic_smem((const void *) k_nib_gemv_group<true>, device_info().smem_optin, device_info().smem_optin, "nib group");
+}
+
 // dense NIBBLE products of up to 8 columns can share a grid
 bool gemv_groupable(const bf16n_weight & w, const bf16n_mmv_args & a) {
     const int C = (int) (w.K / CHUNK);
@@ -886,7 +900,7 @@ void gemv_group(const bf16n_weight * w, const bf16n_mmv_args * a, int n, cudaStr
             blocks += it.blocks * it.ncols;
             i++;
         }
-        launch_chained(wide ? k_nib_gemv_group<true> : k_nib_gemv_group<false>, dim3((unsigned) blocks), dim3(256), 0, st, g);
+        launch_chained(wide ? k_nib_gemv_group<true> : k_nib_gemv_group<false>, dim3((unsigned) blocks), dim3(256), even_smem(0, blocks), st, g);
         check_launch();
     }
 }
