@@ -288,7 +288,7 @@ int bf16n_mmv(const bf16n_weight * w, const bf16n_mmv_args * a, void * stream, i
 size_t bf16n_marks_bytes(const bf16n_weight * w) { return w ? marks_bytes(*w) : 0; }
 int bf16n_marks_build(const bf16n_weight * w, void * marks, void * stream) {
     return guarded([&] {
-        ensure_init();
+        // no initialisation: a loader may upload to a GPU before the process settles on its own
         require(w && marks, "marks_build: null argument");
         check_weight(*w);
         require(marks_bytes(*w) > 0, "marks_build: this layout has no marks");

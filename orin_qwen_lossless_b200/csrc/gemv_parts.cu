@@ -330,7 +330,7 @@ size_t marks_bytes(const bf16n_weight & w) {
 
 void marks_build(const bf16n_weight & w, uint16_t * marks, cudaStream_t st) {
     const int64_t units = w.rows / w.R;
-    k_marks<<<(unsigned) std::min<int64_t>((units + 7) / 8, (int64_t) device_info().sms * 8), 256, 0, st>>>(pair_view(w), unit_parts(w), units, marks);
+    k_marks<<<(unsigned) std::min<int64_t>((units + 7) / 8, 1184), 256, 0, st>>>(pair_view(w), unit_parts(w), units, marks);
     check_launch();
 }
 
