@@ -264,7 +264,9 @@ void launch_gemv_parts(const bf16n_weight & w, const uint16_t * marks, const Col
     const Parts p = make_parts(w, marks);
     const int per = units_per_block(p.parts), warps = per * p.parts;
     const int64_t units = q.nrows / w.R, blocks = (units + per - 1) / per;
-    const size_t shm = part_smem(warps, per, p.cap).end + (size_t) NC * w.K * sizeof(TX);
+    // spread evenly (even_smem): 256 blocks of 8192 x 1024 and 4096 x 2048, two / four columns: 8.7 / 10.8 and 8.3 / 10.6 us crowded, 7.3 / 8.9 and
+    // 7.0 / 8.4 so; expert parts, gathers and fragment-order products were level
+    const size_t shm = even_smem(part_smem(warps, per, p.cap).end + (size_t) NC * w.K * sizeof(TX), blocks);
     const Opaque k = {1u, 4u};
     launch_chained(k_gemv_parts<C, NC, TX>, dim3((unsigned) (parts_loop(NC) ? std::min(blocks, (int64_t) device_info().sms * parts_resident(C, NC)) : blocks)), dim3(warps * 32), shm, st, p, q, w.R, ncols, k);
 }
