@@ -134,8 +134,9 @@ int bf16n_mmv(const bf16n_weight * w, const bf16n_mmv_args * a, void * stream, i
  * memory (about 1.2 % of the matrix; 0: this layout has none) that the caller owns and bf16n_marks_build fills on the stream, once
  * per matrix. With them a product or a reconstruction of few units walks a lane stream from several places at once. They are hints:
  * every place is checked against where the codes before it ended, and where one does not agree (a matrix written since, marks not
- * written yet, any bytes at all) the unit is decoded from its start. Results never depend on them, and marks = NULL is the call
- * without them. They have no counterpart in the reference. */
+ * written yet, any bytes at all) the unit is decoded from its start. Results never depend on what they hold. How many there are is not
+ * checked here: the marks of a call are bf16n_marks_bytes(w) bytes for the w of that call, 2-byte aligned, or NULL (the call without
+ * them). They have no counterpart in the reference. */
 size_t bf16n_marks_bytes(const bf16n_weight * w);
 int bf16n_marks_build(const bf16n_weight * w, void * marks, void * stream);
 int bf16n_mmv_marked(const bf16n_weight * w, const void * marks, const bf16n_mmv_args * a, void * stream, int multi_col);

@@ -70,7 +70,8 @@ bool matrix_of(PyObject * w, Matrix & m) {
     if (marks.p != Py_None) {
         if (!plain(marks.p)) { return false; }
         const at::Tensor & k = THPVariable_Unpack(marks.p);
-        if (k.device() == m.device) { m.marks = k.const_data_ptr(); }
+        const bool whole = k.is_contiguous() && (size_t) k.numel() * k.element_size() == bf16n_marks_bytes(&m.c);
+        if (k.device() == m.device && whole && (uintptr_t) k.const_data_ptr() % 2 == 0) { m.marks = k.const_data_ptr(); }
     }
     return true;
 }

@@ -45,6 +45,13 @@ class Meta:
         flags = (FLAG_CHUNK_MAJOR if self.chunk_major else 0) | (FLAG_FRAG_ORDER if self.frag_order else 0)
         return [self.format, self.K, self.rows, self.R, flags, self.off_a, self.off_b, self.off_c, self.off_d]
 
+    def marks_bytes(self) -> int:
+        """bf16n_marks_bytes without the call: a lane-major pair-Huffman unit is cut into parts of 4096 weights, 2 to 16 of them."""
+        weights = self.R * self.K
+        if self.format != FMT_HUFPAIR or self.frag_order or weights % 4096 or not 2 * 4096 <= weights <= 16 * 4096:
+            return 0
+        return self.rows // self.R * (weights // 4096 - 1) * 64
+
 
 def parse_header(aux: torch.Tensor) -> Meta:
     """Metadata from the first 256 bytes of a CPU aux tensor; raises ValueError on a malformed header."""
@@ -62,7 +69,7 @@ class Weight:
     plane: torch.Tensor
     aux: torch.Tensor
     meta: Meta
-    marks: torch.Tensor | None = None    # where the lane streams can be entered (bf16n_marks_build): a hint, checked on the device
+    marks: torch.Tensor | None = None    # where the lane streams can be entered (bf16n_marks_build): their bytes are checked on the device
 
     @property
     def m(self) -> list[int]:
@@ -73,7 +80,13 @@ class Weight:
         return self.plane.numel() + self.aux.numel()
 
     def marks_ptr(self) -> int | None:
-        return None if self.marks is None or self.marks.device != self.plane.device else self.marks.data_ptr()
+        """The marks for a call; None for marks that are not of this matrix's size (another matrix was put in) or not in this memory. What
+        they hold is checked where they are used; how many there are is checked here and nowhere behind."""
+        k = self.marks
+        if k is None or k.device != self.plane.device or not k.is_contiguous() or k.numel() * k.element_size() != self.meta.marks_bytes():
+            return None
+        p = k.data_ptr()
+        return p if p and p % 2 == 0 else None
 
     def c(self) -> CWeight:
         m = self.meta
