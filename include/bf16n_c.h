@@ -139,6 +139,8 @@ int bf16n_mmv(const bf16n_weight * w, const bf16n_mmv_args * a, void * stream, i
  * them). They have no counterpart in the reference. */
 size_t bf16n_marks_bytes(const bf16n_weight * w);
 int bf16n_marks_build(const bf16n_weight * w, void * marks, void * stream);
+/* The same for an aux buffer of aux_bytes that may not hold the matrix yet: nothing behind it is read, whatever it holds. */
+int bf16n_marks_build_within(const bf16n_weight * w, uint64_t aux_bytes, void * marks, void * stream);
 int bf16n_mmv_marked(const bf16n_weight * w, const void * marks, const bf16n_mmv_args * a, void * stream, int multi_col);
 int bf16n_dequant_marked(const bf16n_weight * w, const void * marks, int64_t row0, int64_t nrows, uint16_t * out, void * stream);
 int bf16n_get_rows_marked(const bf16n_weight * w, const void * marks, const void * ids, int64_t ids_s0, int64_t n, void * dst, int dst_bf16,

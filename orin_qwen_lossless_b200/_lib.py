@@ -64,6 +64,7 @@ SIGNATURES = {
     "bf16n_mmv": (C.c_int, [C.POINTER(Weight), C.POINTER(MmvArgs), C.c_void_p, C.c_int]),
     "bf16n_marks_bytes": (C.c_size_t, [C.POINTER(Weight)]),
     "bf16n_marks_build": (C.c_int, [C.POINTER(Weight), C.c_void_p, C.c_void_p]),
+    "bf16n_marks_build_within": (C.c_int, [C.POINTER(Weight), C.c_uint64, C.c_void_p, C.c_void_p]),
     "bf16n_mmv_marked": (C.c_int, [C.POINTER(Weight), C.c_void_p, C.POINTER(MmvArgs), C.c_void_p, C.c_int]),
     "bf16n_dequant_marked": (C.c_int, [C.POINTER(Weight), C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
     "bf16n_get_rows_marked": (C.c_int, [C.POINTER(Weight), C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_int, C.c_int64, C.c_void_p, C.c_int64]),

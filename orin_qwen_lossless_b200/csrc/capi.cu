@@ -286,15 +286,16 @@ int bf16n_mmv(const bf16n_weight * w, const bf16n_mmv_args * a, void * stream, i
 }
 
 size_t bf16n_marks_bytes(const bf16n_weight * w) { return w ? marks_bytes(*w) : 0; }
-int bf16n_marks_build(const bf16n_weight * w, void * marks, void * stream) {
+int bf16n_marks_build_within(const bf16n_weight * w, uint64_t aux_bytes, void * marks, void * stream) {
     return guarded([&] {
         // no initialisation: a loader may upload to a GPU before the process settles on its own
         require(w && marks, "marks_build: null argument");
         check_weight(*w);
         require(marks_bytes(*w) > 0, "marks_build: this layout has no marks");
-        marks_build(*w, (uint16_t *) marks, (cudaStream_t) stream);
+        marks_build(*w, aux_bytes, (uint16_t *) marks, (cudaStream_t) stream);
     });
 }
+int bf16n_marks_build(const bf16n_weight * w, void * marks, void * stream) { return bf16n_marks_build_within(w, UINT64_MAX, marks, stream); }
 
 int bf16n_mmv_group(const bf16n_weight * w, const bf16n_mmv_args * a, int n, void * stream) {
     return guarded([&] {

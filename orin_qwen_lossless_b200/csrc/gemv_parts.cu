@@ -233,23 +233,36 @@ __global__ void __launch_bounds__(512) k_rows_parts(const Parts p, int R, const 
     }
 }
 
-// One warp per unit, once per matrix: where every 64 codes of a lane begin.
-__global__ void __launch_bounds__(256) k_marks(const PairView w, int parts, int64_t units, uint16_t * marks) {
+// One warp per unit, once per matrix: where every 64 codes of a lane begin. `last`: the last stream word that may be read. A loader may
+// upload memory that it fills later, so nothing that the aux buffer holds is taken for right here: words behind `last` are not
+// read, and a length counts as at most HP_LMAX bits.
+__global__ void __launch_bounds__(256) k_marks(const PairView w, int parts, int64_t units, uint16_t * marks, uint32_t last) {
     __shared__ uint32_t lut[HP_MAX_PAIRS];
     for (int i = threadIdx.x; i < HP_MAX_PAIRS; i += 256) { lut[i] = __ldg(w.lut + i); }
     __syncthreads();
     const int lane = threadIdx.x & 31;
     for (int64_t u = (int64_t) blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += (int64_t) gridDim.x * 8) {
-        PairReader rd;
-        rd.open(w, u, lane);
-        uint32_t bits = 0;
+        uint32_t next = __ldg(w.ubase + u) + __ldg(w.lrel + u * 32 + lane);
+        auto word = [&] { return __ldg(w.stream + min(next++, last)); };
+        uint64_t buf = (uint64_t) word() << 32;
+        buf |= word();
+        uint32_t ahead = word(), bits = 0;
+        int have = 64;
         for (int s = 1; s < parts; s++) {
 #pragma unroll 1
-            for (int i = 0; i < PART_STEPS; i++) {
-                uint32_t e[8];
-                rd.take8(lut, e);
+            for (int i = 0; i < 32 * PART_STEPS / 8; i++) { // two codes
+                if (have <= 32) {
+                    buf |= (uint64_t) ahead << (32 - have);
+                    have += 32;
+                    ahead = word();
+                }
 #pragma unroll
-                for (int q = 0; q < 8; q++) { bits += e[q] & 31u; }
+                for (int q = 0; q < 2; q++) {
+                    const int n = min((int) (lut[(uint32_t) (buf >> (64 - HP_LMAX))] & 31u), HP_LMAX);
+                    buf <<= n;
+                    have -= n;
+                    bits += n;
+                }
             }
             marks[(u * (parts - 1) + s - 1) * 32 + lane] = (uint16_t) bits;
         }
@@ -330,9 +343,15 @@ size_t marks_bytes(const bf16n_weight & w) {
     return parts ? (size_t) (w.rows / w.R) * (parts - 1) * 32 * sizeof(uint16_t) : 0;
 }
 
-void marks_build(const bf16n_weight & w, uint16_t * marks, cudaStream_t st) {
-    const int64_t units = w.rows / w.R;
-    k_marks<<<(unsigned) std::min<int64_t>((units + 7) / 8, 1184), 256, 0, st>>>(pair_view(w), unit_parts(w), units, marks);
+void marks_build(const bf16n_weight & w, uint64_t aux_bytes, uint16_t * marks, cudaStream_t st) {
+    const uint64_t units = (uint64_t) (w.rows / w.R);
+    auto holds = [&](uint64_t off, uint64_t n, uint64_t align) { return off % align == 0 && off <= aux_bytes && n <= aux_bytes - off; };
+    require(holds(w.off_a, 4 * HP_MAX_PAIRS, 4) && holds(w.off_b, units * 4, 4) && holds(w.off_c, units * 64, 2) && holds(w.off_d, 4, 4),
+            "marks_build: aux shorter than its offsets");
+    const uint64_t words = (aux_bytes - w.off_d) / 4;
+    if (units == 0) { return; }
+    k_marks<<<(unsigned) std::min<uint64_t>((units + 7) / 8, 1184), 256, 0, st>>>(pair_view(w), unit_parts(w), (int64_t) units, marks,
+                                                                                  (uint32_t) std::min<uint64_t>(words - 1, UINT32_MAX));
     check_launch();
 }
 

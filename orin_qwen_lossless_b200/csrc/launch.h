@@ -87,7 +87,7 @@ void expand_rows(const bf16n_weight & w, int64_t row0, int64_t nrows, const dev:
 void gemv_parts_init();
 int unit_parts(const bf16n_weight & w);    // parts of a unit, 0 when this layout is not cut
 size_t marks_bytes(const bf16n_weight & w); // 0: this layout has none
-void marks_build(const bf16n_weight & w, uint16_t * marks, cudaStream_t st);
+void marks_build(const bf16n_weight & w, uint64_t aux_bytes, uint16_t * marks, cudaStream_t st); // reads nothing behind aux_bytes
 bool gemv_parts_applies(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a);
 void gemv_parts(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a, cudaStream_t st);
 bool expand_parts_applies(const bf16n_weight & w, const uint16_t * marks, int64_t nrows);

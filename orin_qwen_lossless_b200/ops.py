@@ -197,7 +197,10 @@ def choose(rows: int, K: int, n_matrices: int = 1, *, engine: str = "vllm", mode
 
 def upload(plane: torch.Tensor, aux: torch.Tensor, meta: Meta, device: torch.device | str) -> Weight:
     w = Weight(plane.to(device), aux.to(device), meta)
-    w.marks = _make_marks(w)
+    try:
+        w.marks = _make_marks(w)
+    except Exception:       # marks only make calls faster: no memory for them, or a matrix that its first use refuses, does not refuse the upload
+        pass
     return w
 
 
@@ -211,7 +214,7 @@ def _make_marks(w: Weight) -> torch.Tensor | None:
         return None
     with torch.cuda.device(w.plane.device):
         marks = torch.empty(n, dtype=torch.uint8, device=w.plane.device)
-        return marks if lib().bf16n_marks_build(C.byref(cw), marks.data_ptr(), _stream()) == _lib.OK else None
+        return marks if lib().bf16n_marks_build_within(C.byref(cw), w.aux.numel(), marks.data_ptr(), _stream()) == _lib.OK else None
 
 
 # ------------------------------------------------------------------ device: dequant / verify
