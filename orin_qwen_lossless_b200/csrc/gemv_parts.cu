@@ -3,8 +3,8 @@
 // one block.
 //
 // What bounds them is latency: the code table, the unit's streams (one bulk copy) and the part's first plane bytes (straight into
-// registers, the others into L2) are one trip to memory together, then come 64 dependent lookups. 8192 x 2048, one token: 20.2 us
-// with a warp to each of the 512 units, 9.1 with 4096 parts (2.4 TB/s of stored bytes; 0.37 of what HBM gives). Activations lie in
+// registers, the others into L2) are one trip to memory together, then come 64 dependent lookups. 8192 x 2048, one token: 20.4 us
+// with a warp to each of the 512 units, 10.8 with 4096 parts (2.1 TB/s of stored bytes; 0.32 of what HBM gives). Activations lie in
 // shared memory as they are given; a quad of a column is read where it is multiplied, off the chain. Four blocks fit an SM at 64
 // registers, so 512 units of eight parts are one wave. Two and four columns take units in turn (16384 x 2048, 2 columns: 23.7 us
 // with a block to each unit, 20.4 so); one and eight do not, whose registers that overflows (9.1 against 10.1, 42 against 44).
@@ -54,9 +54,12 @@ __global__ void __launch_bounds__(C == 8 ? 512 : 256, parts_resident(C, NC)) k_g
     unsigned char * xs = smem + part_smem(blockDim.x >> 5, (blockDim.x >> 5) / p.parts, p.cap).end;
     const uint32_t xa = smem_u32(xs);
     float mine[NC]; // lane r: row r of the part
+    // Before anything of the matrix: a kernel of the caller's in front may have written it. 8192 x 2048, products one after the other, one /
+    // two / eight tokens: 9.0 / 13.5 / 20.9 us with the matrix read above the wait, 10.8 / 13.4 / 21.8 so; with the release of the next kernel
+    // here too (walk_parts has it behind the streams' arrival) 10.9 / 15.0 / 22.3, as an ordinary launch 11.2 / 13.8 / 22.4.
+    bare_grid_dependency_wait();
     auto prologue = [&] {
         stage_table(smem, p.w.lut);
-        grid_dependency_wait(); // the activations may be the kernel's before this one
         constexpr int VEC = 8 / (int) sizeof(TX); // eight bytes a load: what the interface asks of x and its strides
         for (int i = threadIdx.x; i < NC * (K / VEC); i += blockDim.x) {
             const int n = i / (K / VEC), c = i - n * (K / VEC);

@@ -1,0 +1,35 @@
+"""The kernels that walk units in parts share their loads (parts.cuh): where each of them waits for the kernel in front, and that what they
+read through the read-only path belongs to the matrix. Checked on the sources."""
+import re
+
+import pytest
+from test_dependent_launch_loads import MATRIX, SOURCES, _block, _kernel
+
+WALKERS = sorted(m.group(1) for f, s in SOURCES.items() if f.endswith(".cu") for m in re.finditer(r"__global__[^;{]*?\b(k_\w+)\([^{;]*\)\s*\{", s)
+                 if "walk_parts<" in _block(s, m.end() - 1))
+
+
+def test_the_walkers_are_found():
+    assert WALKERS == ["k_down_combine", "k_expand_parts", "k_expert_parts", "k_gemv_parts"]
+
+
+def test_dense_products_wait_before_they_read_the_matrix():
+    body = _kernel("k_gemv_parts")[1]
+    wait = body.index("grid_dependency_wait()")
+    assert wait < min(body.index(read) for read in ("stage_table(", "walk_parts<", "p.w.", "p.marks") if read in body)
+
+
+def test_rows_are_gathered_behind_the_callers_kernels():
+    assert "k_rows_parts" not in re.findall(r"launch_chained\((\w+)", SOURCES["gemv_parts.cu"])
+    launch = SOURCES["gemv_parts.cu"]
+    launch = _block(launch, launch.index("void rows_parts("))
+    assert re.search(r"launch_behind\(behind_own, kernel", launch) and launch.count("go(k_rows_parts<") == 3 and "<<<" not in launch
+
+
+@pytest.mark.parametrize("name", ["parts.cuh", "k_rows_parts"])
+def test_read_only_loads_are_the_matrix(name):
+    body = SOURCES[name] if name in SOURCES else _kernel(name)[1]
+    found = re.findall(r"(?:__ldg|ld_stream16)\(((?:[^()]|\([^()]*\))*)\)", body)
+    assert found
+    for arg in found:
+        assert MATRIX.search(arg) or re.search(r"\b(marks|from|cur|next)\b", arg), arg     # from, cur, next: PartPlane's pointers into the plane
