@@ -28,11 +28,13 @@ struct Parts {                                // the cut units of one matrix
     const AuxHeader * hdr;
     const uint16_t * marks;                   // [unit][part 1 ..][lane]
     int parts;                                // parts of a unit: R K / 4096
-    uint32_t cap;                             // bytes of streams that a unit's buffer holds
+    uint32_t cap;                             // bytes of streams that half of a unit's buffer holds: 3 bits a weight
+    // The whole of it: 6 bits a weight, the most that codes of HP_LMAX bits for two take, and what lanes and unit are rounded up by
+    __host__ __device__ constexpr uint32_t whole() const { return 2 * cap + PART_SLACK; }
 };
 
-// shared memory of a block that walks `units` units at a time with `warps` warps: table | barriers | starts | two buffers of
-// streams per unit | what the caller adds
+// shared memory of a block that walks `units` units at a time with `warps` warps: table | barriers | starts | a buffer of
+// streams per unit (two halves in turn, or one of twice the size) | what the caller adds
 struct PartSmem { uint32_t bars, starts, streams, end; };
 __host__ __device__ inline PartSmem part_smem(int warps, int units, uint32_t cap) {
     PartSmem s;
@@ -87,7 +89,11 @@ __device__ __forceinline__ int64_t first_unit(const Parts & p) {
 }
 
 // Every block takes units in turn, one warp to a part, all parts of a unit at once; the next unit's streams are copied, its plane
-// asked for and its start looked up while this one is decoded, and one block barrier a unit carries the check of its marks.
+// asked for and its start looked up while this one is decoded, and one block barrier a unit carries the check of its marks. Units that
+// fit half of the buffer (3 bits a weight; the benchmark's take 2.6) are copied into the halves in turn. A longer one takes the whole
+// buffer, so that it and its neighbours are copied when the unit before them is done: 62080 x 2048 of 3.4 bits, eight columns (one
+// turn), 159 us without marks, 667 where such units were left to one warp, 129 so; two columns, 16384 x 2048, 30.0, 114 and 22.5. Codes
+// that all have the same length put the lanes' words into one bank: 16384 x 2048 of 32 exponents that are equally likely, two columns, 29.8 and 43.8.
 //   u, units, unit0             this warp's (first) unit, where units end, and the matrix's unit that is unit 0
 //   prologue()                  what else the block needs, and the wait for the kernel in front; the barrier behind it is here. The
 //                               code table (stage_table) is at the front of the shared memory before that barrier
@@ -108,12 +114,14 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t u, int64_t u
     const uint8_t * plane = p.w.plane + part * (PART_STEPS * CHUNK) + 16 * lane;
 
     bool dead = false; // a copy never arrived (reported): this warp's units are decoded from global memory from then on
-    // the part's start into shared memory for the check, and the unit's streams on their way into buffer b
-    auto announce = [&](const PartStart & t, int b) {
-        asm volatile("st.shared.u32 [%0], %1;" ::"r"(starts0 + b * nwarp * 128), "r"(t.at) : "memory");
-        if (part == 0 && lane == 0 && t.bytes <= p.cap && !dead) {
+    auto place = [&](const PartStart & t, int b) { return buf0 + (LOOP && b && t.bytes <= p.cap ? p.cap + PART_SLACK : 0u); };
+    // the part's start into shared memory for the check, a block barrier before it is read there
+    auto announce = [&](const PartStart & t, int b) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(starts0 + b * nwarp * 128), "r"(t.at) : "memory"); };
+    // the unit's streams on their way, barrier b to tell of it
+    auto copy = [&](const PartStart & t, int b) {
+        if (part == 0 && lane == 0 && t.bytes <= p.whole() && !dead) {
             mbar_expect_tx(bar + 8 * b, t.bytes);
-            bulk_g2s(buf0 + b * (p.cap + PART_SLACK), p.w.stream + t.first, t.bytes, bar + 8 * b);
+            bulk_g2s(place(t, b), p.w.stream + t.first, t.bytes, bar + 8 * b);
         }
     };
     if (part == 0 && lane == 0) {
@@ -127,6 +135,7 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t u, int64_t u
         pl.load(plane + (unit0 + u) * unit_bytes); // ahead of the start, whose trip to memory the streams' copy waits for
         cur.load(p, unit0 + u, part, lane);
         announce(cur, 0);
+        copy(cur, 0);
         if (lane == 0) { bulk_prefetch_l2(pl.cur - 16 * lane + PART_AHEAD * CHUNK, (PART_STEPS - PART_AHEAD) * CHUNK); }
     }
     if (threadIdx.x < 3 * PART_UNITS) { ((int *) broken)[threadIdx.x] = 0; }
@@ -135,17 +144,20 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t u, int64_t u
     uint32_t phases = 0;
     for (int r = 0, slot = 0; r < rounds; r++, u += stride, slot = slot == 2 ? 0 : slot + 1) {
         const int b = r & 1;
-        const bool active = u < units, staged = cur.bytes <= p.cap;
+        const bool active = u < units, staged = cur.bytes <= p.whole(), more = LOOP && u + stride < units;
         PartStart nxt = {};
         pl.next = pl.cur;
-        if (LOOP && u + stride < units) {
+        bool behind = false; // the next unit's streams have no room beside this one's
+        if (more) {
             nxt.load(p, unit0 + u + stride, part, lane);
             announce(nxt, b ^ 1);
+            behind = max(cur.bytes, nxt.bytes) > p.cap;
+            if (!behind) { copy(nxt, b ^ 1); }
             pl.next = plane + (unit0 + u + stride) * unit_bytes;
             if (lane == 0) { bulk_prefetch_l2(pl.next, PART_STEPS * CHUNK); }
         }
         if (active && staged) {
-            const uint32_t landed = dead ? 0u : mbar_wait(bar + 8 * b, (phases >> b) & 1u), words = buf0 + b * (p.cap + PART_SLACK);
+            const uint32_t landed = dead ? 0u : mbar_wait(bar + 8 * b, (phases >> b) & 1u), words = place(cur, b);
             if (!LOOP) { grid_launch_dependents(); }
             phases ^= 1u << b;
             bool joined = false;
@@ -164,10 +176,11 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t u, int64_t u
             if (!joined && lane == 0) { broken[slot][ul] = 1; }
         }
         __syncthreads();
+        if (behind) { copy(nxt, b ^ 1); } // no warp reads this unit's streams any more
         if (threadIdx.x < PART_UNITS) { broken[slot == 0 ? 2 : slot - 1][threadIdx.x] = 0; } // read before this barrier, used after the next
         if (active && staged && !broken[slot][ul]) {
             store(u, part, false);
-        } else if (active && part == 0) { // streams longer than the buffer, or marks that are not this matrix's: the unit from its start
+        } else if (active && part == 0) { // marks that are not this matrix's, or streams longer than any code makes them: the unit from its start
             GlobalReader rd;
             rd.lut = (const uint32_t *) smem;
             rd.rd.open(p.w, unit0 + u, lane);
