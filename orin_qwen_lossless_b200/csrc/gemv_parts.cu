@@ -366,6 +366,10 @@ void marks_build(const bf16n_weight & w, uint64_t aux_bytes, uint16_t * marks, c
 //   4:         16384 x 2048 32.3 / 25.2, 24576 x 2048 36.5 / 36.2, 32768 x 2048 41.2 / 44.8 (3 columns: decoded twice without parts)
 //   8:         8192 x 2048 55 / 20.8, 62080 x 2048 156.7 / 126.9 (two decodes of four columns without parts)
 //   4096 columns of weights have no other form that stages streams: 8192 x 4096 82 / 18, 16384 x 4096 89 / 34.
+// With marks of another matrix (overwritten since, by a program that makes no new ones) every unit is decoded twice, the second time by one warp:
+// without marks / with wrong ones, 8192 x 2048, one and eight columns 20 / 48 and 51 / 101, 62080 x 2048, eight columns 161 / 710, reconstructed
+// 86 / 410, a decode step of one and eight tokens 24 / 55 and 101 / 333. So the marks are made again behind an update (45 us for 1024 x 2048
+// under a profiler), by the Python layer where it sees one. Kernels that wrote the true marks themselves were tried: 1 to 5 % on every call.
 bool gemv_parts_applies(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a) {
     const int C = (int) (w.K / CHUNK), parts = unit_parts(w);
     if (!marks || !parts || parts > (C == 8 ? 2 : 1) * PART_WARPS || w.cm || a.ids || a.ncols > 8 || !(C == 1 || C == 2 || C == 4 || C == 8)) { return false; }

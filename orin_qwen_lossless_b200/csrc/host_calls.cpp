@@ -20,7 +20,7 @@
 namespace {
 
 PyTypeObject * g_weight, * g_meta; // ops.Weight, ops.Meta
-PyObject * s_plane, * s_aux, * s_meta, * s_marks;
+PyObject * s_plane, * s_aux, * s_meta, * s_marks, * s_marks_at;
 const char * const META_FIELDS[10] = {"format", "K", "rows", "R", "chunk_major", "frag_order", "off_a", "off_b", "off_c", "off_d"};
 PyObject * s_fields[10];
 
@@ -70,6 +70,13 @@ bool matrix_of(PyObject * w, Matrix & m) {
     if (marks.p != Py_None) {
         if (!plain(marks.p)) { return false; }
         const at::Tensor & k = THPVariable_Unpack(marks.p);
+        Ref at(PyObject_GetAttr(w, s_marks_at));
+        if (!at.p) { PyErr_Clear(); return false; }
+        if (at.p != Py_None) { // aux was written since they were made: the Python function makes them again
+            const long long made = PyLong_AsLongLong(at.p);
+            if (made == -1 && PyErr_Occurred()) { PyErr_Clear(); return false; }
+            if (a.is_inference() || (long long) a._version() != made) { return false; }
+        }
         const bool whole = k.is_contiguous() && (size_t) k.numel() * k.element_size() == bf16n_marks_bytes(&m.c);
         if (k.device() == m.device && whole && (uintptr_t) k.const_data_ptr() % 2 == 0) { m.marks = k.const_data_ptr(); }
     }
@@ -230,6 +237,7 @@ PyMODINIT_FUNC PyInit__calls(void) {
     s_aux = PyUnicode_InternFromString("aux");
     s_meta = PyUnicode_InternFromString("meta");
     s_marks = PyUnicode_InternFromString("marks");
+    s_marks_at = PyUnicode_InternFromString("marks_at");
     for (int i = 0; i < 10; i++) { s_fields[i] = PyUnicode_InternFromString(META_FIELDS[i]); }
     return PyModule_Create(&module);
 }

@@ -70,6 +70,7 @@ class Weight:
     aux: torch.Tensor
     meta: Meta
     marks: torch.Tensor | None = None    # where the lane streams can be entered (bf16n_marks_build): their bytes are checked on the device
+    marks_at: int | None = None          # aux's version counter when they were made; None: not known
 
     @property
     def m(self) -> list[int]:
@@ -81,12 +82,17 @@ class Weight:
 
     def marks_ptr(self) -> int | None:
         """The marks for a call; None for marks that are not of this matrix's size (another matrix was put in) or not in this memory. What
-        they hold is checked where they are used; how many there are is checked here and nowhere behind."""
+        they hold is checked where they are used; how many there are is checked here and nowhere behind. After an in-place update of
+        aux they are made again first: results would be the same without, but every call slower than without marks."""
         k = self.marks
         if k is None or k.device != self.plane.device or not k.is_contiguous() or k.numel() * k.element_size() != self.meta.marks_bytes():
             return None
         p = k.data_ptr()
-        return p if p and p % 2 == 0 else None
+        if p == 0 or p % 2:
+            return None
+        if self.marks_at is not None and self.marks_at != _version(self.aux):
+            make_marks(self)
+        return self.marks.data_ptr()
 
     def c(self) -> CWeight:
         m = self.meta
@@ -102,6 +108,10 @@ class Weight:
             raise RuntimeError(f"bf16n: aux ({self.aux.numel()} bytes) shorter than its offsets")
         return CWeight(self.plane.data_ptr(), self.aux.data_ptr(), m.format, m.R, m.K, m.rows, int(m.chunk_major),
                        int(m.frag_order), m.off_a, m.off_b, m.off_c, m.off_d)
+
+
+def _version(t: torch.Tensor) -> int | None:
+    return None if t.is_inference() else t._version     # inference tensors count no versions
 
 
 _calls = None
@@ -198,23 +208,31 @@ def choose(rows: int, K: int, n_matrices: int = 1, *, engine: str = "vllm", mode
 def upload(plane: torch.Tensor, aux: torch.Tensor, meta: Meta, device: torch.device | str) -> Weight:
     w = Weight(plane.to(device), aux.to(device), meta)
     try:
-        w.marks = _make_marks(w)
+        make_marks(w)
     except Exception:       # marks only make calls faster: no memory for them, or a matrix that its first use refuses, does not refuse the upload
         pass
     return w
 
 
-def _make_marks(w: Weight) -> torch.Tensor | None:
-    """The marks of a matrix that was just uploaded; None for layouts without them, off the process's GPU and under capture."""
-    if w.meta.format != FMT_HUFPAIR or w.meta.frag_order or not w.plane.is_cuda or torch.cuda.is_current_stream_capturing():
-        return None
-    cw = w.c()
-    n = lib().bf16n_marks_bytes(C.byref(cw))
-    if n == 0:
-        return None
+def make_marks(w: Weight) -> bool:
+    """Makes the marks of a matrix on the GPU (w.marks) from what aux holds now, in the memory of those that it has where they are as many, so
+    that captured calls find them too. False, and nothing done, for layouts without marks, off the process's GPU and under capture.
+
+    upload() calls it, and so does the first call through a Weight whose aux torch has written since. A program that overwrites a matrix in
+    another way (a raw pointer, .data, inside a captured graph), or has only captured calls, calls it itself: with old marks results stay
+    right, but every unit is decoded twice, the second time by one warp."""
+    n = w.meta.marks_bytes()
+    if n == 0 or not w.plane.is_cuda or torch.cuda.is_current_stream_capturing():
+        return False
+    cw, at = w.c(), _version(w.aux)
     with torch.cuda.device(w.plane.device):
-        marks = torch.empty(n, dtype=torch.uint8, device=w.plane.device)
-        return marks if lib().bf16n_marks_build_within(C.byref(cw), w.aux.numel(), marks.data_ptr(), _stream()) == _lib.OK else None
+        old = w.marks
+        fits = old is not None and old.device == w.plane.device and old.is_contiguous() and old.numel() * old.element_size() == n and old.data_ptr() % 2 == 0
+        marks = old if fits else torch.empty(n, dtype=torch.uint8, device=w.plane.device)
+        if lib().bf16n_marks_build_within(C.byref(cw), w.aux.numel(), marks.data_ptr(), _stream()) != _lib.OK:
+            return False
+    w.marks, w.marks_at = marks, at
+    return True
 
 
 # ------------------------------------------------------------------ device: dequant / verify
