@@ -298,7 +298,9 @@ constexpr int SEL_BLOCKS = 8, SEL_THREADS = 1024, SEL_BINS = 2048;
 // Most of that is the barriers and the trips to the other blocks' histograms, and few keys matter: a block whose n_cand-th largest key lies in
 // a bin of the first digit has n_cand keys from that bin on, so no key below the largest of the blocks' bins is wanted. Each block
 // lists its keys from there on (a hundred or two of 7760 for 62080 rows and 128 candidates), and the first block finds the n_cand largest of the
-// lists on its own: a draft step of 62080 rows 43.1 -> 36.0 us, of four tokens 90 -> 70. Where a list does not fit (scores that are all alike), the digits are found by the whole cluster.
+// lists on its own: a draft step of 62080 rows 43.1 -> 36.0 us, of four tokens 90 -> 70. Where a list does not fit (scores of many rows that are all alike), the
+// digits are found by the whole cluster. Scores that are all alike and fit (a hidden state of zeros, up to 8192 rows): a step
+// of 8192 rows 47 us by the whole cluster, 2109 with each tie compared with every entry, 29 with the rows found digit by digit too.
 constexpr int SEL_LIST = 1024;            // keys of a block's list
 constexpr int SEL_KEYS_MAX = 48 * 1024;   // keys of a block that shared memory holds; beyond, every pass reads the scores again
 
@@ -404,32 +406,38 @@ k_select(const float * __restrict__ scores, int rows, int n_cand, int32_t * __re
                 const uint2 * l = cluster.map_shared_rank(&list[0], r);
                 for (int i = tid; i < (int) (first[r + 1] - first[r]); i += SEL_THREADS) { all[first[r] + i] = l[i]; }
             }
-            for (int i = tid; i < SEL_BINS; i += SEL_THREADS) { hist[0][i] = 0u; }
             cluster.sync();
+            // digit by digit the n_cand-th largest key, and where more entries have it than are wanted, the first rows of those: the
+            // need-th largest of their rows' complements, in the same three passes
+            uint32_t last_row = 0xffffffffu;
 #pragma unroll 1
-            for (int pass = 0; pass < 3; pass++) {
-                int shift, width;
-                digit(pass, shift, width);
-                for (int i = tid; i < total; i += SEL_THREADS) {
-                    const uint32_t v = all[i].x;
-                    if (pass == 0 || (v >> (shift + width)) == prefix) { atomicAdd(&hist[pass][(v >> shift) & ((1u << width) - 1u)], 1u); }
-                }
+            for (int by_row = 0; by_row < 2; by_row++) {
+                for (int i = tid; i < 3 * SEL_BINS; i += SEL_THREADS) { hist[0][i] = 0u; }
                 __syncthreads();
-                const int b = (1 << width) - 1 - 2 * tid;
-                find(b, b >= 0 ? hist[pass][b] : 0u, b >= 0 ? hist[pass][b - 1] : 0u, need);
-                prefix = prefix << width | s_bin;
-                need -= s_above;
-                equal = s_equal;
+                uint32_t found = 0;
+#pragma unroll 1
+                for (int pass = 0; pass < 3; pass++) {
+                    int shift, width;
+                    digit(pass, shift, width);
+                    for (int i = tid; i < total; i += SEL_THREADS) {
+                        const uint2 e = all[i];
+                        const uint32_t v = by_row ? ~e.y : e.x;
+                        if ((!by_row || e.x == prefix) && (pass == 0 || (v >> (shift + width)) == found)) { atomicAdd(&hist[pass][(v >> shift) & ((1u << width) - 1u)], 1u); }
+                    }
+                    __syncthreads();
+                    const int b = (1 << width) - 1 - 2 * tid;
+                    find(b, b >= 0 ? hist[pass][b] : 0u, b >= 0 ? hist[pass][b - 1] : 0u, need);
+                    found = found << width | s_bin;
+                    need -= s_above;
+                    equal = s_equal;
+                }
+                if (by_row) { last_row = ~found; break; }
+                prefix = found;
+                if (equal == need) { break; }
             }
             for (int i = tid; i < total; i += SEL_THREADS) {
                 const uint2 v = all[i];
-                bool take = v.x > prefix || (v.x == prefix && equal == need);
-                if (v.x == prefix && equal != need) { // the first rows of those that are the same
-                    uint32_t before = 0;
-                    for (int j = 0; j < total; j++) { before += all[j].x == prefix && all[j].y < v.y; }
-                    take = before < need;
-                }
-                if (take) { mine[atomicAdd(&s_count, 1u)] = (int32_t) v.y; }
+                if (v.x > prefix || (v.x == prefix && v.y <= last_row)) { mine[atomicAdd(&s_count, 1u)] = (int32_t) v.y; }
             }
             return;
         }
