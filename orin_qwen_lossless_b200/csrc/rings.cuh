@@ -74,11 +74,13 @@ __device__ __forceinline__ uint32_t cp_async_wait_all() { // returns the token r
 // (hi, lo, ahead) and a bit offset `o` into hi whose low five bits position the view and whose bit 5 toggles when the
 // offset passes a word. Only bits 0..5 of `o` are meaningful (table entries carry their length in the low bits and
 // exponents above), which is all the funnel shifts and the word-crossing test read.
-struct RingReader {
+// BOUNDED: a reader that a wrong mark may have started, which copies nothing from behind `limit`; the others carry none of it.
+template <bool BOUNDED>
+struct RingReaderOf {
     const uint8_t * base; // global
     uint32_t key;         // ring base | lane swizzle
     uint32_t fetched;     // offset of the next granule to copy
-    uint32_t limit;       // offset of the last granule that the aux buffer holds: a reader started by a wrong mark stays below it
+    uint32_t limit;       // BOUNDED: offset of the last granule that the aux buffer holds
     uint32_t next;        // offset of the next word to read
     uint32_t hi, lo, ahead, o;
     uint32_t token;       // from the last cp.async wait
@@ -90,7 +92,7 @@ struct RingReader {
 #pragma unroll
         for (int i = 0; i < ROUNDS; i++) {
             if (avail <= (int32_t) RING_TARGET) {
-                cp_async16(ring_addr(fetched, key), base + min(fetched, limit));
+                cp_async16(ring_addr(fetched, key), base + (BOUNDED ? min(fetched, limit) : fetched));
                 fetched = imad(k.sixteen, k.one, fetched);
                 avail = (int32_t) imad(k.sixteen, k.one, (uint32_t) avail);
             }
@@ -128,6 +130,7 @@ struct RingReader {
         o = o2;
     }
 };
+using RingReader = RingReaderOf<false>;
 
 } // namespace ring
 } // namespace b16
