@@ -538,7 +538,7 @@ static void moe_decode_checked(const bf16n_weight * gate, const bf16n_weight * u
         return;
     }
     moe_decode(*gate, *up, *down, x, x_bf16 != 0, x_tok, topk_ids, topk_weights, n_tok, n_used, n_experts_local, expert_lo,
-               scratch, y, y_bf16 != 0, (cudaStream_t) stream, peers, marks);
+               scratch, y, y_bf16 != 0, (cudaStream_t) stream, peers, n_experts, marks);
 }
 
 int bf16n_moe_decode_marked(const bf16n_weight * gate, const bf16n_weight * up, const bf16n_weight * down, const void * gate_marks,

@@ -358,14 +358,22 @@ void marks_build(const bf16n_weight & w, uint64_t aux_bytes, uint16_t * marks, c
     check_launch();
 }
 
-// Where the parts are the faster form, by units of the product. Whole units / parts in us (16 rows to a unit):
-//   1 column:  8192 x 2048 20.2 / 9.1, 16384 x 2048 22.1 / 17.0, 24576 x 2048 25.3 / 25.9; 16384 x 1024 12.7 / 9.0, 32768 x 1024
-//              15.7 / 16.6: up to 1024 units. FP32 activations the same: 23.3 / 20.5 and 26.8 / 30.9 for 1024 and 1536 units.
-//   2:         24576 x 2048 32.0 / 28.4, 32768 x 2048 35.6 / 35.2, 47360 x 2048 42.0 / 50.2; 65536 x 1024 45.5 / 37.8 (36.5 with the last
-//              round of whole units in parts), 65536 x 512 28.7 / 23.2
-//   4:         16384 x 2048 32.3 / 25.2, 24576 x 2048 36.5 / 36.2, 32768 x 2048 41.2 / 44.8 (3 columns: decoded twice without parts)
-//   8:         8192 x 2048 55 / 20.8, 62080 x 2048 156.7 / 126.9 (two decodes of four columns without parts)
-//   4096 columns of weights have no other form that stages streams: 8192 x 4096 82 / 18, 16384 x 4096 89 / 34.
+// Where the parts are the faster form, by units of the product. Time with parts over time without marks, units of 16 x 2048 (20 to 90 us; other K,
+// and units of 8 and 4 rows, alike):
+//   units            512  1024  1280  1536  2048  2560  3072  3584  4096
+//   1 column, BF16  0.55  0.82  0.96  1.09  1.29  1.23  1.30  1.29  1.41
+//   2               0.59  0.77  0.77  0.89  1.03  1.09  1.14  0.87  0.97
+//   3               0.36  0.48  0.49  0.58  0.68  0.73  0.76  0.66  0.72
+//   4               0.63  0.83  0.82  0.96  1.10  1.14  0.88  0.99  1.07
+//   5 / 6           0.46  0.61  0.69  0.82  0.92  1.02  0.88  0.98  1.05 / 0.89 (2960 units: 1.11 / 1.08; 4096 units of 4 x 2048 0.86 / 0.78)
+//   7 / 8           0.44  0.58  0.63  0.75  0.83  0.91  0.70  0.79  0.85 (of the two the slower)
+//   1 column, FP32  0.57  0.94  1.03  1.20  1.40  1.07  1.28  1.28  1.33
+//   2               0.68  0.56  0.57  0.67  0.83  0.48  0.56  0.65  0.75 (2048 units of 512 to 1024 columns or 4 rows 1.03 to 1.08)
+//   3               0.77  0.83  0.82  0.98  1.17  0.66  0.77  0.91  1.04 (1536 units of 8 and 4 rows 1.5)
+//   5 to 8          0.67  0.60  0.69  0.80  0.92  0.56  0.65  0.77  0.87
+// The kernels without marks take units in rounds, of 28, 24 and 20 per SM for one, two and four columns of BF16 and of 16 for FP32, and
+// are at their best when a round is just full. Differences of up to 8 % either way come with where the buffers lie. 4096 columns of weights have no other form that stages streams: 0.14 to 0.94 up to 4096
+// units, but three to six of FP32 up to 1.12 just before their round is full.
 // With marks of another matrix (overwritten since, by a program that makes no new ones) every unit is decoded twice, the second time by one warp:
 // without marks / with wrong ones, 8192 x 2048, one and eight columns 20 / 48 and 51 / 101, 62080 x 2048, eight columns 161 / 710, reconstructed
 // 86 / 410, a decode step of one and eight tokens 24 / 55 and 101 / 333. So the marks are made again behind an update (45 us for 1024 x 2048
@@ -374,8 +382,17 @@ bool gemv_parts_applies(const bf16n_weight & w, const uint16_t * marks, const bf
     const int C = (int) (w.K / CHUNK), parts = unit_parts(w);
     if (!marks || !parts || parts > (C == 8 ? 2 : 1) * PART_WARPS || w.cm || a.ids || a.ncols > 8 || !(C == 1 || C == 2 || C == 4 || C == 8)) { return false; }
     const int64_t units = a.nrows / w.R;
-    if (C < 8 && a.ncols == 2) { return units <= 4096 && units * C <= 6144; }
-    return units <= (C < 8 && (a.ncols == 1 || a.ncols == 4) ? 1024 : 4096);
+    const bool large = w.R * C >= 64; // units of 16 x 2048 weights and more
+    auto fills = [&](int64_t from, int per_sm) { return units > from && units <= per_sm * device_info().sms; };
+    if (units > 4096) { return false; }
+    if (C == 8) { return a.x_bf16 || a.ncols < 3 || a.ncols > 6 || !fills(1536, 16); }
+    switch (a.ncols) {
+        case 1: case 4: return units <= 1024;
+        case 2: return units * C <= 6144;
+        case 3: return a.x_bf16 || units <= (large ? 1536 : 1024) || (w.R >= 16 && units <= 3584 && !fills(1024, 16));
+        case 5: case 6: return !a.x_bf16 || !large || !fills(2304, 20);
+        default: return true;
+    }
 }
 
 void gemv_parts(const bf16n_weight & w, const uint16_t * marks, const bf16n_mmv_args & a, cudaStream_t st) {

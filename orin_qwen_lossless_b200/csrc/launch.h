@@ -177,7 +177,7 @@ void expert_units_mmv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStre
 bool moe_decode_supported(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_weight & down);
 void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_weight & down, const void * x, bool x_bf16,
                 int64_t x_tok, const int32_t * ids, const float * weights, int n_tok, int n_used, int n_experts_local, int e_lo,
-                float * scratch, void * y, bool y_bf16, cudaStream_t st, const bf16n_peer_out * peers = nullptr, const ExpertMarks & marks = {});
+                float * scratch, void * y, bool y_bf16, cudaStream_t st, const bf16n_peer_out * peers, int n_experts, const ExpertMarks & marks);
 void moe_decode_frag_order(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_weight & down, const void * x, bool x_bf16,
                            int64_t x_tok, const int32_t * ids, const float * weights, int n_tok, int n_used, int n_experts,
                            float * scratch, void * y, bool y_bf16, cudaStream_t st, bool behind_own);

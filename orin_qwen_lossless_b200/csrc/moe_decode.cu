@@ -377,9 +377,10 @@ ExpertMat expert_mat(const bf16n_weight & w, float * y, const uint16_t * marks =
 
 uint32_t unit_cap(const bf16n_weight & w) { return (uint32_t) ((w.R * w.K * 3 / 8 + 64 + 15) & ~15ll); }
 
-// Parts while a launch has few columns: a step of 1 / 2 / 3 / 4 / 6 / 8 tokens of 8 slots takes 26.6 / 42.0 / 61 / 64 / 86 / 105.7 us a warp to
-// a unit and 20.0 / 32.4 / 45.6 / 56.8 / 81.0 / 100.7 a warp to a part; 16 and 32 tokens 179 and 336 against 190 and 358 (the blocks' openings).
-constexpr int g_parts_max_cols = 64;
+// Parts while a launch has few columns: a step of 1 / 2 / 3 / 4 / 6 / 8 tokens of 8 slots and 64 experts takes 24.4 / 35.9 / 52 / 58 / 80 / 101 us a warp
+// to a unit and 0.78 / 0.82 / 0.80 / 0.92 / 0.94 / 0.93 of that a warp to a part; 10 and 12 tokens 1.0 (the blocks' openings); of 16 experts, whose
+// columns share more, 4 / 5 / 6 / 8 tokens 0.96 / 1.00 / 1.02 / 1.04. n_experts: of the whole layer.
+bool parts_pay(int ncols, int n_experts) { return ncols <= (n_experts <= 16 ? 40 : 64); }
 int g_plane_staged_warps_per_sm = 8; // stage the plane too while the launch has at most this many warps per SM
 
 template <int C, int R, bool CM, typename TX, bool GLU_IN>
@@ -404,7 +405,7 @@ void launch_units(const ExpertMat & m0, const ExpertMat & m1, int n_mats, const 
         attr_done = true;
     }
     if (ncols == 0) { return; }
-    if (m0.marks && m1.marks && ncols <= g_parts_max_cols) {
+    if (m0.marks && m1.marks) {
         constexpr int PARTS = R * C / PART_STEPS, PER = 8 / PARTS;
         const size_t shm = part_smem(8, PER, p.cap_bytes).end + (CM ? PER * PARTS * R * 32 * sizeof(float) : 0);
         launch_chained(k_expert_parts<C, R, CM, TX, GLU_IN>, dim3((unsigned) ((units + PER - 1) / PER), (unsigned) ncols, (unsigned) n_mats), dim3(256), shm, st, m0, m1, p,
@@ -468,7 +469,10 @@ void expert_units_mmv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStre
     p.ids = (const char *) a.ids; p.ids_s0 = a.ids_s0; p.ids_s1 = a.ids_s1;
     p.n_used = a.n_used; p.rows_per_expert = a.rows_per_matrix; p.e_lo = 0; p.e_n = (int) (w.rows / a.rows_per_matrix);
     p.cap_bytes = unit_cap(w);
-    const ExpertMat m = expert_mat(w, (float *) a.y, marks);
+    // A product by itself, time with parts over time without: gate and up 0.64 to 1.05 as far as a step takes parts; down, 16 columns 0.88 to 0.97,
+    // 32 columns of FP32 0.88, but 24 columns of BF16 1.11 and 40 columns 1.14.
+    const bool parts = w.cm ? parts_pay(a.ncols, p.e_n) : a.ncols <= (a.x_bf16 ? 16 : 32);
+    const ExpertMat m = expert_mat(w, (float *) a.y, parts ? marks : nullptr);
     if (w.cm) {
         if (a.x_bf16) { launch_units<4, 8, true, bf16, false>(m, m, 1, p, a.ncols, st); }
         else { launch_units<4, 8, true, float, false>(m, m, 1, p, a.ncols, st); }
@@ -482,7 +486,8 @@ void expert_units_mmv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStre
 // scratch: FP32 [2 * n_tok * n_used * N + n_tok * n_used * H] (N, H = rows per expert of gate and down).
 void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_weight & down, const void * x, bool x_bf16,
                 int64_t x_tok, const int32_t * ids, const float * weights, int n_tok, int n_used, int n_experts_local, int e_lo,
-                float * scratch, void * y, bool y_bf16, cudaStream_t st, const bf16n_peer_out * peers, const ExpertMarks & marks) {
+                float * scratch, void * y, bool y_bf16, cudaStream_t st, const bf16n_peer_out * peers, int n_experts, const ExpertMarks & given) {
+    const ExpertMarks marks = parts_pay(n_tok * n_used, n_experts) ? given : ExpertMarks{};
     const int64_t N = gate.rows / n_experts_local, H = down.rows / n_experts_local;
     const int ncols = n_tok * n_used;
     float * g = scratch, * u = g + (int64_t) ncols * N, * ys = u + (int64_t) ncols * N;
@@ -500,7 +505,7 @@ void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_
     q.x = (const char *) g; q.x2 = u; q.x_tok = 4ll * n_used * N; q.x_slot = 4ll * N;
     q.rows_per_expert = H; q.cap_bytes = unit_cap(down);
     q.early_ids = true; // the ids precede the gate / up launch, whose outputs are the only thing this launch waits for
-    if (marks.down && n_used <= COMBINE_SLOTS && ncols <= g_parts_max_cols && !(peers && peers->n_peers > 0)) {
+    if (marks.down && n_used <= COMBINE_SLOTS && !(peers && peers->n_peers > 0)) {
         launch_chained(k_down_combine, dim3((unsigned) (H / down.R), (unsigned) n_tok), dim3((unsigned) n_used * 64),
                        even_smem(part_smem(2 * n_used, n_used, q.cap_bytes).end, H / down.R * n_tok), st, expert_mat(down, nullptr, marks.down), q, weights, (char *) y, y_bf16, Opaque{1u, 4u});
         check_launch();
@@ -590,7 +595,7 @@ void moe_decode_static(const bf16n_weight & gate, const bf16n_weight & up, const
                        int64_t x_tok, const int32_t * ids, const float * weights, int n_tok, int n_used, int n_experts_local,
                        int e_lo, void * y, bool y_bf16, cudaStream_t st) {
     moe_decode(gate, up, down, x, x_bf16, x_tok, ids, weights, n_tok, n_used, n_experts_local, e_lo,
-               static_scratch_of_current_device(), y, y_bf16, st);
+               static_scratch_of_current_device(), y, y_bf16, st, nullptr, n_experts_local, {});
 }
 
 } // namespace b16
