@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(512) k_rows_parts(const Parts p, int R, const 
         }
         cur.load(p, unit, warp, lane);
         asm volatile("st.shared.u32 [%0], %1;" ::"r"(starts), "r"(cur.at) : "memory");
-        if (threadIdx.x == 0 && cur.bytes <= p.whole()) {
+        if (threadIdx.x == 0 && cur.bytes <= p.whole) {
             mbar_expect_tx(bar, cur.bytes);
             bulk_g2s(words, p.w.stream + cur.first, cur.bytes, bar);
         }
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(512) k_rows_parts(const Parts p, int R, const 
     };
     if (warp <= part) {
         bool good = false;
-        if (cur.bytes <= p.whole()) {
+        if (cur.bytes <= p.whole) {
             const uint32_t landed = mbar_wait(bar, 0u);
             if (landed) {
                 WindowReader rd;

@@ -36,7 +36,7 @@ struct ExpertCols {
     int n_used;
     int64_t rows_per_expert;
     int e_lo, e_n;                             // experts held by this weight: global ids [e_lo, e_lo + e_n)
-    uint32_t cap_bytes;
+    uint32_t cap_bytes, whole_bytes; // parts: of half and of all of a unit's buffer
     bool early_ids;                            // the expert ids were complete before the PREVIOUS kernel on the stream
                                                // began its dependent work (they come from a kernel before that one):
                                                // ids, unit geometry and the bulk copies need not wait for it; only the
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(256, 4) k_expert_parts(const ExpertMat m0, con
         if (threadIdx.x < PER * R && r < p.rows_per_expert) { y[r] = 0.f; }
         return;
     }
-    const Parts parts = {m.v, m.hdr, m.marks, PARTS, p.cap_bytes};
+    const Parts parts = {m.v, m.hdr, m.marks, PARTS, p.cap_bytes, p.whole_bytes};
     float * sums = (float *) (smem + part_smem(8, PER, p.cap_bytes).end) + (warp / PARTS) * (PARTS * R * 32) + lane; // CM: [part][row][lane]
     float4 x[4];     // the lane's activations of one chunk: of the part's (CM), or all there are
     auto load_x = [&](int c) {
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(512, 2) k_down_combine(const ExpertMat m, cons
     if (warp % PARTS == 0 && lane == 0) { ws[s] = weights[(int64_t) t * p.n_used + s]; }
     const bool held = e >= 0 && e < p.e_n;
     const int64_t units = p.rows_per_expert / R;
-    const Parts parts = {m.v, m.hdr, m.marks, PARTS, p.cap_bytes};
+    const Parts parts = {m.v, m.hdr, m.marks, PARTS, p.cap_bytes, p.whole_bytes};
     if (lane < PART_STEPS) { ys[s][(warp % PARTS) * PART_STEPS + lane] = 0.f; } // another rank's expert adds exact zeros
     float4 x[4];
     float mine = 0.f;
@@ -443,7 +443,7 @@ void moe_decode_init() {
     // instantiate and set the shared-memory attribute of every variant outside of any stream capture
     ExpertMat none = {};
     ExpertCols p = {};
-    p.rows_per_expert = 16; p.cap_bytes = 16;
+    p.rows_per_expert = 16; p.cap_bytes = 16; p.whole_bytes = part_whole(16);
     launch_units<4, 8, true, bf16, false>(none, none, 2, p, 0, nullptr);
     launch_units<4, 8, true, float, false>(none, none, 2, p, 0, nullptr);
     launch_units<1, 16, false, float, true>(none, none, 1, p, 0, nullptr);
@@ -468,7 +468,7 @@ void expert_units_mmv(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStre
     p.x = (const char *) a.x; p.x_tok = a.x_tok; p.x_slot = a.x_per_slot == 1 ? 0 : a.x_slot;
     p.ids = (const char *) a.ids; p.ids_s0 = a.ids_s0; p.ids_s1 = a.ids_s1;
     p.n_used = a.n_used; p.rows_per_expert = a.rows_per_matrix; p.e_lo = 0; p.e_n = (int) (w.rows / a.rows_per_matrix);
-    p.cap_bytes = unit_cap(w);
+    p.cap_bytes = unit_cap(w); p.whole_bytes = part_whole(p.cap_bytes);
     // A product by itself, time with parts over time without: gate and up 0.64 to 1.05 as far as a step takes parts; down, 16 columns 0.88 to 0.97,
     // 32 columns of FP32 0.88, but 24 columns of BF16 1.11 and 40 columns 1.14.
     const bool parts = w.cm ? parts_pay(a.ncols, p.e_n) : a.ncols <= (a.x_bf16 ? 16 : 32);
@@ -495,7 +495,7 @@ void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_
     p.x = (const char *) x; p.x_tok = x_tok; p.x_slot = 0;
     p.ids = (const char *) ids; p.ids_s0 = 4; p.ids_s1 = 4ll * n_used;
     p.n_used = n_used; p.rows_per_expert = N; p.e_lo = e_lo; p.e_n = n_experts_local;
-    p.cap_bytes = unit_cap(gate);
+    p.cap_bytes = unit_cap(gate); p.whole_bytes = part_whole(p.cap_bytes);
     if (x_bf16) {
         launch_units<4, 8, true, bf16, false>(expert_mat(gate, g, marks.gate), expert_mat(up, u, marks.up), 2, p, ncols, st);
     } else {
@@ -503,7 +503,7 @@ void moe_decode(const bf16n_weight & gate, const bf16n_weight & up, const bf16n_
     }
     ExpertCols q = p;
     q.x = (const char *) g; q.x2 = u; q.x_tok = 4ll * n_used * N; q.x_slot = 4ll * N;
-    q.rows_per_expert = H; q.cap_bytes = unit_cap(down);
+    q.rows_per_expert = H; q.cap_bytes = unit_cap(down); q.whole_bytes = part_whole(q.cap_bytes);
     q.early_ids = true; // the ids precede the gate / up launch, whose outputs are the only thing this launch waits for
     if (marks.down && n_used <= COMBINE_SLOTS && !(peers && peers->n_peers > 0)) {
         launch_chained(k_down_combine, dim3((unsigned) (H / down.R), (unsigned) n_tok), dim3((unsigned) n_used * 64),

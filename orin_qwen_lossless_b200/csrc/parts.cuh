@@ -29,9 +29,11 @@ struct Parts {                                // the cut units of one matrix
     const uint16_t * marks;                   // [unit][part 1 ..][lane]
     int parts;                                // parts of a unit: R K / 4096
     uint32_t cap;                             // bytes of streams that half of a unit's buffer holds: 3 bits a weight
-    // The whole of it: 6 bits a weight, the most that codes of HP_LMAX bits for two take, and what lanes and unit are rounded up by
-    __host__ __device__ constexpr uint32_t whole() const { return 2 * cap + PART_SLACK; }
+    uint32_t whole;                           // and all of it: part_whole(cap)
 };
+// 6 bits a weight, the most that codes of HP_LMAX bits for two take, and what lanes and unit are rounded up by. From the host: worked out in
+// the kernels it cost a decode step of one token 0.3 us.
+constexpr uint32_t part_whole(uint32_t cap) { return 2 * cap + PART_SLACK; }
 
 // shared memory of a block that walks `units` units at a time with `warps` warps: table | barriers | starts | a buffer of
 // streams per unit (two halves in turn, or one of twice the size) | what the caller adds
@@ -119,7 +121,7 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t u, int64_t u
     auto announce = [&](const PartStart & t, int b) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(starts0 + b * nwarp * 128), "r"(t.at) : "memory"); };
     // the unit's streams on their way, barrier b to tell of it
     auto copy = [&](const PartStart & t, int b) {
-        if (part == 0 && lane == 0 && t.bytes <= p.whole() && !dead) {
+        if (part == 0 && lane == 0 && t.bytes <= p.whole && !dead) {
             mbar_expect_tx(bar + 8 * b, t.bytes);
             bulk_g2s(place(t, b), p.w.stream + t.first, t.bytes, bar + 8 * b);
         }
@@ -144,7 +146,7 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t u, int64_t u
     uint32_t phases = 0;
     for (int r = 0, slot = 0; r < rounds; r++, u += stride, slot = slot == 2 ? 0 : slot + 1) {
         const int b = r & 1;
-        const bool active = u < units, staged = cur.bytes <= p.whole(), more = LOOP && u + stride < units;
+        const bool active = u < units, staged = cur.bytes <= p.whole, more = LOOP && u + stride < units;
         PartStart nxt = {};
         pl.next = pl.cur;
         bool behind = false; // the next unit's streams have no room beside this one's
@@ -203,7 +205,8 @@ __device__ __forceinline__ void walk_parts(const Parts & p, int64_t u, int64_t u
 } // namespace dev
 
 inline dev::Parts make_parts(const bf16n_weight & w, const uint16_t * marks) {
-    return {dev::pair_view(w), (const AuxHeader *) w.aux, marks, unit_parts(w), (uint32_t) ((w.R * w.K * 3 / 8 + 64 + 15) & ~15ll)};
+    const uint32_t cap = (uint32_t) ((w.R * w.K * 3 / 8 + 64 + 15) & ~15ll);
+    return {dev::pair_view(w), (const AuxHeader *) w.aux, marks, unit_parts(w), cap, dev::part_whole(cap)};
 }
 
 } // namespace b16
