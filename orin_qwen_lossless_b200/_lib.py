@@ -6,6 +6,7 @@ There is no Python, PyTorch or CPU fallback for any operator.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 
 from . import build as _build
@@ -133,8 +134,8 @@ def lib():
     global _lib
     if _lib is None:
         path = _build.LIB
-        if not (os.path.exists(path) and os.path.exists(_build.CALLS)):
-            _build.build()
+        if not os.path.exists(path):
+            _build.build_library()
         _lib = C.CDLL(path)
         for name, (res, args) in SIGNATURES.items():
             fn = getattr(_lib, name)  # AttributeError here = the library does not export what the header declares
@@ -144,10 +145,15 @@ def lib():
 
 
 def calls():
-    """The extension module of the calls that the host bounds (csrc/host_calls.cpp)."""
+    """The extension module of the calls that the host bounds (csrc/host_calls.cpp), built first when this Python and torch have none."""
     lib()
-    from . import _calls
-    return _calls
+    path = _build.calls_path()
+    if not os.path.exists(path):
+        _build.build_calls()
+    spec = importlib.util.spec_from_file_location(__package__ + "._calls", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
 
 
 def check(rc: int) -> None:

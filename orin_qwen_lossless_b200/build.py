@@ -10,6 +10,7 @@ import concurrent.futures as cf
 import os
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(PKG, "csrc")
@@ -21,7 +22,6 @@ CUDA_SOURCES = ["gemv.cu", "gemv_staged.cu", "gemv_rings.cu", "gemv_parts.cu", "
 HOST_SOURCES = ["encode.cpp", "policy.cpp"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-pthread",
               "-I", INC]
-CALLS = os.path.join(PKG, "_calls.so")       # csrc/host_calls.cpp: an extension module over torch's C++ interface
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-pthread", "-Wall", "-Wextra", "-I", INC]
 
 
@@ -45,7 +45,13 @@ def _run(cmd: list[str]) -> None:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile what is out of date and link; returns the library path."""
+    """Compile what is out of date and link, the library and the extension module; returns the library path."""
+    build_library(force, verbose)
+    build_calls(force)
+    return LIB
+
+
+def build_library(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     deps = _deps()
     jobs = []
@@ -64,25 +70,29 @@ def build(force: bool = False, verbose: bool = False) -> str:
     objs = [os.path.join(OBJ, s + ".o") for s in CUDA_SOURCES + HOST_SOURCES]
     if force or jobs or _stale(LIB, objs):
         _run(["nvcc", "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", LIB, *objs, "-lpthread"])
-    build_calls(force)
     return LIB
+
+
+def calls_path() -> str:
+    """csrc/host_calls.cpp, an extension module over torch's C++ interface: it is bound to the Python and the torch that it was built for, so
+    each pair has a file of its own."""
+    import torch
+    return os.path.join(PKG, f"_calls-{sysconfig.get_config_var('SOABI')}-torch{torch.__version__}.so")
 
 
 def build_calls(force: bool = False) -> str:
     """The extension module of the calls that the host bounds; linked against the library beside it."""
-    src = os.path.join(SRC, "host_calls.cpp")
-    if force or _stale(CALLS, [src, os.path.join(INC, "bf16n_c.h")]):
-        import sysconfig
-
+    src, path = os.path.join(SRC, "host_calls.cpp"), calls_path()
+    if force or _stale(path, [src, os.path.join(INC, "bf16n_c.h")]):
         import torch
         root = os.path.dirname(torch.__file__)
         cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
         inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
                os.path.join(cuda, "include")]
         _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-              *(f"-isystem{i}" for i in inc), src, "-o", CALLS, "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+              *(f"-isystem{i}" for i in inc), src, "-o", path, "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
               "-L" + PKG, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN"])
-    return CALLS
+    return path
 
 
 if __name__ == "__main__":

@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes as C
 import struct
 import time
+import warnings
 from dataclasses import dataclass
 
 import torch
@@ -117,12 +118,22 @@ def _version(t: torch.Tensor) -> int | None:
 _calls = None
 
 
+class _NoCalls:     # leaves every call to the Python functions
+    mmv = linear = draft_logits = staticmethod(lambda *a: None)
+
+
 def _native():
-    """mmv, linear and draft_logits in native code; they return None for calls that the Python functions are to see."""
+    """mmv, linear and draft_logits in native code; they return None for calls that the Python functions are to see. Where the module
+    cannot be had (no compiler, another torch) the Python functions, which call the same library, see all of them."""
     global _calls
     if _calls is None:
-        m = _lib.calls()
-        m.register(Weight, Meta)
+        lib()
+        try:
+            m = _lib.calls()
+            m.register(Weight, Meta)
+        except Exception as e:
+            warnings.warn(f"bf16n: no native form of mmv, linear and draft_logits (about 15 us more host time a call): {e}", RuntimeWarning)
+            m = _NoCalls
         _calls = m
     return _calls
 
