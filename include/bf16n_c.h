@@ -117,8 +117,10 @@ int bf16n_sm_count(int * out);
 /* Every wait inside a kernel is bounded (bulk copies completing on an mbarrier, tensor-core commits). When one runs out
  * the kernel sets a status word, writes NaN where the affected work item's outputs go and finishes, so the context stays
  * usable. This call synchronises the stream, returns the status words since the last call as a bit mask and clears
- * them: bit 0 the bulk-copy staged GEMV, bit 1 the MoE decode unit kernels, bit 2 the fragment-order kernels, bit 3 the
- * batched (prefill) kernel. 0 means every launch so far wrote complete outputs. Not capturable (it synchronises).
+ * them: bit 0 the bulk-copy staged GEMV, dense products and reconstruction with marks, bit 1 the MoE decode unit kernels, bit 2 the
+ * fragment-order kernels, bit 3 the batched (prefill) kernel, bit 4 the row gather and a draft step's candidates. 0 means every launch so
+ * far wrote complete outputs. Kernels that were given marks set their bit too, but write the right values: they read the unit from
+ * global memory instead. Not capturable (it synchronises).
  * The reference has no bounded waits and nothing like this. */
 #define BF16N_FAULT_GEMV_STAGED 1u
 #define BF16N_FAULT_MOE_DECODE 2u

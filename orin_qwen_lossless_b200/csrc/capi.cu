@@ -17,10 +17,10 @@ std::once_flag g_once;
 int g_init_status = BF16N_OK;
 std::string g_init_error;
 int g_device = -1;                         // the device bf16n_init ran on: the only one this process may launch on
-constexpr int FAULT_WORDS = 6;
+constexpr int FAULT_WORDS = 7;
 unsigned int * g_fault_words[FAULT_WORDS] = {};
 constexpr unsigned int FAULT_BITS[FAULT_WORDS] = {BF16N_FAULT_GEMV_STAGED, BF16N_FAULT_MOE_DECODE, BF16N_FAULT_FRAG_ORDER, BF16N_FAULT_PREFILL,
-                                                  BF16N_FAULT_ROW_GATHER, BF16N_FAULT_GEMV_STAGED};
+                                                  BF16N_FAULT_ROW_GATHER, BF16N_FAULT_GEMV_STAGED, BF16N_FAULT_ROW_GATHER};
 std::atomic<uint64_t> g_peer_wait_ns{2000000000ull};
 
 template <typename F>
@@ -60,6 +60,7 @@ void ensure_init() {
             g_fault_words[3] = prefill_fault_word();
             g_fault_words[4] = row_gather_fault_word();
             g_fault_words[5] = gemv_parts_fault_word();
+            g_fault_words[6] = rows_parts_fault_word();
         } catch (const std::exception & e) {
             g_init_status = BF16N_ECUDA;
             g_init_error = e.what();

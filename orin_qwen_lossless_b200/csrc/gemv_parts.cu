@@ -153,6 +153,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_expand_parts(const 
 // passes over the rows before it there and decodes it, the warps of the parts before that only walk their codes, so that the row's
 // start is known to be right when the block meets. 128 candidates of 62080 x 2048: 19.7 us by a walk of up to 15 rows from the unit's
 // start (with a table of the codes that end in 12 bits of stream), 4.7 so. SCORED: the row is multiplied with its token's activations as well.
+__device__ unsigned int g_row_wait_expired; // a copy of a gathered row's unit never arrived: the row gather's word, not the products'
 template <int C, bool BF, bool SCORED>
 __global__ void __launch_bounds__(512) k_rows_parts(const Parts p, int R, const char * ids, int64_t ids_s0, int64_t row0, char * dst, int64_t dst_s1,
                                                     const RowScores scores, const Opaque k) {
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(512) k_rows_parts(const Parts p, int R, const 
                     good = __all_sync(FULL, rd.position(words + 4 * cur.my) == lds32(starts + 128, rd.next));
                 }
             } else if (lane == 0) {
-                atomicOr(&g_wait_expired, 1u);
+                atomicOr(&g_row_wait_expired, 1u);
             }
         }
         if (!good && lane == 0) { broken = 1; }
@@ -299,6 +300,11 @@ void gemv_parts_c(const bf16n_weight & w, const uint16_t * marks, const Cols & q
 } // namespace
 
 BF16N_DEFINE_FAULT_WORD(gemv_parts_fault_word)
+unsigned int * rows_parts_fault_word() {
+    unsigned int * p = nullptr;
+    cuda_ok(cudaGetSymbolAddress((void **) &p, g_row_wait_expired), "fault word address");
+    return p;
+}
 
 void gemv_parts_init() {
     const int optin = device_info().smem_optin;

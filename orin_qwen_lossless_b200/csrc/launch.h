@@ -119,6 +119,7 @@ unsigned int * fo_fault_word();
 unsigned int * prefill_fault_word();
 unsigned int * row_gather_fault_word();
 unsigned int * gemv_parts_fault_word();
+unsigned int * rows_parts_fault_word();
 
 // gemv_staged.cu
 void gemv_staged_init();

@@ -149,8 +149,9 @@ def init() -> None:
 
 def fault_status() -> int:
     """Synchronises the current stream and returns (and clears) the bit mask of the kernels' bounded waits that ran out
-    since the last call: 1 staged GEMV, 2 MoE decode units, 4 fragment-order kernels, 8 batched kernel, 16 row gather. 0: all outputs
-    complete; otherwise the outputs of the affected work items are NaN."""
+    since the last call: 1 staged GEMV, dense products and reconstruction with marks, 2 MoE decode units, 4 fragment-order kernels, 8 batched
+    kernel, 16 row gather and draft candidates. 0: all outputs complete; otherwise the outputs of the affected work items are NaN (not in
+    kernels with marks, which read the unit again from global memory)."""
     v = C.c_uint(0)
     check(lib().bf16n_fault_status(C.byref(v), _stream()))
     return int(v.value)

@@ -33,3 +33,12 @@ def test_read_only_loads_are_the_matrix(name):
     assert found
     for arg in found:
         assert MATRIX.search(arg) or re.search(r"\b(marks|from|cur|next)\b", arg), arg     # from, cur, next: PartPlane's pointers into the plane
+
+
+def test_an_expired_wait_of_a_gathered_row_is_the_row_gathers():
+    assert "g_wait_expired" not in _kernel("k_rows_parts")[1] and "g_row_wait_expired" in _kernel("k_rows_parts")[1]
+    s = SOURCES["capi.cu"]
+    bits = re.search(r"FAULT_BITS\[FAULT_WORDS\] = \{([^}]*)\}", s).group(1).replace(" ", "").split(",")
+    words = dict(re.findall(r"g_fault_words\[(\d)\] = (\w+)\(\)", s))
+    of = {words[str(i)]: b.strip() for i, b in enumerate(bits)}
+    assert of["rows_parts_fault_word"] == of["row_gather_fault_word"] == "BF16N_FAULT_ROW_GATHER" and of["gemv_parts_fault_word"] == "BF16N_FAULT_GEMV_STAGED"
