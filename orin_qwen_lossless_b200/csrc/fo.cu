@@ -536,7 +536,8 @@ __global__ void __launch_bounds__(FO_COMBINE_SLOTS * 32) k_fo_down_combine(const
 // fall into 32 different banks; columns beyond ncols are zero.
 constexpr int XPAD = 8;
 constexpr int STAGED_WARPS = 28;
-constexpr int FO_BARS = 512; // room for two mbarriers per warp of the staged kernel (up to 32 warps)
+constexpr int FO_BARS = 256; // room for one mbarrier per warp of the staged kernel
+static_assert(STAGED_WARPS * 8 <= FO_BARS, "mbarriers of the staged kernel");
 __global__ void __launch_bounds__(512) k_fo_gemv_mma(const PairView w, int C, Cols p, int ncols, int64_t n_units) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t * lut = (uint32_t *) smem;
@@ -1031,7 +1032,7 @@ void fo_gemv_t(const bf16n_weight & w, const bf16n_mmv_args & a, cudaStream_t st
         return;
     }
     if (a.x_bf16 && (a.ncols >= 2 || p.nrows / BAND >= (int64_t) device_info().sms * big_per_sm)) {
-        // BF16 activations: the tensor-core kernels, 8 columns per decode. Large matrices (at least 16 bands per SM) take
+        // BF16 activations: the tensor-core kernels, 8 columns per decode. Large matrices (from 6 bands per SM on, one column from 16) take
         // the persistent kernel with staged streams, also for a single column.
         const int C = (int) (w.K / CHUNK);
         const int64_t bands = p.nrows / BAND, sms = device_info().sms;

@@ -146,7 +146,10 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_expand_parts(const 
             }
         }
     };
-    walk_parts<false>(p, first_unit(p), units, unit0, R * C * CHUNK, smem, [&] { stage_table(smem, p.w.lut); }, chunks, [](int64_t, int, bool) {});
+    walk_parts<false>(p, first_unit(p), units, unit0, R * C * CHUNK, smem, [&] {
+        stage_table(smem, p.w.lut);
+        bare_grid_dependency_wait(); // an ordinary launch, to which this is nothing; walk_parts lets the next kernel start
+    }, chunks, [](int64_t, int, bool) {});
 }
 
 // Few rows (a draft step's candidates, the tokens of a decode batch), one block each: the warp of the part that the row lies in

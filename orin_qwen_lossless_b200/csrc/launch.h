@@ -34,7 +34,9 @@ inline void allow_dynamic_smem(const void * kernel, int bytes, int optin, const 
 
 // Shared memory that keeps a launch of a few blocks per SM spread evenly: blocks of a dependent launch are placed while the kernel in front
 // still holds some SMs, and would crowd on the others (the down launch of a one-token decode step: 13 us with up to four blocks on an
-// SM, 9 with one on each). `bytes` at least, and more than lets one block beyond the even share on an SM.
+// SM, 9 with one on each). `bytes` at least, and more than lets one block beyond the even share on an SM. What a second stream finds: 20 chains of
+// nine small NIBBLE products of one token 430 -> 300 us alone, beside the same on a second stream 451 -> 448, beside GEMMs 891 -> 824,
+// beside elementwise kernels 563 -> 592; products of 4 tokens and of 8192 rows within 3 %.
 inline size_t even_smem(size_t bytes, int64_t blocks) {
     const int64_t share = (blocks + device_info().sms - 1) / device_info().sms;
     return std::max(bytes, share <= 3 ? (size_t) device_info().smem_optin / (share + 1) : 0);
@@ -45,7 +47,7 @@ inline size_t even_smem(size_t bytes, int64_t blocks) {
 // launch): such a kernel calls grid_dependency_wait() before it touches anything an earlier kernel wrote or still reads,
 // and does only independent work (barriers, a matrix's own tables) above that line. Works under stream capture as well.
 // A kernel that reads a matrix above the line is not ordered behind a kernel of the caller's that wrote the matrix. Where the
-// public interface says so (products of NIBBLE matrices, expert units of a decode step) the caller sees to that; all others
+// public interface says so (products of NIBBLE matrices, expert units and parts of a decode step) the caller sees to that; all others
 // are launched with launch_behind, whose `own` says that the kernel in front is this library's, launched by the same call and
 // waiting for its own predecessors before it lets this one start: whatever wrote the matrix has then completed.
 template <typename... KArgs, typename... Args>

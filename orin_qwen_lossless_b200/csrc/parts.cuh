@@ -97,7 +97,8 @@ __device__ __forceinline__ int64_t first_unit(const Parts & p) {
 // turn), 159 us without marks, 667 where such units were left to one warp, 129 so; two columns, 16384 x 2048, 30.0, 114 and 22.5. Codes
 // that all have the same length put the lanes' words into one bank: 16384 x 2048 of 32 exponents that are equally likely, two columns, 29.8 and 43.8.
 //   u, units, unit0             this warp's (first) unit, where units end, and the matrix's unit that is unit 0
-//   prologue()                  what else the block needs, and the wait for the kernel in front; the barrier behind it is here. The
+//   prologue()                  what else the block needs, and the wait for the kernel in front (unless the kernel waited before): single-turn
+//                               kernels let the next one start from here on. The barrier behind it is here. The
 //                               code table (stage_table) is at the front of the shared memory before that barrier
 //   decode(rd, lut, pl, u, s)   the 64 codes of part s
 //   store(u, s, alone)          after the check: results that decode() kept; alone: this warp decodes all parts, s is the last so far

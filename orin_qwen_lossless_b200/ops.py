@@ -79,6 +79,7 @@ class Weight:
 
     @property
     def nbytes(self) -> int:
+        """Stored bytes of the matrix; its marks (up to 1.2 % more) come on top: meta.marks_bytes()."""
         return self.plane.numel() + self.aux.numel()
 
     def marks_ptr(self) -> int | None:
@@ -406,7 +407,8 @@ def mmv(x: torch.Tensor, w: Weight, ids: torch.Tensor | None = None, rows_per_ma
 
 def mmv_group(xs, ws, outs=None, out_dtype: torch.dtype = torch.float32):
     """Independent dense products ys[i] = ws[i] xs[i] in as few launches as possible: small NIBBLE matrices share one
-    grid (eight products per launch), other formats are launched as mmv launches them. Same bits as mmv per product."""
+    grid (eight products per launch), other formats are launched one by one, without the marks that mmv passes (8192 x 2048: 20 us here, 11
+    there). Same bits as mmv per product."""
     n = len(ws)
     if len(xs) != n or (outs is not None and len(outs) != n):
         raise RuntimeError("bf16n.mmv_group: one activation (and output) per matrix")

@@ -19,6 +19,27 @@ def test_dense_products_wait_before_they_read_the_matrix():
     assert wait < min(body.index(read) for read in ("stage_table(", "walk_parts<", "p.w.", "p.marks") if read in body)
 
 
+@pytest.mark.parametrize("name", WALKERS + ["k_rows_parts"])
+def test_they_wait_before_their_successor_starts(name):
+    assert "grid_dependency_wait()" in _kernel(name)[1]
+
+
+def test_what_the_down_kernels_read_above_the_wait():
+    """Ids and weights are older than the gate / up launch in front, which waited for them before it let these start; nothing else may be read there."""
+    for name, older in (("k_down_combine", {"p.ids", "weights"}), ("k_fo_down_combine", {"ids", "weights"})):
+        params, body = _kernel(name)
+        above = body[:body.index("grid_dependency_wait()")]
+        for p in re.findall(r"(?:const )?(?:float|int32_t) \* (?:__restrict__ )?(\w+)", params):
+            assert p in older or not re.search(rf"\b{p}\b", above), (name, p)
+        for read in ("p.x", "ldg_x4", "ld_act"):
+            assert read not in above, (name, read)
+    for f, function, kernel, front in (("moe_decode.cu", "void moe_decode(", "k_down_combine", "launch_units<4, 8, true"), ("moe_decode.cu", "void moe_decode_frag_order(", "fo_down_combine(", "fo_gemv_two(")):
+        s = SOURCES[f]
+        body = _block(s, s.index(function))
+        assert 0 <= body.index(front) < body.index(kernel)
+        assert sum(k.count("launch_chained(" + kernel) for k in SOURCES.values()) <= 1
+
+
 def test_rows_are_gathered_behind_the_callers_kernels():
     assert "k_rows_parts" not in re.findall(r"launch_chained\((\w+)", SOURCES["gemv_parts.cu"])
     launch = SOURCES["gemv_parts.cu"]
