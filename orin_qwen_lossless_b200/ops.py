@@ -874,8 +874,8 @@ def moe_decode(x: torch.Tensor, gate: Weight, up: Weight, down: Weight, n_expert
                topk_ids: torch.Tensor | None = None, expert_lo: int = 0, n_experts_local: int | None = None,
                scratch: torch.Tensor | None = None, out: torch.Tensor | None = None,
                out_dtype: torch.dtype = torch.float32, peers=None):
-    """One MoE decode step of the routed experts in four launches (router, gate+up, down with SwiGLU on load,
-    combine). Either router_logits (FP32 [T, n_experts]) or topk_weights / topk_ids (FP32 / int32 [T, top_k]) is given.
+    """One MoE decode step of the routed experts in three launches (router, gate+up, down with SwiGLU on load and the slots' weighted sum), four
+    where the sum is one of its own (without marks, of many columns, to peers). Either router_logits (FP32 [T, n_experts]) or topk_weights / topk_ids (FP32 / int32 [T, top_k]) is given.
     The weights hold experts [expert_lo, expert_lo + n_experts_local); other slots add zeros (expert parallelism).
     peers (a bf16n_peer_out): the combine also stores y into the peers' exchange buffers and announces it.
     Returns (y [T, H], topk_weights, topk_ids)."""
