@@ -232,8 +232,9 @@ def make_marks(w: Weight) -> bool:
     that captured calls find them too. False, and nothing done, for layouts without marks, off the process's GPU and under capture.
 
     upload() calls it, and so does the first call through a Weight whose aux torch has written since. A program that overwrites a matrix in
-    another way (a raw pointer, .data, inside a captured graph), or has only captured calls, calls it itself: with old marks results stay
-    right, but every unit is decoded twice, the second time by one warp."""
+    another way (a raw pointer, .data, inside a captured graph), gives the Weight other tensors of the same shape, or has only captured
+    calls, calls it itself: with old marks results stay right, but every unit is decoded twice, the second time by one warp. Marks belong
+    to one Weight: two that share them (dataclasses.replace) find each other's."""
     n = w.meta.marks_bytes()
     if n == 0 or not w.plane.is_cuda or torch.cuda.is_current_stream_capturing():
         return False
