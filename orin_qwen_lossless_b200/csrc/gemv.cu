@@ -885,7 +885,7 @@ void gemv_group(const bf16n_weight * w, const bf16n_mmv_args * a, int n, cudaStr
     while (i < n) {
         NibGroup g = {};
         int blocks = 0;
-        bool wide = false;
+        bool wide = false, one_chunk = true;
         while (i < n && g.n < GROUP_MAX) {
             NibItem & it = g.item[g.n++];
             it.v = nib_view(w[i]);
@@ -896,11 +896,14 @@ void gemv_group(const bf16n_weight * w, const bf16n_mmv_args * a, int n, cudaStr
             const dim3 geo = row_geometry(a[i].nrows, a[i].ncols);
             it.first_block = blocks;
             wide = wide || it.chunks > 4;
+            one_chunk = one_chunk && it.chunks == 1;
             it.blocks = (int) geo.x;
             blocks += it.blocks * it.ncols;
             i++;
         }
-        launch_chained(wide ? k_nib_gemv_group<true> : k_nib_gemv_group<false>, dim3((unsigned) blocks), dim3(256), even_smem(0, blocks), st, g);
+        // Spread evenly (even_smem) unless all rows are of 512 columns, whose blocks are gone before crowding tells: crowded / spread, groups of
+        // eight of 64 x 512, two tokens, 1.28 / 1.64 us, of four of 256 x 512, one token, 1.35 / 1.47; of four of 256 x 2048 2.57 / 1.98.
+        launch_chained(wide ? k_nib_gemv_group<true> : k_nib_gemv_group<false>, dim3((unsigned) blocks), dim3(256), one_chunk ? 0 : even_smem(0, blocks), st, g);
         check_launch();
     }
 }
